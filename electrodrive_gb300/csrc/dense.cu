@@ -1,241 +1,411 @@
 // Dense single-layer operator (the reference's torch-tiled A(x),
 // electrodrive/core/bem_kernel.py:157-230 and :341-381):
 //   V_i = k_e sum_{j != i} sigma_j A_j / sqrt(max(|c_i - c_j|^2, 1e-24))
-//         + self_integrals_i sigma_i A_i        (self term only if given)
-//   non-finite V_i -> 0.
+//         + self_integrals_i sigma_i A_i        (self term only if given);
+//   non-finite V_i -> 0,
+// and the induced potential and field at separate targets.
 //
-// The source index is split into chunks so that small N (5,120 panels) still
-// fills every SM: block (row tile, chunk) accumulates its chunk's sources for
-// 256 targets from (x, y, z, sigma A) tiles staged in shared memory and
-// writes one partial sum per target; a second kernel adds the partials of a
-// row in chunk order (deterministic) and applies k_e, the self term and the
-// non-finite clamp.  With a single chunk the first kernel finishes the rows
-// itself.
+// One block owns a tile of targets; the sources are split over the blocks of
+// a thread-block cluster and, inside a block, over its warps, so that small
+// problems fill every SM.  The partial sums are added in a fixed order, over
+// the block's warps and then over the cluster's blocks through distributed
+// shared memory: no scratch in device memory, no second launch.
+//
+// FP32 (k_dense_f32): each lane keeps several targets, so that a source pair
+// read from shared memory (two 16-byte broadcasts) serves all of them;
+// distances run as packed pairs.  An interaction is 7 FMA-pipe operations,
+// one maximum and one MUFU.RSQ (16 per SM and clock: the bound).  19,997
+// panels, one matvec: 175 -> 123 us (5.03e12 rsqrt/s: 79 us).
+//
+// FP64 (k_dense_f64): the distances run on the FP32 pipe at FP64 accuracy
+// (gridpoint.cuh); two FP64 operations per interaction remain, beside 16 in
+// IEEE arithmetic, whose pipe bounded the kernel (15.8 operations at 2 per SM
+// and clock).  5,120 panels, one matvec: 770 -> 173 us.  A tile of sources
+// whose coordinates are not finite, or all zero, and pairs too close for the
+// split run in IEEE FP64.
 #include <algorithm>
-#include <mutex>
 
 #include "edfmm_internal.cuh"
+#include "gridpoint.cuh"
 
 namespace edfmm {
 
 namespace {
 
-constexpr int kRows = 256;  // targets per block (one per thread)
-constexpr int kTile = 256;  // sources staged per shared-memory tile
+enum DenseKind { kMatvec = 0, kPotential = 1, kField = 2 };
+
+constexpr int kThreads = 128;     // 4 warps
+constexpr int kTile32 = 256;      // sources staged per shared-memory tile, FP32
+constexpr int kTile64 = 128;      // FP64
+constexpr int kRows64 = 64;       // FP64 targets per block: 2 warps, times 2 source halves
+constexpr int kMaxCluster = 8;    // the portable cluster size
 
 __device__ __forceinline__ float inv_r(float r2) { return rsqrt_normal(fmaxf(r2, 1e-24f)); }
 __device__ __forceinline__ double inv_r(double r2) { return rsqrt(fmax(r2, 1e-24)); }
 
-template <typename T>
-__device__ __forceinline__ T finish(T acc, int64_t i, T k_e, const T *self_int, const T *sigma, const T *areas) {
-    T v = acc * k_e;
-    if (self_int) v += self_int[i] * sigma[i] * areas[i];
-    return isfinite(v) ? v : (T)0;
+template <typename T> struct DenseArgs {
+    const T *tgt;  // (m, 3) targets (the centroids themselves for kMatvec)
+    int64_t m;
+    const T *c, *sigma, *areas;  // (n, 3), (n), (n)
+    int64_t n;
+    int64_t chunk;  // sources per block of the cluster (even)
+    int cs;         // cluster size
+    T k_e;
+    const T *self_int;  // kMatvec only
+    T *out;
+};
+
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// element of the same shared-memory variable in block `rank` of the cluster
+__device__ __forceinline__ float dsm_load(const float *p, int rank) {
+    unsigned a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ double dsm_load(const double *p, int rank) {
+    unsigned a;
+    double v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+    return v;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kRows) k_dense_partial(const T *__restrict__ c, const T *__restrict__ sigma,
-                                                         const T *__restrict__ areas, int64_t n, int64_t chunk,
-                                                         T *__restrict__ partial, int finish_rows, T k_e,
-                                                         const T *__restrict__ self_int, T *__restrict__ out) {
-    using T4 = typename Vec4<T>::type;
-    __shared__ T4 src[kTile];
-    const int64_t i = (int64_t)blockIdx.x * kRows + threadIdx.x;
-    const int64_t j0 = (int64_t)blockIdx.y * chunk;
-    const int64_t j1 = min(n, j0 + chunk);
-    T xi = 0, yi = 0, zi = 0;
-    if (i < n) {
-        xi = c[3 * i];
-        yi = c[3 * i + 1];
-        zi = c[3 * i + 2];
+// Sum over the block's source groups and the cluster's blocks, and write the
+// rows.  part[(g * ROWS + row) * COMP + comp]: group g's sums of this block.
+template <typename T, int KIND, int ROWS, int GROUPS>
+__device__ __forceinline__ void dense_finish(const DenseArgs<T> &A, T *part, int64_t row0, int rank) {
+    constexpr int COMP = KIND == kField ? 3 : 1, NV = ROWS * COMP;
+    __syncthreads();
+    for (int q = threadIdx.x; q < NV; q += kThreads) {
+        T v = part[q];
+#pragma unroll
+        for (int g = 1; g < GROUPS; ++g) v += part[g * NV + q];
+        part[q] = v;
     }
-    T acc = 0;
-    for (int64_t jb = j0; jb < j1; jb += kTile) {
-        const int64_t j = jb + threadIdx.x;
-        T4 s;
-        if (j < j1) {
-            s.x = c[3 * j];
-            s.y = c[3 * j + 1];
-            s.z = c[3 * j + 2];
-            s.w = sigma[j] * areas[j];
-        } else {
-            s.x = s.y = s.z = s.w = 0;
+    if (A.cs > 1) cluster_sync_all();
+    else __syncthreads();
+    if (rank == 0) {
+        for (int q = threadIdx.x; q < NV; q += kThreads) {
+            const int64_t i = row0 + q / COMP;
+            if (i >= A.m) continue;
+            T v = part[q];
+            for (int r = 1; r < A.cs; ++r) v += dsm_load(part + q, r);
+            if (KIND == kMatvec) {
+                v *= A.k_e;
+                if (A.self_int) v += A.self_int[i] * A.sigma[i] * A.areas[i];
+                A.out[i] = isfinite(v) ? v : (T)0;
+            } else if (KIND == kPotential) {
+                A.out[i] = v * A.k_e;
+            } else {
+                A.out[row0 * 3 + q] = isfinite(v) ? v : (T)0;
+            }
+        }
+    }
+    if (A.cs > 1) cluster_sync_all();  // the other blocks' shared memory stays until it has been read
+}
+
+// the block's target tile and its share of the sources (rank of the cluster)
+template <typename T>
+__device__ __forceinline__ void dense_ranges(const DenseArgs<T> &A, int rows, int64_t &row0, int &rank, int64_t &j0,
+                                             int64_t &j1) {
+    row0 = (int64_t)(blockIdx.x / (unsigned)A.cs) * rows;
+    rank = (int)(blockIdx.x % (unsigned)A.cs);
+    j0 = min(A.n, rank * A.chunk);
+    j1 = min(A.n, j0 + A.chunk);
+}
+
+// ---------------------------------------------------------------------------
+// FP32: 32 * TPT targets per block, the four warps take every fourth source
+// pair of a tile.  The field weight is formed in the reference's order (k_e
+// times 1/r^3, times sigma A), so a near-coincident pair overflows where the
+// reference's does, and non-finite components become zero at the end
+// (bem_kernel.py:990-997).
+// ---------------------------------------------------------------------------
+template <int KIND> __host__ __device__ constexpr int tpt32() { return KIND == kField ? 2 : 4; }
+
+template <int KIND, bool SELF, int TPT>
+__device__ __forceinline__ void dense_tile_f32(const float4 *src, int npairs, int wid, float k_e, const float2 (&nx)[TPT],
+                                               const float2 (&ny)[TPT], const float2 (&nz)[TPT], int self0,
+                                               float2 (&ax)[TPT], float2 (&ay)[TPT], float2 (&az)[TPT]) {
+#pragma unroll 2
+    for (int k = wid; k < npairs; k += 4) {
+        const float4 u = src[2 * k], v = src[2 * k + 1];  // (x, x', y, y'), (z, z', q, q')
+        const float2 qw = make_float2(v.z, v.w);
+#pragma unroll
+        for (int t = 0; t < TPT; ++t) {
+            const float2 dx = __fadd2_rn(make_float2(u.x, u.y), nx[t]), dy = __fadd2_rn(make_float2(u.z, u.w), ny[t]),
+                         dz = __fadd2_rn(make_float2(v.x, v.y), nz[t]);
+            const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+            float2 ir = make_float2(inv_r(r2.x), inv_r(r2.y));
+            if (SELF) {  // self0 + 32 t: the target's position in this tile
+                if (2 * k == self0 + 32 * t) ir.x = 0.0f;
+                if (2 * k + 1 == self0 + 32 * t) ir.y = 0.0f;
+            }
+            if (KIND == kField) {
+                const float2 ke2 = make_float2(k_e, k_e);
+                const float2 w = __fmul2_rn(__fmul2_rn(ke2, __fmul2_rn(__fmul2_rn(ir, ir), ir)), qw);
+                ax[t] = __ffma2_rn(w, dx, ax[t]);  // source minus target: the sign is taken at the end
+                ay[t] = __ffma2_rn(w, dy, ay[t]);
+                az[t] = __ffma2_rn(w, dz, az[t]);
+            } else {
+                ax[t] = __ffma2_rn(qw, ir, ax[t]);
+            }
+        }
+    }
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(kThreads) k_dense_f32(const DenseArgs<float> A) {
+    constexpr int TPT = tpt32<KIND>(), ROWS = 32 * TPT, COMP = KIND == kField ? 3 : 1;
+    __shared__ float4 src[kTile32];
+    __shared__ float part[4 * ROWS * COMP];
+    int64_t row0, j0, j1;
+    int rank;
+    dense_ranges(A, ROWS, row0, rank, j0, j1);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float2 nx[TPT], ny[TPT], nz[TPT];
+    float ex[TPT], ey[TPT], ez[TPT];
+#pragma unroll
+    for (int t = 0; t < TPT; ++t) {
+        const int64_t i = min(row0 + lane + 32 * t, A.m - 1);
+        nx[t].x = nx[t].y = -A.tgt[3 * i];
+        ny[t].x = ny[t].y = -A.tgt[3 * i + 1];
+        nz[t].x = nz[t].y = -A.tgt[3 * i + 2];
+        ex[t] = ey[t] = ez[t] = 0.0f;
+    }
+    float *sf = reinterpret_cast<float *>(src);
+    for (int64_t jb = j0; jb < j1; jb += kTile32) {
+        const int cnt = (int)min((int64_t)kTile32, j1 - jb);
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int q = threadIdx.x + h * kThreads;
+            float x = 0, y = 0, z = 0, w = 0;  // an odd tile ends with a source of no charge
+            if (q < cnt) {
+                const int64_t j = jb + q;
+                x = A.c[3 * j];
+                y = A.c[3 * j + 1];
+                z = A.c[3 * j + 2];
+                w = A.sigma[j] * A.areas[j];
+            }
+            float *o = sf + (q >> 1) * 8 + (q & 1);
+            o[0] = x;
+            o[2] = y;
+            o[4] = z;
+            o[6] = w;
         }
         __syncthreads();
-        src[threadIdx.x] = s;
-        __syncthreads();
-        const int cnt = (int)((j1 - jb) < (int64_t)kTile ? (j1 - jb) : (int64_t)kTile);
-        const bool diag_here = i >= jb && i < jb + cnt;
         // two-level sum (tile, then chunk) bounds FP32 rounding growth
-        T tacc = 0;
-#pragma unroll 8
-        for (int k = 0; k < cnt; ++k) {
-            const T4 q = src[k];
-            const T dx = xi - q.x, dy = yi - q.y, dz = zi - q.z;
-            T w = q.w * inv_r(dx * dx + dy * dy + dz * dz);
-            if (diag_here && jb + k == i) w = 0;
-            tacc += w;
+        float2 ax[TPT], ay[TPT], az[TPT];
+#pragma unroll
+        for (int t = 0; t < TPT; ++t) ax[t] = ay[t] = az[t] = make_float2(0.0f, 0.0f);
+        const int np = (cnt + 1) >> 1;
+        if (KIND == kMatvec && jb < row0 + ROWS && row0 < jb + cnt)
+            dense_tile_f32<KIND, true>(src, np, wid, A.k_e, nx, ny, nz, (int)(row0 - jb) + lane, ax, ay, az);
+        else
+            dense_tile_f32<KIND, false>(src, np, wid, A.k_e, nx, ny, nz, 0, ax, ay, az);
+#pragma unroll
+        for (int t = 0; t < TPT; ++t) {
+            ex[t] += ax[t].x + ax[t].y;
+            if (KIND == kField) {
+                ey[t] += ay[t].x + ay[t].y;
+                ez[t] += az[t].x + az[t].y;
+            }
         }
-        acc += tacc;
     }
-    if (i >= n) return;
-    if (finish_rows)
-        out[i] = finish(acc, i, k_e, self_int, sigma, areas);
-    else
-        partial[(int64_t)blockIdx.y * n + i] = acc;
+#pragma unroll
+    for (int t = 0; t < TPT; ++t) {
+        float *p = part + (wid * ROWS + lane + 32 * t) * COMP;
+        if (KIND == kField) {
+            p[0] = -ex[t];
+            p[1] = -ey[t];
+            p[2] = -ez[t];
+        } else {
+            p[0] = ex[t];
+        }
+    }
+    dense_finish<float, KIND, ROWS, 4>(A, part, row0, rank);
 }
 
-// induced potential at separate targets (no diagonal): bem_kernel.py:233-270
-template <typename T>
-__global__ void __launch_bounds__(kRows) k_targets_partial(const T *__restrict__ tgt, int64_t m,
-                                                           const T *__restrict__ c, const T *__restrict__ sigma,
-                                                           const T *__restrict__ areas, int64_t n, int64_t chunk,
-                                                           T *__restrict__ partial, int finish_rows, T k_e,
-                                                           T *__restrict__ out) {
-    using T4 = typename Vec4<T>::type;
-    __shared__ T4 src[kTile];
-    const int64_t i = (int64_t)blockIdx.x * kRows + threadIdx.x;
-    const int64_t j0 = (int64_t)blockIdx.y * chunk;
-    const int64_t j1 = min(n, j0 + chunk);
-    T xi = 0, yi = 0, zi = 0;
-    if (i < m) {
-        xi = tgt[3 * i];
-        yi = tgt[3 * i + 1];
-        zi = tgt[3 * i + 2];
-    }
-    T acc = 0;
-    for (int64_t jb = j0; jb < j1; jb += kTile) {
-        const int64_t j = jb + threadIdx.x;
-        T4 s;
-        if (j < j1) {
-            s.x = c[3 * j];
-            s.y = c[3 * j + 1];
-            s.z = c[3 * j + 2];
-            s.w = sigma[j] * areas[j];
-        } else {
-            s.x = s.y = s.z = s.w = 0;
-        }
-        __syncthreads();
-        src[threadIdx.x] = s;
-        __syncthreads();
-        const int cnt = (int)((j1 - jb) < (int64_t)kTile ? (j1 - jb) : (int64_t)kTile);
-        T tacc = 0;
-#pragma unroll 8
-        for (int k = 0; k < cnt; ++k) {
-            const T4 q = src[k];
-            const T dx = xi - q.x, dy = yi - q.y, dz = zi - q.z;
-            tacc += q.w * inv_r(dx * dx + dy * dy + dz * dz);
-        }
-        acc += tacc;
-    }
-    if (i >= m) return;
-    if (finish_rows)
-        out[i] = acc * k_e;
-    else
-        partial[(int64_t)blockIdx.y * m + i] = acc;
-}
+// ---------------------------------------------------------------------------
+// FP64: 64 targets per block, one per thread and source half of a tile
+// ---------------------------------------------------------------------------
+struct Src64 {
+    float4 u, v, w;  // (xa, xb, xc, ya), (yb, yc, za, zb), (zc, -, charge as two words)
+};
+struct Tgt64 {
+    double x, y, z;
+    GridCoord gx, gy, gz;  // scaled
+};
 
-// induced field at separate targets: E_i = sum_j (K_E / max(|x_i - r_j|^2,
-// 1e-24)^(3/2)) (sigma_j A_j) (x_i - r_j)  (bem_kernel.py:280-335, Laplace
-// fast path).  The weight is formed in the working dtype in the reference's
-// order (K_E times 1/r^3, times sigma A), so a near-coincident pair overflows
-// where the reference's does, and non-finite components become zero at the
-// end (bem_kernel.py:990-997).
-template <typename T>
-__global__ void __launch_bounds__(kRows) k_field_partial(const T *__restrict__ tgt, int64_t m,
-                                                         const T *__restrict__ c, const T *__restrict__ sigma,
-                                                         const T *__restrict__ areas, int64_t n, int64_t chunk,
-                                                         T *__restrict__ partial, int finish_rows, T k_e,
-                                                         T *__restrict__ out) {
-    using T4 = typename Vec4<T>::type;
-    __shared__ T4 src[kTile];
-    const int64_t i = (int64_t)blockIdx.x * kRows + threadIdx.x;
-    const int64_t j0 = (int64_t)blockIdx.y * chunk;
-    const int64_t j1 = min(n, j0 + chunk);
-    T xi = 0, yi = 0, zi = 0;
-    if (i < m) {
-        xi = tgt[3 * i];
-        yi = tgt[3 * i + 1];
-        zi = tgt[3 * i + 2];
-    }
-    T ex = 0, ey = 0, ez = 0;
-    for (int64_t jb = j0; jb < j1; jb += kTile) {
-        const int64_t j = jb + threadIdx.x;
-        T4 s;
-        if (j < j1) {
-            s.x = c[3 * j];
-            s.y = c[3 * j + 1];
-            s.z = c[3 * j + 2];
-            s.w = sigma[j] * areas[j];
-        } else {
-            s.x = s.y = s.z = s.w = 0;
-        }
-        __syncthreads();
-        src[threadIdx.x] = s;
-        __syncthreads();
-        const int cnt = (int)((j1 - jb) < (int64_t)kTile ? (j1 - jb) : (int64_t)kTile);
-        T tx = 0, ty = 0, tz = 0;
-#pragma unroll 8
-        for (int k = 0; k < cnt; ++k) {
-            const T4 q = src[k];
-            const T dx = xi - q.x, dy = yi - q.y, dz = zi - q.z;
-            const T ir = inv_r(dx * dx + dy * dy + dz * dz);
-            const T w = (k_e * (ir * ir * ir)) * q.w;
-            tx += w * dx;
-            ty += w * dy;
-            tz += w * dz;
-        }
-        ex += tx;
-        ey += ty;
-        ez += tz;
-    }
-    if (i >= m) return;
-    if (finish_rows) {
-        out[3 * i] = isfinite(ex) ? ex : (T)0;
-        out[3 * i + 1] = isfinite(ey) ? ey : (T)0;
-        out[3 * i + 2] = isfinite(ez) ? ez : (T)0;
+__device__ __forceinline__ unsigned high_abs(double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; }
+
+// one source in IEEE FP64, from device memory (w: the charge)
+template <int KIND>
+__device__ __noinline__ void dense_pair_ieee(const double *c, int64_t j, int64_t self, double x, double y, double z,
+                                             double w, double k_e, double &ex, double &ey, double &ez) {
+    ex = ey = ez = 0.0;
+    if (KIND == kMatvec && j == self) return;
+    const double dx = x - c[3 * j], dy = y - c[3 * j + 1], dz = z - c[3 * j + 2];
+    const double ir = inv_r(dx * dx + dy * dy + dz * dz);
+    if (KIND == kField) {
+        const double f = (k_e * (ir * ir * ir)) * w;
+        ex = f * dx;
+        ey = f * dy;
+        ez = f * dz;
     } else {
-        T *p = partial + ((int64_t)blockIdx.y * m + i) * 3;
-        p[0] = ex;
+        ex = w * ir;
+    }
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> A) {
+    constexpr int COMP = KIND == kField ? 3 : 1;
+    __shared__ Src64 src[kTile64];
+    __shared__ double xyz[KIND == kField ? 3 * kTile64 : 1];
+    __shared__ double part[2 * kRows64 * COMP];
+    __shared__ unsigned s_hi[4];
+    int64_t row0, j0, j1;
+    int rank;
+    dense_ranges(A, kRows64, row0, rank, j0, j1);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, half = threadIdx.x >> 6;
+    const int64_t i = row0 + (threadIdx.x & 63);
+    Tgt64 T;
+    {
+        const int64_t q = min(i, A.m - 1);
+        T.x = A.tgt[3 * q];
+        T.y = A.tgt[3 * q + 1];
+        T.z = A.tgt[3 * q + 2];
+    }
+    const unsigned thi = max(high_abs(T.x), max(high_abs(T.y), high_abs(T.z)));
+    int kprev = INT32_MIN;
+    double ex = 0, ey = 0, ez = 0;
+    for (int64_t jb = j0; jb < j1; jb += kTile64) {
+        const int cnt = (int)min((int64_t)kTile64, j1 - jb);
+        double x = 0, y = 0, z = 0, w = 0;
+        if ((int)threadIdx.x < cnt) {
+            const int64_t j = jb + threadIdx.x;
+            x = A.c[3 * j];
+            y = A.c[3 * j + 1];
+            z = A.c[3 * j + 2];
+            w = A.sigma[j] * A.areas[j];
+        }
+        // the tile's scale: a power of two above every |coordinate| of its sources and targets
+        const unsigned hi = __reduce_max_sync(0xffffffffu, max(max(thi, high_abs(x)), max(high_abs(y), high_abs(z))));
+        __syncthreads();  // the previous tile has been read
+        if (lane == 0) s_hi[wid] = hi;
+        __syncthreads();
+        int k;
+        const bool split = grid_exponent(max(max(s_hi[0], s_hi[1]), max(s_hi[2], s_hi[3])), k);
+        if (!split) {
+            if ((int)threadIdx.x < cnt) reinterpret_cast<double *>(&src[threadIdx.x])[0] = w;
+            __syncthreads();
+            for (int s = half; s < cnt; s += 2) {
+                double px, py, pz;
+                dense_pair_ieee<KIND>(A.c, jb + s, i, T.x, T.y, T.z, reinterpret_cast<double *>(&src[s])[0], A.k_e, px,
+                                      py, pz);
+                ex += px;
+                ey += py;
+                ez += pz;
+            }
+            continue;
+        }
+        const double down = grid_pow2(-k);
+        if (k != kprev) {
+            T.gx = grid_split(T.x * down);
+            T.gy = grid_split(T.y * down);
+            T.gz = grid_split(T.z * down);
+            kprev = k;
+        }
+        if ((int)threadIdx.x < cnt) {
+            const GridCoord a = grid_split(x * down), b = grid_split(y * down), c = grid_split(z * down);
+            Src64 &S = src[threadIdx.x];
+            S.u = make_float4(a.a, a.b, a.c, b.a);
+            S.v = make_float4(b.b, b.c, c.a, c.b);
+            S.w = make_float4(c.c, 0.0f, __int_as_float(__double2loint(w)), __int_as_float(__double2hiint(w)));
+            if (KIND == kField) {
+                xyz[3 * threadIdx.x] = x;
+                xyz[3 * threadIdx.x + 1] = y;
+                xyz[3 * threadIdx.x + 2] = z;
+            }
+        } else if ((int)threadIdx.x < ((cnt + 3) & ~3)) {  // no charge, outside the scaled box
+            Src64 &S = src[threadIdx.x];
+            S.u = make_float4(3.0f, 0.0f, 0.0f, 3.0f);
+            S.v = make_float4(0.0f, 0.0f, 3.0f, 0.0f);
+            S.w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (KIND == kField) xyz[3 * threadIdx.x] = xyz[3 * threadIdx.x + 1] = xyz[3 * threadIdx.x + 2] = 0.0;
+        }
+        __syncthreads();
+        // closer than the split resolves, or than the clamp: IEEE
+        const float near2 = fmaxf(kGridNear2, (float)(1.0001e-24 * down * down));
+        double tx = 0, ty = 0, tz = 0;  // two-level sum: tile, then chunk; the split pairs in scaled units
+        double sx = 0, sy = 0, sz = 0;
+        auto load = [&](int s, GridDiff &dx, GridDiff &dy, GridDiff &dz, double &w) {
+            const float4 u = src[s].u, v = src[s].v, q = src[s].w;
+            w = __hiloint2double(__float_as_int(q.w), __float_as_int(q.z));
+            dx = grid_diff(T.gx, GridCoord{u.x, u.y, u.z});
+            dy = grid_diff(T.gy, GridCoord{u.w, v.x, v.y});
+            dz = grid_diff(T.gz, GridCoord{v.z, v.w, q.x});
+        };
+        auto add = [&](int s, const GridR2 &r2, double w) {
+            float y0;
+            unsigned ci;
+            grid_rsqrt(r2, y0, ci);
+            if (KIND == kField) {
+                const double ir = grid_double(y0) * grid_one_plus(ci);
+                const double f = (A.k_e * (ir * ir * ir)) * w;
+                tx = fma(f, T.x - xyz[3 * s], tx);
+                ty = fma(f, T.y - xyz[3 * s + 1], ty);
+                tz = fma(f, T.z - xyz[3 * s + 2], tz);
+            } else {
+                tx = fma(w * grid_double(y0), grid_one_plus(ci), tx);
+            }
+        };
+        auto add_any = [&](int s, const GridR2 &r2, double w) {
+            if (r2.R1 < near2) {
+                if (s >= cnt) return;  // padding
+                double px, py, pz;
+                dense_pair_ieee<KIND>(A.c, jb + s, i, T.x, T.y, T.z, w, A.k_e, px, py, pz);
+                sx += px;
+                sy += py;
+                sz += pz;
+            } else {
+                add(s, r2, w);
+            }
+        };
+        for (int s = half; s < cnt; s += 4) {  // two sources side by side; the tile is padded to a multiple of 4
+            GridDiff dx, dy, dz;
+            double w0, w1;
+            load(s, dx, dy, dz, w0);
+            const GridR2 r0 = grid_r2(dx, dy, dz);
+            load(s + 2, dx, dy, dz, w1);
+            const GridR2 r1 = grid_r2(dx, dy, dz);
+            if (fminf(r0.R1, r1.R1) < near2) {
+                add_any(s, r0, w0);
+                add_any(s + 2, r1, w1);
+            } else {
+                add(s, r0, w0);
+                add(s + 2, r1, w1);
+            }
+        }
+        const double unscale = KIND == kField ? down * down * down : down;
+        ex += tx * unscale + sx;
+        if (KIND == kField) {
+            ey += ty * unscale + sy;
+            ez += tz * unscale + sz;
+        }
+    }
+    double *p = part + (half * kRows64 + (threadIdx.x & 63)) * COMP;
+    p[0] = ex;
+    if (KIND == kField) {
         p[1] = ey;
         p[2] = ez;
     }
-}
-
-template <typename T>
-__global__ void k_field_reduce(const T *__restrict__ partial, int chunks, int64_t m, T *__restrict__ out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    T ex = 0, ey = 0, ez = 0;
-    for (int c = 0; c < chunks; ++c) {
-        const T *p = partial + ((int64_t)c * m + i) * 3;
-        ex += p[0];
-        ey += p[1];
-        ez += p[2];
-    }
-    out[3 * i] = isfinite(ex) ? ex : (T)0;
-    out[3 * i + 1] = isfinite(ey) ? ey : (T)0;
-    out[3 * i + 2] = isfinite(ez) ? ez : (T)0;
-}
-
-template <typename T>
-__global__ void k_targets_reduce(const T *__restrict__ partial, int chunks, int64_t m, T k_e, T *__restrict__ out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    T acc = 0;
-    for (int c = 0; c < chunks; ++c) acc += partial[(int64_t)c * m + i];
-    out[i] = acc * k_e;
-}
-
-template <typename T>
-__global__ void k_dense_reduce(const T *__restrict__ partial, int chunks, int64_t n, T k_e,
-                               const T *__restrict__ self_int, const T *__restrict__ sigma,
-                               const T *__restrict__ areas, T *__restrict__ out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    T acc = 0;
-    for (int c = 0; c < chunks; ++c) acc += partial[(int64_t)c * n + i];
-    out[i] = finish(acc, i, k_e, self_int, sigma, areas);
+    dense_finish<double, KIND, kRows64, 2>(A, part, row0, rank);
 }
 
 int sm_count() {
@@ -249,197 +419,97 @@ int sm_count() {
     return sms;
 }
 
-}  // namespace
-
-// Source chunking: enough blocks for ~8 per SM, at most 64 chunks, chunks a
-// multiple of the shared-memory tile.
-void dense_plan(int64_t n, int &chunks, int64_t &chunk) {
-    const int64_t rows = (n + kRows - 1) / kRows;
-    const int64_t want = 8LL * sm_count();
-    int64_t c = rows >= want ? 1 : (want + rows - 1) / rows;
-    c = std::min<int64_t>(std::max<int64_t>(c, 1), 64);
-    chunk = ((n + c - 1) / c + kTile - 1) / kTile * kTile;
-    if (chunk <= 0) chunk = kTile;
-    chunks = (int)((n + chunk - 1) / chunk);
-    if (chunks < 1) chunks = 1;
-}
-
-size_t dense_scratch_bytes(int64_t n, int dtype) {
-    int chunks;
-    int64_t chunk;
-    dense_plan(n, chunks, chunk);
-    if (chunks <= 1) return 0;
-    return (size_t)chunks * (size_t)n * (dtype == EDFMM_F64 ? 8 : 4);
-}
-
-template <typename T>
-int dense_run(const T *c, const T *sigma, const T *areas, const T *self_int, int64_t n, T k_e, T *out, T *partial,
-              cudaStream_t s) {
-    int chunks;
-    int64_t chunk;
-    dense_plan(n, chunks, chunk);
-    dim3 grid((unsigned)((n + kRows - 1) / kRows), (unsigned)chunks);
-    k_dense_partial<T><<<grid, kRows, 0, s>>>(c, sigma, areas, n, chunk, partial, chunks == 1, k_e, self_int, out);
-    EDFMM_LAUNCH_CHECK("k_dense_partial");
-    if (chunks > 1) {
-        k_dense_reduce<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(partial, chunks, n, k_e, self_int, sigma, areas,
-                                                                     out);
-        EDFMM_LAUNCH_CHECK("k_dense_reduce");
+// Cluster size: the number of blocks that share a target tile's sources.  An
+// SM's time is the blocks it gets times a block's (its sources, plus about 40
+// sources' worth of set-up and reduction), so the choice minimises
+// ceil(tiles * cs / SMs) * (n / cs + 40); from eight blocks per SM on, a
+// split gains nothing.
+int cluster_size(int64_t tiles, int64_t n) {
+    const int64_t sms = sm_count();
+    if (tiles >= 8 * sms) return 1;
+    int best = 1;
+    int64_t cost = INT64_MAX;
+    for (int cs = 1; cs <= kMaxCluster; ++cs) {
+        const int64_t t = (tiles * cs + sms - 1) / sms * ((n + cs - 1) / cs + 40);
+        if (t < cost) {
+            cost = t;
+            best = cs;
+        }
     }
+    return best;
+}
+
+template <typename T, int KIND>
+int dense_launch(const T *tgt, int64_t m, const T *c, const T *sigma, const T *areas, int64_t n, T k_e,
+                 const T *self_int, T *out, cudaStream_t s) {
+    constexpr int ROWS = sizeof(T) == 4 ? 32 * tpt32<KIND>() : kRows64;
+    const int64_t tiles = (m + ROWS - 1) / ROWS;
+    DenseArgs<T> A{tgt, m, c, sigma, areas, n, 0, cluster_size(tiles, n), k_e, self_int, out};
+    A.chunk = ((n + A.cs - 1) / A.cs + 1) & ~(int64_t)1;
+    if (tiles * A.cs > INT32_MAX) return fail(EDFMM_ERR_ARG, "too many targets for one launch");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles * A.cs));
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)A.cs;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = A.cs > 1 ? 1 : 0;
+    cudaError_t e;
+    if constexpr (sizeof(T) == 4) e = cudaLaunchKernelEx(&cfg, k_dense_f32<KIND>, A);
+    else e = cudaLaunchKernelEx(&cfg, k_dense_f64<KIND>, A);
+    if (e != cudaSuccess) return fail(EDFMM_ERR_CUDA, std::string("launch of k_dense failed: ") + cudaGetErrorString(e));
+    EDFMM_LAUNCH_CHECK("k_dense");
     return EDFMM_OK;
 }
 
-int dense_matvec(const void *c, const void *sigma, const void *areas, const void *self_int, int64_t n, int dtype,
-                 double k_e, void *out, void *scratch, cudaStream_t s) {
+template <int KIND>
+int dense_any(const void *tgt, int64_t m, const void *c, const void *sigma, const void *areas, int64_t n, int dtype,
+              double k_e, const void *self_int, void *out, cudaStream_t s) {
     if (dtype == EDFMM_F64)
-        return dense_run<double>(static_cast<const double *>(c), static_cast<const double *>(sigma),
-                                 static_cast<const double *>(areas), static_cast<const double *>(self_int), n, k_e,
-                                 static_cast<double *>(out), static_cast<double *>(scratch), s);
-    return dense_run<float>(static_cast<const float *>(c), static_cast<const float *>(sigma),
-                            static_cast<const float *>(areas), static_cast<const float *>(self_int), n, (float)k_e,
-                            static_cast<float *>(out), static_cast<float *>(scratch), s);
+        return dense_launch<double, KIND>((const double *)tgt, m, (const double *)c, (const double *)sigma,
+                                          (const double *)areas, n, k_e, (const double *)self_int, (double *)out, s);
+    return dense_launch<float, KIND>((const float *)tgt, m, (const float *)c, (const float *)sigma, (const float *)areas,
+                                     n, (float)k_e, (const float *)self_int, (float *)out, s);
 }
+
+}  // namespace
 
 }  // namespace edfmm
 
 using namespace edfmm;
 
-// ---------------------------------------------------------------------------
-// Allocation-free variant.
-//
-// Some callers cannot allocate device memory while they apply the operator:
-// an application whose framework allocator has already reserved the GPU's
-// free memory (so a cudaMalloc/cudaMallocAsync from this library would fail
-// or fragment that pool), or a host language binding that exposes no CUDA
-// allocator and cannot release device memory it did not create.  For them,
-// the partial sums live in one fixed, file-scope device array instead of
-// stream-ordered scratch.  The array (8 MiB) is part of the library's
-// device image: every GPU that loads the library holds it until the process
-// exits.  Host code must not pass the array's name to a kernel (on the host
-// it is only a stand-in symbol); its device address is looked up once per
-// device with cudaGetSymbolAddress, with that device current, and kept for
-// the life of the process (a cudaDeviceReset would make it stale, so the
-// entry point is not for use after one).
-// ---------------------------------------------------------------------------
-#define EDFMM_DENSE_NOALLOC_SCRATCH_BYTES (8u << 20)
 #define EDFMM_DENSE_NOALLOC_MAX_N 262144
 
-static __device__ __align__(256) unsigned char g_dense_noalloc_scratch[EDFMM_DENSE_NOALLOC_SCRATCH_BYTES];
-
-namespace {
-std::mutex g_noalloc_mu;
-constexpr int kMaxDevices = 64;
-void *g_noalloc_addr[kMaxDevices] = {nullptr};
-
-// Device address of g_dense_noalloc_scratch on the current device (looked up
-// on the first call per device).
-int noalloc_scratch(void **addr) {
-    int dev = 0;
-    EDFMM_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDevices) return fail(EDFMM_ERR_ARG, "device ordinal out of range");
-    std::lock_guard<std::mutex> lock(g_noalloc_mu);
-    if (!g_noalloc_addr[dev]) {
-        void *p = nullptr;
-        cudaError_t e = cudaGetSymbolAddress(&p, g_dense_noalloc_scratch);
-        if (e != cudaSuccess || !p)
-            return fail(EDFMM_ERR_CUDA,
-                        std::string("cudaGetSymbolAddress(g_dense_noalloc_scratch) failed: ") + cudaGetErrorString(e));
-        g_noalloc_addr[dev] = p;
-    }
-    *addr = g_noalloc_addr[dev];
-    return EDFMM_OK;
+extern "C" EDFMM_API int edfmm_dense_matvec(const void *centroids, const void *sigma, const void *areas,
+                                            const void *self_integrals, int64_t n, int dtype, double k_e, void *out,
+                                            void *stream) {
+    if (n < 0) return fail(EDFMM_ERR_ARG, "n must be >= 0");
+    if (dtype != EDFMM_F32 && dtype != EDFMM_F64) return fail(EDFMM_ERR_ARG, "dtype must be EDFMM_F32 or EDFMM_F64");
+    if (n == 0) return EDFMM_OK;
+    if (!centroids || !sigma || !areas || !out) return fail(EDFMM_ERR_ARG, "centroids, sigma, areas, out must be non-NULL");
+    return dense_any<kMatvec>(centroids, n, centroids, sigma, areas, n, dtype, k_e, self_integrals, out,
+                              static_cast<cudaStream_t>(stream));
 }
-}  // namespace
 
 extern "C" EDFMM_API int edfmm_dense_matvec_noalloc(const void *centroids, const void *sigma, const void *areas,
                                                     const void *self_integrals, int64_t n, int dtype, double k_e,
                                                     void *out, void *stream) {
-    if (n < 0) return fail(EDFMM_ERR_ARG, "n must be >= 0");
-    if (dtype != EDFMM_F32 && dtype != EDFMM_F64) return fail(EDFMM_ERR_ARG, "dtype must be EDFMM_F32 or EDFMM_F64");
     if (n > EDFMM_DENSE_NOALLOC_MAX_N)
         return fail(EDFMM_ERR_ARG, "edfmm_dense_matvec_noalloc: n = " + std::to_string(n) + " exceeds its limit of " +
-                                       std::to_string(EDFMM_DENSE_NOALLOC_MAX_N) +
-                                       " panels (fixed 8 MiB device scratch); use edfmm_dense_matvec");
-    if (n == 0) return EDFMM_OK;
-    if (!centroids || !sigma || !areas || !out) return fail(EDFMM_ERR_ARG, "centroids, sigma, areas, out must be non-NULL");
-    const size_t bytes = dense_scratch_bytes(n, dtype);
-    if (bytes > EDFMM_DENSE_NOALLOC_SCRATCH_BYTES)
-        return fail(EDFMM_ERR_ARG, "edfmm_dense_matvec_noalloc: this device needs " + std::to_string(bytes) +
-                                       " bytes of partial sums, above the fixed 8 MiB scratch; use edfmm_dense_matvec");
-    void *scratch = nullptr;
-    if (bytes) {
-        if (int rc = noalloc_scratch(&scratch)) return rc;
-    }
-    // every partial-sum slot the reduction reads is written by this call, so
-    // nothing left by an earlier call needs clearing
-    return dense_matvec(centroids, sigma, areas, self_integrals, n, dtype, k_e, out, scratch,
-                        static_cast<cudaStream_t>(stream));
+                                       std::to_string(EDFMM_DENSE_NOALLOC_MAX_N) + " panels; use edfmm_dense_matvec");
+    return edfmm_dense_matvec(centroids, sigma, areas, self_integrals, n, dtype, k_e, out, stream);
 }
 
-namespace {
-template <typename T>
-int targets_run(const T *tgt, int64_t m, const T *c, const T *sigma, const T *areas, int64_t n, T k_e, T *out,
-                cudaStream_t s) {
-    // target rows of 256, source chunks so that there are ~8 blocks per SM
-    const int64_t rows = (m + kRows - 1) / kRows;
-    const int64_t want = 8LL * sm_count();
-    int64_t nch = rows >= want ? 1 : (want + rows - 1) / rows;
-    nch = std::min<int64_t>(std::max<int64_t>(nch, 1), 64);
-    int64_t chunk = ((n + nch - 1) / nch + kTile - 1) / kTile * kTile;
-    if (chunk <= 0) chunk = kTile;
-    int chunks = (int)((n + chunk - 1) / chunk);
-    if (chunks < 1) chunks = 1;
-    T *partial = nullptr;
-    if (chunks > 1) EDFMM_CUDA_TRY(cudaMallocAsync((void **)&partial, sizeof(T) * (size_t)chunks * (size_t)m, s));
-    dim3 grid((unsigned)((m + kRows - 1) / kRows), (unsigned)chunks);
-    k_targets_partial<T><<<grid, kRows, 0, s>>>(tgt, m, c, sigma, areas, n, chunk, partial, chunks == 1, k_e, out);
-    int rc = EDFMM_OK;
-    {
-        count_launch();
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) rc = fail(EDFMM_ERR_CUDA, std::string("k_targets_partial: ") + cudaGetErrorString(e));
-    }
-    if (!rc && chunks > 1) {
-        k_targets_reduce<T><<<(unsigned)((m + 255) / 256), 256, 0, s>>>(partial, chunks, m, k_e, out);
-        count_launch();
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) rc = fail(EDFMM_ERR_CUDA, std::string("k_targets_reduce: ") + cudaGetErrorString(e));
-    }
-    if (partial) cudaFreeAsync(partial, s);
-    return rc;
+extern "C" EDFMM_API size_t edfmm_dense_workspace_bytes(int64_t, int) { return 0; }
+
+extern "C" EDFMM_API int edfmm_dense_matvec_ws(const void *centroids, const void *sigma, const void *areas,
+                                               const void *self_integrals, int64_t n, int dtype, double k_e, void *out,
+                                               void *, size_t, void *stream) {
+    return edfmm_dense_matvec(centroids, sigma, areas, self_integrals, n, dtype, k_e, out, stream);
 }
-template <typename T>
-int field_run(const T *tgt, int64_t m, const T *c, const T *sigma, const T *areas, int64_t n, T k_e, T *out,
-              cudaStream_t s) {
-    const int64_t rows = (m + kRows - 1) / kRows;
-    const int64_t want = 8LL * sm_count();
-    int64_t nch = rows >= want ? 1 : (want + rows - 1) / rows;
-    nch = std::min<int64_t>(std::max<int64_t>(nch, 1), 64);
-    int64_t chunk = ((n + nch - 1) / nch + kTile - 1) / kTile * kTile;
-    if (chunk <= 0) chunk = kTile;
-    int chunks = (int)((n + chunk - 1) / chunk);
-    if (chunks < 1) chunks = 1;
-    T *partial = nullptr;
-    if (chunks > 1)
-        EDFMM_CUDA_TRY(cudaMallocAsync((void **)&partial, sizeof(T) * 3 * (size_t)chunks * (size_t)m, s));
-    dim3 grid((unsigned)((m + kRows - 1) / kRows), (unsigned)chunks);
-    k_field_partial<T><<<grid, kRows, 0, s>>>(tgt, m, c, sigma, areas, n, chunk, partial, chunks == 1, k_e, out);
-    int rc = EDFMM_OK;
-    {
-        count_launch();
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) rc = fail(EDFMM_ERR_CUDA, std::string("k_field_partial: ") + cudaGetErrorString(e));
-    }
-    if (!rc && chunks > 1) {
-        k_field_reduce<T><<<(unsigned)((m + 255) / 256), 256, 0, s>>>(partial, chunks, m, out);
-        count_launch();
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) rc = fail(EDFMM_ERR_CUDA, std::string("k_field_reduce: ") + cudaGetErrorString(e));
-    }
-    if (partial) cudaFreeAsync(partial, s);
-    return rc;
-}
-}  // namespace
 
 extern "C" EDFMM_API int edfmm_dense_field_targets(const void *targets, int64_t m, const void *centroids,
                                                    const void *sigma, const void *areas, int64_t n, int dtype,
@@ -453,11 +523,7 @@ extern "C" EDFMM_API int edfmm_dense_field_targets(const void *targets, int64_t 
         return EDFMM_OK;
     }
     if (!targets || !centroids || !sigma || !areas || !out) return fail(EDFMM_ERR_ARG, "NULL argument");
-    if (dtype == EDFMM_F64)
-        return field_run<double>((const double *)targets, m, (const double *)centroids, (const double *)sigma,
-                                 (const double *)areas, n, k_e, (double *)out, s);
-    return field_run<float>((const float *)targets, m, (const float *)centroids, (const float *)sigma,
-                            (const float *)areas, n, (float)k_e, (float *)out, s);
+    return dense_any<kField>(targets, m, centroids, sigma, areas, n, dtype, k_e, nullptr, out, s);
 }
 
 extern "C" EDFMM_API int edfmm_dense_potential_targets(const void *targets, int64_t m, const void *centroids,
@@ -472,46 +538,5 @@ extern "C" EDFMM_API int edfmm_dense_potential_targets(const void *targets, int6
         return EDFMM_OK;
     }
     if (!targets || !centroids || !sigma || !areas || !out) return fail(EDFMM_ERR_ARG, "NULL argument");
-    if (dtype == EDFMM_F64)
-        return targets_run<double>((const double *)targets, m, (const double *)centroids, (const double *)sigma,
-                                   (const double *)areas, n, k_e, (double *)out, s);
-    return targets_run<float>((const float *)targets, m, (const float *)centroids, (const float *)sigma,
-                              (const float *)areas, n, (float)k_e, (float *)out, s);
-}
-
-extern "C" EDFMM_API size_t edfmm_dense_workspace_bytes(int64_t n, int dtype) {
-    return n > 0 ? dense_scratch_bytes(n, dtype) : 0;
-}
-
-extern "C" EDFMM_API int edfmm_dense_matvec_ws(const void *centroids, const void *sigma, const void *areas,
-                                               const void *self_integrals, int64_t n, int dtype, double k_e, void *out,
-                                               void *workspace, size_t workspace_bytes, void *stream) {
-    if (n < 0) return fail(EDFMM_ERR_ARG, "n must be >= 0");
-    if (dtype != EDFMM_F32 && dtype != EDFMM_F64) return fail(EDFMM_ERR_ARG, "dtype must be EDFMM_F32 or EDFMM_F64");
-    if (n == 0) return EDFMM_OK;
-    if (!centroids || !sigma || !areas || !out) return fail(EDFMM_ERR_ARG, "centroids, sigma, areas, out must be non-NULL");
-    const size_t bytes = dense_scratch_bytes(n, dtype);
-    if (bytes && (!workspace || workspace_bytes < bytes))
-        return fail(EDFMM_ERR_ARG, "workspace smaller than edfmm_dense_workspace_bytes(n, dtype)");
-    return dense_matvec(centroids, sigma, areas, self_integrals, n, dtype, k_e, out, workspace,
-                        static_cast<cudaStream_t>(stream));
-}
-
-extern "C" EDFMM_API int edfmm_dense_matvec(const void *centroids, const void *sigma, const void *areas,
-                                            const void *self_integrals, int64_t n, int dtype, double k_e, void *out,
-                                            void *stream) {
-    if (n < 0) return fail(EDFMM_ERR_ARG, "n must be >= 0");
-    if (dtype != EDFMM_F32 && dtype != EDFMM_F64) return fail(EDFMM_ERR_ARG, "dtype must be EDFMM_F32 or EDFMM_F64");
-    if (n == 0) return EDFMM_OK;
-    if (!centroids || !sigma || !areas || !out) return fail(EDFMM_ERR_ARG, "centroids, sigma, areas, out must be non-NULL");
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const size_t bytes = dense_scratch_bytes(n, dtype);
-    void *scratch = nullptr;
-    if (bytes) EDFMM_CUDA_TRY(cudaMallocAsync(&scratch, bytes, s));
-    int rc = dense_matvec(centroids, sigma, areas, self_integrals, n, dtype, k_e, out, scratch, s);
-    if (scratch) {
-        cudaError_t e = cudaFreeAsync(scratch, s);
-        if (!rc && e != cudaSuccess) rc = fail(EDFMM_ERR_CUDA, std::string("cudaFreeAsync: ") + cudaGetErrorString(e));
-    }
-    return rc;
+    return dense_any<kPotential>(targets, m, centroids, sigma, areas, n, dtype, k_e, nullptr, out, s);
 }

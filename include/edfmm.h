@@ -239,8 +239,11 @@ EDFMM_API int edfmm_plan_get_expansions(const edfmm_plan *plan, void *multipoles
  *   out_i = k_e sum_{j != i} sigma_j areas_j / sqrt(max(|c_i - c_j|^2, 1e-24))
  *           + self_integrals_i sigma_i areas_i   (self term only if non-NULL);
  *   non-finite entries -> 0.  centroids (n, 3) row-major, vectors (n,).
- * Partial sums live in stream-ordered scratch (cudaMallocAsync/cudaFreeAsync
- * on `stream`).
+ * Partial sums live in the shared memory of thread-block clusters: the call
+ * allocates nothing and may be captured in a CUDA graph.  In EDFMM_F64 the
+ * distances are evaluated on the FP32 pipe from coordinates split exactly into
+ * three floats, with the accuracy of IEEE FP64 (about 2^-53 per term); terms
+ * and sums are FP64.
  */
 EDFMM_API int edfmm_dense_matvec(const void *centroids_dev, const void *sigma_dev, const void *areas_dev,
                                  const void *self_integrals_dev, int64_t n, int dtype, double k_e, void *out_dev,
@@ -253,19 +256,9 @@ EDFMM_API int edfmm_dense_matvec(const void *centroids_dev, const void *sigma_de
  * and cannot free device memory it did not create.  No counterpart in the
  * reference (it has no device code for this operator).
  *
- * Allocates nothing: the partial sums live in a fixed 8 MiB file-scope
- * device array that every GPU loading the library keeps until exit.
  * Limit: n <= 262144 panels; larger n returns EDFMM_ERR_ARG with a message
- * (use edfmm_dense_matvec).  The caller still provides all inputs and `out`.
- * The first call on each device looks up the array's device address with
- * cudaGetSymbolAddress; make that first call before any stream capture.
- * The address is kept for the life of the process, so do not call this
- * entry point after cudaDeviceReset (or anything else that recreates the
- * device's primary context) in the same process.
- * All calls share the array, so calls whose work overlaps on the GPU (on
- * different streams, or on different host threads without ordering) race;
- * order them on one stream.  Each call rewrites every scratch slot it reads,
- * so no clearing is needed between calls.
+ * (use edfmm_dense_matvec, which allocates nothing either).  The caller
+ * provides all inputs and `out`.
  */
 EDFMM_API int edfmm_dense_matvec_noalloc(const void *centroids_dev, const void *sigma_dev, const void *areas_dev,
                                          const void *self_integrals_dev, int64_t n, int dtype, double k_e,
@@ -275,7 +268,7 @@ EDFMM_API int edfmm_dense_matvec_noalloc(const void *centroids_dev, const void *
  * Induced potential at separate targets (bem_potential_targets,
  * electrodrive/core/bem_kernel.py:233-270):
  *   out_t = k_e sum_j sigma_j areas_j / sqrt(max(|x_t - c_j|^2, 1e-24)).
- * targets (m, 3); stream-ordered scratch.
+ * targets (m, 3).
  */
 EDFMM_API int edfmm_dense_potential_targets(const void *targets_dev, int64_t m, const void *centroids_dev,
                                             const void *sigma_dev, const void *areas_dev, int64_t n, int dtype,
@@ -291,8 +284,8 @@ EDFMM_API int edfmm_dense_field_targets(const void *targets_dev, int64_t m, cons
 
 /*
  * Dense operator with a caller-provided workspace of
- * edfmm_dense_workspace_bytes(n, dtype) bytes (may be 0): allocates nothing,
- * so it can be captured in a CUDA graph.  Same math as edfmm_dense_matvec.
+ * edfmm_dense_workspace_bytes(n, dtype) bytes (0: the kernels need none, and
+ * the workspace may be NULL).  The same as edfmm_dense_matvec.
  */
 EDFMM_API size_t edfmm_dense_workspace_bytes(int64_t n, int dtype);
 EDFMM_API int edfmm_dense_matvec_ws(const void *centroids_dev, const void *sigma_dev, const void *areas_dev,
