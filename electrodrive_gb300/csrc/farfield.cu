@@ -92,47 +92,86 @@ __global__ void k_set_charges_split(double4 *pts, float4 *pts_tf, const int32_t 
 }
 
 // ---------------------------------------------------------------------------
-// P2M: warp per leaf, lanes over points
+// P2M: warp per leaf, lanes over points.  A lane's terms q R_n^m go straight to
+// shared memory (row v = 2 tri(n, m) + part, one column per lane), and one
+// lane per row adds the columns that hold points: at p = 8 and 20 points 90
+// stores and 60 adds per lane, where a shuffle tree over register arrays
+// takes 450 shuffles and 450 adds (and FP64 arrays of 180 values spill; an
+// FP64 add takes 64 issue cycles).  Beside the near field, FP64, 2,468 leaves
+// of 20 points: 282 -> 209 us; FP32, 9,856 leaves of 20 points (order 6): 39 ->
+// 22 us.
 // ---------------------------------------------------------------------------
+template <typename T> constexpr int p2m_warps() { return sizeof(T) == 4 ? 4 : 2; }
+
 template <typename T, int P>
-__global__ void __launch_bounds__(128) k_p2m(const int32_t *__restrict__ leaves, int64_t n_leaves,
-                                             const typename Vec4<T>::type *__restrict__ pts,
-                                             const typename Vec4<T>::type *__restrict__ center,
-                                             const typename Vec4<T>::type *__restrict__ half, const int2 *range,
-                                             Cplx<T> *Mexp, int nc_pad) {
-    constexpr int NC = ncoef(P);
+__global__ void __launch_bounds__(32 * p2m_warps<T>())
+    k_p2m(const int32_t *__restrict__ leaves, int64_t n_leaves, const typename Vec4<T>::type *__restrict__ pts,
+          const typename Vec4<T>::type *__restrict__ center, const typename Vec4<T>::type *__restrict__ half,
+          const int2 *__restrict__ range, Cplx<T> *__restrict__ Mexp, int nc_pad) {
+    constexpr int NV = 2 * ncoef(P), NR = (NV + 31) / 32;
+    extern __shared__ __align__(16) unsigned char p2m_smem[];
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= n_leaves) return;
+    T *sm = reinterpret_cast<T *>(p2m_smem) + (threadIdx.x >> 5) * (NV * 33);
     const int leaf = leaves[w];
     const typename Vec4<T>::type c = center[leaf];
     const T ia = (T)1 / half[leaf].w;
     const int2 rg = range[leaf];
-    T accr[NC], acci[NC];
+    T acc[NR];
 #pragma unroll
-    for (int k = 0; k < NC; ++k) accr[k] = acci[k] = (T)0;
-    for (int i = rg.x + lane; i < rg.y; i += 32) {
-        const typename Vec4<T>::type p = pts[i];
-        T Rr[NC], Ri[NC];
-        regular_harmonics<T, P>((p.x - c.x) * ia, (p.y - c.y) * ia, (p.z - c.z) * ia, Rr, Ri);
+    for (int j = 0; j < NR; ++j) acc[j] = (T)0;
+    for (int b = rg.x; b < rg.y; b += 32) {
+        const int na = min(32, rg.y - b);
+        __syncwarp();
+        if (lane < na) {
+            const typename Vec4<T>::type p = pts[b + lane];
+            const T x = (p.x - c.x) * ia, y = (p.y - c.y) * ia, z = (p.z - c.z) * ia, q = p.w;
+            const T r2 = x * x + y * y + z * z;
+            T dr = (T)1, di = (T)0;
 #pragma unroll
-        for (int k = 0; k < NC; ++k) {
-            accr[k] += p.w * Rr[k];
-            acci[k] -= p.w * Ri[k];
+            for (int m = 0; m <= P; ++m) {
+                if (m > 0) {
+                    const T sc = (T)(-1.0 / (2.0 * (m > 0 ? m : 1)));
+                    const T nr = sc * (x * dr - y * di), ni = sc * (x * di + y * dr);
+                    dr = nr;
+                    di = ni;
+                }
+                T pr = dr, pi = di, qr = (T)0, qi = (T)0;
+                sm[(2 * tri(m, m)) * 33 + lane] = q * pr;
+                sm[(2 * tri(m, m) + 1) * 33 + lane] = -(q * pi);
+#pragma unroll
+                for (int n = m + 1; n <= P; ++n) {
+                    const T c1 = (T)(2 * n - 1) / (T)((n + m) * (n - m)), c2 = (T)1 / (T)((n + m) * (n - m));
+                    T nr = c1 * z * pr, ni = c1 * z * pi;
+                    if (n > m + 1) {
+                        nr -= c2 * r2 * qr;
+                        ni -= c2 * r2 * qi;
+                    }
+                    qr = pr;
+                    qi = pi;
+                    pr = nr;
+                    pi = ni;
+                    sm[(2 * tri(n, m)) * 33 + lane] = q * pr;
+                    sm[(2 * tri(n, m) + 1) * 33 + lane] = -(q * pi);
+                }
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < NR; ++j) {
+            const int v = lane + 32 * j;
+            if (v < NV) {
+                T t = acc[j];
+                for (int l = 0; l < na; ++l) t += sm[v * 33 + l];
+                acc[j] = t;
+            }
         }
     }
+    T *out = reinterpret_cast<T *>(Mexp + (int64_t)leaf * nc_pad);
 #pragma unroll
-    for (int k = 0; k < NC; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            accr[k] += __shfl_xor_sync(0xffffffffu, accr[k], o);
-            acci[k] += __shfl_xor_sync(0xffffffffu, acci[k], o);
-        }
-    }
-    Cplx<T> *out = Mexp + (int64_t)leaf * nc_pad;
-#pragma unroll
-    for (int k = 0; k < NC; ++k)
-        if ((k & 31) == lane) out[k] = Cplx<T>{accr[k], acci[k]};
+    for (int j = 0; j < NR; ++j)
+        if (lane + 32 * j < NV) out[lane + 32 * j] = acc[j];
 }
 
 // ---------------------------------------------------------------------------
@@ -212,47 +251,10 @@ __device__ __forceinline__ void fma2_into(float &sr, float &si, float xr, float 
     sr = r.x;
     si = r.y;
 }
-__device__ __forceinline__ void fma2_into(double &sr, double &si, double xr, double xi, double2 c) {
-    sr = fma(xr, c.x, sr);
-    si = fma(xi, c.y, si);
-}
-
-// FP64 coefficient arrays in the thread's shared-memory slots (element i at
-// b[i * STRIDE]: one word per thread per coefficient, conflict-free): the
-// 180 doubles of a translation do not fit in registers.  Elements are read
-// and written with volatile shared-memory accesses, which the compiler keeps
-// in program order and may neither hoist into registers nor merge, so the
-// arrays stay in shared memory (FP64 FMAs are the cost here, not the loads).
-__device__ __forceinline__ double lds_vol(const double *p) {
-    double v;
-    asm volatile("ld.volatile.shared.f64 %0, [%1];" : "=d"(v) : "r"((unsigned)__cvta_generic_to_shared(p)));
-    return v;
-}
-__device__ __forceinline__ void sts_vol(double *p, double v) {
-    asm volatile("st.volatile.shared.f64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p)), "d"(v));
-}
-struct DRef {
-    double *p;
-    __device__ __forceinline__ operator double() const { return lds_vol(p); }
-    __device__ __forceinline__ DRef &operator=(double v) {
-        sts_vol(p, v);
-        return *this;
-    }
-    __device__ __forceinline__ DRef &operator=(const DRef &o) { return *this = (double)o; }
-    __device__ __forceinline__ DRef &operator+=(double v) { return *this = lds_vol(p) + v; }
-};
-template <int STRIDE> struct DArr {
-    double *b;
-    __device__ __forceinline__ DRef operator[](int i) const { return DRef{b + i * STRIDE}; }
-};
-__device__ __forceinline__ void fma2_into(DRef sr, DRef si, double xr, double xi, double2 c) {
-    sr = fma(xr, c.x, (double)sr);
-    si = fma(xi, c.y, (double)si);
-}
-
 // ---------------------------------------------------------------------------
-// M2M / L2L fast paths (compile-time order): one thread per node of a level,
-// FP32 in registers with packed FMAs, FP64 in shared-memory slots.  Both
+// M2M / L2L fast paths (compile-time order), one launch per level.  Two forms:
+// one thread per node (FP32, levels of many nodes: registers, packed FMAs),
+// and one warp per node (FP64, and small FP32 levels; below).  Both
 // translations factor the azimuth out like the M2L.  With
 // d = (c_C - c_P) / a_P = (s cos phi, s sin phi, z) and the real regular
 // harmonics rho_k^l := R_k^l(s, 0, z) (R_k^l(d) = e^{i l phi} rho_k^l,
@@ -509,55 +511,258 @@ __device__ __forceinline__ void l2l_node(int node, const int32_t *__restrict__ p
     store_row<P>(Lexp + (int64_t)node * nc_pad, xr, xi);
 }
 
-constexpr int kFastThreads32 = 128, kFastThreads64 = 64;
+constexpr int kFastThreads = 128;
 
-template <typename T> constexpr int fast_threads() { return sizeof(T) == 4 ? kFastThreads32 : kFastThreads64; }
-template <typename T, int P> constexpr size_t fast_smem() {
-    return sizeof(T) == 4 ? 0 : (size_t)4 * ncoef(P) * kFastThreads64 * sizeof(double);
+template <int P>
+__global__ void __launch_bounds__(kFastThreads) k_m2m_fast(
+    const int32_t *__restrict__ nodes, int count, const uint8_t *__restrict__ is_leaf,
+    const int32_t *__restrict__ children, const int32_t *__restrict__ parent, const float4 *__restrict__ center,
+    const float4 *__restrict__ half, float2 *__restrict__ Mexp, float2 *__restrict__ moved, int nc_pad) {
+    constexpr int NC = ncoef(P);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    float xr[NC], xi[NC], Sr[NC], Si[NC];
+    m2m_node<float, P>(nodes[i], is_leaf, children, parent, center, half, Mexp, moved, nc_pad, xr, xi, Sr, Si);
+}
+
+template <int P>
+__global__ void __launch_bounds__(kFastThreads) k_l2l_fast(const int32_t *__restrict__ nodes, int count,
+                                                            const int32_t *__restrict__ parent,
+                                                            const float4 *__restrict__ center,
+                                                            const float4 *__restrict__ half, float2 *__restrict__ Lexp,
+                                                            int nc_pad) {
+    constexpr int NC = ncoef(P);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    float xr[NC], xi[NC], Sr[NC], Si[NC];
+    l2l_node<float, P>(nodes[i], parent, center, half, Lexp, nc_pad, xr, xi, Sr, Si);
+}
+
+// ---------------------------------------------------------------------------
+// The same translations with one warp per node, lanes over output
+// coefficients.  A thread that owns a node walks about 2,600 dependent
+// operations: 10 us however few nodes a level has in FP32, and 130 to 280 us in
+// FP64, whose pipe issues a warp's operation in 64 cycles whether one lane is
+// active or all (two FP64 lanes per SM and clock).  Spread over the lanes a
+// node takes about 45 multiply-adds per lane.  The lanes' outputs are paired
+// long with short, so that the warp's longest chain (the number of (k, l)
+// terms of its outputs) is within a few terms of the mean.  FP64, 50k-panel
+// torus, six levels: M2M 1,060 -> 127 us, L2L 640 -> 119 us.
+// ---------------------------------------------------------------------------
+constexpr int kWarpNodes = 4;  // nodes (warps) per block
+
+// number of terms (k, l) of output (n, m): |l| <= k and |m - l| <= n - k (M2M),
+// or k <= P - n, |l| <= k (L2L)
+__host__ __device__ constexpr int shift_terms(int P, bool l2l, int n, int m) {
+    int t = 0;
+    for (int k = 0; k <= (l2l ? P - n : n); ++k)
+        for (int l = -k; l <= k; ++l) {
+            const int u = l2l ? m + l : m - l, j = l2l ? n + k : n - k;
+            if (u >= -j && u <= j) ++t;
+        }
+    return t;
+}
+// the outputs of each lane, (n, m) packed as n * 16 + m, 255 for none: the
+// outputs by decreasing term count take the lanes in turn, back and forth
+template <int P, bool L2L> struct ShiftPlan {
+    static constexpr int NR = (ncoef(P) + 31) / 32;
+    unsigned char out[NR][32];
+    __host__ __device__ constexpr ShiftPlan() : out() {
+        int key[ncoef(P)] = {}, nm[ncoef(P)] = {};
+        int c = 0;
+        for (int n = 0; n <= P; ++n)
+            for (int m = 0; m <= n; ++m, ++c) {
+                const int t = shift_terms(P, L2L, n, m);
+                int i = c;
+                for (; i > 0 && key[i - 1] < t; --i) {
+                    key[i] = key[i - 1];
+                    nm[i] = nm[i - 1];
+                }
+                key[i] = t;
+                nm[i] = n * 16 + m;
+            }
+        for (int r = 0; r < NR; ++r)
+            for (int l = 0; l < 32; ++l) {
+                const int q = r * 32 + l;
+                out[r][(r & 1) ? 31 - l : l] = q < ncoef(P) ? (unsigned char)nm[q] : 255;
+            }
+    }
+};
+template <int P, bool L2L> __device__ const ShiftPlan<P, L2L> d_shift_plan{};
+
+template <typename T, int P> struct WarpShift {
+    typename Pair<T>::type x[(P + 1) * (P + 1)];  // rotated input, all orders: (n, m) at n^2 + n + m
+    T rho[(P + 1) * (P + 1)];                     // rho_k^l at k^2 + k + l
+    typename Pair<T>::type ph[P + 1];             // e^{i m phi}
+    T fr[P + 1];                                  // (a_C / a_P)^n
+};
+
+// lanes 0..P: e^{i m phi}, ratio^m and column m of rho
+template <typename T, int P>
+__device__ __forceinline__ void warp_shift_frame(WarpShift<T, P> &S, const Shift<T> &f, int lane) {
+    if (lane <= P) {
+        const int m = lane;
+        T wr = 1, wi = 0, fm = 1, diag = 1, ar = f.ec, ai = f.es, ra = f.ratio, sa = -f.s;
+#pragma unroll
+        for (int bit = 1; bit <= P; bit <<= 1) {  // powers by their binary digits
+            if (m & bit) {
+                const T nr = wr * ar - wi * ai, ni = wr * ai + wi * ar;
+                wr = nr;
+                wi = ni;
+                fm *= ra;
+                diag *= sa;
+            }
+            const T nr = ar * ar - ai * ai, ni = (T)2 * ar * ai;
+            ar = nr;
+            ai = ni;
+            ra *= ra;
+            sa *= sa;
+        }
+        S.ph[m] = mk2(wr, wi);
+        S.fr[m] = fm;
+        T inv = (T)1;
+#pragma unroll
+        for (int i = 1; i <= P; ++i)
+            if (i <= m) inv *= (T)(1.0 / (2.0 * i));
+        T cm1 = diag * inv, cm2 = 0;  // rho_m^m = (-s / 2)^m / m!
+        const T sg = (m & 1) ? (T)-1 : (T)1;
+        S.rho[m * m + 2 * m] = cm1;
+        S.rho[m * m] = sg * cm1;
+        for (int k = m + 1; k <= P; ++k) {
+            const T d = (T)1 / (T)((k + m) * (k - m));
+            const T c = ((T)(2 * k - 1) * f.z * cm1 - f.r2 * cm2) * d;
+            cm2 = cm1;
+            cm1 = c;
+            S.rho[k * k + k + m] = c;
+            S.rho[k * k + k - m] = sg * c;
+        }
+    }
+}
+
+// x_n^m e^{i m phi} g, stored for orders m and -m (X^{-m} = (-1)^m conj X^m)
+template <typename T, int P>
+__device__ __forceinline__ void warp_shift_put(WarpShift<T, P> &S, int n, int m, T xr, T xi, T g) {
+    const auto w = S.ph[m];
+    const T fr = w.x * g, fi = w.y * g;
+    const T yr = xr * fr - xi * fi, yi = xr * fi + xi * fr;
+    const T sg = (m & 1) ? (T)-1 : (T)1;
+    S.x[n * n + n - m] = mk2(sg * yr, -sg * yi);
+    S.x[n * n + n + m] = mk2(yr, yi);
+}
+
+// sum over the terms of output (n, m)
+template <typename T, int P, bool L2L>
+__device__ __forceinline__ typename Pair<T>::type warp_shift_sum(const WarpShift<T, P> &S, int n, int m) {
+    T sr = 0, si = 0;
+    const int kmax = L2L ? P - n : n;
+    int k = 0, ri = 0, xi = n * n + n + m, left = 1;  // k = 0: the single term l = 0
+    while (true) {
+        const auto x = S.x[xi];
+        const T r = S.rho[ri];
+        sr = fma(r, x.x, sr);
+        si = fma(r, x.y, si);
+        ++ri;
+        xi += L2L ? 1 : -1;
+        if (--left == 0) {
+            if (++k > kmax) break;
+            const int j = L2L ? n + k : n - k;
+            // l from max(-k, m - j) (M2M) or max(-k, -j - m) (L2L) to min(k, m + j) or min(k, j - m)
+            const int lo = max(-k, L2L ? -j - m : m - j), hi = min(k, L2L ? j - m : m + j);
+            left = hi - lo + 1;
+            ri = k * k + k + lo;
+            xi = j * j + j + (L2L ? m + lo : m - lo);
+        }
+    }
+    return mk2(sr, si);
 }
 
 template <typename T, int P>
-__global__ void __launch_bounds__(fast_threads<T>()) k_m2m_fast(
+__global__ void __launch_bounds__(32 * kWarpNodes) k_m2m_warp(
     const int32_t *__restrict__ nodes, int count, const uint8_t *__restrict__ is_leaf,
     const int32_t *__restrict__ children, const int32_t *__restrict__ parent,
     const typename Vec4<T>::type *__restrict__ center, const typename Vec4<T>::type *__restrict__ half,
     typename Pair<T>::type *__restrict__ Mexp, typename Pair<T>::type *__restrict__ moved, int nc_pad) {
-    constexpr int NC = ncoef(P);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    using T2 = typename Pair<T>::type;
+    constexpr int NR = ShiftPlan<P, false>::NR;
+    __shared__ WarpShift<T, P> shifts[kWarpNodes];
+    const int lane = threadIdx.x & 31, i = blockIdx.x * kWarpNodes + (threadIdx.x >> 5);
     if (i >= count) return;
-    const int node = nodes[i];
-    if constexpr (sizeof(T) == 4) {
-        float xr[NC], xi[NC], Sr[NC], Si[NC];
-        m2m_node<T, P>(node, is_leaf, children, parent, center, half, Mexp, moved, nc_pad, xr, xi, Sr, Si);
-    } else {
-        extern __shared__ double fast_dsm[];
-        constexpr int S = kFastThreads64;
-        DArr<S> xr{fast_dsm + threadIdx.x}, xi{fast_dsm + NC * S + threadIdx.x}, Sr{fast_dsm + 2 * NC * S + threadIdx.x},
-            Si{fast_dsm + 3 * NC * S + threadIdx.x};
-        m2m_node<T, P>(node, is_leaf, children, parent, center, half, Mexp, moved, nc_pad, xr, xi, Sr, Si);
+    WarpShift<T, P> &S = shifts[threadIdx.x >> 5];
+    const int node = nodes[i], par = parent[node];
+    T2 x[NR];
+    int nm[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        nm[r] = d_shift_plan<P, false>.out[r][lane];
+        x[r] = mk2((T)0, (T)0);
+        if (nm[r] == 255) continue;
+        const int q = tri(nm[r] >> 4, nm[r] & 15);
+        if (is_leaf[node]) {
+            x[r] = Mexp[(int64_t)node * nc_pad + q];
+        } else {
+            for (int o = 0; o < 8; ++o) {
+                const int ch = children[8 * node + o];
+                if (ch < 0) continue;
+                const T2 v = moved[(int64_t)ch * nc_pad + q];
+                x[r].x += v.x;
+                x[r].y += v.y;
+            }
+            Mexp[(int64_t)node * nc_pad + q] = x[r];
+        }
+    }
+    if (par < 0) return;
+    const Shift<T> f = shift_of<T>(center[node], center[par], half[node].w, half[par].w);
+    warp_shift_frame<T, P>(S, f, lane);
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+        if (nm[r] != 255) warp_shift_put<T, P>(S, nm[r] >> 4, nm[r] & 15, x[r].x, x[r].y, S.fr[nm[r] >> 4]);
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        if (nm[r] == 255) continue;
+        const int n = nm[r] >> 4, m = nm[r] & 15;
+        const T2 v = warp_shift_sum<T, P, false>(S, n, m), w = S.ph[m];
+        moved[(int64_t)node * nc_pad + tri(n, m)] = mk2(v.x * w.x + v.y * w.y, v.y * w.x - v.x * w.y);  // e^{-i m phi}
     }
 }
 
 template <typename T, int P>
-__global__ void __launch_bounds__(fast_threads<T>()) k_l2l_fast(const int32_t *__restrict__ nodes, int count,
-                                                                 const int32_t *__restrict__ parent,
-                                                                 const typename Vec4<T>::type *__restrict__ center,
-                                                                 const typename Vec4<T>::type *__restrict__ half,
-                                                                 typename Pair<T>::type *__restrict__ Lexp,
-                                                                 int nc_pad) {
-    constexpr int NC = ncoef(P);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(32 * kWarpNodes) k_l2l_warp(
+    const int32_t *__restrict__ nodes, int count, const int32_t *__restrict__ parent,
+    const typename Vec4<T>::type *__restrict__ center, const typename Vec4<T>::type *__restrict__ half,
+    typename Pair<T>::type *__restrict__ Lexp, int nc_pad) {
+    using T2 = typename Pair<T>::type;
+    constexpr int NR = ShiftPlan<P, true>::NR;
+    __shared__ WarpShift<T, P> shifts[kWarpNodes];
+    const int lane = threadIdx.x & 31, i = blockIdx.x * kWarpNodes + (threadIdx.x >> 5);
     if (i >= count) return;
-    const int node = nodes[i];
-    if constexpr (sizeof(T) == 4) {
-        float xr[NC], xi[NC], Sr[NC], Si[NC];
-        l2l_node<T, P>(node, parent, center, half, Lexp, nc_pad, xr, xi, Sr, Si);
-    } else {
-        extern __shared__ double fast_dsm[];
-        constexpr int S = kFastThreads64;
-        DArr<S> xr{fast_dsm + threadIdx.x}, xi{fast_dsm + NC * S + threadIdx.x}, Sr{fast_dsm + 2 * NC * S + threadIdx.x},
-            Si{fast_dsm + 3 * NC * S + threadIdx.x};
-        l2l_node<T, P>(node, parent, center, half, Lexp, nc_pad, xr, xi, Sr, Si);
+    WarpShift<T, P> &S = shifts[threadIdx.x >> 5];
+    const int node = nodes[i], par = parent[node];
+    if (par < 0) return;
+    T2 x[NR];
+    int nm[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        nm[r] = d_shift_plan<P, true>.out[r][lane];
+        if (nm[r] != 255) x[r] = Lexp[(int64_t)par * nc_pad + tri(nm[r] >> 4, nm[r] & 15)];
+    }
+    const Shift<T> f = shift_of<T>(center[node], center[par], half[node].w, half[par].w);
+    warp_shift_frame<T, P>(S, f, lane);
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+        if (nm[r] != 255) warp_shift_put<T, P>(S, nm[r] >> 4, nm[r] & 15, x[r].x, x[r].y, (T)1);
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        if (nm[r] == 255) continue;
+        const int n = nm[r] >> 4, m = nm[r] & 15;
+        const T2 v = warp_shift_sum<T, P, true>(S, n, m), w = S.ph[m];
+        const T g = S.fr[n];  // (a_C / a_P)^j e^{-i u phi}
+        T2 *o = Lexp + (int64_t)node * nc_pad + tri(n, m);
+        const T2 old = *o;
+        *o = mk2(old.x + g * (v.x * w.x + v.y * w.y), old.y + g * (v.y * w.x - v.x * w.y));
     }
 }
 
@@ -751,13 +956,21 @@ __global__ void __launch_bounds__(128) k_l2l(const int32_t *__restrict__ nodes, 
 template <typename T> int p2m_impl(const DevTree &tree, FmmBuffers &buf, cudaStream_t s) {
     using T4 = typename Vec4<T>::type;
     if (tree.n_leaves == 0) return EDFMM_OK;
-    const unsigned grid = nblk(tree.n_leaves * 32, 128);
+    constexpr int NT = 32 * p2m_warps<T>();
+    const unsigned grid = nblk(tree.n_leaves * 32, NT);
+    const size_t smem = sizeof(T) * 33 * 2 * (size_t)ncoef(buf.p) * p2m_warps<T>();
 #define EDFMM_P2M_CASE(PP)                                                                                          \
-    case PP:                                                                                                        \
-        k_p2m<T, PP><<<grid, 128, 0, s>>>(dptr<int32_t>(tree.leaves), tree.n_leaves, dptr<T4>(tree.pts),              \
-                                          dptr<T4>(tree.center), dptr<T4>(tree.half), dptr<int2>(tree.range),          \
-                                          dptr<Cplx<T>>(buf.multipoles), buf.nc_pad);                                \
-        break;
+    case PP: {                                                                                                      \
+        static const cudaError_t attr =                                                                             \
+            cudaFuncSetAttribute(k_p2m<T, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize,                         \
+                                 (int)(sizeof(T) * 33 * 2 * ncoef(PP) * p2m_warps<T>()));                            \
+        if (attr != cudaSuccess)                                                                                    \
+            return fail(EDFMM_ERR_CUDA, std::string("k_p2m shared memory: ") + cudaGetErrorString(attr));           \
+        k_p2m<T, PP><<<grid, NT, smem, s>>>(dptr<int32_t>(tree.leaves), tree.n_leaves, dptr<T4>(tree.pts),           \
+                                            dptr<T4>(tree.center), dptr<T4>(tree.half), dptr<int2>(tree.range),       \
+                                            dptr<Cplx<T>>(buf.multipoles), buf.nc_pad);                              \
+        break;                                                                                                      \
+    }
     switch (buf.p) {
         EDFMM_P2M_CASE(1)
         EDFMM_P2M_CASE(2)
@@ -777,26 +990,32 @@ template <typename T> int p2m_impl(const DevTree &tree, FmmBuffers &buf, cudaStr
     return EDFMM_OK;
 }
 
-template <typename T, int P> int fast_smem_attr(const void *fn) {
-    if (fast_smem<T, P>() <= 48 * 1024) return EDFMM_OK;
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fast_smem<T, P>());
-    return e == cudaSuccess ? EDFMM_OK : fail(EDFMM_ERR_CUDA, std::string("fast M2M/L2L shared memory: ") +
-                                                                   cudaGetErrorString(e));
-}
+// FP32 levels up to this many nodes take a warp per node.  At order 6 a level
+// of about 3,000 nodes takes 5.3 us with a warp per node and 10.8 with a
+// thread, one of about 7,000 nodes 9.3 us with a thread; a warp's work per node
+// is ten times a thread's share, so the forms meet between the two.
+constexpr int kWarpLevel = 6144;
 
 template <typename T, int P> int launch_m2m_fast(const DevTree &tree, FmmBuffers &buf, cudaStream_t s) {
     using T4 = typename Vec4<T>::type;
     using T2 = typename Pair<T>::type;
-    static const int attr = fast_smem_attr<T, P>((const void *)k_m2m_fast<T, P>);
-    if (attr) return attr;
-    constexpr int NT = fast_threads<T>();
     for (int lev = tree.max_level; lev >= 0; --lev) {
         const int lo = tree.level_offsets[lev], hi = tree.level_offsets[lev + 1];
         if (hi <= lo) continue;
-        k_m2m_fast<T, P><<<nblk(hi - lo, NT), NT, fast_smem<T, P>(), s>>>(
-            dptr<int32_t>(tree.level_nodes) + lo, hi - lo, dptr<uint8_t>(tree.is_leaf), dptr<int32_t>(tree.children),
-            dptr<int32_t>(tree.parent), dptr<T4>(tree.center), dptr<T4>(tree.half), dptr<T2>(buf.multipoles),
-            dptr<T2>(buf.translated), buf.nc_pad);
+        const int32_t *nodes = dptr<int32_t>(tree.level_nodes) + lo;
+        bool warp = sizeof(T) == 8 || hi - lo <= kWarpLevel;
+        if constexpr (sizeof(T) == 4) {
+            if (!warp)
+                k_m2m_fast<P><<<nblk(hi - lo, kFastThreads), kFastThreads, 0, s>>>(
+                    nodes, hi - lo, dptr<uint8_t>(tree.is_leaf), dptr<int32_t>(tree.children),
+                    dptr<int32_t>(tree.parent), dptr<float4>(tree.center), dptr<float4>(tree.half),
+                    dptr<float2>(buf.multipoles), dptr<float2>(buf.translated), buf.nc_pad);
+        }
+        if (warp)
+            k_m2m_warp<T, P><<<nblk(hi - lo, kWarpNodes), 32 * kWarpNodes, 0, s>>>(
+                nodes, hi - lo, dptr<uint8_t>(tree.is_leaf), dptr<int32_t>(tree.children), dptr<int32_t>(tree.parent),
+                dptr<T4>(tree.center), dptr<T4>(tree.half), dptr<T2>(buf.multipoles), dptr<T2>(buf.translated),
+                buf.nc_pad);
         if (lev > 0) count_launch();
     }
     return EDFMM_OK;
@@ -805,15 +1024,21 @@ template <typename T, int P> int launch_m2m_fast(const DevTree &tree, FmmBuffers
 template <typename T, int P> int launch_l2l_fast(const DevTree &tree, FmmBuffers &buf, cudaStream_t s) {
     using T4 = typename Vec4<T>::type;
     using T2 = typename Pair<T>::type;
-    static const int attr = fast_smem_attr<T, P>((const void *)k_l2l_fast<T, P>);
-    if (attr) return attr;
-    constexpr int NT = fast_threads<T>();
     for (int lev = 1; lev <= tree.max_level; ++lev) {
         const int lo = tree.level_offsets[lev], hi = tree.level_offsets[lev + 1];
         if (hi <= lo) continue;
-        k_l2l_fast<T, P><<<nblk(hi - lo, NT), NT, fast_smem<T, P>(), s>>>(
-            dptr<int32_t>(tree.level_nodes) + lo, hi - lo, dptr<int32_t>(tree.parent), dptr<T4>(tree.center),
-            dptr<T4>(tree.half), dptr<T2>(buf.locals), buf.nc_pad);
+        const int32_t *nodes = dptr<int32_t>(tree.level_nodes) + lo;
+        bool warp = sizeof(T) == 8 || hi - lo <= kWarpLevel;
+        if constexpr (sizeof(T) == 4) {
+            if (!warp)
+                k_l2l_fast<P><<<nblk(hi - lo, kFastThreads), kFastThreads, 0, s>>>(
+                    nodes, hi - lo, dptr<int32_t>(tree.parent), dptr<float4>(tree.center), dptr<float4>(tree.half),
+                    dptr<float2>(buf.locals), buf.nc_pad);
+        }
+        if (warp)
+            k_l2l_warp<T, P><<<nblk(hi - lo, kWarpNodes), 32 * kWarpNodes, 0, s>>>(
+                nodes, hi - lo, dptr<int32_t>(tree.parent), dptr<T4>(tree.center), dptr<T4>(tree.half),
+                dptr<T2>(buf.locals), buf.nc_pad);
         if (lev < tree.max_level) count_launch();
     }
     return EDFMM_OK;
