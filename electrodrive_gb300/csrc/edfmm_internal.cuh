@@ -187,6 +187,15 @@ __device__ __forceinline__ float rsqrt_normal(float x) {
 #endif
 
 // Device-resident tree in DFS pre-order (the reference's node numbering).
+// Scale of an FP64 tree's split coordinates (gridpoint.cuh): 2^-k, 2^k, the
+// scaled r^2 below which a pair is evaluated in IEEE FP64, and the high word
+// of the largest |coordinate|.
+struct GridInfo {
+    double down, up;
+    float near2;
+    unsigned hi;
+};
+
 struct DevTree {
     int dtype = EDFMM_F32;
     int64_t n_points = 0;
@@ -206,11 +215,15 @@ struct DevTree {
     DevBuf leaves;     // int32 ids of leaf nodes (ascending)
     std::vector<int32_t> level_offsets;  // host: level l nodes = level_nodes[off[l], off[l+1])
     DevBuf level_nodes;                  // int32 node ids grouped by level
-    // FP64 trees in two-float mode: per point (x, y, z, charge) split into
-    // FP32 (hi, lo) pairs, 8 floats, refreshed with the charges; per node
-    // (cx, cy, cz, expansion scale a) split the same way
-    DevBuf pts_tf;
+    // FP64 trees in two-float mode: per node (cx, cy, cz, expansion scale a)
+    // split into FP32 (hi, lo) pairs
     DevBuf nodes_tf;
+    // FP64 trees: per point the exact coordinate split of gridpoint.cuh and
+    // the charge (three float4; the charge as a double, or as two floats in
+    // two-float mode), and the split's scale
+    DevBuf pts_grid;
+    DevBuf grid_info;
+    bool grid_tf = false;
     // batched plans: instance k owns nodes inst_node_off[k] .. inst_node_off[k+1]-1
     int n_inst = 0;
     DevBuf inst_node_off;  // int32 x (n_inst + 1)
@@ -333,25 +346,24 @@ int prepare_extreme_rows(const DevTree &tree, const DevLists &lists, FmmBuffers 
 // when the order changes
 int prepare_two_float(DevTree &tree, FmmBuffers &buf, cudaStream_t s);
 
-struct NearArgs {
-    const void *sigma = nullptr;      // original order (nullable)
-    const void *areas = nullptr;      // original order (nullable)
-    const void *self_int = nullptr;   // original order (nullable)
+struct L2pArgs {
+    const void *sigma = nullptr;     // original order (nullable)
+    const void *areas = nullptr;     // original order (nullable)
+    const void *self_int = nullptr;  // original order (nullable)
     double k_e = 1.0;
-    void *out = nullptr;              // original order if scatter, else tree order
-    bool scatter = false;             // write out[index_map[i]] with k_e, self term, clamp
-    bool near = true;                 // include P2P
-    bool far = true;                  // include L2P
-    const void *add_in = nullptr;     // tree-order sums added before the epilogue (nullable)
-    // sources of the P2P when they are another tree's points (targets
-    // evaluated against a source plan): no self exclusion then
-    const struct DevTree *src_tree = nullptr;
+    void *out = nullptr;           // original order if scatter, else tree order
+    bool scatter = false;          // write out[index_map[i]] with k_e, self term, clamp
+    bool far = true;               // evaluate the local expansions
+    const void *add_in = nullptr;  // near sums in tree order (nullable)
 };
-// field at the points of a target tree (evaluation from a source plan)
 int run_targets_field(const DevTree &tree, const DevLists &lists, const FmmBuffers &buf, const DevTree &stree,
                       double k_e, bool near, bool far, void *out, cudaStream_t s);
-int run_p2p_l2p(const DevTree &tree, const DevLists &lists, const FmmBuffers &buf,
-                const NearArgs &args, cudaStream_t s);
+// near sums in tree order; src_tree: the sources when they are another
+// tree's points (targets evaluated against a source plan: no self exclusion)
+int run_p2p(const DevTree &tree, const DevLists &lists, const FmmBuffers &buf, const DevTree *src_tree, void *out,
+            cudaStream_t s);
+int run_l2p(const DevTree &tree, const FmmBuffers &buf, const L2pArgs &args, cudaStream_t s);
+int grid_prepare(DevTree &tree, cudaStream_t s);
 int upload_tables();
 
 }  // namespace edfmm

@@ -44,13 +44,32 @@ __device__ __forceinline__ void coef_nm(int c, int &n, int &m) {
 // ---------------------------------------------------------------------------
 // charges
 // ---------------------------------------------------------------------------
+// grid: the split points of an FP64 tree (three float4 per point, the charge in
+// the last two words, as a double or (tf) as two floats), or NULL; a == NULL
+// keeps the charges that are set
 template <typename T>
-__global__ void k_set_charges(typename Vec4<T>::type *pts, const int32_t *__restrict__ idx, int64_t n,
-                              const T *__restrict__ a, const T *__restrict__ b) {
+__global__ void k_set_charges(typename Vec4<T>::type *pts, float4 *grid, int tf, const int32_t *__restrict__ idx,
+                              int64_t n, const T *__restrict__ a, const T *__restrict__ b) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    int o = idx[i];
-    pts[i].w = b ? a[o] * b[o] : a[o];
+    T q;
+    if (a) {
+        const int o = idx[i];
+        q = b ? a[o] * b[o] : a[o];
+        pts[i].w = q;
+    } else {
+        q = pts[i].w;
+    }
+    if constexpr (sizeof(T) == 8) {
+        if (grid) {
+            float2 w = make_float2(__int_as_float(__double2loint(q)), __int_as_float(__double2hiint(q)));
+            if (tf) {
+                const tf32x2 t = tf_from_double(q);
+                w = make_float2(t.hi, t.lo);
+            }
+            *reinterpret_cast<float2 *>(&grid[3 * i + 2].z) = w;
+        }
+    }
 }
 
 // two-float mode: node geometry (cx, cy, cz, a) and FP64 complex
@@ -71,24 +90,6 @@ __global__ void k_split_coeffs(const double2 *__restrict__ in, int64_t n, float4
     const double2 c = in[i];
     const tf32x2 re = tf_from_double(c.x), im = tf_from_double(c.y);
     out[i] = make_float4(re.hi, re.lo, im.hi, im.lo);
-}
-
-// FP64 trees in two-float mode: the charges as above (a == NULL keeps them)
-// and every point split into (hi, lo) FP32 pairs, 8 floats per point
-__global__ void k_set_charges_split(double4 *pts, float4 *pts_tf, const int32_t *__restrict__ idx, int64_t n,
-                                    const double *__restrict__ a, const double *__restrict__ b) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double4 x = pts[i];
-    if (a) {
-        const int o = idx[i];
-        x.w = b ? a[o] * b[o] : a[o];
-        pts[i].w = x.w;
-    }
-    const tf32x2 sx = tf_from_double(x.x), sy = tf_from_double(x.y), sz = tf_from_double(x.z),
-                 sq = tf_from_double(x.w);
-    pts_tf[2 * i] = make_float4(sx.hi, sx.lo, sy.hi, sy.lo);
-    pts_tf[2 * i + 1] = make_float4(sz.hi, sz.lo, sq.hi, sq.lo);
 }
 
 // ---------------------------------------------------------------------------
@@ -1207,21 +1208,15 @@ int m2l_impl(const DevTree &tree, const DevTree &stree, const DevLists &lists, c
 
 int set_charges(const DevTree &tree, const void *a, const void *b, cudaStream_t s) {
     if (tree.n_points == 0) return EDFMM_OK;
-    if (tree.dtype == EDFMM_F64 && tree.pts_tf.p) {
-        k_set_charges_split<<<nblk(tree.n_points, 256), 256, 0, s>>>(
-            dptr<double4>(tree.pts), dptr<float4>(tree.pts_tf), dptr<int32_t>(tree.index_map), tree.n_points,
-            static_cast<const double *>(a), static_cast<const double *>(b));
-        EDFMM_LAUNCH_CHECK("k_set_charges_split");
-        return EDFMM_OK;
-    }
+    const unsigned grid = nblk(tree.n_points, 256);
     if (tree.dtype == EDFMM_F64)
-        k_set_charges<double><<<nblk(tree.n_points, 256), 256, 0, s>>>(dptr<double4>(tree.pts), dptr<int32_t>(tree.index_map),
-                                                                      tree.n_points, static_cast<const double *>(a),
-                                                                      static_cast<const double *>(b));
+        k_set_charges<double><<<grid, 256, 0, s>>>(dptr<double4>(tree.pts), dptr<float4>(tree.pts_grid), tree.grid_tf,
+                                                   dptr<int32_t>(tree.index_map), tree.n_points,
+                                                   static_cast<const double *>(a), static_cast<const double *>(b));
     else
-        k_set_charges<float><<<nblk(tree.n_points, 256), 256, 0, s>>>(dptr<float4>(tree.pts), dptr<int32_t>(tree.index_map),
-                                                                     tree.n_points, static_cast<const float *>(a),
-                                                                     static_cast<const float *>(b));
+        k_set_charges<float><<<grid, 256, 0, s>>>(dptr<float4>(tree.pts), nullptr, 0, dptr<int32_t>(tree.index_map),
+                                                  tree.n_points, static_cast<const float *>(a),
+                                                  static_cast<const float *>(b));
     EDFMM_LAUNCH_CHECK("k_set_charges");
     return EDFMM_OK;
 }

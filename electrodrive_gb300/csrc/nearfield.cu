@@ -1,23 +1,18 @@
-// Near field (P2P) fused with the local-expansion evaluation (L2P) and the
-// matvec epilogue.
+// Near field (P2P) and the local-expansion evaluation with the matvec
+// epilogue (L2P).
 //
-// One warp owns one target leaf.  Source leaves of the target's P2P row are
-// staged in shared memory 64 points at a time (the next chunk loaded while
-// the current one is computed) and read by broadcast.  The leaf's targets
-// are split into slots that each fill the warp (32 targets with one lane
-// each, 16 with two, 8 with four, 4 with eight); FP32 runs the distances as
-// packed pairs.  The kernel is the reference's kernels_cpu.py:83-153
-// contribution
+// P2P is the reference's kernels_cpu.py:83-153 contribution
 //     q_s / max(|x_t - x_s|, eps)   (eps = machine epsilon of the dtype)
 // evaluated as q_s * rsqrt(max(r^2, eps^2)), with the diagonal dropped only
-// inside the self leaf pair.  The same warp then evaluates the leaf's local
-// expansion at its points and, for a full matvec, applies the epilogue of
+// inside the self leaf pair.  L2P evaluates the leaf's local expansion at its
+// points, adds the near sums and, for a full matvec, applies the epilogue of
 // bem_fmm.py:718-749 (K_E, original order, self term, non-finite -> 0), so
 // each output is written exactly once.
 #include <cfloat>
 #include <type_traits>
 
 #include "edfmm_internal.cuh"
+#include "gridpoint.cuh"
 #include "harmonics.cuh"
 #include "twofloat.cuh"
 
@@ -25,25 +20,540 @@ namespace edfmm {
 
 namespace {
 
-__constant__ float c_rdiv_f[kPMax + 1][kPMax + 1];
-__constant__ double c_rdiv_d[kPMax + 1][kPMax + 1];
-__constant__ float2 c_rdiv_tf[kPMax + 1][kPMax + 1];  // (hi, lo) of the FP64 table
+__constant__ float2 c_rdiv_tf[kPMax + 1][kPMax + 1];  // (hi, lo) of 1 / ((n + m)(n - m)), 1 / n^2 at m = 0
 
-template <typename T> __device__ __forceinline__ T rdiv(int n, int m);
-template <> __device__ __forceinline__ float rdiv<float>(int n, int m) { return c_rdiv_f[n][m]; }
-template <> __device__ __forceinline__ double rdiv<double>(int n, int m) { return c_rdiv_d[n][m]; }
+// ---------------------------------------------------------------------------
+// P2P.  One warp owns up to 64 targets of a leaf (a whole leaf at the usual
+// leaf sizes); with few leaves the four warps of a block share one leaf, each
+// walking a quarter of its row.
+//
+// Lanes: the nt targets are held R per lane by L = ceil(nt / R) lanes, and
+// G = 32 / L such groups of lanes split the sources.  R is chosen per nt (table
+// below) for the least time per interaction: a source read from shared memory
+// serves R targets, and few lanes idle whatever nt is.  20 targets: R = 2, ten
+// lanes, three groups; one lane per target would leave a third of the warp idle.
+//
+// Sources: the leaves of a row hold about 20 to 40 points each, so their
+// points are packed back to back into chunks of 64 or 128 staged in shared
+// memory: the ranges of 32 row entries are scanned over the warp, and a
+// position's entry is found by counting the entries that start at or before
+// it (one OR-reduction and population count per 32 positions).  Staging one
+// leaf at a time, the fixed work per leaf was about half of the kernel on
+// surface meshes.
+// Alone: FP32, 200k-panel torus 295 -> 143 us, a million points in a cube 2,352
+// -> 1,738 us (16 rsqrt per SM and clock: 58 and 935 us); FP64, 20,011 points
+// on a sphere 2,486 -> 277 us (gridpoint.cuh; 63 us at full issue); two-float,
+// 50k-panel torus 1,089 -> 327 us (140 us at full issue).
+// ---------------------------------------------------------------------------
+enum NearMode {
+    kF32,   // packed pairs of sources on the FP32 pipe
+    kTF,    // FP64 plan in two-float mode: the split coordinates to two-float accuracy
+    kGrid,  // FP64 on the FP32 pipe from exactly split coordinates (gridpoint.cuh)
+    kIeee   // FP64 between two trees (no common grid)
+};
+
+constexpr int kNearWarps = 4;
+
+template <int MODE> struct NearCfg;
+template <> struct NearCfg<kF32> {
+    using T = float;
+    // RS: the values of R compiled (bit R); A + B R: issue slots per source step.
+    // R = 2, 3, 4: with 5 and 6 too a million points take 1,722 instead of 1,738 us,
+    // but the warps of an SM then run six copies of the loop, and on surface
+    // leaves (200k-panel torus 190 instead of 143 us, 24 dimers 427 instead of
+    // 326) the instruction fetches cost more than the idle lanes.
+    static constexpr int CH = 128, REC = 1, RS = 0x1c, A = 5, B = 11;
+};
+template <> struct NearCfg<kTF> {
+    using T = double;
+    static constexpr int CH = 64, REC = 3, RS = 0xe, A = 6, B = 75;
+};
+template <> struct NearCfg<kGrid> {
+    using T = double;
+    static constexpr int CH = 64, REC = 3, RS = 0xe, A = 6, B = 150;
+};
+template <> struct NearCfg<kIeee> {
+    using T = double;
+    static constexpr int CH = 64, REC = 2, RS = 0xe, A = 5, B = 128;
+};
+
+// targets per lane for nt targets: the least (A + B R) / G with G = 32 / ceil(nt / R)
+template <int MODE> struct NearShape {
+    unsigned char r[65];
+    constexpr NearShape() : r() {
+        using C = NearCfg<MODE>;
+        for (int nt = 0; nt <= 64; ++nt) {
+            r[nt] = 0;
+            long best = 1L << 60;
+            for (int R = 1; R < 8; ++R) {
+                const int L = (nt + R - 1) / R;
+                if (!(C::RS >> R & 1) || L < 1 || L > 32) continue;
+                const long cost = (C::A + C::B * R) * 100000L / (32 / L);
+                if (cost < best) {
+                    best = cost;
+                    r[nt] = (unsigned char)R;
+                }
+            }
+        }
+    }
+};
+template <int MODE> __device__ const NearShape<MODE> d_near_shape{};
+
+template <typename T> struct NearParams {
+    const int32_t *leaves;
+    int64_t n_leaves;
+    const int32_t *off;
+    const int32_t *src;
+    const typename Vec4<T>::type *pts;   // targets
+    const int2 *range;                   // target leaves' point ranges
+    const typename Vec4<T>::type *spts;  // sources (== pts for one tree)
+    const float4 *spts_split;            // kTF, kGrid: three float4 per point
+    const GridInfo *grid;                // kTF, kGrid
+    const int2 *srange;
+    int same;  // one tree: drop i == j in self pairs
+    T eps2;
+    InstMask mask;  // batched plans: leaves of inactive instances are skipped
+    T *out;         // near sums, tree order
+};
+
+// the part of a leaf's row a warp walks, 32 entries at a time
+struct RowBatch {
+    int first, len, total;  // this lane's entry: position of its first point, number of points; points of the batch
+    int seen;               // entries with points that start before the next window
+};
+
+template <typename T>
+__device__ __forceinline__ void load_batch(const NearParams<T> &P, int k0, int kend, int skip, int lane, int *soff,
+                                           RowBatch &b, bool &self) {
+    const int k = k0 + lane;
+    const int s = k < kend ? P.src[k] : -1;
+    const int2 r = s >= 0 ? P.srange[s] : make_int2(0, 0);
+    b.len = r.y - r.x;
+    if (s >= 0 && s == skip) {
+        self = true;
+        b.len = 0;
+    }
+    int incl = b.len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    b.first = incl - b.len;
+    b.total = __shfl_sync(0xffffffffu, incl, 31);
+    b.seen = 0;
+    const unsigned nz = __ballot_sync(0xffffffffu, b.len > 0);
+    __syncwarp();
+    if (b.len > 0) soff[__popc(nz & ((1u << lane) - 1u))] = r.x - b.first;
+    __syncwarp();
+}
+
+// source indices of positions w + 2 lane and w + 2 lane + 1 of the batch (-1
+// past its end), for consecutive windows w = 0, 64, 128, ...
+__device__ __forceinline__ void window_sources(RowBatch &b, int w, int lane, const int *soff, int &i0, int &i1) {
+    const int t = b.first - w;
+    const bool in = b.len > 0 && t >= 0;
+    const unsigned m0 = __reduce_or_sync(0xffffffffu, in && t < 32 ? 1u << (t & 31) : 0u);
+    const unsigned m1 = __reduce_or_sync(0xffffffffu, in && t >= 32 && t < 64 ? 1u << (t & 31) : 0u);
+    const unsigned m = lane < 16 ? m0 : m1;
+    const int p = (2 * lane) & 31;
+    const int e0 = b.seen + (lane < 16 ? 0 : __popc(m0)) + __popc(m & ((2u << p) - 1u)) - 1;
+    const int e1 = e0 + (int)((m >> (p + 1)) & 1u);
+    b.seen += __popc(m0) + __popc(m1);
+    const int q = w + 2 * lane;
+    i0 = q < b.total ? soff[e0] + q : -1;
+    i1 = q + 1 < b.total ? soff[e1] + q + 1 : -1;
+}
+
+// a lane's targets
+template <int MODE, int R> struct Targets;
+template <int R> struct Targets<kF32, R> {
+    float2 nx[R], ny[R], nz[R];  // -x of the target, in both halves
+    float acc[R];
+};
+template <int R> struct Targets<kTF, R> {
+    GridCoord x[R], y[R], z[R];
+    double acc[R];
+};
+template <int R> struct Targets<kGrid, R> {
+    GridCoord x[R], y[R], z[R];
+    double acc[R];
+};
+template <int R> struct Targets<kIeee, R> {
+    double x[R], y[R], z[R], acc[R];
+};
+
+// staged sources to registers (the lane's two sources of a window) and on to shared memory
+template <int MODE> struct Staged;
+template <> struct Staged<kF32> {
+    float4 a, b;
+};
+template <> struct Staged<kIeee> {
+    double4 a, b;
+};
+template <> struct Staged<kTF> {
+    float4 a[3], b[3];
+};
+template <> struct Staged<kGrid> {
+    float4 a[3], b[3];
+};
+template <int MODE, typename T>
+__device__ __forceinline__ void fetch(const NearParams<T> &P, int i0, int i1, Staged<MODE> &f) {
+    if constexpr (MODE == kF32) {
+        const float4 z = make_float4(0, 0, 0, 0);
+        f.a = i0 >= 0 ? P.spts[i0] : z;
+        f.b = i1 >= 0 ? P.spts[i1] : z;
+    } else if constexpr (MODE == kIeee) {
+        f.a = i0 >= 0 ? P.spts[i0] : double4{0, 0, 0, 0};
+        f.b = i1 >= 0 ? P.spts[i1] : double4{0, 0, 0, 0};
+    } else {
+        constexpr int N = NearCfg<MODE>::REC;
+#pragma unroll
+        for (int c = 0; c < N; ++c) {
+            f.a[c] = i0 >= 0 ? P.spts_split[(int64_t)N * i0 + c] : make_float4(0, 0, 0, 0);
+            f.b[c] = i1 >= 0 ? P.spts_split[(int64_t)N * i1 + c] : make_float4(0, 0, 0, 0);
+        }
+        f.a[2].y = __int_as_float(i0);
+        f.b[2].y = __int_as_float(i1);
+    }
+}
+template <int MODE> __device__ __forceinline__ void stage(float4 *buf, int pair, const Staged<MODE> &f) {
+    if constexpr (MODE == kF32) {  // (x, x', y, y'), (z, z', q, q')
+        buf[2 * pair] = make_float4(f.a.x, f.b.x, f.a.y, f.b.y);
+        buf[2 * pair + 1] = make_float4(f.a.z, f.b.z, f.a.w, f.b.w);
+    } else if constexpr (MODE == kIeee) {
+        double4 *d = reinterpret_cast<double4 *>(buf);
+        d[2 * pair] = f.a;
+        d[2 * pair + 1] = f.b;
+    } else {
+        constexpr int N = NearCfg<MODE>::REC;
+#pragma unroll
+        for (int c = 0; c < N; ++c) {
+            buf[N * (2 * pair) + c] = f.a[c];
+            buf[N * (2 * pair + 1) + c] = f.b[c];
+        }
+    }
+}
+
+template <int MODE, int R, typename T>
+__device__ __forceinline__ void load_target(const NearParams<T> &P, int ti, int r, const GridInfo &g, Targets<MODE, R> &X) {
+    const typename Vec4<T>::type x = P.pts[ti];
+    if constexpr (MODE == kF32) {
+        X.nx[r] = make_float2(-x.x, -x.x);
+        X.ny[r] = make_float2(-x.y, -x.y);
+        X.nz[r] = make_float2(-x.z, -x.z);
+        X.acc[r] = 0.0f;
+    } else if constexpr (MODE == kTF || MODE == kGrid) {
+        X.x[r] = grid_split(x.x * g.down);
+        X.y[r] = grid_split(x.y * g.down);
+        X.z[r] = grid_split(x.z * g.down);
+        X.acc[r] = 0.0;
+    } else {
+        X.x[r] = x.x;
+        X.y[r] = x.y;
+        X.z[r] = x.z;
+        X.acc[r] = 0.0;
+    }
+}
 
 __device__ __forceinline__ double inv_dist(double r2, double eps2) { return rsqrt(fmax(r2, eps2)); }
 
+// kGrid: a pair too close for the split, in IEEE FP64 (scaled by 2^k)
+__device__ __noinline__ double grid_pair_ieee(const double4 *pts, int s, int t, double eps2, double up) {
+    if (s < 0 || s == t) return 0.0;
+    const double4 a = pts[t], b = pts[s];
+    const double dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+    return b.w * inv_dist(dx * dx + dy * dy + dz * dz, eps2) * up;
+}
 
+// hi + lo += (qh + ql) (y0 + z)
+__device__ __forceinline__ void grid_add_tf(float qh, float ql, float y0, float z, float &hi, float &lo) {
+    const float p = g_mul(qh, y0);
+    const float e = g_fma(ql, y0, g_fma(qh, z, g_fma(qh, y0, -p)));
+    float s, f;
+    grid_two_sum(hi, p, s, f);
+    hi = s;
+    lo = g_add(lo, g_add(f, e));
+}
+
+// sources part, part + G, ... of a staged chunk of cnt sources; SELF: the
+// chunk holds points sbase .. of the targets' own leaf, and t0 + L r is the
+// lane's target r (of targets up to last)
+template <int MODE, int R, bool SELF, typename T>
+__device__ __forceinline__ void accumulate(const NearParams<T> &P, const float4 *buf, int cnt, int part, int G, int sbase,
+                                           int t0, int L, int last, const GridInfo &g,
+                                           Targets<MODE, R> &X) {
+    if constexpr (MODE == kF32) {
+        const float eps2 = P.eps2;
+        float2 ps[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) ps[r] = make_float2(0.0f, 0.0f);
+        const int np = (cnt + 1) >> 1;
+#pragma unroll 2
+        for (int j = part; j < np; j += G) {
+            const float4 u = buf[2 * j], v = buf[2 * j + 1];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const float2 dx = __fadd2_rn(make_float2(u.x, u.y), X.nx[r]),
+                             dy = __fadd2_rn(make_float2(u.z, u.w), X.ny[r]),
+                             dz = __fadd2_rn(make_float2(v.x, v.y), X.nz[r]);
+                const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+                float i0 = rsqrt_normal(fmaxf(r2.x, eps2)), i1 = rsqrt_normal(fmaxf(r2.y, eps2));
+                if (SELF) {
+                    if (sbase + 2 * j == t0 + L * r) i0 = 0.0f;
+                    if (sbase + 2 * j + 1 == t0 + L * r) i1 = 0.0f;
+                }
+                ps[r] = __ffma2_rn(make_float2(v.z, v.w), make_float2(i0, i1), ps[r]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) X.acc[r] += ps[r].x + ps[r].y;  // per-chunk partial, then one add
+    } else if constexpr (MODE == kTF) {
+        float hi[R], lo[R];  // a chunk's sum, hi + lo, of at most 64 terms; then FP64
+        double ps[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            hi[r] = lo[r] = 0.0f;
+            ps[r] = 0.0;
+        }
+        for (int j = part; j < cnt; j += G) {
+            const float4 u = buf[3 * j], v = buf[3 * j + 1], q = buf[3 * j + 2];
+            float R1[R], M[R];
+            bool close = false;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                R1[r] = grid_r2_tf(grid_diff2(X.x[r], GridCoord{u.x, u.y, u.z}),
+                                   grid_diff2(X.y[r], GridCoord{u.w, v.x, v.y}),
+                                   grid_diff2(X.z[r], GridCoord{v.z, v.w, q.x}), M[r]);
+                close = close || !(R1[r] >= g.near2);
+            }
+            if (close) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if (!(R1[r] >= g.near2)) {
+                        ps[r] += grid_pair_ieee(P.pts, __float_as_int(q.y), min(t0 + L * r, last), P.eps2, g.up);
+                    } else {
+                        float y0, z;
+                        grid_rsqrt_tf(R1[r], M[r], y0, z);
+                        grid_add_tf(q.z, q.w, y0, z, hi[r], lo[r]);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    float y0, z;
+                    grid_rsqrt_tf(R1[r], M[r], y0, z);
+                    grid_add_tf(q.z, q.w, y0, z, hi[r], lo[r]);
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) X.acc[r] += ps[r] + ((double)hi[r] + (double)lo[r]);
+    } else if constexpr (MODE == kGrid) {
+        double ps[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) ps[r] = 0.0;
+        for (int j = part; j < cnt; j += G) {
+            const float4 u = buf[3 * j], v = buf[3 * j + 1], q = buf[3 * j + 2];
+            const double w = __hiloint2double(__float_as_int(q.w), __float_as_int(q.z));
+            GridR2 r2[R];
+            bool close = false;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                r2[r] = grid_r2(grid_diff(X.x[r], GridCoord{u.x, u.y, u.z}), grid_diff(X.y[r], GridCoord{u.w, v.x, v.y}),
+                                grid_diff(X.z[r], GridCoord{v.z, v.w, q.x}));
+                close = close || !(r2[r].R1 >= g.near2);
+            }
+            if (close) {  // the target itself, or a pair the split does not resolve
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if (!(r2[r].R1 >= g.near2)) {
+                        ps[r] += grid_pair_ieee(P.pts, __float_as_int(q.y), min(t0 + L * r, last), P.eps2, g.up);
+                    } else {
+                        float y0;
+                        unsigned ci;
+                        grid_rsqrt(r2[r], y0, ci);
+                        ps[r] = fma(w * grid_double(y0), grid_one_plus(ci), ps[r]);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    float y0;
+                    unsigned ci;
+                    grid_rsqrt(r2[r], y0, ci);
+                    ps[r] = fma(w * grid_double(y0), grid_one_plus(ci), ps[r]);
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) X.acc[r] += ps[r];
+    } else {
+        const double eps2 = P.eps2;
+        const double4 *sp = reinterpret_cast<const double4 *>(buf);
+        double ps[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) ps[r] = 0.0;
+        for (int j = part; j < cnt; j += G) {
+            const double4 q = sp[j];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const double dx = X.x[r] - q.x, dy = X.y[r] - q.y, dz = X.z[r] - q.z;
+                double inv = inv_dist(dx * dx + dy * dy + dz * dz, eps2);
+                if (SELF && sbase + j == t0 + L * r) inv = 0.0;
+                ps[r] += q.w * inv;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) X.acc[r] += ps[r];
+    }
+}
+
+// targets tb .. tb + nt - 1 of leaf t; WPL warps share them (this is warp
+// `wid` of the block)
+template <int MODE, int R, int WPL, typename T>
+__device__ __forceinline__ void near_targets(const NearParams<T> &P, int t, int tb, int nt, int2 rg, int wid,
+                                             float4 *buf, int *soff, T *part, const GridInfo &g) {
+    using C = NearCfg<MODE>;
+    constexpr int NW = C::CH / 64;  // windows per chunk
+    const int lane = threadIdx.x & 31;
+    const int L = (nt + R - 1) / R, G = 32 / L;
+    const int grp = lane / L, l = lane - grp * L;
+    Targets<MODE, R> X;
+#pragma unroll
+    for (int r = 0; r < R; ++r) load_target<MODE, R>(P, tb + min(l + L * r, nt - 1), r, g, X);
+    const int t0 = tb + l;
+    const int first = grp < G ? grp : C::CH;  // lanes beyond the last group take no source
+    int kbeg = P.off[t], kend = P.off[t + 1];
+    if constexpr (WPL > 1) {
+        const int per = (kend - kbeg + WPL - 1) / WPL;
+        kbeg = min(kend, kbeg + wid * per);
+        kend = min(kend, kbeg + per);
+    }
+    // the split forms drop the diagonal through their close-pair test
+    const int skip = MODE != kGrid && MODE != kTF && P.same ? t : -2;
+    bool self = false;
+    for (int k0 = kbeg; k0 < kend; k0 += 32) {
+        RowBatch b;
+        load_batch(P, k0, kend, skip, lane, soff, b, self);
+        Staged<MODE> f[NW];
+#pragma unroll
+        for (int i = 0; i < NW; ++i) {
+            int i0, i1;
+            window_sources(b, 64 * i, lane, soff, i0, i1);
+            fetch<MODE>(P, i0, i1, f[i]);
+        }
+        for (int c = 0; c < b.total; c += C::CH) {
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < NW; ++i) stage<MODE>(buf, lane + 32 * i, f[i]);
+            __syncwarp();
+            if (c + C::CH < b.total) {  // the next chunk's points are loaded behind this one's arithmetic
+#pragma unroll
+                for (int i = 0; i < NW; ++i) {
+                    int i0, i1;
+                    window_sources(b, c + C::CH + 64 * i, lane, soff, i0, i1);
+                    fetch<MODE>(P, i0, i1, f[i]);
+                }
+            }
+            accumulate<MODE, R, false>(P, buf, min(C::CH, b.total - c), first, G, 0, t0, L, tb + nt - 1, g, X);
+        }
+    }
+    if (__any_sync(0xffffffffu, self)) {
+        for (int sb = rg.x; sb < rg.y; sb += C::CH) {
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < NW; ++i) {
+                const int q = sb + 64 * i + 2 * lane;
+                Staged<MODE> f;
+                fetch<MODE>(P, q < rg.y ? q : -1, q + 1 < rg.y ? q + 1 : -1, f);
+                stage<MODE>(buf, lane + 32 * i, f);
+            }
+            __syncwarp();
+            accumulate<MODE, R, true>(P, buf, min(C::CH, rg.y - sb), first, G, sb, t0, L, tb + nt - 1, g, X);
+        }
+    }
+    // the groups' sums per target, in group order (and in warp order)
+    __syncwarp();
+    T *red = reinterpret_cast<T *>(buf);  // G * nt <= 32 R values
+    if (grp < G) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (l + L * r >= nt) continue;
+            T v;
+            if constexpr (MODE == kTF || MODE == kGrid) v = X.acc[r] * g.down;
+            else v = X.acc[r];
+            red[grp * nt + l + L * r] = v;
+        }
+    }
+    __syncwarp();
+    for (int i = lane; i < nt; i += 32) {
+        T v = red[i];
+        for (int q = 1; q < G; ++q) v += red[q * nt + i];
+        if constexpr (WPL > 1) part[wid * 64 + i] = v;
+        else P.out[tb + i] = v;
+    }
+    if constexpr (WPL > 1) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < nt; i += 32 * WPL) {
+            T v = part[i];
+#pragma unroll
+            for (int q = 1; q < WPL; ++q) v += part[q * 64 + i];
+            P.out[tb + i] = v;
+        }
+        __syncthreads();
+    } else {
+        __syncwarp();
+    }
+}
+
+template <int MODE> __host__ __device__ constexpr int near_blocks() { return MODE == kF32 ? 5 : 4; }
+
+template <int MODE, int WPL>
+__global__ void __launch_bounds__(32 * kNearWarps, near_blocks<MODE>())
+    k_p2p(const NearParams<typename NearCfg<MODE>::T> P) {
+    using C = NearCfg<MODE>;
+    using T = typename C::T;
+    __shared__ float4 buf[kNearWarps][C::CH * C::REC];
+    __shared__ int soff[kNearWarps][32];
+    __shared__ T part[WPL > 1 ? WPL * 64 : 1];
+    const int wid = threadIdx.x >> 5;
+    const int64_t w = WPL > 1 ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * kNearWarps + wid;
+    if (w >= P.n_leaves) return;
+    const int t = P.leaves[w];
+    if (!inst_active(P.mask, t)) return;  // uniform over the warps that share a leaf
+    const int2 rg = P.range[t];
+    GridInfo g{};
+    if constexpr (MODE == kGrid || MODE == kTF) g = *P.grid;
+    for (int tb = rg.x; tb < rg.y; tb += 64) {
+        const int nt = min(64, rg.y - tb);
+        const int R = d_near_shape<MODE>.r[nt];
+#define EDFMM_NEAR_R(RR)                                                                                     \
+    if constexpr ((C::RS >> RR) & 1) {                                                                           \
+        if (R == RR) near_targets<MODE, RR, WPL>(P, t, tb, nt, rg, wid, buf[wid], soff[wid], part, g);       \
+    }
+        EDFMM_NEAR_R(1)
+        EDFMM_NEAR_R(2)
+        EDFMM_NEAR_R(3)
+        EDFMM_NEAR_R(4)
+        EDFMM_NEAR_R(5)
+        EDFMM_NEAR_R(6)
+#undef EDFMM_NEAR_R
+    }
+}
+
+// ---------------------------------------------------------------------------
+// L2P and epilogue: one warp per leaf, one lane per target
+// ---------------------------------------------------------------------------
 // Re sum_{n,m} L_n^m R_n^m(x, y, z) over m in [-n, n]
-template <typename T>
-__device__ __forceinline__ T l2p_point(const Cplx<T> *L, int p, T x, T y, T z) {
+template <typename T, int P>
+__device__ __forceinline__ T l2p_point(const Cplx<T> *L, T x, T y, T z) {
     const T r2 = x * x + y * y + z * z;
     T acc = (T)0, dr = (T)1, di = (T)0;
-    for (int m = 0; m <= p; ++m) {
+#pragma unroll
+    for (int m = 0; m <= P; ++m) {
         if (m > 0) {
-            const T s = -(T)0.5 * rdiv<T>(m, 0) * (T)m;  // -1 / (2m): rdiv(m, 0) = 1 / m^2
+            const T s = (T)(-0.5 / (m > 0 ? m : 1));
             const T nr = s * (x * dr - y * di), ni = s * (x * di + y * dr);
             dr = nr;
             di = ni;
@@ -52,8 +562,9 @@ __device__ __forceinline__ T l2p_point(const Cplx<T> *L, int p, T x, T y, T z) {
         T pr = dr, pi = di, qr = (T)0, qi = (T)0;
         Cplx<T> lv = L[tri(m, m)];
         T col = lv.re * pr - lv.im * pi;
-        for (int n = m + 1; n <= p; ++n) {
-            const T d = rdiv<T>(n, m);
+#pragma unroll
+        for (int n = m + 1; n <= P; ++n) {
+            const T d = (T)(1.0 / ((n + m) * (n - m)));
             const T c1 = (T)(2 * n - 1) * z;
             const T nr = (c1 * pr - r2 * qr) * d, ni = (c1 * pi - r2 * qi) * d;
             lv = L[tri(n, m)];
@@ -101,27 +612,18 @@ __device__ __forceinline__ tf32x2 l2p_point_tf(const tf32x2c *L, int p, tf32x2 x
     return acc;
 }
 
-template <typename T> struct NearParams {
+template <typename T> struct L2pParams {
     const int32_t *leaves;
     int64_t n_leaves;
-    const int32_t *off;
-    const int32_t *src;
-    const typename Vec4<T>::type *pts;   // targets
-    const int2 *range;                   // target leaves' point ranges
-    const typename Vec4<T>::type *spts;  // sources (== pts for one tree)
-    const float4 *spts_tf;               // two-float mode: sources as (xh, xl, yh, yl), (zh, zl, qh, ql)
-    const int2 *srange;
-    int same;                            // one tree: drop i == j in self pairs
+    const typename Vec4<T>::type *pts;
+    const int2 *range;
     const typename Vec4<T>::type *center;
     const typename Vec4<T>::type *half;
     const Cplx<T> *Lexp;
-    int p;
     int nc_pad;
-    T eps2;
-    int near;
-    int far;
-    const T *add_in;  // tree-order near sums computed by an earlier pass (nullable)
-    InstMask mask;    // batched plans: leaves of inactive instances are skipped
+    int far;          // 0: the epilogue alone
+    const T *add_in;  // near sums, tree order (nullable)
+    InstMask mask;
     // epilogue
     int scatter;
     const int32_t *index_map;
@@ -132,330 +634,41 @@ template <typename T> struct NearParams {
     T *out;
 };
 
-// Target slots.  A block of nt <= 64 targets of a leaf is split by the
-// binary digits of nt rounded up to a multiple of 4: up to two slots of 32
-// targets with one lane each, then 16 targets with 2 lanes each, 8 with 4
-// and 4 with 8.  Every slot fills the warp, so the lanes stay busy whatever
-// the leaf size; the lanes of a target take every G-th source (FP32: source
-// pair) of a chunk and a fixed shuffle tree combines them.
-template <typename T> struct Slot;
-template <> struct Slot<float> {
-    float2 nx, ny, nz;  // -x of the lane's target, in both halves
-    float2 ps;          // packed partial sums
-    int ti;             // target point index, -1 for a padding lane
-};
-template <> struct Slot<double> {
-    double x, y, z;
-    double ps;
-    int ti;
-};
-template <> struct Slot<tf32x2> {
-    tf32x2 x, y, z;
-    tf32x2 ps;
-    int ti;
-};
-
-// FP32: sources two at a time as packed pairs (FADD2 / FMUL2 / FFMA2); only
-// the reciprocal square roots and the eps clamp are scalar.  An odd chunk is
-// padded with a zero-charge source.
-template <int G, bool SELF>
-__device__ __forceinline__ void accumulate_slot(const float *sx, int cnt, int sbase, int part, Slot<float> &S,
-                                                float eps2) {
-    const float *sy = sx + 64, *sz = sx + 128, *sw = sx + 192;
-    const int np = (cnt + 1) >> 1;
-    float2 ps = S.ps;
-#pragma unroll 2  // measured: 2.31 ms against 2.39 (unroll 4) at 1M uniform points
-    for (int j = part; j < np; j += G) {
-        const float2 qx = *reinterpret_cast<const float2 *>(sx + 2 * j);
-        const float2 qy = *reinterpret_cast<const float2 *>(sy + 2 * j);
-        const float2 qz = *reinterpret_cast<const float2 *>(sz + 2 * j);
-        const float2 qw = *reinterpret_cast<const float2 *>(sw + 2 * j);
-        const float2 dx = __fadd2_rn(qx, S.nx), dy = __fadd2_rn(qy, S.ny), dz = __fadd2_rn(qz, S.nz);
-        const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-        float i0 = rsqrt_normal(fmaxf(r2.x, eps2)), i1 = rsqrt_normal(fmaxf(r2.y, eps2));
-        if (SELF) {
-            if (sbase + 2 * j == S.ti) i0 = 0.0f;
-            if (sbase + 2 * j + 1 == S.ti) i1 = 0.0f;
-        }
-        ps = __ffma2_rn(qw, make_float2(i0, i1), ps);
-    }
-    S.ps = ps;
-}
-
-// FP64: one source per step from the staged (x, y, z, q) chunk
-template <int G, bool SELF>
-__device__ __forceinline__ void accumulate_slot(const double4 *sp, int cnt, int sbase, int part, Slot<double> &S,
-                                                double eps2) {
-    double ps = 0.0;
-#pragma unroll 4
-    for (int j = part; j < cnt; j += G) {
-        const double4 q = sp[j];
-        const double dx = S.x - q.x, dy = S.y - q.y, dz = S.z - q.z;
-        double inv = inv_dist(dx * dx + dy * dy + dz * dz, eps2);
-        if (SELF && sbase + j == S.ti) inv = 0.0;
-        ps += q.w * inv;
-    }
-    S.ps += ps;  // per-chunk partial, then one add: two-level summation
-}
-
-// Two-float: one source per step from the staged split points
-// (s4[2j] = (xh, xl, yh, yl), s4[2j + 1] = (zh, zl, qh, ql): two 16-byte
-// shared loads).  The coordinate differences are formed from the split
-// parts, so the cancellation of nearby points loses nothing; 1 / r takes one
-// Newton step from the FP32 estimate.
-template <int G, bool SELF>
-__device__ __forceinline__ void accumulate_slot(const float4 *s4, int cnt, int sbase, int part, Slot<tf32x2> &S,
-                                                float eps2) {
-    tf32x2 ps = tf32x2(0);
-#pragma unroll 2
-    for (int j = part; j < cnt; j += G) {
-        const float4 a = s4[2 * j], b = s4[2 * j + 1];
-        const tf32x2 dx = S.x - tf32x2(a.x, a.y);
-        const tf32x2 dy = S.y - tf32x2(a.z, a.w);
-        const tf32x2 dz = S.z - tf32x2(b.x, b.y);
-        tf32x2 r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-        if (!(r2.hi >= eps2)) r2 = tf32x2(eps2, 0.0f);
-        tf32x2 inv = tf_rsqrt(r2, rsqrt_normal(r2.hi));
-        if (SELF && sbase + j == S.ti) inv = tf32x2(0);
-        ps = fma(tf32x2(b.z, b.w), inv, ps);
-    }
-    S.ps = S.ps + ps;  // per-chunk partial, then one add: two-level summation
-}
-
-template <typename T, int G>
-__device__ __forceinline__ void slot_init(const NearParams<T> &P, int tb, int te, int base, int lane, Slot<T> &S) {
-    const int ti = tb + base + lane / G;
-    S.ti = ti < te ? ti : -1;
-    const typename Vec4<T>::type x = P.pts[ti < te ? ti : tb];
-    if constexpr (sizeof(T) == 4) {
-        S.nx = make_float2(-x.x, -x.x);
-        S.ny = make_float2(-x.y, -x.y);
-        S.nz = make_float2(-x.z, -x.z);
-        S.ps = make_float2(0.0f, 0.0f);
-    } else {
-        S.x = x.x;
-        S.y = x.y;
-        S.z = x.z;
-        S.ps = 0.0;
-    }
-}
-
-template <int G>
-__device__ __forceinline__ void slot_init(const NearParams<double> &P, int tb, int te, int base, int lane,
-                                          Slot<tf32x2> &S) {
-    const int ti = tb + base + lane / G;
-    S.ti = ti < te ? ti : -1;
-    const double4 x = P.pts[ti < te ? ti : tb];
-    S.x = tf_from_double(x.x);
-    S.y = tf_from_double(x.y);
-    S.z = tf_from_double(x.z);
-    S.ps = tf32x2(0);
-}
-
-template <int G>
-__device__ __forceinline__ void slot_finish(Slot<tf32x2> &S, int lane, int tb, double *pot) {
-    tf32x2 a = S.ps;
-#pragma unroll
-    for (int o = 1; o < G; o <<= 1) a = a + tf_shfl_xor(a, o);
-    if (lane % G == 0 && S.ti >= 0) pot[S.ti - tb] = tf_to_double(a);
-}
-
-template <typename T, int G>
-__device__ __forceinline__ void slot_finish(Slot<T> &S, int lane, int tb, T *pot) {
-    T a;
-    if constexpr (sizeof(T) == 4)
-        a = S.ps.x + S.ps.y;
-    else
-        a = S.ps;
-#pragma unroll
-    for (int o = 1; o < G; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (lane % G == 0 && S.ti >= 0) pot[S.ti - tb] = a;
-}
-
-template <typename T, bool SELF, typename C, typename E>
-__device__ __forceinline__ void accumulate_slots(const C *chunk, int cnt, int sb, int lane, const bool (&on)[5],
-                                                 Slot<T> (&S)[5], E eps2) {
-    if (on[0]) accumulate_slot<1, SELF>(chunk, cnt, sb, 0, S[0], eps2);
-    if (on[1]) accumulate_slot<1, SELF>(chunk, cnt, sb, 0, S[1], eps2);
-    if (on[2]) accumulate_slot<2, SELF>(chunk, cnt, sb, lane % 2, S[2], eps2);
-    if (on[3]) accumulate_slot<4, SELF>(chunk, cnt, sb, lane % 4, S[3], eps2);
-    if (on[4]) accumulate_slot<8, SELF>(chunk, cnt, sb, lane % 8, S[4], eps2);
-}
-
-// Targets tb..te-1 (at most 64) of leaf t: near field by slots, then the
-// local expansion and the epilogue with one lane per target.  Source chunks
-// of up to 64 points (one leaf, or a 64-point piece of a larger one) are
-// staged in shared memory (FP32 as x / y / z / q arrays, two-float as split
-// points, FP64 as points).
-// The leaf ids and ranges of the row are read 32 entries at a time (one per
-// lane) and broadcast by shuffles, and the next chunk's points are loaded
-// before the current chunk is computed, so the dependent global loads
-// overlap the arithmetic.
-struct SplitPt {  // two-float source point: (xh, xl, yh, yl), (zh, zl, qh, ql)
-    float4 a, b;
-};
-
-template <typename T, bool TF>
-__device__ __forceinline__ void leaf_slots(const NearParams<T> &P, int t, int tb, int te,
-                                           typename Vec4<T>::type *sp, T *pot, const Cplx<T> *sL) {
+template <typename T, bool TF, int PP>
+__global__ void __launch_bounds__(128) k_l2p(const L2pParams<T> P) {
     using T4 = typename Vec4<T>::type;
-    using ST = std::conditional_t<TF, tf32x2, T>;      // slot arithmetic
-    using Pre = std::conditional_t<TF, SplitPt, T4>;  // prefetched source point
-    constexpr bool F32 = !TF && sizeof(T) == 4;
-    const int lane = threadIdx.x & 31;
-    const int nt = te - tb;
-    bool on[5];
-    int base[5];
-    {
-        int rem = (nt + 3) & ~3, o = 0;
-        on[0] = rem >= 32;
-        base[0] = o;
-        if (on[0]) o += 32, rem -= 32;
-        on[1] = rem >= 32;
-        base[1] = o;
-        if (on[1]) o += 32, rem -= 32;
-        on[2] = (rem & 16) != 0;
-        base[2] = o;
-        if (on[2]) o += 16;
-        on[3] = (rem & 8) != 0;
-        base[3] = o;
-        if (on[3]) o += 8;
-        on[4] = (rem & 4) != 0;
-        base[4] = o;
-    }
-    Slot<ST> S[5];
-    if constexpr (TF) {
-        slot_init<1>(P, tb, te, base[0], lane, S[0]);
-        slot_init<1>(P, tb, te, base[1], lane, S[1]);
-        slot_init<2>(P, tb, te, base[2], lane, S[2]);
-        slot_init<4>(P, tb, te, base[3], lane, S[3]);
-        slot_init<8>(P, tb, te, base[4], lane, S[4]);
-    } else {
-        slot_init<T, 1>(P, tb, te, base[0], lane, S[0]);
-        slot_init<T, 1>(P, tb, te, base[1], lane, S[1]);
-        slot_init<T, 2>(P, tb, te, base[2], lane, S[2]);
-        slot_init<T, 4>(P, tb, te, base[3], lane, S[3]);
-        slot_init<T, 8>(P, tb, te, base[4], lane, S[4]);
-    }
-    if (P.near) {
-        const T eps2 = P.eps2;
-        const int kbeg = P.off[t], kend = P.off[t + 1];
-        int kb = kbeg, s_l = 0, sa_l = 0, se_l = 0;
-        auto load_batch = [&](int b0) {
-            kb = b0;
-            const int k = b0 + lane;
-            s_l = k < kend ? P.src[k] : 0;
-            const int2 r = k < kend ? P.srange[s_l] : make_int2(0, 0);
-            sa_l = r.x;
-            se_l = r.y;
-        };
-        auto fetch = [&](int sb, int se, int i) -> Pre {
-            if constexpr (TF) {
-                if (i < se - sb) return SplitPt{P.spts_tf[2 * (sb + i)], P.spts_tf[2 * (sb + i) + 1]};
-                return SplitPt{make_float4(0, 0, 0, 0), make_float4(0, 0, 0, 0)};
-            } else {
-                return i < se - sb ? P.spts[sb + i] : T4{0, 0, 0, 0};
-            }
-        };
-        if (kbeg < kend) {
-            load_batch(kbeg);
-            int k = kbeg;
-            int s = __shfl_sync(0xffffffffu, s_l, 0), sb = __shfl_sync(0xffffffffu, sa_l, 0),
-                se = __shfl_sync(0xffffffffu, se_l, 0);
-            Pre qa = fetch(sb, se, lane), qb = fetch(sb, se, lane + 32);
-            while (true) {
-                const int cs = s, csb = sb, cnt = min(64, se - sb);
-                __syncwarp();
-                if constexpr (TF) {
-                    float4 *s4 = reinterpret_cast<float4 *>(sp);
-                    s4[2 * lane] = qa.a;
-                    s4[2 * lane + 1] = qa.b;
-                    s4[2 * lane + 64] = qb.a;
-                    s4[2 * lane + 65] = qb.b;
-                } else if constexpr (F32) {
-                    float *sx = reinterpret_cast<float *>(sp);
-                    sx[lane] = qa.x;
-                    sx[64 + lane] = qa.y;
-                    sx[128 + lane] = qa.z;
-                    sx[192 + lane] = qa.w;
-                    sx[lane + 32] = qb.x;
-                    sx[64 + lane + 32] = qb.y;
-                    sx[128 + lane + 32] = qb.z;
-                    sx[192 + lane + 32] = qb.w;
-                } else {
-                    sp[lane] = qa;
-                    sp[lane + 32] = qb;
-                }
-                __syncwarp();
-                bool more = true;
-                if (sb + 64 < se) {
-                    sb += 64;
-                } else if (++k >= kend) {
-                    more = false;
-                } else {
-                    if (k >= kb + 32) load_batch(k);
-                    s = __shfl_sync(0xffffffffu, s_l, k - kb);
-                    sb = __shfl_sync(0xffffffffu, sa_l, k - kb);
-                    se = __shfl_sync(0xffffffffu, se_l, k - kb);
-                }
-                if (more) {
-                    qa = fetch(sb, se, lane);
-                    qb = fetch(sb, se, lane + 32);
-                }
-                if constexpr (TF) {
-                    const float4 *s4 = reinterpret_cast<const float4 *>(sp);
-                    if (P.same && cs == t)
-                        accumulate_slots<tf32x2, true>(s4, cnt, csb, lane, on, S, (float)eps2);
-                    else
-                        accumulate_slots<tf32x2, false>(s4, cnt, csb, lane, on, S, (float)eps2);
-                } else if constexpr (F32) {
-                    const float *sx = reinterpret_cast<const float *>(sp);
-                    if (P.same && cs == t)
-                        accumulate_slots<T, true>(sx, cnt, csb, lane, on, S, eps2);
-                    else
-                        accumulate_slots<T, false>(sx, cnt, csb, lane, on, S, eps2);
-                } else {
-                    if (P.same && cs == t)
-                        accumulate_slots<T, true>(sp, cnt, csb, lane, on, S, eps2);
-                    else
-                        accumulate_slots<T, false>(sp, cnt, csb, lane, on, S, eps2);
-                }
-                if (!more) break;
-            }
-        }
-    }
-    if constexpr (TF) {
-        slot_finish<1>(S[0], lane, tb, pot);
-        slot_finish<1>(S[1], lane, tb, pot);
-        slot_finish<2>(S[2], lane, tb, pot);
-        slot_finish<4>(S[3], lane, tb, pot);
-        slot_finish<8>(S[4], lane, tb, pot);
-    } else {
-        slot_finish<T, 1>(S[0], lane, tb, pot);
-        slot_finish<T, 1>(S[1], lane, tb, pot);
-        slot_finish<T, 2>(S[2], lane, tb, pot);
-        slot_finish<T, 4>(S[3], lane, tb, pot);
-        slot_finish<T, 8>(S[4], lane, tb, pot);
-    }
-    __syncwarp();
-    T4 c;
+    constexpr int NC = ncoef(PP);
+    __shared__ Cplx<T> sL[4][NC];
+    const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t w = (int64_t)blockIdx.x * 4 + wl;
+    if (w >= P.n_leaves) return;
+    const int t = P.leaves[w];
+    if (!inst_active(P.mask, t)) return;
+    T4 c{};
     T ia = (T)1;
     if (P.far) {
+        for (int k = lane; k < NC; k += 32) {
+            const Cplx<T> v = P.Lexp[(int64_t)t * P.nc_pad + k];
+            if constexpr (TF)  // staged as two-float (the same 16 bytes per coefficient)
+                reinterpret_cast<tf32x2c *>(sL[wl])[k] = tf32x2c{tf_from_double(v.re), tf_from_double(v.im)};
+            else
+                sL[wl][k] = v;
+        }
         c = P.center[t];
         ia = (T)1 / P.half[t].w;
+        __syncwarp();
     }
-    for (int i = lane; i < nt; i += 32) {
-        const int ti = tb + i;
-        const T4 x = P.pts[ti];
-        T v = P.near ? pot[i] : (T)0;
-        if (P.add_in) v += P.add_in[ti];
+    const int2 rg = P.range[t];
+    for (int ti = rg.x + lane; ti < rg.y; ti += 32) {
+        T v = P.add_in ? P.add_in[ti] : (T)0;
         if (P.far) {
+            const T4 x = P.pts[ti];
             if constexpr (TF)
-                v += tf_to_double(l2p_point_tf(reinterpret_cast<const tf32x2c *>(sL), P.p,
+                v += tf_to_double(l2p_point_tf(reinterpret_cast<const tf32x2c *>(sL[wl]), PP,
                                                tf_from_double((x.x - c.x) * ia), tf_from_double((x.y - c.y) * ia),
                                                tf_from_double((x.z - c.z) * ia)));
             else
-                v += l2p_point<T>(sL, P.p, (x.x - c.x) * ia, (x.y - c.y) * ia, (x.z - c.z) * ia);
+                v += l2p_point<T, PP>(sL[wl], (x.x - c.x) * ia, (x.y - c.y) * ia, (x.z - c.z) * ia);
         }
         if (P.scatter) {
             const int o = P.index_map[ti];
@@ -467,92 +680,147 @@ __device__ __forceinline__ void leaf_slots(const NearParams<T> &P, int t, int tb
             P.out[ti] = v;
         }
     }
-    __syncwarp();
 }
 
-template <typename T, bool TF>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 4) k_p2p_l2p(const NearParams<T> P) {
-    using T4 = typename Vec4<T>::type;
-    __shared__ T4 sp[4][64];  // a staged chunk of up to 64 sources
-    __shared__ Cplx<T> sL[4][ncoef(kPMax)];
-    __shared__ T spot[4][64];  // the near-field sums of a block of targets
-    const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t w = (int64_t)blockIdx.x * 4 + wl;
-    if (w >= P.n_leaves) return;
-    const int t = P.leaves[w];
-    if (!inst_active(P.mask, t)) return;  // uniform over the warp; the kernel has no block barrier
-    if (P.far) {
-        const int nc = ncoef(P.p);
-        for (int k = lane; k < nc; k += 32) {
-            const Cplx<T> c = P.Lexp[(int64_t)t * P.nc_pad + k];
-            if constexpr (TF)  // staged as two-float (the same 16 bytes per coefficient)
-                reinterpret_cast<tf32x2c *>(sL[wl])[k] = tf32x2c{tf_from_double(c.re), tf_from_double(c.im)};
-            else
-                sL[wl][k] = c;
-        }
-        __syncwarp();
+// ---------------------------------------------------------------------------
+// FP64 trees: the exact split of the points (gridpoint.cuh)
+// ---------------------------------------------------------------------------
+__global__ void k_grid_max(const double4 *__restrict__ pts, int64_t n, GridInfo *info) {
+    unsigned hi = 0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double4 p = pts[i];
+        hi = max(hi, (unsigned)__double2hiint(p.x) & 0x7fffffffu);
+        hi = max(hi, (unsigned)__double2hiint(p.y) & 0x7fffffffu);
+        hi = max(hi, (unsigned)__double2hiint(p.z) & 0x7fffffffu);
     }
-    const int2 rg = P.range[t];
-    for (int tb = rg.x; tb < rg.y; tb += 64)
-        leaf_slots<T, TF>(P, t, tb, min(rg.y, tb + 64), sp[wl], spot[wl], sL[wl]);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0) atomicMax(&info->hi, hi);
+}
+// three float4 per point: (xa, xb, xc, ya), (yb, yc, za, zb), (zc, -, charge);
+// set_charges writes the charge
+__global__ void k_grid_points(const double4 *__restrict__ pts, int64_t n, GridInfo *info, float4 *__restrict__ out) {
+    int k;
+    const bool ok = grid_exponent(info->hi, k);
+    if (!ok) k = 0;
+    const double down = grid_pow2(-k);
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        info->down = down;
+        info->up = grid_pow2(k);
+        // without a usable scale every pair is evaluated in IEEE FP64: no r^2 is >= NaN
+        info->near2 = ok ? fmaxf(kGridNear2, (float)(1.0001 * DBL_EPSILON * DBL_EPSILON * down * down)) : NAN;
+    }
+    if (i >= n) return;
+    const double4 p = pts[i];
+    GridCoord x{}, y{}, z{};
+    if (ok) {
+        x = grid_split(p.x * down);
+        y = grid_split(p.y * down);
+        z = grid_split(p.z * down);
+    }
+    out[3 * i] = make_float4(x.a, x.b, x.c, y.a);
+    out[3 * i + 1] = make_float4(y.b, y.c, z.a, z.b);
+    out[3 * i + 2] = make_float4(z.c, 0.0f, 0.0f, 0.0f);
 }
 
 }  // namespace
 
-// 1 / ((n + m)(n - m)) tables (1 / n^2 at m = 0); __constant__ data lives in
-// each device context, so every plan creation uploads it on its device.
+// The split points of an FP64 tree (48 bytes per point), without their charges
+int grid_prepare(DevTree &tree, cudaStream_t s) {
+    if (tree.dtype != EDFMM_F64 || tree.n_points == 0) return EDFMM_OK;
+    int rc;
+    if ((rc = tree.pts_grid.reserve(sizeof(float4) * 3 * (size_t)tree.n_points)) ||
+        (rc = tree.grid_info.reserve(sizeof(GridInfo))))
+        return rc;
+    GridInfo *info = dptr<GridInfo>(tree.grid_info);
+    EDFMM_CUDA_TRY(cudaMemsetAsync(info, 0, sizeof(GridInfo), s));
+    const int64_t nb = (tree.n_points + 255) / 256;
+    k_grid_max<<<(unsigned)(nb < 608 ? nb : 608), 256, 0, s>>>(dptr<double4>(tree.pts), tree.n_points, info);
+    EDFMM_LAUNCH_CHECK("k_grid_max");
+    k_grid_points<<<(unsigned)nb, 256, 0, s>>>(dptr<double4>(tree.pts), tree.n_points, info, dptr<float4>(tree.pts_grid));
+    EDFMM_LAUNCH_CHECK("k_grid_points");
+    return EDFMM_OK;
+}
+
+// The two-float table; __constant__ data lives in each device context, so
+// every plan creation uploads it on its device.
 int upload_tables() {
-    float hf[kPMax + 1][kPMax + 1];
-    double hd[kPMax + 1][kPMax + 1];
+    float2 ht[kPMax + 1][kPMax + 1];
     for (int n = 0; n <= kPMax; ++n)
         for (int m = 0; m <= kPMax; ++m) {
             int d = (n + m) * (n - m);
             if (m == 0 && n > 0) d = n * n;
-            hd[n][m] = d != 0 ? 1.0 / d : 0.0;
-            hf[n][m] = (float)hd[n][m];
+            const double v = d != 0 ? 1.0 / d : 0.0;
+            ht[n][m].x = (float)v;
+            ht[n][m].y = (float)(v - (double)ht[n][m].x);
         }
-    float2 ht[kPMax + 1][kPMax + 1];
-    for (int n = 0; n <= kPMax; ++n)
-        for (int m = 0; m <= kPMax; ++m) {
-            ht[n][m].x = (float)hd[n][m];
-            ht[n][m].y = (float)(hd[n][m] - (double)ht[n][m].x);
-        }
-    EDFMM_CUDA_TRY(cudaMemcpyToSymbol(c_rdiv_f, hf, sizeof(hf)));
-    EDFMM_CUDA_TRY(cudaMemcpyToSymbol(c_rdiv_d, hd, sizeof(hd)));
     EDFMM_CUDA_TRY(cudaMemcpyToSymbol(c_rdiv_tf, ht, sizeof(ht)));
     return EDFMM_OK;
 }
 
 namespace {
 
+// Below this many leaves the four warps of a block share a leaf.  With one warp
+// per leaf 2,003 points (64 leaves) keep 64 warps busy: 84 us against 23.  The
+// FP64 forms take ten times as long per interaction, so their last wave
+// weighs more: 2,468 leaves in two-float (at 106 operations an interaction)
+// 874 us with a warp per leaf, 406 shared; FP32 with 9,856 leaves 143 and 162 us.
+template <int MODE> constexpr int64_t shared_leaves() { return MODE == kF32 ? 152 * 16 : 152 * 64; }
+
+template <int MODE, typename T> int near_launch(const NearParams<T> &P, cudaStream_t s) {
+    if (P.n_leaves < shared_leaves<MODE>())
+        k_p2p<MODE, kNearWarps><<<(unsigned)P.n_leaves, 32 * kNearWarps, 0, s>>>(P);
+    else
+        k_p2p<MODE, 1><<<(unsigned)((P.n_leaves + kNearWarps - 1) / kNearWarps), 32 * kNearWarps, 0, s>>>(P);
+    EDFMM_LAUNCH_CHECK("k_p2p");
+    return EDFMM_OK;
+}
+
 template <typename T>
-int near_impl(const DevTree &tree, const DevLists &lists, const FmmBuffers &buf, const NearArgs &a, cudaStream_t s) {
+int near_impl(const DevTree &tree, const DevLists &lists, const FmmBuffers &buf, const DevTree *src_tree, void *out,
+              cudaStream_t s) {
     using T4 = typename Vec4<T>::type;
     if (tree.n_leaves == 0) return EDFMM_OK;
-    NearParams<T> P;
+    NearParams<T> P{};
     P.leaves = lists.p2p_leaves.p ? dptr<int32_t>(lists.p2p_leaves) : dptr<int32_t>(tree.leaves);
     P.n_leaves = tree.n_leaves;
     P.off = dptr<int32_t>(lists.p2p_off);
     P.src = dptr<int32_t>(lists.p2p_src);
     P.pts = dptr<T4>(tree.pts);
     P.range = dptr<int2>(tree.range);
-    P.spts = a.src_tree ? dptr<T4>(a.src_tree->pts) : P.pts;
-    // two-float near field: an FP64 plan (one tree) whose split points exist
-    const bool tf = sizeof(T) == 8 && !a.src_tree && buf.arith == EDFMM_ARITH_TWO_FLOAT && tree.pts_tf.p;
-    P.spts_tf = tf ? dptr<float4>(tree.pts_tf) : nullptr;
-    P.srange = a.src_tree ? dptr<int2>(a.src_tree->range) : P.range;
-    P.same = a.src_tree ? 0 : 1;
+    P.spts = src_tree ? dptr<T4>(src_tree->pts) : P.pts;
+    P.srange = src_tree ? dptr<int2>(src_tree->range) : P.range;
+    P.same = src_tree ? 0 : 1;
+    const T eps = sizeof(T) == 8 ? (T)DBL_EPSILON : (T)FLT_EPSILON;
+    P.eps2 = eps * eps;
+    P.mask = src_tree ? InstMask{} : buf.mask;
+    P.out = static_cast<T *>(out);
+    if constexpr (sizeof(T) == 4) {
+        return near_launch<kF32>(P, s);
+    } else {
+        if (src_tree) return near_launch<kIeee>(P, s);
+        P.spts_split = dptr<float4>(tree.pts_grid);
+        P.grid = dptr<GridInfo>(tree.grid_info);
+        return tree.grid_tf ? near_launch<kTF>(P, s) : near_launch<kGrid>(P, s);
+    }
+}
+
+template <typename T>
+int l2p_impl(const DevTree &tree, const FmmBuffers &buf, const L2pArgs &a, cudaStream_t s) {
+    using T4 = typename Vec4<T>::type;
+    if (tree.n_leaves == 0) return EDFMM_OK;
+    L2pParams<T> P{};
+    P.leaves = dptr<int32_t>(tree.leaves);
+    P.n_leaves = tree.n_leaves;
+    P.pts = dptr<T4>(tree.pts);
+    P.range = dptr<int2>(tree.range);
     P.center = dptr<T4>(tree.center);
     P.half = dptr<T4>(tree.half);
     P.Lexp = dptr<Cplx<T>>(buf.locals);
-    P.p = buf.p;
     P.nc_pad = buf.nc_pad;
-    const T eps = sizeof(T) == 8 ? (T)DBL_EPSILON : (T)FLT_EPSILON;
-    P.eps2 = eps * eps;
-    P.near = a.near ? 1 : 0;
     P.far = a.far ? 1 : 0;
     P.add_in = static_cast<const T *>(a.add_in);
-    P.mask = a.src_tree ? InstMask{} : buf.mask;
+    P.mask = buf.mask;
     P.scatter = a.scatter ? 1 : 0;
     P.index_map = dptr<int32_t>(tree.index_map);
     P.sigma = static_cast<const T *>(a.sigma);
@@ -560,24 +828,42 @@ int near_impl(const DevTree &tree, const DevLists &lists, const FmmBuffers &buf,
     P.self_int = static_cast<const T *>(a.self_int);
     P.k_e = (T)a.k_e;
     P.out = static_cast<T *>(a.out);
-    if constexpr (sizeof(T) == 8) {
-        if (tf) {
-            k_p2p_l2p<T, true><<<(unsigned)((tree.n_leaves + 3) / 4), 128, 0, s>>>(P);
-            EDFMM_LAUNCH_CHECK("k_p2p_l2p (two-float)");
-            return EDFMM_OK;
-        }
+    const unsigned grid = (unsigned)((tree.n_leaves + 3) / 4);
+    const bool tf = sizeof(T) == 8 && buf.arith == EDFMM_ARITH_TWO_FLOAT;
+    switch (buf.p) {
+#define EDFMM_L2P_CASE(PP)                                                  \
+    case PP:                                                                \
+        if (sizeof(T) == 8 && tf) k_l2p<T, (sizeof(T) == 8), PP><<<grid, 128, 0, s>>>(P); \
+        else k_l2p<T, false, PP><<<grid, 128, 0, s>>>(P);                   \
+        break;
+        EDFMM_L2P_CASE(1)
+        EDFMM_L2P_CASE(2)
+        EDFMM_L2P_CASE(3)
+        EDFMM_L2P_CASE(4)
+        EDFMM_L2P_CASE(5)
+        EDFMM_L2P_CASE(6)
+        EDFMM_L2P_CASE(7)
+        EDFMM_L2P_CASE(8)
+        EDFMM_L2P_CASE(9)
+        EDFMM_L2P_CASE(10)
+#undef EDFMM_L2P_CASE
+        default:
+            return fail(EDFMM_ERR_UNSUPPORTED, "expansion order out of range");
     }
-    k_p2p_l2p<T, false><<<(unsigned)((tree.n_leaves + 3) / 4), 128, 0, s>>>(P);
-    EDFMM_LAUNCH_CHECK("k_p2p_l2p");
+    EDFMM_LAUNCH_CHECK("k_l2p");
     return EDFMM_OK;
 }
 
 }  // namespace
 
-int run_p2p_l2p(const DevTree &tree, const DevLists &lists, const FmmBuffers &buf, const NearArgs &args,
-                cudaStream_t s) {
-    return tree.dtype == EDFMM_F64 ? near_impl<double>(tree, lists, buf, args, s)
-                                   : near_impl<float>(tree, lists, buf, args, s);
+int run_p2p(const DevTree &tree, const DevLists &lists, const FmmBuffers &buf, const DevTree *src_tree, void *out,
+            cudaStream_t s) {
+    return tree.dtype == EDFMM_F64 ? near_impl<double>(tree, lists, buf, src_tree, out, s)
+                                   : near_impl<float>(tree, lists, buf, src_tree, out, s);
+}
+
+int run_l2p(const DevTree &tree, const FmmBuffers &buf, const L2pArgs &args, cudaStream_t s) {
+    return tree.dtype == EDFMM_F64 ? l2p_impl<double>(tree, buf, args, s) : l2p_impl<float>(tree, buf, args, s);
 }
 
 namespace {

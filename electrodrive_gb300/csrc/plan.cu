@@ -123,7 +123,8 @@ int shrink_tree_lists(DevTree &t, DevLists &l, cudaStream_t s) {
     DevBuf *bufs[] = {&t.pts,      &t.index_map,     &t.center,      &t.half,    &t.range,
                       &t.parent,   &t.children,      &t.level,       &t.is_leaf, &t.leaves,
                       &t.level_nodes, &t.inst_node_off, &l.p2p_off,  &l.p2p_src, &l.m2l_off,
-                      &l.m2l_src,  &l.m2l_swapped_off, &l.m2l_swapped_src, &l.p2p_leaves, &l.m2l_rows};
+                      &l.m2l_src,  &l.m2l_swapped_off, &l.m2l_swapped_src, &l.p2p_leaves, &l.m2l_rows,
+                      &t.pts_grid, &t.grid_info};
     for (DevBuf *b : bufs)
         if (int rc = b->shrink_to_fit(s)) return rc;
     return EDFMM_OK;
@@ -224,6 +225,7 @@ int edfmm_plan_create(const void *points_dev, int64_t n, int dtype, int leaf_siz
     BlockCacheScope cache_scope;  // the build runs on `s` alone
     rc = tree_build(points_dev, n, dtype, leaf_size, max_depth, p->tree, s);
     if (!rc) rc = lists_build(p->tree, mac_theta, p->lists, s);
+    if (!rc) rc = grid_prepare(p->tree, s);
     if (!rc) rc = shrink_tree_lists(p->tree, p->lists, s);
     if (!rc) {
         p->fmm.p = expansion_order;
@@ -283,6 +285,7 @@ int edfmm_plan_create_batch(const void *points_dev, const int64_t *offsets, int 
     }
     rc = tree_build_forest(points_dev, offsets, n_instances, dtype, leaf_size, max_depth, p->tree, s);
     if (!rc) rc = lists_build(p->tree, mac_theta, p->lists, s);
+    if (!rc) rc = grid_prepare(p->tree, s);
     if (!rc) rc = shrink_tree_lists(p->tree, p->lists, s);
     if (!rc) {
         p->fmm.p = expansion_order;
@@ -352,6 +355,8 @@ int edfmm_plan_convert(const edfmm_plan *src, int dtype, int expansion_order, vo
                     &t.level_nodes, &t.inst_node_off, &l.p2p_off, &l.p2p_src, &l.m2l_off, &l.m2l_src,
                     &l.m2l_swapped_off, &l.m2l_swapped_src, &l.p2p_leaves, &l.m2l_rows};
     for (size_t i = 0; !rc && i < sizeof(from) / sizeof(from[0]); ++i) rc = clone_buf(*from[i], *to[i], s);
+    if (!rc) rc = grid_prepare(t, s);
+    if (!rc && dtype == EDFMM_F64) rc = set_charges(t, nullptr, nullptr, s);
     if (!rc) rc = alloc_expansions(p, dtype, expansion_order, s);  // synchronises the stream
     if (rc) {
         delete p;
@@ -400,18 +405,19 @@ int edfmm_plan_set_arithmetic(edfmm_plan *p, int mode, void *stream) {
     if (mode != EDFMM_ARITH_NATIVE && mode != EDFMM_ARITH_TWO_FLOAT)
         return fail(EDFMM_ERR_ARG, "mode must be EDFMM_ARITH_NATIVE or EDFMM_ARITH_TWO_FLOAT");
     cudaStream_t s = S(stream);
+    // the split points' charges are doubles or pairs of floats
+    auto split_charges = [&](bool tf) {
+        p->tree.grid_tf = tf;
+        return set_charges(p->tree, nullptr, nullptr, s);
+    };
     if (mode == EDFMM_ARITH_NATIVE) {
-        p->tree.pts_tf.release();
         p->tree.nodes_tf.release();
         p->fmm.mult_tf.release();
         p->fmm.arith = EDFMM_ARITH_NATIVE;
-        return EDFMM_OK;
+        return p->tree.grid_tf ? split_charges(false) : EDFMM_OK;
     }
     if (p->tree.dtype != EDFMM_F64) return fail(EDFMM_ERR_UNSUPPORTED, "two-float arithmetic applies to FP64 plans");
-    if (p->tree.n_points > 0) {
-        if (int rc = p->tree.pts_tf.reserve(sizeof(float) * 8 * (size_t)p->tree.n_points)) return rc;
-        if (int rc = set_charges(p->tree, nullptr, nullptr, s)) return rc;  // splits the points and charges
-    }
+    if (int rc = split_charges(true)) return rc;
     if (int rc = prepare_two_float(p->tree, p->fmm, s)) return rc;  // split nodes, split-multipole buffer
     // the pairs the two-float M2L leaves to the FP64 kernel, built now (it
     // synchronises the stream) rather than inside a later matvec
@@ -623,21 +629,15 @@ int edfmm_plan_l2l(edfmm_plan *p, void *stream) {
 int edfmm_plan_l2p(edfmm_plan *p, void *phi_far_tree, void *stream) {
     if (int rc = check_plan(p)) return rc;
     if (p->tree.n_points > 0 && !phi_far_tree) return fail(EDFMM_ERR_ARG, "output is NULL");
-    NearArgs a;
+    L2pArgs a;
     a.out = phi_far_tree;
-    a.near = false;
-    a.far = true;
-    return run_p2p_l2p(p->tree, p->lists, p->fmm, a, S(stream));
+    return run_l2p(p->tree, p->fmm, a, S(stream));
 }
 
 int edfmm_plan_p2p(edfmm_plan *p, void *phi_near_tree, void *stream) {
     if (int rc = check_plan(p)) return rc;
     if (p->tree.n_points > 0 && !phi_near_tree) return fail(EDFMM_ERR_ARG, "output is NULL");
-    NearArgs a;
-    a.out = phi_near_tree;
-    a.near = true;
-    a.far = false;
-    return run_p2p_l2p(p->tree, p->lists, p->fmm, a, S(stream));
+    return run_p2p(p->tree, p->lists, p->fmm, nullptr, phi_near_tree, S(stream));
 }
 
 int edfmm_plan_matvec(edfmm_plan *p, const void *sigma, const void *areas, const void *self_integrals, double k_e,
@@ -651,59 +651,52 @@ int edfmm_plan_matvec(edfmm_plan *p, const void *sigma, const void *areas, const
     const bool swapped = (flags & EDFMM_REFERENCE_PAIR_ORDER) != 0;
     int rc;
     if (swapped && (rc = lists_build_swapped(p->tree, p->lists, s))) return rc;
+    const size_t elt = p->tree.dtype == EDFMM_F64 ? sizeof(double) : sizeof(float);
+    if (near && (rc = p->near_sum.reserve(elt * (size_t)p->tree.n_points))) return rc;
     if ((rc = set_charges(p->tree, sigma, areas, s))) return rc;
-    if (far && near && p->fmm.near_overlap) {
-        // The near field depends only on the charges: it runs on a second
-        // stream beside P2M -> M2M -> M2L -> L2L, into tree-order sums that
-        // the final pass (L2P + epilogue) adds.  Fork and join through
-        // events, so the pattern is also valid inside a stream capture.
+    // The near field depends only on the charges: the far-field chain
+    // P2M -> M2M -> M2L -> L2L runs beside it on a second stream and the final
+    // pass (L2P + epilogue) adds both.  Fork and join through events, so the
+    // pattern is also valid inside a stream capture.  The far field's stream
+    // has the higher priority: its small level-by-level launches are
+    // latency-bound and start as soon as a block of the near field retires.
+    // With the near field on the second stream at the caller's priority they
+    // waited until its last wave had started (P2M began 186 us into the 200k-panel
+    // torus's FP32 matvec); at equal priorities that matvec takes 397 us, with
+    // the far field first 366 (24 dimers: 796 and 725 us).
+    const bool fork = far && near && p->fmm.near_overlap;
+    cudaStream_t f = s;
+    if (fork) {
         if (!p->side) {
-            EDFMM_CUDA_TRY(cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking));
+            int least = 0, greatest = 0;
+            EDFMM_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+            EDFMM_CUDA_TRY(cudaStreamCreateWithPriority(&p->side, cudaStreamNonBlocking, greatest));
             EDFMM_CUDA_TRY(cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming));
             EDFMM_CUDA_TRY(cudaEventCreateWithFlags(&p->ev_join, cudaEventDisableTiming));
         }
-        const size_t elt = p->tree.dtype == EDFMM_F64 ? sizeof(double) : sizeof(float);
-        if ((rc = p->near_sum.reserve(elt * (size_t)p->tree.n_points))) return rc;
+        f = p->side;
         EDFMM_CUDA_TRY(cudaEventRecord(p->ev_fork, s));
-        EDFMM_CUDA_TRY(cudaStreamWaitEvent(p->side, p->ev_fork, 0));
-        NearArgs an;
-        an.out = p->near_sum.p;
-        an.scatter = false;
-        an.near = true;
-        an.far = false;
-        if ((rc = run_p2p_l2p(p->tree, p->lists, p->fmm, an, p->side))) return rc;
-        EDFMM_CUDA_TRY(cudaEventRecord(p->ev_join, p->side));
-        if ((rc = run_p2m(p->tree, p->fmm, s)) || (rc = run_m2m(p->tree, p->fmm, s)) ||
-            (rc = run_m2l(p->tree, p->lists, p->fmm, swapped, s)) || (rc = run_l2l(p->tree, p->fmm, s)))
-            return rc;
+        EDFMM_CUDA_TRY(cudaStreamWaitEvent(f, p->ev_fork, 0));
+    }
+    if (far && (rc = run_p2m(p->tree, p->fmm, f))) return rc;
+    if (near && (rc = run_p2p(p->tree, p->lists, p->fmm, nullptr, p->near_sum.p, s))) return rc;
+    if (far && ((rc = run_m2m(p->tree, p->fmm, f)) || (rc = run_m2l(p->tree, p->lists, p->fmm, swapped, f)) ||
+                (rc = run_l2l(p->tree, p->fmm, f))))
+        return rc;
+    if (fork) {
+        EDFMM_CUDA_TRY(cudaEventRecord(p->ev_join, f));
         EDFMM_CUDA_TRY(cudaStreamWaitEvent(s, p->ev_join, 0));
-        NearArgs a;
-        a.sigma = sigma;
-        a.areas = areas;
-        a.self_int = self_integrals;
-        a.k_e = k_e;
-        a.out = out;
-        a.scatter = true;
-        a.near = false;
-        a.far = true;
-        a.add_in = p->near_sum.p;
-        return run_p2p_l2p(p->tree, p->lists, p->fmm, a, s);
     }
-    if (far) {
-        if ((rc = run_p2m(p->tree, p->fmm, s)) || (rc = run_m2m(p->tree, p->fmm, s)) ||
-            (rc = run_m2l(p->tree, p->lists, p->fmm, swapped, s)) || (rc = run_l2l(p->tree, p->fmm, s)))
-            return rc;
-    }
-    NearArgs a;
+    L2pArgs a;
     a.sigma = sigma;
     a.areas = areas;
     a.self_int = self_integrals;
     a.k_e = k_e;
     a.out = out;
     a.scatter = true;
-    a.near = near;
     a.far = far;
-    return run_p2p_l2p(p->tree, p->lists, p->fmm, a, s);
+    a.add_in = near ? p->near_sum.p : nullptr;
+    return run_l2p(p->tree, p->fmm, a, s);
 }
 
 struct edfmm_targets {
@@ -711,6 +704,7 @@ struct edfmm_targets {
     DevTree tree;                // tree of the target points
     DevLists lists;              // rows: target nodes; sources: source-plan nodes
     FmmBuffers buf;              // target locals
+    DevBuf near_sum;             // near sums at the targets, tree order
 };
 
 int edfmm_targets_create(edfmm_plan *p, const void *targets_dev, int64_t m, void *stream, edfmm_targets **out) {
@@ -809,12 +803,10 @@ int edfmm_targets_stage(edfmm_targets *t, int stage, void *out_dev, void *stream
     case EDFMM_TARGETS_P2P: {
         if (t->tree.n_points == 0) return EDFMM_OK;
         if (!out_dev) return fail(EDFMM_ERR_ARG, "output is NULL");
-        NearArgs a;
+        if (stage == EDFMM_TARGETS_P2P) return run_p2p(t->tree, t->lists, t->buf, &p->tree, out_dev, s);
+        L2pArgs a;
         a.out = out_dev;
-        a.near = stage == EDFMM_TARGETS_P2P;
-        a.far = stage == EDFMM_TARGETS_L2P;
-        a.src_tree = &p->tree;
-        return run_p2p_l2p(t->tree, t->lists, t->buf, a, s);
+        return run_l2p(t->tree, t->buf, a, s);
     }
     case EDFMM_TARGETS_LOCALS: {
         if (M == 0) return EDFMM_OK;
@@ -886,14 +878,19 @@ int edfmm_targets_potential(edfmm_targets *t, const void *sigma, const void *are
             (rc = run_m2l_two(t->tree, p->tree, t->lists, p->fmm, t->buf, s)) || (rc = run_l2l(t->tree, t->buf, s)))
             return rc;
     }
-    NearArgs a;
+    if (near) {
+        const size_t elt = t->tree.dtype == EDFMM_F64 ? sizeof(double) : sizeof(float);
+        if ((rc = t->near_sum.reserve(elt * (size_t)t->tree.n_points)) ||
+            (rc = run_p2p(t->tree, t->lists, t->buf, &p->tree, t->near_sum.p, s)))
+            return rc;
+    }
+    L2pArgs a;
     a.k_e = k_e;
     a.out = out;
     a.scatter = true;
-    a.near = near;
     a.far = far;
-    a.src_tree = &p->tree;
-    return run_p2p_l2p(t->tree, t->lists, t->buf, a, s);
+    a.add_in = near ? t->near_sum.p : nullptr;
+    return run_l2p(t->tree, t->buf, a, s);
 }
 
 int edfmm_targets_field(edfmm_targets *t, const void *sigma, const void *areas, double k_e, void *out, int flags,

@@ -138,9 +138,10 @@ EDFMM_API int edfmm_plan_rebuild_lists(edfmm_plan *plan, double mac_theta, void 
  * significant bits; within about 1e-13 of the FP64 result, far inside the
  * expansion's truncation error), which on this GPU runs several times faster
  * than FP64; the expansions, P2M, M2M, L2L and every input and output stay
- * FP64.  EDFMM_ARITH_NATIVE (the default) restores IEEE FP64.  Two-float mode
- * keeps a split copy of the points (32 bytes per point) and synchronises
- * `stream` once while it prepares.  FP32 plans accept only EDFMM_ARITH_NATIVE.
+ * FP64.  EDFMM_ARITH_NATIVE (the default) restores IEEE FP64 (the near field
+ * evaluates its distances on the FP32 pipe from exactly split coordinates, 48
+ * bytes per point kept by every FP64 plan, with the accuracy of IEEE FP64).
+ * Setting two-float mode synchronises `stream` once while it prepares.  FP32 plans accept only EDFMM_ARITH_NATIVE.
  */
 EDFMM_API int edfmm_plan_set_arithmetic(edfmm_plan *plan, int mode, void *stream);
 
