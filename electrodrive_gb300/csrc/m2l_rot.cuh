@@ -130,61 +130,15 @@ template <typename T, int STRIDE> struct SmemV {
     __device__ __forceinline__ void set(int i, T x) { sts_keep(base + i * STRIDE, x); }
 };
 
-template <typename T> struct Vec2 {};
-template <> struct Vec2<float> { using type = float2; };
-template <> struct Vec2<double> { using type = double2; };
-
-__device__ __forceinline__ float2 lds_keep(const float2 *p) {
-    float2 v;
-    asm volatile("ld.volatile.shared.v2.f32 {%0, %1}, [%2];"
-                 : "=f"(v.x), "=f"(v.y)
-                 : "r"((unsigned)__cvta_generic_to_shared(p)));
-    return v;
-}
-__device__ __forceinline__ double2 lds_keep(const double2 *p) {
-    double2 v;
-    asm volatile("ld.volatile.shared.v2.f64 {%0, %1}, [%2];"
-                 : "=d"(v.x), "=d"(v.y)
-                 : "r"((unsigned)__cvta_generic_to_shared(p)));
-    return v;
-}
-__device__ __forceinline__ void sts_keep(float2 *p, float2 v) {
-    asm volatile("st.volatile.shared.v2.f32 [%0], {%1, %2};" ::"r"((unsigned)__cvta_generic_to_shared(p)), "f"(v.x),
-                 "f"(v.y));
-}
-__device__ __forceinline__ void sts_keep(double2 *p, double2 v) {
-    asm volatile("st.volatile.shared.v2.f64 [%0], {%1, %2};" ::"r"((unsigned)__cvta_generic_to_shared(p)), "d"(v.x),
-                 "d"(v.y));
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ double2 add2(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-// x * h + a on both halves
-__device__ __forceinline__ float2 fma2(float2 x, float h, float2 a) { return __ffma2_rn(x, make_float2(h, h), a); }
-__device__ __forceinline__ double2 fma2(double2 x, double h, double2 a) {
-    return make_double2(fma(x.x, h, a.x), fma(x.y, h, a.y));
-}
-
-// Per-lane accumulator of the translated locals: complex slot tri(n, m) at
-// base[tri(n, m) * STRIDE] (one 8- or 16-byte word per lane, so a warp's
-// access is conflict-free and each coefficient pair is one load and one store).
-// FP32 uses plain accesses (the compiler keeps the slots in shared memory at
-// 167 registers; volatile stores measured 5% slower); FP64 uses volatile ones
-// so that its 45 complex slots are not pulled into registers.
-template <typename T, int STRIDE> struct AccC {
-    using T2 = typename Vec2<T>::type;
-    T2 *base;
-    __device__ __forceinline__ T2 get(int q) const {
-        if constexpr (sizeof(T) == 8)
-            return lds_keep(base + q * STRIDE);
-        else
-            return base[q * STRIDE];
-    }
-    __device__ __forceinline__ void set(int q, T2 x) {
-        if constexpr (sizeof(T) == 8)
-            sts_keep(base + q * STRIDE, x);
-        else
-            base[q * STRIDE] = x;
-    }
+// Per-lane accumulator of the translated locals (FP32): complex slot tri(n, m)
+// at base[tri(n, m) * STRIDE] (one 8-byte word per lane, so a warp's access is
+// conflict-free and each coefficient pair is one load and one store).  Plain
+// accesses: the compiler keeps the slots in shared memory at 167 registers
+// (volatile stores measured 5% slower).
+template <int STRIDE> struct AccC {
+    float2 *base;
+    __device__ __forceinline__ float2 get(int q) const { return base[q * STRIDE]; }
+    __device__ __forceinline__ void set(int q, float2 x) { base[q * STRIDE] = x; }
 };
 
 // forward rotation of degree n: scale by fn, R_z(+phi), Q_p, R_z(+theta), Q_m.
@@ -206,38 +160,35 @@ __device__ __forceinline__ void forward(V &v, T cr, T fn, const Frame<T, P> &F) 
 
 // backward rotation of degree n (transposes in reverse order), added to acc;
 // BINOM: scaled by hn = n! / rho^(n+1) as it is added
-template <typename T, int P, bool BINOM, int n, typename V, typename A>
-__device__ __forceinline__ void backward(V &v, A &acc, const Frame<T, P> &F, T hn, T irho) {
+template <int P, bool BINOM, int n, typename V, typename A>
+__device__ __forceinline__ void backward(V &v, A &acc, const Frame<float, P> &F, float hn, float irho) {
     constexpr int N = 2 * n + 1, OV = n * n, OFF = kRotOff[n];
-    T b[N], o[N];
+    float b[N], o[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) b[i] = v.get(OV + i);
-    rot_apply<T, 3, N, OFF, 0>(b, o);
-    zrot<T, N, P>(o, F.ct, F.st, T(-1));
-    rot_apply<T, 2, N, OFF, 0>(o, b);
-    zrot<T, N, P>(b, F.cp, F.sp, T(-1));
-    using T2 = typename Vec2<T>::type;
+    rot_apply<float, 3, N, OFF, 0>(b, o);
+    zrot<float, N, P>(o, F.ct, F.st, -1.0f);
+    rot_apply<float, 2, N, OFF, 0>(o, b);
+    zrot<float, N, P>(b, F.cp, F.sp, -1.0f);
     {
-        T2 a = acc.get(tri(n, 0));
+        float2 a = acc.get(tri(n, 0));
         a.x = BINOM ? fma(b[0], hn, a.x) : a.x + b[0];
         acc.set(tri(n, 0), a);
     }
 #pragma unroll
     for (int m = 1; m <= n; ++m) {
-        T2 x;
-        x.x = b[2 * m - 1];
-        x.y = b[2 * m];
-        acc.set(tri(n, m), BINOM ? fma2(x, hn, acc.get(tri(n, m))) : add2(acc.get(tri(n, m)), x));
+        const float2 x = make_float2(b[2 * m - 1], b[2 * m]), a = acc.get(tri(n, m));
+        acc.set(tri(n, m), BINOM ? __ffma2_rn(x, make_float2(hn, hn), a) : __fadd2_rn(a, x));
     }
-    if constexpr (n < P) backward<T, P, BINOM, n + 1>(v, acc, F, hn * T(n + 1) * irho, irho);
+    if constexpr (n < P) backward<P, BINOM, n + 1>(v, acc, F, hn * float(n + 1) * irho, irho);
 }
 
 // The axial translation with the factor table f[j] = j! / rho^(j+1):
-// L'_n^m = (-1)^(n+m) sum_{k=m..P} M'_k^m f[n+k], in place.  FP32 runs the
-// complex (m >= 1) terms as packed pairs: f2[j] = (f[j], f[j]).
-template <typename T, int P, int m, typename V>
-__device__ __forceinline__ void axial_table(V &v, const T (&f)[2 * P + 1], const float2 (&f2)[2 * P + 1]) {
-    if constexpr (m > 0 && sizeof(T) == 4) {
+// L'_n^m = (-1)^(n+m) sum_{k=m..P} M'_k^m f[n+k], in place; the complex
+// (m >= 1) terms as packed pairs, f2[j] = (f[j], f[j]).
+template <int P, int m, typename V>
+__device__ __forceinline__ void axial_table(V &v, const float (&f)[2 * P + 1], const float2 (&f2)[2 * P + 1]) {
+    if constexpr (m > 0) {
         float2 u[P + 1];
 #pragma unroll
         for (int k = m; k <= P; ++k) u[k] = make_float2(v.get(k * k + 2 * m - 1), v.get(k * k + 2 * m));
@@ -251,30 +202,20 @@ __device__ __forceinline__ void axial_table(V &v, const T (&f)[2 * P + 1], const
             v.set(n * n + 2 * m, sg * sum.y);
         }
     } else {
-        T ur[P + 1], ui[P + 1], wr[P + 1], wi[P + 1];
+        float u[P + 1], w[P + 1];
 #pragma unroll
-        for (int k = m; k <= P; ++k) {
-            ur[k] = v.get(k * k + (m == 0 ? 0 : 2 * m - 1));
-            ui[k] = m == 0 ? T(0) : v.get(k * k + 2 * m);
+        for (int k = 0; k <= P; ++k) u[k] = v.get(k * k);
+#pragma unroll
+        for (int n = 0; n <= P; ++n) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int k = 0; k <= P; ++k) sum = fma(u[k], f[n + k], sum);
+            w[n] = (n & 1) ? -sum : sum;
         }
 #pragma unroll
-        for (int n = m; n <= P; ++n) {
-            T sr = T(0), si = T(0);
-#pragma unroll
-            for (int k = m; k <= P; ++k) {
-                sr = fma(ur[k], f[n + k], sr);
-                if (m > 0) si = fma(ui[k], f[n + k], si);
-            }
-            wr[n] = ((n + m) & 1) ? -sr : sr;
-            wi[n] = ((n + m) & 1) ? -si : si;
-        }
-#pragma unroll
-        for (int n = m; n <= P; ++n) {
-            v.set(n * n + (m == 0 ? 0 : 2 * m - 1), wr[n]);
-            if (m > 0) v.set(n * n + 2 * m, wi[n]);
-        }
+        for (int n = 0; n <= P; ++n) v.set(n * n, w[n]);
     }
-    if constexpr (m < P) axial_table<T, P, m + 1>(v, f, f2);
+    if constexpr (m < P) axial_table<P, m + 1>(v, f, f2);
 }
 
 // The axial translation in binomial form (the FP32 kernel at p <= 7 and the
@@ -349,29 +290,20 @@ __device__ __forceinline__ void axial(V &v, const T (&h)[P + 1]) {
 // 3.82 ms at p = 8)
 template <typename T, int P> __host__ __device__ constexpr bool rot_binomial() { return !(sizeof(T) == 4 && P >= 8); }
 
-// One pair: translated locals of source s added to acc.
-template <typename T, int P, typename V, typename A>
-__device__ __forceinline__ void rot_pair(V &v, A &acc, const typename Vec2<T>::type *__restrict__ Mrow, T c, T dx, T dy,
-                                         T dz) {
-    // FP32 rows are read two coefficients per 16-byte load (rows of an even
-    // number of coefficients, 16-byte aligned): half the scattered loads
+// One pair (FP32): translated locals of source row Mrow added to acc.
+template <int P, typename V, typename A>
+__device__ __forceinline__ void rot_pair(V &v, A &acc, const float2 *__restrict__ Mrow, float c, float dx, float dy,
+                                         float dz) {
+    // rows are read two coefficients per 16-byte load (rows of an even number
+    // of coefficients, 16-byte aligned): half the scattered loads
     float4 x4{};
 #pragma unroll
     for (int n = 0; n <= P; ++n) {
 #pragma unroll
         for (int m = 0; m <= n; ++m) {
             const int q = tri(n, m);
-            typename Vec2<T>::type x;
-            if constexpr (sizeof(T) == 4) {
-                if ((q & 1) == 0) {
-                    x4 = reinterpret_cast<const float4 *>(Mrow)[q >> 1];
-                    x = make_float2(x4.x, x4.y);
-                } else {
-                    x = make_float2(x4.z, x4.w);
-                }
-            } else {
-                x = Mrow[q];
-            }
+            if ((q & 1) == 0) x4 = reinterpret_cast<const float4 *>(Mrow)[q >> 1];
+            const float2 x = (q & 1) == 0 ? make_float2(x4.x, x4.y) : make_float2(x4.z, x4.w);
             if (m == 0) {
                 v.set(n * n, x.x);
             } else {
@@ -380,35 +312,33 @@ __device__ __forceinline__ void rot_pair(V &v, A &acc, const typename Vec2<T>::t
             }
         }
     }
-    const T s2 = dx * dx + dy * dy, r2 = s2 + dz * dz;
-    const T s = sqrt(s2), rho = sqrt(r2), irho = T(1) / rho;
-    Frame<T, P> F;
-    T cphi = T(1), sphi = T(0);
-    if (s2 > T(0)) {
-        const T is = T(1) / s;
+    const float s2 = dx * dx + dy * dy, r2 = s2 + dz * dz;
+    const float s = sqrt(s2), rho = sqrt(r2), irho = 1.0f / rho;
+    Frame<float, P> F;
+    float cphi = 1.0f, sphi = 0.0f;
+    if (s2 > 0.0f) {
+        const float is = 1.0f / s;
         cphi = dx * is;
         sphi = dy * is;
     }
-    powers<T, P>(cphi, sphi, F.cp, F.sp);
-    powers<T, P>(dz * irho, s * irho, F.ct, F.st);
-    constexpr bool BINOM = rot_binomial<T, P>();
-    forward<T, P, BINOM, 0>(v, BINOM ? c * irho : c, T(1), F);
+    powers<float, P>(cphi, sphi, F.cp, F.sp);
+    powers<float, P>(dz * irho, s * irho, F.ct, F.st);
+    constexpr bool BINOM = rot_binomial<float, P>();
+    forward<float, P, BINOM, 0>(v, BINOM ? c * irho : c, 1.0f, F);
     if constexpr (BINOM) {
-        const T none[P + 1] = {};
-        axial<T, P, 0, false>(v, none);
+        const float none[P + 1] = {};
+        axial<float, P, 0, false>(v, none);
     } else {
-        T f[2 * P + 1];
+        float f[2 * P + 1];
         f[0] = irho;
 #pragma unroll
-        for (int j = 1; j <= 2 * P; ++j) f[j] = f[j - 1] * (T)j * irho;
+        for (int j = 1; j <= 2 * P; ++j) f[j] = f[j - 1] * (float)j * irho;
         float2 f2[2 * P + 1];
-        if constexpr (sizeof(T) == 4) {
 #pragma unroll
-            for (int j = 0; j <= 2 * P; ++j) f2[j] = make_float2((float)f[j], (float)f[j]);
-        }
-        axial_table<T, P, 0>(v, f, f2);
+        for (int j = 0; j <= 2 * P; ++j) f2[j] = make_float2(f[j], f[j]);
+        axial_table<P, 0>(v, f, f2);
     }
-    backward<T, P, BINOM, 0>(v, acc, F, irho, irho);
+    backward<P, BINOM, 0>(v, acc, F, irho, irho);
 }
 
 // ---------------------------------------------------------------------------
@@ -452,26 +382,25 @@ __host__ __device__ constexpr bool pk_started(int I) {
 // a block run the same number of rounds of pairs, with a barrier between
 // rounds, so that the warps of an SM walk the long straight-line pair code
 // close together and share its instruction fetches.
-template <typename T, int P, bool V_IN_SMEM>
-__global__ void __launch_bounds__(kRotThreads, sizeof(T) == 4 ? (rot_binomial<T, P>() ? 4 : 3) : 1)
+template <int P>
+__global__ void __launch_bounds__(kRotThreads, rot_binomial<float, P>() ? 4 : 3)
     k_m2l_rot(int64_t n_nodes, const int32_t *__restrict__ off, const int32_t *__restrict__ src,
-              const int32_t *__restrict__ rows,
-              const typename Vec4<T>::type *__restrict__ tcenter, const typename Vec4<T>::type *__restrict__ thalf,
-              const typename Vec4<T>::type *__restrict__ center, const typename Vec4<T>::type *__restrict__ half,
-              const typename Vec2<T>::type *__restrict__ Mexp, typename Vec2<T>::type *__restrict__ Lexp,
-              int nc_pad, const InstMask mask) {
-    using T2 = typename Vec2<T>::type;
+              const int32_t *__restrict__ rows, const float4 *__restrict__ tcenter, const float4 *__restrict__ thalf,
+              const float4 *__restrict__ center, const float4 *__restrict__ half, const float2 *__restrict__ Mexp,
+              float2 *__restrict__ Lexp, int nc_pad, const InstMask mask) {
+    using T = float;
+    using T2 = float2;
     constexpr int NV = (P + 1) * (P + 1), NQ = (P + 1) * (P + 2) / 2, NT = kRotThreads;
     extern __shared__ __align__(16) unsigned char rot_smem[];
     __shared__ int max_rounds;
     T2 *sq = reinterpret_cast<T2 *>(rot_smem);
-    AccC<T, NT> acc{sq + threadIdx.x};
+    AccC<NT> acc{sq + threadIdx.x};
     // warp w takes target row rows[w] (rows by decreasing pair count), or row w
     const int64_t w = ((int64_t)blockIdx.x * NT + threadIdx.x) >> 5;
     const int64_t t = rows && w < n_nodes ? (int64_t)rows[w] : w;
     const int lane = threadIdx.x & 31;
     const bool live = t < n_nodes && inst_active(mask, (int)t);
-    typename Vec4<T>::type ct{};
+    float4 ct{};
     T iaL = T(1);
     int b = 0, e = 0;
     if (live) {
@@ -492,17 +421,12 @@ __global__ void __launch_bounds__(kRotThreads, sizeof(T) == 4 ? (rot_binomial<T,
         const int k = b + r * 32 + lane;
         if (k >= e) continue;
         const int s = __ldg(src + k);
-        const typename Vec4<T>::type cs = center[s];
+        const float4 cs = center[s];
         const T c = half[s].w * iaL;
-        if (sizeof(T) == 4 && c > (T)kRotExtremeRatio) continue;  // translated by k_m2l_generic
-        const T2 *Mrow = Mexp + (int64_t)s * nc_pad;
-        if constexpr (V_IN_SMEM) {
-            SmemV<T, NT> v{reinterpret_cast<T *>(sq + NQ * NT) + threadIdx.x};
-            rot_pair<T, P>(v, acc, Mrow, c, (ct.x - cs.x) * iaL, (ct.y - cs.y) * iaL, (ct.z - cs.z) * iaL);
-        } else {
-            RegV<T, NV> v;
-            rot_pair<T, P>(v, acc, Mrow, c, (ct.x - cs.x) * iaL, (ct.y - cs.y) * iaL, (ct.z - cs.z) * iaL);
-        }
+        if (c > kRotExtremeRatio) continue;  // translated by k_m2l_generic
+        RegV<T, NV> v;
+        rot_pair<P>(v, acc, Mexp + (int64_t)s * nc_pad, c, (ct.x - cs.x) * iaL, (ct.y - cs.y) * iaL,
+                    (ct.z - cs.z) * iaL);
     }
     if (!live) return;
     T2 *out = Lexp + t * nc_pad;
@@ -543,19 +467,19 @@ __global__ void __launch_bounds__(kRotThreads, sizeof(T) == 4 ? (rot_binomial<T,
 // scale exceeds 256x the target's are left to the caller (FP32 exponent
 // range), as in the FP32 kernel.
 // ---------------------------------------------------------------------------
-template <int P, int n, typename V>
-__device__ __forceinline__ void backward_tf(V &v, const Frame<tf32x2, P> &F) {
+template <typename T, int P, int n, typename V>
+__device__ __forceinline__ void backward_v(V &v, const Frame<T, P> &F) {
     constexpr int N = 2 * n + 1, OV = n * n, OFF = kRotOff[n];
-    tf32x2 b[N], o[N];
+    T b[N], o[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) b[i] = v.get(OV + i);
-    rot_apply<tf32x2, 3, N, OFF, 0>(b, o);
-    zrot<tf32x2, N, P>(o, F.ct, F.st, tf32x2(-1));
-    rot_apply<tf32x2, 2, N, OFF, 0>(o, b);
-    zrot<tf32x2, N, P>(b, F.cp, F.sp, tf32x2(-1));
+    rot_apply<T, 3, N, OFF, 0>(b, o);
+    zrot<T, N, P>(o, F.ct, F.st, T(-1));
+    rot_apply<T, 2, N, OFF, 0>(o, b);
+    zrot<T, N, P>(b, F.cp, F.sp, T(-1));
 #pragma unroll
     for (int i = 0; i < N; ++i) v.set(OV + i, b[i]);
-    if constexpr (n < P) backward_tf<P, n + 1>(v, F);
+    if constexpr (n < P) backward_v<T, P, n + 1>(v, F);
 }
 
 // --- the two-float matrices on packed FP32x2 instructions ---
@@ -823,7 +747,7 @@ __device__ __forceinline__ void rot_pair_tf(V &v, const float4 *__restrict__ Mro
     for (int j = 1; j <= P; ++j) h[j] = h[j - 1] * T(j) * irho;
     axial<T, P, 0, true>(v, h);
     if constexpr (PK) backward_tf_pk<P, 0>(v, F);
-    else backward_tf<P, 0>(v, F);
+    else backward_v<T, P, 0>(v, F);
 }
 
 // tnodes / snodes: per node (cx hi, cx lo, cy hi, cy lo), (cz hi, cz lo, a hi, a lo).
@@ -939,6 +863,122 @@ __global__ void __launch_bounds__(NT, 256 / NT)
     }
 }
 
+// ---------------------------------------------------------------------------
+// FP64 M2L.  The pair's coefficients stay in its lane's shared-memory slots,
+// read with loads the compiler may not hoist (81 doubles and the phases do
+// not fit in registers), and after each round of 32 pairs the warp adds the
+// slots of its lanes, lane i owning coefficients i, i + 32, i + 64.  The FP64
+// pipe (64 cycles per warp operation) is the bound, so what counts is that
+// every scheduler always has a warp to serve, and to the end: two blocks fit
+// an SM, and the four warps of a block take the rounds of one row in turn.
+// With the translated locals accumulated per lane one block filled an SM and
+// its pipe idled through every shared-memory latency; with a row per warp, long
+// rows that shared a scheduler ended long after the others.  180k pairs on a
+// sphere of 20,011 points: 1,174 (accumulators per lane), 1,345 (a row per
+// warp, ten warps per SM), 987 us (four warps a row; 590 us at the pipe's full rate).
+// ---------------------------------------------------------------------------
+template <int P>
+__global__ void __launch_bounds__(kRotThreads, 2)
+    k_m2l_rot_f64(int64_t n_nodes, const int32_t *__restrict__ off, const int32_t *__restrict__ src,
+                  const int32_t *__restrict__ rows, const double4 *__restrict__ tcenter,
+                  const double4 *__restrict__ thalf, const double4 *__restrict__ center,
+                  const double4 *__restrict__ half, const double2 *__restrict__ Mexp, double2 *__restrict__ Lexp,
+                  int nc_pad, const InstMask mask) {
+    constexpr int NV = (P + 1) * (P + 1), NR = (NV + 31) / 32, NT = kRotThreads, NW = NT / 32;
+    extern __shared__ __align__(16) unsigned char rot_smem[];
+    double *slots = reinterpret_cast<double *>(rot_smem);  // slot i of thread u at slots[i * NT + u]
+    const int64_t t = rows ? (int64_t)rows[blockIdx.x] : (int64_t)blockIdx.x;
+    if (t >= n_nodes || !inst_active(mask, (int)t)) return;
+    const int lane = threadIdx.x & 31, wbase = threadIdx.x & ~31;
+    SmemV<double, NT> v{slots + threadIdx.x};
+    const double4 ct = tcenter[t];
+    const double iaL = 1.0 / thalf[t].w;
+    const int b = off[t], e = off[t + 1];
+    double acc[NR];
+#pragma unroll
+    for (int j = 0; j < NR; ++j) acc[j] = 0.0;
+    for (int k0 = b + wbase; k0 < e; k0 += NT) {
+        const int k = k0 + lane;
+        if (k < e) {
+            const int s = __ldg(src + k);
+            const double4 cs = center[s];
+            const double2 *Mrow = Mexp + (int64_t)s * nc_pad;
+#pragma unroll
+            for (int n = 0; n <= P; ++n) {
+#pragma unroll
+                for (int m = 0; m <= n; ++m) {
+                    const double2 x = Mrow[tri(n, m)];
+                    if (m == 0) {
+                        v.set(n * n, x.x);
+                    } else {
+                        v.set(n * n + 2 * m - 1, x.x);
+                        v.set(n * n + 2 * m, x.y);
+                    }
+                }
+            }
+            const double dx = (ct.x - cs.x) * iaL, dy = (ct.y - cs.y) * iaL, dz = (ct.z - cs.z) * iaL;
+            const double s2 = dx * dx + dy * dy, r2 = s2 + dz * dz;
+            const double irho = rsqrt(r2);
+            Frame<double, P> F;
+            double cphi = 1.0, sphi = 0.0, s1 = 0.0;
+            if (s2 > 0.0) {
+                const double is = rsqrt(s2);
+                s1 = s2 * is;
+                cphi = dx * is;
+                sphi = dy * is;
+            }
+            powers<double, P>(cphi, sphi, F.cp, F.sp);
+            powers<double, P>(dz * irho, s1 * irho, F.ct, F.st);
+            forward<double, P, true, 0>(v, half[s].w * iaL * irho, 1.0, F);
+            double h[P + 1];
+            h[0] = irho;
+#pragma unroll
+            for (int j = 1; j <= P; ++j) h[j] = h[j - 1] * (double)j * irho;
+            axial<double, P, 0, true>(v, h);
+            backward_v<double, P, 0>(v, F);
+        } else {
+#pragma unroll
+            for (int i = 0; i < NV; ++i) v.set(i, 0.0);
+        }
+        __syncwarp();
+        // starting at this lane: conflict-free shared-memory reads, a fixed order per coefficient
+#pragma unroll
+        for (int j = 0; j < NR; ++j) {
+            const int i = lane + 32 * j;
+            if (i < NV) {
+                const double *row = slots + i * NT + wbase;
+                double sum = acc[j];
+#pragma unroll 8
+                for (int l = 0; l < 32; ++l) sum += lds_keep(row + ((l + lane) & 31));
+                acc[j] = sum;
+            }
+        }
+        __syncwarp();
+    }
+    // the warps' sums, in warp order
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < NR; ++j)
+        if (lane + 32 * j < NV) slots[(wbase >> 5) * NV + lane + 32 * j] = acc[j];
+    __syncthreads();
+    double *out = reinterpret_cast<double *>(Lexp + t * nc_pad);
+    for (int i = threadIdx.x; i < NV; i += NT) {
+        double val = slots[i];
+#pragma unroll
+        for (int q = 1; q < NW; ++q) val += slots[q * NV + i];
+        val *= iaL;
+        int n = 0;
+        while ((n + 1) * (n + 1) <= i) ++n;
+        const int q = i - n * n;  // 0: Re X0; 2m - 1: Re Xm; 2m: Im Xm
+        if (q == 0) {
+            out[2 * tri(n, 0)] = val;
+            out[2 * tri(n, 0) + 1] = 0.0;
+        } else {
+            out[2 * tri(n, (q + 1) >> 1) + ((q & 1) ? 0 : 1)] = val;
+        }
+    }
+}
+
 inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 template <int P, int NT, bool PK>
@@ -960,21 +1000,37 @@ int launch_rot_tf(int64_t M, const int32_t *off, const int32_t *src, const int32
     return EDFMM_OK;
 }
 
-template <typename T, int P, bool V_IN_SMEM>
-int launch_rot(int64_t M, const int32_t *off, const int32_t *src, const int32_t *rows, const void *tcen,
-               const void *thal, const void *cen,
-               const void *hal, const void *Mx, void *Lx, int nc_pad, const InstMask &mask, cudaStream_t s) {
-    using T4 = typename Vec4<T>::type;
-    using T2 = typename Vec2<T>::type;
-    constexpr int NV = (P + 1) * (P + 1), NQ = (P + 1) * (P + 2) / 2, NT = kRotThreads;
-    constexpr size_t smem = (size_t)NQ * NT * sizeof(T2) + (V_IN_SMEM ? (size_t)NV * NT * sizeof(T) : 0);
+template <int P>
+int launch_rot_f64(int64_t M, const int32_t *off, const int32_t *src, const int32_t *rows, const void *tcen,
+                   const void *thal, const void *cen, const void *hal, const void *Mx, void *Lx, int nc_pad,
+                   const InstMask &mask, cudaStream_t s) {
+    constexpr size_t smem = (size_t)(P + 1) * (P + 1) * kRotThreads * sizeof(double);
     static const cudaError_t attr =
-        cudaFuncSetAttribute(k_m2l_rot<T, P, V_IN_SMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_m2l_rot_f64<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (attr != cudaSuccess)
+        return fail(EDFMM_ERR_CUDA, std::string("k_m2l_rot_f64 shared memory attribute: ") + cudaGetErrorString(attr));
+    k_m2l_rot_f64<P><<<(unsigned)M, kRotThreads, smem, s>>>(
+        M, off, src, rows, static_cast<const double4 *>(tcen), static_cast<const double4 *>(thal),
+        static_cast<const double4 *>(cen), static_cast<const double4 *>(hal), static_cast<const double2 *>(Mx),
+        static_cast<double2 *>(Lx), nc_pad, mask);
+    EDFMM_LAUNCH_CHECK("k_m2l_rot_f64");
+    return EDFMM_OK;
+}
+
+template <int P>
+int launch_rot(int64_t M, const int32_t *off, const int32_t *src, const int32_t *rows, const void *tcen,
+               const void *thal, const void *cen, const void *hal, const void *Mx, void *Lx, int nc_pad,
+               const InstMask &mask, cudaStream_t s) {
+    constexpr int NQ = (P + 1) * (P + 2) / 2, NT = kRotThreads;
+    constexpr size_t smem = (size_t)NQ * NT * sizeof(float2);
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(k_m2l_rot<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (attr != cudaSuccess)
         return fail(EDFMM_ERR_CUDA, std::string("k_m2l_rot shared memory attribute: ") + cudaGetErrorString(attr));
-    k_m2l_rot<T, P, V_IN_SMEM><<<nblk(M * 32, NT), NT, smem, s>>>(
-        M, off, src, rows, static_cast<const T4 *>(tcen), static_cast<const T4 *>(thal), static_cast<const T4 *>(cen),
-        static_cast<const T4 *>(hal), static_cast<const T2 *>(Mx), static_cast<T2 *>(Lx), nc_pad, mask);
+    k_m2l_rot<P><<<nblk(M * 32, NT), NT, smem, s>>>(
+        M, off, src, rows, static_cast<const float4 *>(tcen), static_cast<const float4 *>(thal),
+        static_cast<const float4 *>(cen), static_cast<const float4 *>(hal), static_cast<const float2 *>(Mx),
+        static_cast<float2 *>(Lx), nc_pad, mask);
     EDFMM_LAUNCH_CHECK("k_m2l_rot");
     return EDFMM_OK;
 }

@@ -7,14 +7,14 @@ int m2l_rot_f32(int p, int64_t M, const int32_t *off, const int32_t *src, const 
                 const void *c, const void *d, const void *Mx, void *Lx, int nc_pad, const InstMask &mask,
                 cudaStream_t s) {
     switch (p) {
-        case 1: return launch_rot<float, 1, false>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
-        case 2: return launch_rot<float, 2, false>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
-        case 3: return launch_rot<float, 3, false>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
-        case 4: return launch_rot<float, 4, false>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
-        case 5: return launch_rot<float, 5, false>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
-        case 6: return launch_rot<float, 6, false>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
-        case 7: return launch_rot<float, 7, false>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
-        case 8: return launch_rot<float, 8, false>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 1: return launch_rot<1>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 2: return launch_rot<2>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 3: return launch_rot<3>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 4: return launch_rot<4>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 5: return launch_rot<5>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 6: return launch_rot<6>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 7: return launch_rot<7>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 8: return launch_rot<8>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
         default: return fail(EDFMM_ERR_UNSUPPORTED, "rotation M2L supports orders 1..8");
     }
 }

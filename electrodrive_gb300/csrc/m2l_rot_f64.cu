@@ -7,14 +7,14 @@ int m2l_rot_f64(int p, int64_t M, const int32_t *off, const int32_t *src, const 
                 const void *c, const void *d, const void *Mx, void *Lx, int nc_pad, const InstMask &mask,
                 cudaStream_t s) {
     switch (p) {
-        case 1: return launch_rot<double, 1, true>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
-        case 2: return launch_rot<double, 2, true>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
-        case 3: return launch_rot<double, 3, true>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
-        case 4: return launch_rot<double, 4, true>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
-        case 5: return launch_rot<double, 5, true>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
-        case 6: return launch_rot<double, 6, true>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
-        case 7: return launch_rot<double, 7, true>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
-        case 8: return launch_rot<double, 8, true>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 1: return launch_rot_f64<1>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 2: return launch_rot_f64<2>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 3: return launch_rot_f64<3>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 4: return launch_rot_f64<4>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 5: return launch_rot_f64<5>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 6: return launch_rot_f64<6>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 7: return launch_rot_f64<7>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
+        case 8: return launch_rot_f64<8>(M, off, src, rows, a, b, c, d, Mx, Lx, nc_pad, mask, s);
         default: return fail(EDFMM_ERR_UNSUPPORTED, "rotation M2L supports orders 1..8");
     }
 }
