@@ -12,8 +12,7 @@
 // Arnoldi step two batched projections instead of the reference's j+1
 // sequential modified-Gram-Schmidt passes; in exact arithmetic the basis is
 // the same.  Reductions are deterministic: each block writes a partial sum
-// and the partials are added in a fixed order (by a separate kernel, or by
-// the last block to finish).
+// and the last block to finish adds the partials in a fixed order.
 //
 // Layout: V is (restart + 1, n) row-major in T; H is (restart + 1, restart)
 // row-major FP64; g, cs, sn are FP64 vectors; `scal` (FP64) holds
@@ -28,10 +27,19 @@ namespace edfmm {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kItems = 4;
-constexpr int kChunkN = kThreads * kItems;  // vector elements per block
 
-inline unsigned nblocks(int64_t n) { return (unsigned)((n + kChunkN - 1) / kChunkN); }
+// Vector elements per block: the largest of 64, 128, ..., 1,024 that gives two
+// blocks per SM.  The products of a step are few, but FP64 ones issue at two
+// per SM and clock: 5,120 elements in blocks of 1,024 kept five SMs busy for
+// 12 us per projection or update at 25 basis vectors (63 us an Arnoldi step);
+// in blocks of 64, with the final sums and the rotations in the last block
+// instead of launches of their own, a step takes 33 us.
+inline int chunk_of(int64_t n) {
+    int c = 1024;
+    while (c > 64 && (n + c - 1) / c < 304) c >>= 1;
+    return c;
+}
+inline unsigned nblocks(int64_t n) { return (unsigned)((n + chunk_of(n) - 1) / chunk_of(n)); }
 
 // work area: [counter (uint, padded to 16 doubles)][h1 (R+1)][h2 (R+1)][y (R)][partials nb*(R+1)]
 struct Work {
@@ -66,6 +74,7 @@ __device__ __forceinline__ double block_sum(double v, double *sm) {
 __device__ __forceinline__ bool last_block(unsigned *counter) {
     __shared__ bool is_last;
     __threadfence();
+    __syncthreads();  // every warp's partials are written before the count
     if (threadIdx.x == 0) {
         unsigned prev = atomicAdd(counter, 1u);
         is_last = prev == gridDim.x - 1;
@@ -79,14 +88,13 @@ __device__ __forceinline__ bool last_block(unsigned *counter) {
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_start(int64_t n, const T *__restrict__ b, const T *__restrict__ ax,
                                                     const T *__restrict__ pinv, T *__restrict__ v0, double *g,
-                                                    int restart, double *scal, void *work) {
+                                                    int restart, double *scal, void *work, int chunk) {
     __shared__ double sm[32];
     Work W = work_view(work, restart);
-    T s_true = 0, s_pre = 0;  // per-thread sums of kItems squares in T, then FP64
-    const int64_t base = (int64_t)blockIdx.x * kChunkN;
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        const int64_t i = base + (int64_t)k * kThreads + threadIdx.x;
+    T s_true = 0, s_pre = 0;  // per-thread sums of up to 4 squares in T, then FP64
+    const int64_t base = (int64_t)blockIdx.x * chunk;
+    for (int q = threadIdx.x; q < chunk; q += kThreads) {
+        const int64_t i = base + q;
         if (i < n) {
             const T rt = b[i] - ax[i];
             const T r = pinv ? pinv[i] * rt : rt;
@@ -136,120 +144,113 @@ __global__ void k_scale_by(int64_t n, T *v, const T *src, const double *scal, in
     v[i] = src[i] * (T)inv;
 }
 
-// Partial h[r] = <V_r, w> over one chunk of kChunkN rows per block, r <= j
-// (w = pinv * av on the first pass, written back).  The chunk of w is staged
-// in shared memory and each warp takes whole rows r, so a block needs no
-// barrier per row; the partials are added by k_dots_fin.
+// h[r] = <V_r, w>, r <= j (w = pinv * av on the first pass, written back).
+// The block's chunk of w is staged in shared memory and each warp takes whole
+// rows r, so a block needs no barrier per row; the last block to finish adds
+// the blocks' partials (in a fixed order).
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_dots(int64_t n, int j, int restart, const T *__restrict__ V,
                                                    T *__restrict__ w, const T *__restrict__ av,
-                                                   const T *__restrict__ pinv, void *work) {
-    __shared__ T ws[kChunkN];
+                                                   const T *__restrict__ pinv, void *work, int pass, int chunk) {
+    __shared__ T ws[1024];
     Work W = work_view(work, restart);
-    const int64_t base = (int64_t)blockIdx.x * kChunkN;
-    const int cnt = (int)(n - base < kChunkN ? n - base : kChunkN);
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        const int q = k * kThreads + threadIdx.x;
+    const int64_t base = (int64_t)blockIdx.x * chunk;
+    const int cnt = (int)(n - base < chunk ? n - base : chunk);
+    for (int q = threadIdx.x; q < cnt; q += kThreads) {
         const int64_t i = base + q;
-        T x = 0;
-        if (q < cnt) {
-            if (av) {
-                x = pinv ? pinv[i] * av[i] : av[i];
-                w[i] = x;
-            } else {
-                x = w[i];
-            }
+        T x;
+        if (av) {
+            x = pinv ? pinv[i] * av[i] : av[i];
+            w[i] = x;
+        } else {
+            x = w[i];
         }
         ws[q] = x;
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int r = wid; r <= j; r += kThreads / 32) {
-        const T *vr = V + (int64_t)r * n + base;
-        T sl = 0;  // a lane's 32 products in T, then FP64 across lanes and blocks
+    if (chunk <= 128) {
+        // four threads per row: a shuffle tree over a whole warp would take
+        // more FP64 additions than the chunk has products
+        const int sub = threadIdx.x & 3;
+        for (int rb = 0; rb <= j; rb += kThreads / 4) {
+            const int r = rb + (int)(threadIdx.x >> 2);
+            T sl = 0;  // at most 32 products in T
+            if (r <= j) {
+                const T *vr = V + (int64_t)r * n + base;
 #pragma unroll 8
-        for (int q = lane; q < cnt; q += 32) sl += vr[q] * ws[q];
-        double s = (double)sl;
+                for (int q = sub; q < cnt; q += 4) sl += vr[q] * ws[q];
+            }
+            double s = (double)sl;
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            if (sub == 0 && r <= j) W.part[(int64_t)blockIdx.x * (restart + 1) + r] = s;
+        }
+    } else {
+        for (int r = wid; r <= j; r += kThreads / 32) {
+            const T *vr = V + (int64_t)r * n + base;
+            T sl = 0;  // a lane's products (at most 32) in T, then FP64 across lanes and blocks
+#pragma unroll 8
+            for (int q = lane; q < cnt; q += 32) sl += vr[q] * ws[q];
+            double s = (double)sl;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) W.part[(int64_t)blockIdx.x * (restart + 1) + r] = s;
-    }
-}
-
-// h[r] = sum of the blocks' partials (fixed order: lane-strided sums, then a
-// fixed shuffle tree); one warp per row r, one block of 32 warps
-__global__ void __launch_bounds__(1024) k_dots_fin(int nb, int j, int restart, void *work, int pass) {
-    Work W = work_view(work, restart);
-    double *h = pass == 1 ? W.h1 : W.h2;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int r = wid; r <= j; r += 32) {
-        double t = 0;
-        for (int q = lane; q < nb; q += 32) t += W.part[(int64_t)q * (restart + 1) + r];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (lane == 0) h[r] = t;
-    }
-}
-
-// w -= sum_i h[i] V_i; on the second pass also |w| -> H[j+1, j] via scal
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_sub(int64_t n, int j, int restart, const T *__restrict__ V,
-                                                  T *__restrict__ w, void *work, int pass, double *H) {
-    __shared__ double sm[32];
-    __shared__ T hs[257];
-    Work W = work_view(work, restart);
-    const double *h = pass == 1 ? W.h1 : W.h2;
-    for (int r = threadIdx.x; r <= j; r += blockDim.x) hs[r] = (T)h[r];
-    __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kChunkN;
-    T s2 = 0;
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        const int64_t i = base + (int64_t)k * kThreads + threadIdx.x;
-        if (i < n) {
-            T x = w[i];
-            for (int r = 0; r <= j; ++r) x -= hs[r] * V[(int64_t)r * n + i];
-            w[i] = x;
-            s2 += x * x;
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) W.part[(int64_t)blockIdx.x * (restart + 1) + r] = s;
         }
     }
-    if (pass == 1) return;
-    double s2d = block_sum((double)s2, sm);
-    if (threadIdx.x == 0) W.part[blockIdx.x] = s2d;
     if (!last_block(W.counter)) return;
-    double t = 0;
-    for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) t += __ldcg(&W.part[q]);
-    t = block_sum(t, sm);
-    if (threadIdx.x == 0) {
-        H[(int64_t)(j + 1) * restart + j] = sqrt(t);
-        *W.counter = 0;
+    // one thread per row and group of blocks, then the groups in order
+    __shared__ double red[kThreads];
+    double *h = pass == 1 ? W.h1 : W.h2;
+    for (int rb = 0; rb <= j; rb += kThreads) {
+        const int nr = j + 1 - rb < kThreads ? j + 1 - rb : kThreads, G = kThreads / nr;
+        const int r = threadIdx.x % nr, grp = threadIdx.x / nr;
+        double t = 0;
+        if (grp < G) {
+#pragma unroll 4
+            for (unsigned q = grp; q < gridDim.x; q += G) t += __ldcg(&W.part[(int64_t)q * (restart + 1) + rb + r]);
+        }
+        __syncthreads();
+        red[threadIdx.x] = t;
+        __syncthreads();
+        if (threadIdx.x < nr) {
+            for (int k = 1; k < G; ++k) t += red[k * nr + r];
+            h[rb + r] = t;
+        }
     }
+    if (threadIdx.x == 0) *W.counter = 0;
 }
 
-// Hessenberg column j = h1 + h2, Givens rotations, g update, residual estimate.
-// Mirrors bem_solver.py:590-616 (rotation with denom < 1e-14 -> identity).
-// The column is gathered into shared memory by the warp, rotated by one
-// thread there (a dependent chain through shared memory, not global), and
-// written back by the warp.
-__global__ void k_givens(int j, int restart, double *H, double *g, double *cs, double *sn, double *scal, void *work) {
-    __shared__ double col[258];
-    if (blockIdx.x != 0) return;
-    Work W = work_view(work, restart);
-    for (int i = threadIdx.x; i <= j; i += blockDim.x) col[i] = W.h1[i] + W.h2[i];
-    if (threadIdx.x == 0) col[j + 1] = H[(int64_t)(j + 1) * restart + j];
+// Hessenberg column j = h1 + h2 and its subdiagonal hn, Givens rotations, g
+// update, residual estimate (one warp).  Mirrors bem_solver.py:590-616 (rotation
+// with denom < 1e-14 -> identity).  The column and the earlier rotations are
+// gathered into shared memory, the column is rotated by one thread there (a
+// dependent chain), and written back by the warp.
+struct GivensMem {
+    double col[258], cs[256], sn[256];
+};
+__device__ void givens_step(int j, int restart, double hn, double *H, double *g, double *cs, double *sn, double *scal,
+                            const Work &W, GivensMem &M) {
+    const int lane = threadIdx.x;
+    for (int i = lane; i <= j; i += 32) {
+        M.col[i] = __ldcg(&W.h1[i]) + __ldcg(&W.h2[i]);
+        if (i < j) {
+            M.cs[i] = cs[i];
+            M.sn[i] = sn[i];
+        }
+    }
     __syncwarp();
-    if (threadIdx.x == 0) {
-        const double hn = col[j + 1];
+    if (lane == 0) {
         if (!(isfinite(hn) && hn > 0.0)) {
             if (scal[2] < 0) scal[2] = (double)j;
         }
+        double a = M.col[0];
         for (int i = 0; i < j; ++i) {
-            const double a = col[i], b = col[i + 1];
-            col[i] = cs[i] * a + sn[i] * b;
-            col[i + 1] = -sn[i] * a + cs[i] * b;
+            const double b = M.col[i + 1];
+            M.col[i] = M.cs[i] * a + M.sn[i] * b;
+            a = -M.sn[i] * a + M.cs[i] * b;
         }
-        const double a = col[j], b = col[j + 1];
+        const double b = hn;
         const double den = sqrt(a * a + b * b);
         double c = 1.0, s = 0.0;
         if (den >= 1e-14 && isfinite(den)) {
@@ -258,8 +259,8 @@ __global__ void k_givens(int j, int restart, double *H, double *g, double *cs, d
         }
         cs[j] = c;
         sn[j] = s;
-        col[j] = c * a + s * b;
-        col[j + 1] = 0.0;
+        M.col[j] = c * a + s * b;
+        M.col[j + 1] = 0.0;
         const double gj = g[j];
         g[j] = c * gj;
         g[j + 1] = -s * gj;
@@ -270,18 +271,83 @@ __global__ void k_givens(int j, int restart, double *H, double *g, double *cs, d
         scal[4 + restart] = hn;
     }
     __syncwarp();
-    for (int i = threadIdx.x; i <= j + 1; i += blockDim.x) H[(int64_t)i * restart + j] = col[i];
+    for (int i = lane; i <= j + 1; i += 32) H[(int64_t)i * restart + j] = M.col[i];
 }
 
-// y = R^{-1} g[0:m] (upper triangular, FP64)
-__global__ void k_trsv(int m, int restart, const double *H, const double *g, void *work) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// w -= sum_i h[i] V_i; on the second pass the last block also takes |w| and
+// finishes the step.  Chunks below 256 elements give several threads to an
+// element, each with every G-th basis vector.
+template <typename T>
+__global__ void __launch_bounds__(kThreads) k_sub(int64_t n, int j, int restart, const T *__restrict__ V,
+                                                  T *__restrict__ w, void *work, int pass, double *H, double *g,
+                                                  double *cs, double *sn, double *scal, int chunk) {
+    __shared__ double sm[32];
+    __shared__ T hs[257];
+    __shared__ T part[kThreads];
+    __shared__ GivensMem gm;
     Work W = work_view(work, restart);
+    const double *h = pass == 1 ? W.h1 : W.h2;
+    for (int r = threadIdx.x; r <= j; r += blockDim.x) hs[r] = (T)h[r];
+    __syncthreads();
+    const int64_t base = (int64_t)blockIdx.x * chunk;
+    const int G = chunk < kThreads ? kThreads / chunk : 1;
+    T s2 = 0;
+    if (G == 1) {
+        for (int q = threadIdx.x; q < chunk; q += kThreads) {
+            const int64_t i = base + q;
+            if (i < n) {
+                T x = w[i];
+#pragma unroll 4
+                for (int r = 0; r <= j; ++r) x -= hs[r] * V[(int64_t)r * n + i];
+                w[i] = x;
+                s2 += x * x;
+            }
+        }
+    } else {
+        const int q = threadIdx.x % chunk, grp = threadIdx.x / chunk;
+        const int64_t i = base + q;
+        T x = 0;
+        if (i < n) {
+#pragma unroll 4
+            for (int r = grp; r <= j; r += G) x += hs[r] * V[(int64_t)r * n + i];
+        }
+        part[threadIdx.x] = x;
+        __syncthreads();
+        if (grp == 0 && i < n) {
+            for (int k = 1; k < G; ++k) x += part[k * chunk + q];
+            x = w[i] - x;
+            w[i] = x;
+            s2 = x * x;
+        }
+    }
+    if (pass == 1) return;
+    double s2d = block_sum((double)s2, sm);
+    if (threadIdx.x == 0) W.part[blockIdx.x] = s2d;
+    if (!last_block(W.counter)) return;
+    double t = 0;
+    for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) t += __ldcg(&W.part[q]);
+    t = block_sum(t, sm);
+    if (threadIdx.x >= 32) return;
+    t = sqrt(__shfl_sync(0xffffffffu, t, 0));
+    givens_step(j, restart, t, H, g, cs, sn, scal, W, gm);
+    if (threadIdx.x == 0) *W.counter = 0;
+}
+
+// y = R^{-1} g[0:m] (upper triangular, FP64), column by column: one warp
+// subtracts column i times y_i from the rows above it, the right-hand side in
+// shared memory
+__global__ void k_trsv(int m, int restart, const double *H, const double *g, void *work) {
+    __shared__ double b[256];
+    Work W = work_view(work, restart);
+    const int lane = threadIdx.x;
+    for (int i = lane; i < m; i += 32) b[i] = g[i];
+    __syncwarp();
     for (int i = m - 1; i >= 0; --i) {
-        double s = g[i];
-        for (int k = i + 1; k < m; ++k) s -= H[(int64_t)i * restart + k] * W.y[k];
         const double d = H[(int64_t)i * restart + i];
-        W.y[i] = (d != 0.0) ? s / d : 0.0;
+        const double y = (d != 0.0) ? b[i] / d : 0.0;
+        for (int k = lane; k < i; k += 32) b[k] -= H[(int64_t)k * restart + i] * y;
+        if (lane == 0) W.y[i] = y;
+        __syncwarp();
     }
 }
 
@@ -309,7 +375,7 @@ template <typename T>
 int gmres_start(int64_t n, const void *b, const void *ax, const void *pinv, void *v0, void *g, int restart,
                 void *scal, void *work, cudaStream_t s) {
     k_start<T><<<nblocks(n), kThreads, 0, s>>>(n, (const T *)b, (const T *)ax, (const T *)pinv, (T *)v0, (double *)g,
-                                                restart, (double *)scal, work);
+                                                restart, (double *)scal, work, chunk_of(n));
     EDFMM_LAUNCH_CHECK("k_start");
     k_scale_by<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, (T *)v0, (const T *)v0, (const double *)scal, 1);
     EDFMM_LAUNCH_CHECK("k_scale_by");
@@ -320,21 +386,16 @@ template <typename T>
 int gmres_arnoldi(int64_t n, int j, int restart, void *V, const void *av, const void *pinv, void *H, void *g, void *cs,
                   void *sn, void *scal, void *w, void *work, cudaStream_t s) {
     const unsigned nb = nblocks(n);
+    const int chunk = chunk_of(n);
     T *Vt = (T *)V;
-    k_dots<T><<<nb, kThreads, 0, s>>>(n, j, restart, Vt, (T *)w, (const T *)av, (const T *)pinv, work);
-    EDFMM_LAUNCH_CHECK("k_dots");
-    k_dots_fin<<<1, 1024, 0, s>>>((int)nb, j, restart, work, 1);
-    EDFMM_LAUNCH_CHECK("k_dots_fin");
-    k_sub<T><<<nb, kThreads, 0, s>>>(n, j, restart, Vt, (T *)w, work, 1, (double *)H);
-    EDFMM_LAUNCH_CHECK("k_sub");
-    k_dots<T><<<nb, kThreads, 0, s>>>(n, j, restart, Vt, (T *)w, nullptr, nullptr, work);
-    EDFMM_LAUNCH_CHECK("k_dots");
-    k_dots_fin<<<1, 1024, 0, s>>>((int)nb, j, restart, work, 2);
-    EDFMM_LAUNCH_CHECK("k_dots_fin");
-    k_sub<T><<<nb, kThreads, 0, s>>>(n, j, restart, Vt, (T *)w, work, 2, (double *)H);
-    EDFMM_LAUNCH_CHECK("k_sub");
-    k_givens<<<1, 32, 0, s>>>(j, restart, (double *)H, (double *)g, (double *)cs, (double *)sn, (double *)scal, work);
-    EDFMM_LAUNCH_CHECK("k_givens");
+    for (int pass = 1; pass <= 2; ++pass) {
+        k_dots<T><<<nb, kThreads, 0, s>>>(n, j, restart, Vt, (T *)w, pass == 1 ? (const T *)av : nullptr,
+                                          pass == 1 ? (const T *)pinv : nullptr, work, pass, chunk);
+        EDFMM_LAUNCH_CHECK("k_dots");
+        k_sub<T><<<nb, kThreads, 0, s>>>(n, j, restart, Vt, (T *)w, work, pass, (double *)H, (double *)g, (double *)cs,
+                                         (double *)sn, (double *)scal, chunk);
+        EDFMM_LAUNCH_CHECK("k_sub");
+    }
     k_scale_by<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, Vt + (int64_t)(j + 1) * n, (const T *)w,
                                                                (const double *)scal, 4 + restart);
     EDFMM_LAUNCH_CHECK("k_scale_by");
