@@ -49,9 +49,18 @@ struct Ws {
     size_t bytes;
 };
 
-constexpr int kPartRows = 1024;  // rows per weight-gradient partial
+constexpr int kColRows = 1024;  // rows per partial column sum
 
-inline int64_t n_parts(int64_t n) { return std::max<int64_t>(1, (n + kPartRows - 1) / kPartRows); }
+inline int64_t n_col_parts(int64_t n) { return std::max<int64_t>(1, (n + kColRows - 1) / kColRows); }
+
+// Rows per weight-gradient partial: about one partial per SM, at most 1,024
+// rows (a multiple of the 64-row stage).  30,000 panels in 30 partials of 1,024
+// rows left most SMs idle: 83 us per 128-wide layer, 10 in 157 of 192.
+inline int part_rows(int64_t n) {
+    const int64_t r = (n + 151) / 152;
+    return (int)std::min<int64_t>(1024, std::max<int64_t>(64, (r + 63) / 64 * 64));
+}
+inline int64_t n_parts(int64_t n) { return std::max<int64_t>(1, (n + part_rows(n) - 1) / part_rows(n)); }
 
 Ws carve(void *base, int64_t n) {
     Ws w{};
@@ -65,10 +74,10 @@ Ws carve(void *base, int64_t n) {
     size_t a_x0 = take(n * NIN * bf), a_h1 = take(n * W * bf), a_h2 = take(n * W * bf), a_h3 = take(n * W * bf),
            a_dz = take(n * W * bf), a_dz2 = take(n * W * bf), a_w1 = take(W * NIN * bf), a_w2 = take(W * W * bf), a_w3 = take(W * W * bf),
            a_w2t = take(W * W * bf), a_w3t = take(W * W * bf), a_g = take(W * 4), a_c2 = take(W * 4), a_dc = take(W * 4),
-           a_dg = take(W * 4), a_part = take((size_t)n_parts(n) * (W * W + W) * 4), a_st = take(16 * 8);
-    w.bytes = o;
+           a_dg = take(W * 4), a_part = take(std::max((size_t)n_parts(n) * (W * W + W), (size_t)n_col_parts(n) * W) * 4), a_st = take(16 * 8);
+    w.bytes = o + 255;  // the buffers start at the base rounded up to 256 bytes
     if (base) {
-        char *b = static_cast<char *>(base);
+        char *b = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(base) + 255) & ~(uintptr_t)255);
         w.x0 = (__nv_bfloat16 *)(b + a_x0);
         w.h1 = (__nv_bfloat16 *)(b + a_h1);
         w.h2 = (__nv_bfloat16 *)(b + a_h2);
@@ -196,49 +205,85 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-
-__device__ __forceinline__ uint32_t ld32(const __nv_bfloat16 *p) { return *reinterpret_cast<const uint32_t *>(p); }
+// four 8 x 8 BF16 matrices from shared memory; lane l gives row l % 8 of matrix l / 8
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const __nv_bfloat16 *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((unsigned)__cvta_generic_to_shared(p))
+                 : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const __nv_bfloat16 *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((unsigned)__cvta_generic_to_shared(p))
+                 : "memory");
+}
+// 16 bytes to shared memory, zeros when !valid
+__device__ __forceinline__ void cp16(__nv_bfloat16 *dst, const __nv_bfloat16 *src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(valid ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
 
 enum Epi { EPI_RELU = 0, EPI_MASK = 1 };
 
-// One warp computes 16 rows x 128 columns.  Wt (128 x K, K contiguous) is
-// staged in shared memory with a padded row stride (conflict-free fragment
-// loads).  EPI_RELU: out = relu(acc + bias[n]) and optionally y = w4 . out + b4;
-// EPI_MASK: out = mask[r][n] > 0 ? acc + bias[n] : 0 (ReLU backward).
+constexpr int kLinRows = 128;  // rows per block, 16 per warp
+
+// One warp computes 16 rows x 128 columns.  Wt (128 x K, K contiguous) and the
+// block's rows of X are copied to shared memory 16 bytes at a time (padded
+// rows: conflict-free ldmatrix), the results go back through the warp's rows of
+// X.  EPI_RELU: out = relu(acc + bias[n]) and optionally y = w4 . out + b4;
+// EPI_MASK: out = mask[r][n] > 0 ? acc + bias[n] : 0 (ReLU backward).  30,000
+// rows of 128: 13 to 18 us with 4-byte loads of every fragment, 8 to 13 now (8
+// MB in, 8 MB out).
+template <int K> constexpr size_t lin_smem() { return (size_t)(W + kLinRows) * (K + 8) * sizeof(__nv_bfloat16); }
+template <int K> constexpr size_t lin_smem_out() {  // the output rows take over the staging area
+    return std::max(lin_smem<K>(), (size_t)kLinRows * (W + 8) * sizeof(__nv_bfloat16));
+}
+
 template <int K, int EPI, bool HEAD>
-__global__ void __launch_bounds__(128) k_pcn_linear(const __nv_bfloat16 *__restrict__ X, const __nv_bfloat16 *__restrict__ Wt,
+__global__ void __launch_bounds__(256) k_pcn_linear(const __nv_bfloat16 *__restrict__ X, const __nv_bfloat16 *__restrict__ Wt,
                                                     const float *__restrict__ bias, const __nv_bfloat16 *__restrict__ mask,
                                                     int64_t n, __nv_bfloat16 *__restrict__ out,
                                                     const float *__restrict__ prm, float *__restrict__ y) {
-    constexpr int LD = K + 8;  // padded row stride (bf16 elements)
-    __shared__ __align__(16) __nv_bfloat16 sw[W * LD];
-    for (int i = threadIdx.x; i < W * K / 2; i += blockDim.x) {
-        const int r = (2 * i) / K, c = (2 * i) % K;
-        *reinterpret_cast<uint32_t *>(&sw[r * LD + c]) = ld32(Wt + 2 * i);
+    constexpr int LD = K + 8, LO = W + 8;  // padded row strides (bf16 elements)
+    extern __shared__ __align__(16) __nv_bfloat16 lin_sm[];
+    __nv_bfloat16 *sw = lin_sm, *sx = lin_sm + W * LD;
+    const int64_t b0r = (int64_t)blockIdx.x * kLinRows;
+    for (int i = threadIdx.x; i < W * K / 8; i += 256) cp16(sw + (i / (K / 8)) * LD + (i % (K / 8)) * 8, Wt + 8 * i, true);
+    for (int i = threadIdx.x; i < kLinRows * K / 8; i += 256) {
+        const int r = i / (K / 8), c = (i % (K / 8)) * 8;
+        const bool ok = b0r + r < n;
+        cp16(sx + r * LD + c, X + (ok ? (b0r + r) * K + c : 0), ok);
     }
+    cp_wait();
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int64_t r0 = ((int64_t)blockIdx.x * 4 + warp) * 16;
-    if (r0 >= n) return;
+    const int64_t r0 = b0r + warp * 16;
     const int64_t ra = r0 + g, rb = r0 + g + 8;
     const bool va = ra < n, vb = rb < n;
     float acc[16][4];
 #pragma unroll
     for (int j = 0; j < 16; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+    const int lr = lane & 7, lm = lane >> 3;
 #pragma unroll
     for (int k0 = 0; k0 < K; k0 += 16) {
-        uint32_t a[4];
-        a[0] = va ? ld32(X + ra * K + k0 + 2 * t) : 0u;
-        a[1] = vb ? ld32(X + rb * K + k0 + 2 * t) : 0u;
-        a[2] = va ? ld32(X + ra * K + k0 + 2 * t + 8) : 0u;
-        a[3] = vb ? ld32(X + rb * K + k0 + 2 * t + 8) : 0u;
+        uint32_t a[4];  // (rows 0-7, k 0-7), (8-15, 0-7), (0-7, 8-15), (8-15, 8-15)
+        ldsm4(a, sx + (warp * 16 + (lm & 1) * 8 + lr) * LD + k0 + (lm >> 1) * 8);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const __nv_bfloat16 *wr = sw + (8 * j + g) * LD + k0 + 2 * t;
-            mma_bf16(acc[j], a, ld32(wr), ld32(wr + 8));
+        for (int j = 0; j < 16; j += 2) {
+            uint32_t b[4];  // column tiles j, j + 1, k halves 0, 1 of each
+            ldsm4(b, sw + (8 * (j + (lm >> 1)) + lr) * LD + k0 + (lm & 1) * 8);
+            mma_bf16(acc[j], a, b[0], b[1]);
+            mma_bf16(acc[j + 1], a, b[2], b[3]);
         }
     }
+    __syncthreads();  // the output rows overlay W and X
+    __nv_bfloat16 *so = lin_sm + warp * 16 * LO;
     float ya = 0.0f, yb = 0.0f;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
@@ -261,13 +306,20 @@ __global__ void __launch_bounds__(128) k_pcn_linear(const __nv_bfloat16 *__restr
             }
         }
         const __nv_bfloat162 oa = __floats2bfloat162_rn(v[0], v[1]), ob = __floats2bfloat162_rn(v[2], v[3]);
-        if (va) *reinterpret_cast<__nv_bfloat162 *>(out + ra * W + col) = oa;
-        if (vb) *reinterpret_cast<__nv_bfloat162 *>(out + rb * W + col) = ob;
+        *reinterpret_cast<__nv_bfloat162 *>(so + g * LO + col) = oa;
+        *reinterpret_cast<__nv_bfloat162 *>(so + (g + 8) * LO + col) = ob;
         if (HEAD) {  // the head reads the stored (BF16-rounded) activations
             const float w0 = prm[O_W4 + col], w1 = prm[O_W4 + col + 1];
             ya += __bfloat162float(oa.x) * w0 + __bfloat162float(oa.y) * w1;
             yb += __bfloat162float(ob.x) * w0 + __bfloat162float(ob.y) * w1;
         }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {  // 16 rows of 256 bytes, two rows per step
+        const int r = 2 * i + (lane >> 4), c = (lane & 15) * 8;
+        if (r0 + r < n)
+            *reinterpret_cast<uint4 *>(out + (r0 + r) * W + c) = *reinterpret_cast<const uint4 *>(so + r * LO + c);
     }
     if (HEAD) {
 #pragma unroll
@@ -283,20 +335,52 @@ __global__ void __launch_bounds__(128) k_pcn_linear(const __nv_bfloat16 *__restr
     }
 }
 
+template <int K, int EPI, bool HEAD>
+int launch_linear(const __nv_bfloat16 *X, const __nv_bfloat16 *Wt, const float *bias, const __nv_bfloat16 *mask,
+                  int64_t n, __nv_bfloat16 *out, const float *prm, float *y, cudaStream_t s) {
+    constexpr size_t smem = lin_smem_out<K>();
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(k_pcn_linear<K, EPI, HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (attr != cudaSuccess)
+        return fail(EDFMM_ERR_CUDA, std::string("k_pcn_linear shared memory: ") + cudaGetErrorString(attr));
+    k_pcn_linear<K, EPI, HEAD><<<nblk(n, kLinRows), 256, smem, s>>>(X, Wt, bias, mask, n, out, prm, y);
+    EDFMM_LAUNCH_CHECK("k_pcn_linear");
+    return EDFMM_OK;
+}
+
 // ---------------------------------------------------------------------------
 // context: g = mean_i h1_i;  c2 = V2 g + b2
 // ---------------------------------------------------------------------------
-// per-part column sums of a BF16 (n x 128) matrix, optionally weighted by w[r]
-__global__ void __launch_bounds__(W) k_pcn_colsum_part(const __nv_bfloat16 *__restrict__ h, const float *__restrict__ w,
-                                                       int64_t n, float *__restrict__ part) {
+// per-part column sums of a BF16 (n x 128) matrix, optionally weighted by w[r],
+// in row order.  Stages of 128 rows are copied to shared memory by the whole
+// block, and one thread per column adds them: its chain of additions is the
+// same as over device memory, without a load's latency in every few links
+// (30,000 rows: 36 -> 12 us).
+constexpr int kColStage = 128;
+__global__ void __launch_bounds__(512) k_pcn_colsum_part(const __nv_bfloat16 *__restrict__ h, const float *__restrict__ w,
+                                                         int64_t n, float *__restrict__ part) {
+    __shared__ __align__(16) __nv_bfloat16 t[kColStage * W];
+    __shared__ float tw[kColStage];
     const int c = threadIdx.x;
-    const int64_t r0 = (int64_t)blockIdx.x * kPartRows, r1 = (n < r0 + kPartRows) ? n : r0 + kPartRows;
+    const int64_t r0 = (int64_t)blockIdx.x * kColRows, r1 = (n < r0 + kColRows) ? n : r0 + kColRows;
     float s = 0.0f;
-    for (int64_t r = r0; r < r1; ++r) {
-        const float v = __bfloat162float(h[r * W + c]);
-        s += w ? w[r] * v : v;
+    for (int64_t rt = r0; rt < r1; rt += kColStage) {
+        const int rows = (int)(r1 - rt < kColStage ? r1 - rt : kColStage);
+        __syncthreads();
+        for (int i = threadIdx.x; i < rows * (W / 8); i += 512) cp16(t + 8 * i, h + rt * W + 8 * i, true);
+        if (w)
+            for (int i = threadIdx.x; i < rows; i += 512) tw[i] = w[rt + i];
+        cp_wait();
+        __syncthreads();
+        if (c < W) {
+#pragma unroll 16
+            for (int r = 0; r < rows; ++r) {
+                const float v = __bfloat162float(t[r * W + c]);
+                s += w ? tw[r] * v : v;
+            }
+        }
     }
-    part[(int64_t)blockIdx.x * W + c] = s;
+    if (c < W) part[(int64_t)blockIdx.x * W + c] = s;
 }
 
 // out[c] = scale * sum_p part[p][c]  (fixed order)
@@ -312,6 +396,7 @@ __global__ void __launch_bounds__(W) k_pcn_context(const float *__restrict__ prm
                                                    float *__restrict__ c2) {
     const int r = threadIdx.x;
     float s = prm[O_B2 + r];
+#pragma unroll 32
     for (int k = 0; k < W; ++k) s += prm[O_V2 + r * W + k] * g[k];
     c2[r] = s;
 }
@@ -319,87 +404,85 @@ __global__ void __launch_bounds__(W) k_pcn_context(const float *__restrict__ prm
 // ---------------------------------------------------------------------------
 // backward
 // ---------------------------------------------------------------------------
-// dz3[r][c] = (h3 > 0) ? dy[r] w4[c] : 0
+// dz3[r][c] = (h3 > 0) ? dy[r] w4[c] : 0, eight columns (16 bytes) per thread
 __global__ void k_pcn_head_grad(const __nv_bfloat16 *__restrict__ h3, const float *__restrict__ dy,
                                 const float *__restrict__ prm, int64_t n, __nv_bfloat16 *__restrict__ dz) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n * W) return;
-    const int64_t r = i / W;
-    const int c = (int)(i % W);
-    const float v = __bfloat162float(h3[i]) > 0.0f ? dy[r] * prm[O_W4 + c] : 0.0f;
-    dz[i] = __float2bfloat16_rn(v);
+    if (i >= n * (W / 8)) return;
+    const int c = (int)(i % (W / 8)) * 8;
+    const float d = dy[i / (W / 8)];
+    uint4 in = reinterpret_cast<const uint4 *>(h3)[i], o;
+    const __nv_bfloat162 *x = reinterpret_cast<const __nv_bfloat162 *>(&in);
+    __nv_bfloat162 *z = reinterpret_cast<__nv_bfloat162 *>(&o);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        z[q] = __floats2bfloat162_rn(__bfloat162float(x[q].x) > 0.0f ? d * prm[O_W4 + c + 2 * q] : 0.0f,
+                                     __bfloat162float(x[q].y) > 0.0f ? d * prm[O_W4 + c + 2 * q + 1] : 0.0f);
+    reinterpret_cast<uint4 *>(dz)[i] = o;
 }
 
 // partial weight gradients over a block of rows, on the tensor cores:
 //   part[p][o][k] = sum_{r in block p} D[r][o] X[r][k]     (o < 128, k < K)
 //   part[p][128*K + o] = sum_r D[r][o]                   (bias gradient)
-// The product D^T X has the rows r as its reduction dimension, so each stage
-// of RT rows is staged transposed in shared memory (Dt[o][r], Xt[k][r], padded
-// rows: conflict-free fragment loads) and warp w computes output rows
-// 16w..16w+15 against all K columns with mma.sync m16n8k16 (BF16 in, FP32
-// accumulate; the order of the additions is fixed, so the sums are
-// deterministic).  The bias sums run on the FP32 pipe in row order.
+// The product D^T X has the rows r as its reduction dimension: stages of 64
+// rows are copied to shared memory as they are (16 bytes at a time, padded
+// rows, rows past the end zero) and ldmatrix transposes the fragments of both
+// operands.  Warp w computes output rows 16w..16w+15 against all K columns
+// (mma.sync m16n8k16, BF16 in, FP32 accumulate; fixed order).  The bias sums
+// run on the FP32 pipe in row order.
+constexpr int kWgStage = 64;
 template <int K>
 __global__ void __launch_bounds__(256) k_pcn_wgrad_part(const __nv_bfloat16 *__restrict__ D,
-                                                        const __nv_bfloat16 *__restrict__ X, int64_t n,
+                                                        const __nv_bfloat16 *__restrict__ X, int64_t n, int rows_part,
                                                         float *__restrict__ part) {
-    constexpr int RT = 32;       // rows per stage (two MMA k-steps)
-    constexpr int LD = RT + 8;   // padded row stride of the transposed tiles (bf16 elements)
-    constexpr int NT = K / 8;    // n-tiles of 8 columns
-    __shared__ __align__(16) __nv_bfloat16 Dt[W * LD];
-    __shared__ __align__(16) __nv_bfloat16 Xt[K * LD];
+    constexpr int LDD = W + 8, LDX = K + 8;  // padded row strides (bf16 elements)
+    constexpr int NT = K / 8;                // n-tiles of 8 columns
+    __shared__ __align__(16) __nv_bfloat16 Dt[kWgStage * LDD];
+    __shared__ __align__(16) __nv_bfloat16 Xt[kWgStage * LDX];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g = lane >> 2, t = lane & 3;
+    const int g = lane >> 2, t = lane & 3, lr = lane & 7, lm = lane >> 3;
     const int o0 = 16 * warp;
     float acc[NT][4];
 #pragma unroll
     for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
     float bsum = 0.0f;
-    const int64_t r0 = (int64_t)blockIdx.x * kPartRows, r1 = (n < r0 + kPartRows) ? n : r0 + kPartRows;
-    for (int64_t rt = r0; rt < r1; rt += RT) {
-        const int rows = (int)((r1 - rt < RT) ? r1 - rt : RT);
+    const int64_t r0 = (int64_t)blockIdx.x * rows_part, r1 = (n < r0 + rows_part) ? n : r0 + rows_part;
+    for (int64_t rt = r0; rt < r1; rt += kWgStage) {
+        const int rows = (int)((r1 - rt < kWgStage) ? r1 - rt : kWgStage);
         __syncthreads();
-        // transpose RT x 128 of D and RT x K of X into Dt / Xt (pairs of
-        // columns per 32-bit global load; rows past the end are zeros)
-        for (int i = tid; i < RT * (W / 2); i += 256) {
-            const int r = i / (W / 2), c = 2 * (i % (W / 2));
-            __nv_bfloat162 v = __floats2bfloat162_rn(0.0f, 0.0f);
-            if (r < rows) v = *reinterpret_cast<const __nv_bfloat162 *>(D + (rt + r) * W + c);
-            Dt[c * LD + r] = v.x;
-            Dt[(c + 1) * LD + r] = v.y;
+        for (int i = tid; i < kWgStage * (W / 8); i += 256) {
+            const int r = i / (W / 8), c = (i % (W / 8)) * 8;
+            cp16(Dt + r * LDD + c, D + (r < rows ? (rt + r) * W + c : 0), r < rows);
         }
-        for (int i = tid; i < RT * (K / 2); i += 256) {
-            const int r = i / (K / 2), c = 2 * (i % (K / 2));
-            __nv_bfloat162 v = __floats2bfloat162_rn(0.0f, 0.0f);
-            if (r < rows) v = *reinterpret_cast<const __nv_bfloat162 *>(X + (rt + r) * K + c);
-            Xt[c * LD + r] = v.x;
-            Xt[(c + 1) * LD + r] = v.y;
+        for (int i = tid; i < kWgStage * (K / 8); i += 256) {
+            const int r = i / (K / 8), c = (i % (K / 8)) * 8;
+            cp16(Xt + r * LDX + c, X + (r < rows ? (rt + r) * K + c : 0), r < rows);
         }
+        cp_wait();
         __syncthreads();
 #pragma unroll
-        for (int k0 = 0; k0 < RT; k0 += 16) {
-            uint32_t a[4];
-            a[0] = ld32(Dt + (o0 + g) * LD + k0 + 2 * t);
-            a[1] = ld32(Dt + (o0 + g + 8) * LD + k0 + 2 * t);
-            a[2] = ld32(Dt + (o0 + g) * LD + k0 + 2 * t + 8);
-            a[3] = ld32(Dt + (o0 + g + 8) * LD + k0 + 2 * t + 8);
+        for (int k0 = 0; k0 < kWgStage; k0 += 16) {
+            uint32_t a[4];  // (o 0-7, r 0-7), (o 8-15, r 0-7), (o 0-7, r 8-15), (o 8-15, r 8-15)
+            ldsm4t(a, Dt + (k0 + (lm >> 1) * 8 + lr) * LDD + o0 + (lm & 1) * 8);
 #pragma unroll
-            for (int j = 0; j < NT; ++j) {
-                const __nv_bfloat16 *xr = Xt + (8 * j + g) * LD + k0 + 2 * t;
-                mma_bf16(acc[j], a, ld32(xr), ld32(xr + 8));
+            for (int j = 0; j < NT; j += 2) {
+                uint32_t b[4];  // column tiles j, j + 1, row halves 0, 1 of each
+                ldsm4t(b, Xt + (k0 + (lm & 1) * 8 + lr) * LDX + 8 * (j + (lm >> 1)));
+                mma_bf16(acc[j], a, b[0], b[1]);
+                mma_bf16(acc[j + 1], a, b[2], b[3]);
             }
         }
-        if (tid < W)
-            for (int r = 0; r < rows; ++r) bsum += __bfloat162float(Dt[tid * LD + r]);
+        if (tid < W) {
+#pragma unroll 16
+            for (int r = 0; r < rows; ++r) bsum += __bfloat162float(Dt[r * LDD + tid]);
+        }
     }
     float *pp = part + (int64_t)blockIdx.x * (W * K + W);
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
         const int col = 8 * j + 2 * t;
-        pp[(o0 + g) * K + col] = acc[j][0];
-        pp[(o0 + g) * K + col + 1] = acc[j][1];
-        pp[(o0 + g + 8) * K + col] = acc[j][2];
-        pp[(o0 + g + 8) * K + col + 1] = acc[j][3];
+        *reinterpret_cast<float2 *>(pp + (o0 + g) * K + col) = make_float2(acc[j][0], acc[j][1]);
+        *reinterpret_cast<float2 *>(pp + (o0 + g + 8) * K + col) = make_float2(acc[j][2], acc[j][3]);
     }
     if (tid < W) pp[W * K + tid] = bsum;
 }
@@ -411,6 +494,7 @@ __global__ void k_pcn_wgrad_reduce(const float *__restrict__ part, int64_t np, i
     const int stride = W * K + W;
     if (i >= stride) return;
     float s = 0.0f;
+#pragma unroll 16
     for (int64_t p = 0; p < np; ++p) s += part[p * stride + i];
     if (i < W * K)
         grads[off + i] = s;
@@ -433,28 +517,38 @@ __global__ void __launch_bounds__(256) k_pcn_sum(const float *__restrict__ v, in
     }
 }
 
-// context backward: dV2 = dc2 g^T, db2 = dc2, dg = V2^T dc2 / n  (dc2 = column sum of dz2)
+// context backward: dV2 = dc2 g^T, db2 = dc2, dg = V2^T dc2 / n  (dc2 = column
+// sum of dz2); block r < 128 writes row r of dV2, block 128 dg
 __global__ void __launch_bounds__(W) k_pcn_context_grad(const float *__restrict__ prm, const float *__restrict__ g,
                                                         const float *__restrict__ dc, int64_t n, float *__restrict__ grads,
                                                         float *__restrict__ dg) {
-    const int r = threadIdx.x;
-    for (int k = 0; k < W; ++k) grads[O_V2 + r * W + k] = dc[r] * g[k];
+    const int k = threadIdx.x, r = blockIdx.x;
+    if (r < W) {
+        grads[O_V2 + r * W + k] = dc[r] * g[k];
+        return;
+    }
     float s = 0.0f;
-    for (int o = 0; o < W; ++o) s += prm[O_V2 + o * W + r] * dc[o];
-    dg[r] = s / (float)(n > 0 ? n : 1);
+#pragma unroll 32
+    for (int o = 0; o < W; ++o) s += prm[O_V2 + o * W + k] * dc[o];
+    dg[k] = s / (float)(n > 0 ? n : 1);
 }
 
 // ---------------------------------------------------------------------------
-// loss: L = sum A (s (1 + y) - sigma)^2 / sum A sigma^2, dL/dy
+// loss: L = sum A (s (1 + y) - sigma)^2 / sum A sigma^2, dL/dy.  One cluster of
+// eight blocks: dL/dy needs the whole denominator, and the blocks exchange
+// their sums through distributed shared memory (added in block order), so the
+// call needs no scratch.  30,000 panels: one block took 189 us, the cluster
+// 24.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) k_pcn_loss(const float *__restrict__ y, const double *__restrict__ s,
-                                                   const double *__restrict__ sigma, const double *__restrict__ a,
-                                                   int64_t n, float *__restrict__ dy, double *__restrict__ loss) {
+constexpr int kLossBlocks = 8;
+__global__ void __cluster_dims__(kLossBlocks, 1, 1) __launch_bounds__(1024)
+    k_pcn_loss(const float *__restrict__ y, const double *__restrict__ s, const double *__restrict__ sigma,
+               const double *__restrict__ a, int64_t n, float *__restrict__ dy, double *__restrict__ loss) {
     __shared__ double red[2][32];
-    __shared__ double den_s;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    __shared__ double sums[2], inv_s;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, rank = blockIdx.x;
     double num = 0, den = 0;
-    for (int64_t i = tid; i < n; i += blockDim.x) {
+    for (int64_t i = rank * 1024 + tid; i < n; i += kLossBlocks * 1024) {
         const double e = s[i] * (1.0 + (double)y[i]) - sigma[i];
         num += a[i] * e * e;
         den += a[i] * sigma[i] * sigma[i];
@@ -468,20 +562,37 @@ __global__ void __launch_bounds__(1024) k_pcn_loss(const float *__restrict__ y, 
         red[1][wid] = den;
     }
     __syncthreads();
-    if (tid == 0) {
-        double tn = 0, td = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-            tn += red[0][w];
-            td += red[1][w];
-        }
-        den_s = td > 0 ? td : 1.0;
-        *loss = tn / den_s;
+    if (tid < 2) {
+        double t = 0;
+        for (int w = 0; w < 32; ++w) t += red[tid][w];
+        sums[tid] = t;
     }
-    __syncthreads();
-    const double d = den_s;
-    for (int64_t i = tid; i < n; i += blockDim.x) {
+    auto cluster_sync = [] {
+        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    };
+    cluster_sync();
+    if (tid == 0) {
+        double t[2] = {0, 0};
+        for (int r = 0; r < kLossBlocks; ++r) {
+            for (int q = 0; q < 2; ++q) {
+                unsigned at;
+                double v;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                             : "=r"(at)
+                             : "r"((unsigned)__cvta_generic_to_shared(&sums[q])), "r"(r));
+                asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(at) : "memory");
+                t[q] += v;
+            }
+        }
+        const double d = t[1] > 0 ? t[1] : 1.0;
+        if (rank == 0) *loss = t[0] / d;
+        inv_s = 2.0 / d;
+    }
+    cluster_sync();  // the sums have been read (and the block sees inv_s)
+    const double f = inv_s;
+    for (int64_t i = rank * 1024 + tid; i < n; i += kLossBlocks * 1024) {
         const double e = s[i] * (1.0 + (double)y[i]) - sigma[i];
-        dy[i] = (float)(2.0 * a[i] * e * s[i] / d);
+        dy[i] = (float)(a[i] * e * s[i] * f);
     }
 }
 
@@ -539,27 +650,21 @@ extern "C" EDFMM_API int edfmm_pcn_forward(const float *params_dev, const float 
     Ws w = carve(ws_dev, n);
     if (ws_bytes < w.bytes) return fail(EDFMM_ERR_ARG, "edfmm_pcn_forward: workspace too small");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int64_t np = n_parts(n);
+    const int64_t np = n_col_parts(n);
     k_pcn_cast<<<nblk(W * W, 256), 256, 0, s>>>(params_dev, w.w1b, w.w2b, w.w3b, w.w2t, w.w3t);
     EDFMM_LAUNCH_CHECK("k_pcn_cast");
     k_pcn_cast_x<<<nblk(n * NIN, 256), 256, 0, s>>>(features_dev, n, w.x0);
     EDFMM_LAUNCH_CHECK("k_pcn_cast_x");
-    const unsigned grid = nblk(n, 64);
-    k_pcn_linear<NIN, EPI_RELU, false><<<grid, 128, 0, s>>>(w.x0, w.w1b, params_dev + O_B1, nullptr, n, w.h1, params_dev,
-                                                             nullptr);
-    EDFMM_LAUNCH_CHECK("k_pcn_linear");
-    k_pcn_colsum_part<<<(unsigned)np, W, 0, s>>>(w.h1, nullptr, n, w.part);
+    if (int rc = launch_linear<NIN, EPI_RELU, false>(w.x0, w.w1b, params_dev + O_B1, nullptr, n, w.h1, params_dev, nullptr, s))
+        return rc;
+    k_pcn_colsum_part<<<(unsigned)np, 512, 0, s>>>(w.h1, nullptr, n, w.part);
     EDFMM_LAUNCH_CHECK("k_pcn_colsum_part");
     k_pcn_reduce_cols<<<1, W, 0, s>>>(w.part, np, 1.0f / (float)n, w.g);
     EDFMM_LAUNCH_CHECK("k_pcn_reduce_cols");
     k_pcn_context<<<1, W, 0, s>>>(params_dev, w.g, w.c2);
     EDFMM_LAUNCH_CHECK("k_pcn_context");
-    k_pcn_linear<W, EPI_RELU, false><<<grid, 128, 0, s>>>(w.h1, w.w2b, w.c2, nullptr, n, w.h2, params_dev, nullptr);
-    EDFMM_LAUNCH_CHECK("k_pcn_linear");
-    k_pcn_linear<W, EPI_RELU, true><<<grid, 128, 0, s>>>(w.h2, w.w3b, params_dev + O_B3, nullptr, n, w.h3, params_dev,
-                                                          y_dev);
-    EDFMM_LAUNCH_CHECK("k_pcn_linear");
-    return EDFMM_OK;
+    if (int rc = launch_linear<W, EPI_RELU, false>(w.h1, w.w2b, w.c2, nullptr, n, w.h2, params_dev, nullptr, s)) return rc;
+    return launch_linear<W, EPI_RELU, true>(w.h2, w.w3b, params_dev + O_B3, nullptr, n, w.h3, params_dev, y_dev, s);
 }
 
 extern "C" EDFMM_API int edfmm_pcn_backward(const float *params_dev, int64_t n, const float *dy_dev, float *grads_dev,
@@ -569,35 +674,33 @@ extern "C" EDFMM_API int edfmm_pcn_backward(const float *params_dev, int64_t n, 
     Ws w = carve(ws_dev, n);
     if (ws_bytes < w.bytes) return fail(EDFMM_ERR_ARG, "edfmm_pcn_backward: workspace too small");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int64_t np = n_parts(n);
-    const unsigned grid = nblk(n, 64);
+    const int64_t np = n_parts(n), nc = n_col_parts(n);
+    const int pr = part_rows(n);
     // head: dw4 = sum_r dy_r h3_r, db4 = sum dy
-    k_pcn_colsum_part<<<(unsigned)np, W, 0, s>>>(w.h3, dy_dev, n, w.part);
+    k_pcn_colsum_part<<<(unsigned)nc, 512, 0, s>>>(w.h3, dy_dev, n, w.part);
     EDFMM_LAUNCH_CHECK("k_pcn_colsum_part");
-    k_pcn_reduce_cols<<<1, W, 0, s>>>(w.part, np, 1.0f, grads_dev + O_W4);
+    k_pcn_reduce_cols<<<1, W, 0, s>>>(w.part, nc, 1.0f, grads_dev + O_W4);
     EDFMM_LAUNCH_CHECK("k_pcn_reduce_cols");
     k_pcn_sum<<<1, 256, 0, s>>>(dy_dev, n, grads_dev + O_B4);
     EDFMM_LAUNCH_CHECK("k_pcn_sum");
     // layer 3: dz3 = (h3 > 0) dy w4;  dW3 = dz3^T h2;  dz2 = (h2 > 0) dz3 W3
-    k_pcn_head_grad<<<nblk(n * W, 256), 256, 0, s>>>(w.h3, dy_dev, params_dev, n, w.dz);
+    k_pcn_head_grad<<<nblk(n * (W / 8), 256), 256, 0, s>>>(w.h3, dy_dev, params_dev, n, w.dz);
     EDFMM_LAUNCH_CHECK("k_pcn_head_grad");
-    k_pcn_wgrad_part<W><<<(unsigned)np, 256, 0, s>>>(w.dz, w.h2, n, w.part);
+    k_pcn_wgrad_part<W><<<(unsigned)np, 256, 0, s>>>(w.dz, w.h2, n, pr, w.part);
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_part");
     k_pcn_wgrad_reduce<<<nblk(W * W + W, 256), 256, 0, s>>>(w.part, np, W, grads_dev, O_W3, O_B3);
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_reduce");
-    k_pcn_linear<W, EPI_MASK, false><<<grid, 128, 0, s>>>(w.dz, w.w3t, nullptr, w.h2, n, w.dz2, params_dev, nullptr);
-    EDFMM_LAUNCH_CHECK("k_pcn_linear");
+    if (int rc = launch_linear<W, EPI_MASK, false>(w.dz, w.w3t, nullptr, w.h2, n, w.dz2, params_dev, nullptr, s)) return rc;
     // layer 2: dW2 = dz2^T h1, dc2 = colsum(dz2) -> dV2, db2, dg
-    k_pcn_wgrad_part<W><<<(unsigned)np, 256, 0, s>>>(w.dz2, w.h1, n, w.part);
+    k_pcn_wgrad_part<W><<<(unsigned)np, 256, 0, s>>>(w.dz2, w.h1, n, pr, w.part);
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_part");
     k_pcn_wgrad_reduce<<<nblk(W * W + W, 256), 256, 0, s>>>(w.part, np, W, grads_dev, O_W2, O_B2);
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_reduce");
-    k_pcn_context_grad<<<1, W, 0, s>>>(params_dev, w.g, grads_dev + O_B2, n, grads_dev, w.dg);
+    k_pcn_context_grad<<<W + 1, W, 0, s>>>(params_dev, w.g, grads_dev + O_B2, n, grads_dev, w.dg);
     EDFMM_LAUNCH_CHECK("k_pcn_context_grad");
     // layer 1: dz1 = (h1 > 0) (dz2 W2 + dg / n);  dW1 = dz1^T x0
-    k_pcn_linear<W, EPI_MASK, false><<<grid, 128, 0, s>>>(w.dz2, w.w2t, w.dg, w.h1, n, w.dz, params_dev, nullptr);
-    EDFMM_LAUNCH_CHECK("k_pcn_linear");
-    k_pcn_wgrad_part<NIN><<<(unsigned)np, 256, 0, s>>>(w.dz, w.x0, n, w.part);
+    if (int rc = launch_linear<W, EPI_MASK, false>(w.dz2, w.w2t, w.dg, w.h1, n, w.dz, params_dev, nullptr, s)) return rc;
+    k_pcn_wgrad_part<NIN><<<(unsigned)np, 256, 0, s>>>(w.dz, w.x0, n, pr, w.part);
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_part");
     k_pcn_wgrad_reduce<<<nblk(W * NIN + W, 256), 256, 0, s>>>(w.part, np, NIN, grads_dev, O_W1, O_B1);
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_reduce");
@@ -609,7 +712,7 @@ extern "C" EDFMM_API int edfmm_pcn_loss(const float *y_dev, const double *scale_
                                         void *stream) {
     if (n <= 0 || !y_dev || !scale_dev || !sigma_dev || !areas_dev || !dy_dev || !loss_dev)
         return fail(EDFMM_ERR_ARG, "edfmm_pcn_loss: bad arguments");
-    k_pcn_loss<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(y_dev, scale_dev, sigma_dev, areas_dev, n, dy_dev,
+    k_pcn_loss<<<kLossBlocks, 1024, 0, static_cast<cudaStream_t>(stream)>>>(y_dev, scale_dev, sigma_dev, areas_dev, n, dy_dev,
                                                                    loss_dev);
     EDFMM_LAUNCH_CHECK("k_pcn_loss");
     return EDFMM_OK;
