@@ -140,6 +140,7 @@ def _declare(L):
         "edfmm_near_rows": (i32, [_vp, C.POINTER(_vp), C.POINTER(_vp)]),
         "edfmm_near_quadrature_matvec": (i32, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, i64, dbl, i32, i32, _vp, _vp]),
         "edfmm_point_charge_potential": (i32, [_vp, i64, _vp, i32, dbl, i32, _vp, _vp]),
+        "edfmm_point_charges_add": (i32, [_vp, i64, C.POINTER(dbl), i32, dbl, i32, i32, _vp, _vp, _vp]),
         "edfmm_gmres_work_bytes": (C.c_size_t, [i64, i32]),
         "edfmm_gmres_start": (i32, [i64, i32, i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
         "edfmm_gmres_arnoldi": (i32, [i64, i32, i32, i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),

@@ -29,7 +29,7 @@ from torch import Tensor
 from .. import _lib
 from ..utils.config import K_E, BEMConfig
 from .bem_mesh import TriMesh, generate_mesh
-from .bem_near import (NearCorrection, field_at_targets, near_potential_correction, point_charge_field,
+from .bem_near import (NearCorrection, add_point_charges, field_at_targets, near_potential_correction,
                        point_charge_potential, potential_at_targets, self_integrals)
 from .bem_solver import gmres_batched, gmres_restart
 from .operators import DenseOperator, FmmOperator
@@ -162,7 +162,7 @@ class BEMSolution:
                                           distance_factor=self.near_quad_dist_factor,
                                           quad_order=self.near_quad_order, max_depth=self.near_quad_max_depth)
         if self.charges:
-            v = v + point_charge_potential(pts, self.charges)
+            add_point_charges(pts, self.charges, V=v)
         return v
 
     def eval_V_E_batched(self, points: Tensor) -> Tuple[Tensor, Tensor]:
@@ -173,7 +173,7 @@ class BEMSolution:
         v = self.eval(pts)
         e = field_at_targets(pts, self.centroids, self.sigma, self.areas)
         if self.charges:
-            e = e + point_charge_field(pts, self.charges)
+            add_point_charges(pts, self.charges, E=e)
         return v, e
 
 

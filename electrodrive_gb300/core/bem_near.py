@@ -162,17 +162,26 @@ def apply_near_quadrature_matvec_cuda(V_far: Tensor, sigma: Tensor, *, centroids
     return out
 
 
+def add_point_charges(points: Tensor, charges, *, V: Optional[Tensor] = None, E: Optional[Tensor] = None,
+                      overwrite: bool = False, k_e: float = K_E) -> None:
+    """V += sum_k k_e q_k / max(|x - r_k|, 1e-12) and E += the charges' field at
+    CUDA points, in place (``overwrite``: V is written instead)."""
+    L = _lib.load_library()
+    rows = [float(v) for q, pos in charges for v in (q, *pos)]
+    n_ch = len(rows) // 4
+    ch = (C.c_double * max(len(rows), 1))(*rows)
+    pts = points.contiguous()
+    with torch.cuda.device(points.device):
+        _lib.check(L.edfmm_point_charges_add(_lib.ptr(pts), points.shape[0], ch, n_ch, float(k_e),
+                                             _lib.dtype_code(points.dtype), 1 if overwrite else 0, _lib.ptr(V),
+                                             _lib.ptr(E), _lib.stream_handle(points.device)),
+                   "edfmm_point_charges_add")
+
+
 def point_charge_potential(points: Tensor, charges, *, k_e: float = K_E) -> Tensor:
     """sum_k k_e q_k / max(|x - r_k|, 1e-12) at CUDA points (core/bem.py:291-320)."""
-    L = _lib.load_library()
-    dev, dt = points.device, points.dtype
-    ch = np.asarray([[float(q), *map(float, pos)] for q, pos in charges], dtype=np.float64).reshape(-1, 4)
-    chd = torch.as_tensor(ch, device=dev) if ch.size else torch.zeros(1, 4, dtype=torch.float64, device=dev)
-    out = torch.empty(points.shape[0], dtype=dt, device=dev)
-    with torch.cuda.device(dev):
-        _lib.check(L.edfmm_point_charge_potential(_lib.ptr(points.contiguous()), points.shape[0], _lib.ptr(chd),
-                                                  ch.shape[0], float(k_e), _lib.dtype_code(dt), _lib.ptr(out),
-                                                  _lib.stream_handle(dev)), "edfmm_point_charge_potential")
+    out = torch.empty(points.shape[0], dtype=points.dtype, device=points.device)
+    add_point_charges(points, charges, V=out, overwrite=True, k_e=k_e)
     return out
 
 
@@ -238,6 +247,10 @@ def point_charge_field(points: Tensor, charges) -> Tensor:
     (_free_space_E_field_at_points, bem.py:340-370), (M, 3) in the points' dtype."""
     P = points.reshape(-1, 3)
     E = torch.zeros_like(P)
+    if P.is_cuda and P.dtype in (torch.float32, torch.float64) and not P.requires_grad:
+        E = E.contiguous()
+        add_point_charges(P, charges, E=E)
+        return E
     for q, pos in charges:
         R = P - torch.as_tensor(pos, dtype=P.dtype, device=P.device)[None, :]
         r = torch.linalg.norm(R, dim=1, keepdim=True).clamp_min(1e-12)
@@ -245,5 +258,6 @@ def point_charge_field(points: Tensor, charges) -> Tensor:
     return E
 
 
-__all__ = ["self_integrals", "NearCorrection", "apply_near_quadrature_matvec_cuda", "point_charge_potential",
+__all__ = ["self_integrals", "NearCorrection", "apply_near_quadrature_matvec_cuda", "add_point_charges",
+           "point_charge_potential",
            "potential_at_targets", "field_at_targets", "point_charge_field", "near_potential_correction"]

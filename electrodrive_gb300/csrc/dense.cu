@@ -37,7 +37,6 @@ enum DenseKind { kMatvec = 0, kPotential = 1, kField = 2 };
 constexpr int kThreads = 128;     // 4 warps
 constexpr int kTile32 = 256;      // sources staged per shared-memory tile, FP32
 constexpr int kTile64 = 128;      // FP64
-constexpr int kRows64 = 64;       // FP64 targets per block: 2 warps, times 2 source halves
 constexpr int kMaxCluster = 8;    // the portable cluster size
 
 __device__ __forceinline__ float inv_r(float r2) { return rsqrt_normal(fmaxf(r2, 1e-24f)); }
@@ -232,7 +231,8 @@ __global__ void __launch_bounds__(kThreads) k_dense_f32(const DenseArgs<float> A
 }
 
 // ---------------------------------------------------------------------------
-// FP64: 64 targets per block, one per thread and source half of a tile
+// FP64: 128 / GROUPS targets per block, one per thread; the groups of threads
+// take every GROUPS-th source of a tile
 // ---------------------------------------------------------------------------
 struct Src64 {
     float4 u, v, w;  // (xa, xb, xc, ya), (yb, yc, za, zb), (zc, -, charge as two words)
@@ -262,18 +262,18 @@ __device__ __noinline__ void dense_pair_ieee(const double *c, int64_t j, int64_t
     }
 }
 
-template <int KIND>
+template <int KIND, int GROUPS>
 __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> A) {
-    constexpr int COMP = KIND == kField ? 3 : 1;
+    constexpr int COMP = KIND == kField ? 3 : 1, ROWS = kThreads / GROUPS;
     __shared__ Src64 src[kTile64];
     __shared__ double xyz[KIND == kField ? 3 * kTile64 : 1];
-    __shared__ double part[2 * kRows64 * COMP];
+    __shared__ double part[kThreads * COMP];
     __shared__ unsigned s_hi[4];
     int64_t row0, j0, j1;
     int rank;
-    dense_ranges(A, kRows64, row0, rank, j0, j1);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, half = threadIdx.x >> 6;
-    const int64_t i = row0 + (threadIdx.x & 63);
+    dense_ranges(A, ROWS, row0, rank, j0, j1);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, grp = threadIdx.x / ROWS;
+    const int64_t i = row0 + threadIdx.x % ROWS;
     Tgt64 T;
     {
         const int64_t q = min(i, A.m - 1);
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
         if (!split) {
             if ((int)threadIdx.x < cnt) reinterpret_cast<double *>(&src[threadIdx.x])[0] = w;
             __syncthreads();
-            for (int s = half; s < cnt; s += 2) {
+            for (int s = grp; s < cnt; s += GROUPS) {
                 double px, py, pz;
                 dense_pair_ieee<KIND>(A.c, jb + s, i, T.x, T.y, T.z, reinterpret_cast<double *>(&src[s])[0], A.k_e, px,
                                       py, pz);
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
                 xyz[3 * threadIdx.x + 1] = y;
                 xyz[3 * threadIdx.x + 2] = z;
             }
-        } else if ((int)threadIdx.x < ((cnt + 3) & ~3)) {  // no charge, outside the scaled box
+        } else if ((int)threadIdx.x < ((cnt + 2 * GROUPS - 1) & ~(2 * GROUPS - 1))) {  // padding: no charge, outside the scaled box
             Src64 &S = src[threadIdx.x];
             S.u = make_float4(3.0f, 0.0f, 0.0f, 3.0f);
             S.v = make_float4(0.0f, 0.0f, 3.0f, 0.0f);
@@ -377,19 +377,19 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
                 add(s, r2, w);
             }
         };
-        for (int s = half; s < cnt; s += 4) {  // two sources side by side; the tile is padded to a multiple of 4
+        for (int s = grp; s < cnt; s += 2 * GROUPS) {  // two sources side by side in the padded tile
             GridDiff dx, dy, dz;
             double w0, w1;
             load(s, dx, dy, dz, w0);
             const GridR2 r0 = grid_r2(dx, dy, dz);
-            load(s + 2, dx, dy, dz, w1);
+            load(s + GROUPS, dx, dy, dz, w1);
             const GridR2 r1 = grid_r2(dx, dy, dz);
             if (fminf(r0.R1, r1.R1) < near2) {
                 add_any(s, r0, w0);
-                add_any(s + 2, r1, w1);
+                add_any(s + GROUPS, r1, w1);
             } else {
                 add(s, r0, w0);
-                add(s + 2, r1, w1);
+                add(s + GROUPS, r1, w1);
             }
         }
         const double unscale = KIND == kField ? down * down * down : down;
@@ -399,13 +399,13 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
             ez += tz * unscale + sz;
         }
     }
-    double *p = part + (half * kRows64 + (threadIdx.x & 63)) * COMP;
+    double *p = part + threadIdx.x * COMP;
     p[0] = ex;
     if (KIND == kField) {
         p[1] = ey;
         p[2] = ez;
     }
-    dense_finish<double, KIND, kRows64, 2>(A, part, row0, rank);
+    dense_finish<double, KIND, ROWS, GROUPS>(A, part, row0, rank);
 }
 
 int sm_count() {
@@ -442,7 +442,12 @@ int cluster_size(int64_t tiles, int64_t n) {
 template <typename T, int KIND>
 int dense_launch(const T *tgt, int64_t m, const T *c, const T *sigma, const T *areas, int64_t n, T k_e,
                  const T *self_int, T *out, cudaStream_t s) {
-    constexpr int ROWS = sizeof(T) == 4 ? 32 * tpt32<KIND>() : kRows64;
+    // FP64: 64 targets per block, or 32 when those would leave SMs without a block
+    // even in clusters of eight; the smaller tile splits every source for half
+    // the targets (1,000 targets, 5,120 sources: 89 and 290 us, potential and
+    // field, with 64, 76 and 180 with 32)
+    const bool narrow = sizeof(T) == 8 && (m + 63) / 64 * kMaxCluster < 2 * sm_count();
+    const int ROWS = sizeof(T) == 4 ? 32 * tpt32<KIND>() : narrow ? 32 : 64;
     const int64_t tiles = (m + ROWS - 1) / ROWS;
     DenseArgs<T> A{tgt, m, c, sigma, areas, n, 0, cluster_size(tiles, n), k_e, self_int, out};
     A.chunk = ((n + A.cs - 1) / A.cs + 1) & ~(int64_t)1;
@@ -459,7 +464,7 @@ int dense_launch(const T *tgt, int64_t m, const T *c, const T *sigma, const T *a
     cfg.numAttrs = A.cs > 1 ? 1 : 0;
     cudaError_t e;
     if constexpr (sizeof(T) == 4) e = cudaLaunchKernelEx(&cfg, k_dense_f32<KIND>, A);
-    else e = cudaLaunchKernelEx(&cfg, k_dense_f64<KIND>, A);
+    else e = narrow ? cudaLaunchKernelEx(&cfg, k_dense_f64<KIND, 4>, A) : cudaLaunchKernelEx(&cfg, k_dense_f64<KIND, 2>, A);
     if (e != cudaSuccess) return fail(EDFMM_ERR_CUDA, std::string("launch of k_dense failed: ") + cudaGetErrorString(e));
     EDFMM_LAUNCH_CHECK("k_dense");
     return EDFMM_OK;
