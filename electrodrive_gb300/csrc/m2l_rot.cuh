@@ -64,9 +64,16 @@ template <typename T, int N, int P>
 __device__ __forceinline__ void zrot(T (&b)[N], const T (&c)[P + 1], const T (&s)[P + 1], T sign) {
 #pragma unroll
     for (int m = 1; 2 * m < N; ++m) {
-        const T re = b[2 * m - 1], im = b[2 * m], cm = c[m], sm = sign * s[m];
-        b[2 * m - 1] = re * cm - im * sm;
-        b[2 * m] = re * sm + im * cm;
+        const T re = b[2 * m - 1], im = b[2 * m], cm = c[m];
+        if constexpr (std::is_same<T, tf32x2>::value) {
+            const T sm = sign.hi < 0.0f ? -s[m] : s[m];
+            b[2 * m - 1] = tf_cmul(re, cm, im, -sm);
+            b[2 * m] = tf_cmul(im, cm, re, sm);
+        } else {
+            const T sm = sign * s[m];
+            b[2 * m - 1] = re * cm - im * sm;
+            b[2 * m] = re * sm + im * cm;
+        }
     }
 }
 
@@ -519,6 +526,34 @@ __device__ __forceinline__ tfp tfp_mul_const(float2 g, float2 ng, float2 nglo, c
     return tfp{h, f2_sub(f2_sub(p, h), ne)};
 }
 
+// a c + b s on both halves (tf_cmul)
+__device__ __forceinline__ tfp tfp_cmul(const tfp &a, const tfp &c, const tfp &b, const tfp &s) {
+    const float2 m1 = make_float2(-1.0f, -1.0f);
+    const float2 nah = __fmul2_rn(a.hi, m1), nbh = __fmul2_rn(b.hi, m1);
+    const float2 p = __fmul2_rn(a.hi, c.hi), q = __fmul2_rn(b.hi, s.hi);
+    const float2 np = __ffma2_rn(nah, c.hi, p), nq = __ffma2_rn(nbh, s.hi, q);  // rounding errors, negated
+    float2 l = __fmul2_rn(a.hi, c.lo);
+    l = __ffma2_rn(a.lo, c.hi, l);
+    l = __ffma2_rn(b.hi, s.lo, l);
+    l = __ffma2_rn(b.lo, s.hi, l);
+    l = f2_sub(f2_sub(l, np), nq);
+    const float2 t = __fadd2_rn(p, q), bb = f2_sub(t, p);  // two-sum
+    const float2 e = __fadd2_rn(f2_sub(p, f2_sub(t, bb)), f2_sub(q, bb));
+    l = __fadd2_rn(l, e);
+    const float2 h = __fadd2_rn(t, l);
+    return tfp{h, f2_sub(l, f2_sub(h, t))};
+}
+// a * g, g the same two-float value for both halves
+__device__ __forceinline__ tfp tfp_mul_tf(const tfp &a, tf32x2 g) {
+    const float2 gh = make_float2(g.hi, g.hi), ngh = make_float2(-g.hi, -g.hi), ngl = make_float2(-g.lo, -g.lo);
+    const float2 p = __fmul2_rn(a.hi, gh);
+    float2 ne = __ffma2_rn(a.hi, ngh, p);
+    ne = __ffma2_rn(a.hi, ngl, ne);
+    ne = __ffma2_rn(a.lo, ngh, ne);
+    const float2 h = f2_sub(p, ne);
+    return tfp{h, f2_sub(f2_sub(p, h), ne)};
+}
+
 template <int n> struct PkT {  // one degree block of two-float values in a packed layout
     tfp p[n > 0 ? n : 1];
     tf32x2 r;  // Re X_n
@@ -627,19 +662,34 @@ __device__ __forceinline__ void pkt_apply(const PkT<n> &x, PkT<n> &y) {
     pkt_left_row<TAB, n, LIN, 0, false>(x, y.r);
 }
 
-// X_m <- X_m e^{+-i m a} in two-float, x in layout LA, y in layout LB
-template <int n, int LA, int LB, int P, int m>
+// X_m <- X_m e^{+-i m a} in two-float, x in layout LA, y in layout LB: pair j
+// (Re X_j, Im X_{j+1}) at once, from (Re X_j, Im X_{j+1}) and (Im X_j, Re X_{j+1})
+__device__ __forceinline__ tfp tfp_pair(tf32x2 a, tf32x2 b) {
+    return tfp{make_float2(a.hi, b.hi), make_float2(a.lo, b.lo)};
+}
+template <int n, int LA, int LB, int P, int j>
 __device__ __forceinline__ void pkt_zrot(const PkT<n> &x, PkT<n> &y, const tf32x2 (&c)[P + 1],
                                          const tf32x2 (&s)[P + 1], bool neg) {
-    if constexpr (m == 0) {
-        pkt_set<n, LB, 0>(y, pkt_get<n, LA, 0>(x));
+    if constexpr (n == 0) {
+        y.r = x.r;
+    } else if constexpr (j < n) {
+        const tf32x2 re0 = pkt_get<n, LA, ix_re(j)>(x), im1 = pkt_get<n, LA, 2 * (j + 1)>(x),
+                     re1 = pkt_get<n, LA, ix_re(j + 1)>(x);
+        const tf32x2 s1 = neg ? -s[j + 1] : s[j + 1];
+        if constexpr (j == 0) {  // X_0 does not turn
+            pkt_set<n, LB, 0>(y, re0);
+            pkt_set<n, LB, 2>(y, tf_cmul(im1, c[1], re1, s1));
+        } else {
+            const tf32x2 im0 = pkt_get<n, LA, 2 * j>(x), s0 = neg ? s[j] : -s[j];
+            const tfp o = tfp_cmul(tfp_pair(re0, im1), tfp_pair(c[j], c[j + 1]), tfp_pair(im0, re1), tfp_pair(s0, s1));
+            pkt_set<n, LB, ix_re(j)>(y, tf32x2(o.hi.x, o.lo.x));
+            pkt_set<n, LB, 2 * (j + 1)>(y, tf32x2(o.hi.y, o.lo.y));
+        }
+        pkt_zrot<n, LA, LB, P, j + 1>(x, y, c, s, neg);
     } else {
-        const tf32x2 re = pkt_get<n, LA, 2 * m - 1>(x), im = pkt_get<n, LA, 2 * m>(x), cm = c[m];
-        const tf32x2 sm = neg ? -s[m] : s[m];
-        pkt_set<n, LB, 2 * m - 1>(y, re * cm - im * sm);
-        pkt_set<n, LB, 2 * m>(y, re * sm + im * cm);
+        const tf32x2 re = pkt_get<n, LA, ix_re(n)>(x), im = pkt_get<n, LA, 2 * n>(x);
+        pkt_set<n, LB, ix_re(n)>(y, tf_cmul(re, c[n], im, neg ? s[n] : -s[n]));
     }
-    if constexpr (m < n) pkt_zrot<n, LA, LB, P, m + 1>(x, y, c, s, neg);
 }
 
 // all 2n + 1 values of a packed block to / from the slots of v (block index order)
@@ -658,22 +708,11 @@ __device__ __forceinline__ void pkt_load(const V &v, PkT<n> &x) {
 // R_z(+phi), Q_p, R_z(+theta), Q_m
 template <int P, int n, typename V>
 __device__ __forceinline__ void forward_tf_pk(V &v, tf32x2 cr, tf32x2 fn, const Frame<tf32x2, P> &F) {
-    constexpr int OV = n * n;
     PkT<n> a, b;
-    pkt_set<n, 0, 0>(b, v.get(OV) * fn);
+    pkt_load<n, 0, 0>(v, b);
 #pragma unroll
-    for (int m = 1; m <= n; ++m) {
-        // scaled row into layout RI (compile-time indices after unrolling)
-        const tf32x2 re = v.get(OV + 2 * m - 1) * fn, im = v.get(OV + 2 * m) * fn;
-        if (m < n) {
-            b.p[m].hi.x = re.hi;
-            b.p[m].lo.x = re.lo;
-        } else {
-            b.r = re;
-        }
-        b.p[m - 1].hi.y = im.hi;
-        b.p[m - 1].lo.y = im.lo;
-    }
+    for (int j = 0; j < n; ++j) b.p[j] = tfp_mul_tf(b.p[j], fn);
+    b.r = b.r * fn;
     pkt_zrot<n, 0, 1, P, 0>(b, a, F.cp, F.sp, false);
     pkt_apply<0, n, 1, 0>(a, b);
     pkt_zrot<n, 0, 1, P, 0>(b, a, F.ct, F.st, false);
@@ -693,6 +732,46 @@ __device__ __forceinline__ void backward_tf_pk(V &v, const Frame<tf32x2, P> &F) 
     pkt_zrot<n, 1, 0, P, 0>(b, a, F.cp, F.sp, true);
     pkt_store<n, 0, 0>(v, a);
     if constexpr (n < P) backward_tf_pk<P, n + 1>(v, F);
+}
+
+// axial<tf32x2, P, m, true> with the real and imaginary parts of order m >= 1
+// in the halves of packed operations
+template <int P, int N, int K, int m>
+__device__ __forceinline__ void pkt_binom(const tfp (&u)[P + 1], tfp &s) {
+    constexpr float cb = (float)binom(N + K, K);
+    const float2 g = make_float2(cb, cb), ng = make_float2(-cb, -cb), zero = make_float2(0.0f, 0.0f);
+    if constexpr (K == m) s = tfp_mul_const<true>(g, ng, zero, u[K]);
+    else s = tfp_fma_const<true>(g, ng, zero, u[K], s);
+    if constexpr (K < P) pkt_binom<P, N, K + 1, m>(u, s);
+}
+template <int P, int m, int N, typename V>
+__device__ __forceinline__ void axial_tf_rows(V &v, const tfp (&u)[P + 1], const tf32x2 (&h)[P + 1]) {
+    tfp s;
+    pkt_binom<P, N, m, m>(u, s);
+    s = tfp_mul_tf(s, h[N]);
+    const tf32x2 re(s.hi.x, s.lo.x), im(s.hi.y, s.lo.y);
+    v.set(N * N + 2 * m - 1, ((N + m) & 1) ? -re : re);
+    v.set(N * N + 2 * m, ((N + m) & 1) ? -im : im);
+    if constexpr (N < P) axial_tf_rows<P, m, N + 1>(v, u, h);
+}
+template <int P, int m, typename V> __device__ __forceinline__ void axial_tf_pk(V &v, const tf32x2 (&h)[P + 1]) {
+    if constexpr (m == 0) {
+        tf32x2 ur[P + 1], ui[P + 1], wr[P + 1], wi[P + 1];
+#pragma unroll
+        for (int k = 0; k <= P; ++k) {
+            ur[k] = v.get(k * k);
+            ui[k] = tf32x2(0);
+        }
+        binom_rows<tf32x2, P, 0, 0, true>(ur, ui, wr, wi, h);
+#pragma unroll
+        for (int k = 0; k <= P; ++k) v.set(k * k, wr[k]);
+    } else {
+        tfp u[P + 1];
+#pragma unroll
+        for (int k = m; k <= P; ++k) u[k] = tfp_pair(v.get(k * k + 2 * m - 1), v.get(k * k + 2 * m));
+        axial_tf_rows<P, m, m>(v, u, h);
+    }
+    if constexpr (m < P) axial_tf_pk<P, m + 1>(v, h);
 }
 
 // two-float slots split into a hi and a lo array (slot i of this thread at
@@ -745,7 +824,8 @@ __device__ __forceinline__ void rot_pair_tf(V &v, const float4 *__restrict__ Mro
     h[0] = irho;
 #pragma unroll
     for (int j = 1; j <= P; ++j) h[j] = h[j - 1] * T(j) * irho;
-    axial<T, P, 0, true>(v, h);
+    if constexpr (PK) axial_tf_pk<P, 0>(v, h);
+    else axial<T, P, 0, true>(v, h);
     if constexpr (PK) backward_tf_pk<P, 0>(v, F);
     else backward_v<T, P, 0>(v, F);
 }

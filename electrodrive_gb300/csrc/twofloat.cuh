@@ -87,6 +87,18 @@ __device__ __forceinline__ tf32x2 tf_fma_const(float ghi, float glo, tf32x2 a, t
     const tf32x2 s = tf_two_sum(p.hi, c.hi);
     return tf_fast_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(e, c.lo)));
 }
+// a c + b s with one renormalisation (a rotation's output: 20 operations where
+// two products and a sum take 25)
+__device__ __forceinline__ tf32x2 tf_cmul(tf32x2 a, tf32x2 c, tf32x2 b, tf32x2 s) {
+    const tf32x2 p = tf_two_prod(a.hi, c.hi), q = tf_two_prod(b.hi, s.hi);
+    float l = __fmul_rn(a.hi, c.lo);
+    l = __fmaf_rn(a.lo, c.hi, l);
+    l = __fmaf_rn(b.hi, s.lo, l);
+    l = __fmaf_rn(b.lo, s.hi, l);
+    l = __fadd_rn(__fadd_rn(l, p.lo), q.lo);
+    const tf32x2 t = tf_two_sum(p.hi, q.hi);
+    return tf_fast_two_sum(t.hi, __fadd_rn(l, t.lo));
+}
 __device__ __forceinline__ bool operator>(tf32x2 a, tf32x2 b) { return a.hi > b.hi || (a.hi == b.hi && a.lo > b.lo); }
 __device__ __forceinline__ bool operator<(tf32x2 a, tf32x2 b) { return b > a; }
 
