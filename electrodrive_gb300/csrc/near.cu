@@ -695,7 +695,7 @@ EDFMM_API int edfmm_near_create(const void *centroids_dev, const void *areas_dev
         int64_t mx = 0;
         for (int64_t i = 0; i < n; ++i) mx = std::max<int64_t>(mx, hoff[i + 1] - hoff[i]);
         h->max_row = mx;
-        if ((rc = sort_csr_rows(dptr<int32_t>(h->row_off), dptr<int32_t>(h->cols), n, mx, s))) return done(rc);
+        if ((rc = sort_csr_rows(dptr<int32_t>(h->row_off), dptr<int32_t>(h->cols), n, mx, n, s))) return done(rc);
         k_near_weights_pairs<<<nb(np, 128), 128, 0, s>>>(c, a, static_cast<const double *>(panel_vertices_dev), n, np,
                                                          dptr<int32_t>(h->row_off), dptr<int32_t>(h->cols), quad_order,
                                                          depth, k_e, dptr<double>(h->w64));

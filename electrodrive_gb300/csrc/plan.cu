@@ -117,17 +117,51 @@ int alloc_expansions(edfmm_plan *p, int dtype, int expansion_order, cudaStream_t
     return rc;
 }
 
-// Plan buffers built inside a BlockCacheScope may sit in cached blocks larger
-// than they need; move those to exact-size blocks before the plan is handed out.
-int shrink_tree_lists(DevTree &t, DevLists &l, cudaStream_t s) {
+// Slab size of a set-up over n points: about what its temporaries and lists
+// take (900 bytes a point for a cube in FP32), 128 MB at most.
+size_t setup_slab_bytes(int64_t n, int dtype) {
+    const size_t want = (size_t)std::max<int64_t>(n, 1) * (dtype == EDFMM_F64 ? 1280 : 1024);
+    return std::min<size_t>(std::max<size_t>(want, 1 << 20), (size_t)128 << 20);
+}
+
+// The buffers of a tree and its lists that a set-up inside a BlockCacheScope
+// leaves in slabs or in cached blocks larger than they need move to exact
+// blocks before the plan is handed out; expansions of up to 16 MB (three
+// buffers of esz bytes) share the block of the small ones.
+int settle_buffers(DevTree &t, DevLists &l, DevBuf *const *exp, int n_exp, size_t esz, DevBuf &block,
+                   cudaStream_t s) {
     DevBuf *bufs[] = {&t.pts,      &t.index_map,     &t.center,      &t.half,    &t.range,
                       &t.parent,   &t.children,      &t.level,       &t.is_leaf, &t.leaves,
                       &t.level_nodes, &t.inst_node_off, &l.p2p_off,  &l.p2p_src, &l.m2l_off,
                       &l.m2l_src,  &l.m2l_swapped_off, &l.m2l_swapped_src, &l.p2p_leaves, &l.m2l_rows,
                       &t.pts_grid, &t.grid_info};
-    for (DevBuf *b : bufs)
-        if (int rc = b->shrink_to_fit(s)) return rc;
-    return EDFMM_OK;
+    const int n = (int)(sizeof(bufs) / sizeof(bufs[0]));
+    if (n_exp * esz <= ((size_t)16 << 20)) return pack_buffers(bufs, n, exp, n_exp, esz, block, s);
+    int rc = pack_buffers(bufs, n, nullptr, 0, 0, block, s);
+    for (int i = 0; !rc && i < n_exp; ++i) {
+        rc = exp[i]->reserve(esz);
+        if (!rc) rc = exp[i]->shrink_to_fit(s);
+    }
+    return rc;
+}
+
+// tree and lists are built: the rest of a plan's set-up (synchronises the stream)
+int finish_plan(edfmm_plan *p, int dtype, int expansion_order, cudaStream_t s) {
+    p->fmm.p = expansion_order;
+    p->fmm.nc = num_coeffs(expansion_order);
+    p->fmm.nc_pad = (p->fmm.nc + 1) & ~1;
+    const size_t esz = (dtype == EDFMM_F64 ? 16 : 8) * (size_t)p->fmm.nc_pad *
+                       (size_t)std::max<int64_t>(p->tree.n_nodes, 1);
+    DevBuf *exp[] = {&p->fmm.multipoles, &p->fmm.locals, &p->fmm.translated};
+    int rc = grid_prepare(p->tree, s);
+    if (!rc) rc = settle_buffers(p->tree, p->lists, exp, 3, esz, p->block, s);
+    if (!rc) {
+        cudaError_t e = cudaMemsetAsync(p->fmm.multipoles.p, 0, esz, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(p->fmm.locals.p, 0, esz, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) rc = fail(EDFMM_ERR_CUDA, std::string("plan set-up: ") + cudaGetErrorString(e));
+    }
+    return rc;
 }
 
 int check_plan(const edfmm_plan *p) {
@@ -138,30 +172,71 @@ int check_plan(const edfmm_plan *p) {
 }  // namespace
 
 struct BlockCache {
-    std::multimap<size_t, void *> free_blocks;  // by size
+    std::multimap<size_t, DevBlock> free_blocks;  // by size
+    size_t slab_bytes = 0;
+    std::vector<void *> slabs;
+    char *cut = nullptr, *cut_end = nullptr;  // what is left of the last slab
 };
 
 namespace {
 thread_local BlockCache *g_block_cache = nullptr;
+
+constexpr size_t kBlockAlign = 256;
+inline size_t align_up(size_t b) { return (b + kBlockAlign - 1) / kBlockAlign * kBlockAlign; }
+
+// the parts of a packed block: 16-byte words of part blockIdx.y
+constexpr int kMaxParts = 32;
+struct PackArgs {
+    const uint4 *src[kMaxParts];
+    uint4 *dst[kMaxParts];
+    size_t words[kMaxParts];
+};
+__global__ void __launch_bounds__(256) k_pack(PackArgs A) {
+    const int k = blockIdx.y;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.words[k]; i += (size_t)gridDim.x * blockDim.x)
+        A.dst[k][i] = A.src[k][i];
 }
+}  // namespace
 
 BlockCache *block_cache() { return g_block_cache; }
 
-void *block_cache_take(BlockCache *c, size_t nbytes, size_t *got) {
+DevBlock block_cache_take(BlockCache *c, size_t nbytes) {
     // the smallest held block that fits, unless it is more than twice the request
     auto it = c->free_blocks.lower_bound(nbytes);
-    if (it == c->free_blocks.end() || it->first > 2 * nbytes + 256) return nullptr;
-    void *p = it->second;
-    *got = it->first;
-    c->free_blocks.erase(it);
-    return p;
+    if (it != c->free_blocks.end() && it->first <= 2 * nbytes + 256) {
+        const DevBlock b = it->second;
+        c->free_blocks.erase(it);
+        return b;
+    }
+    const size_t want = align_up(nbytes);
+    if (want > c->slab_bytes / 2) return DevBlock{};
+    if (c->cut + want > c->cut_end) {
+        void *p = nullptr;
+        if (cudaMalloc(&p, c->slab_bytes) != cudaSuccess) {
+            (void)cudaGetLastError();  // too little memory for a slab: blocks of their own from here on
+            c->slab_bytes = 0;
+            return DevBlock{};
+        }
+        c->slabs.push_back(p);
+        c->cut = static_cast<char *>(p);
+        c->cut_end = c->cut + c->slab_bytes;
+    }
+    const DevBlock b{c->cut, want, c};
+    c->cut += want;
+    return b;
 }
 
-void block_cache_put(BlockCache *c, void *p, size_t nbytes) { c->free_blocks.emplace(nbytes, p); }
+void block_cache_put(BlockCache *c, const DevBlock &b) { c->free_blocks.emplace(b.bytes, b); }
 
 void block_cache_trim(BlockCache *c) {
-    for (auto &kv : c->free_blocks) cudaFree(kv.second);
-    c->free_blocks.clear();
+    for (auto it = c->free_blocks.begin(); it != c->free_blocks.end();) {
+        if (it->second.slab) {
+            ++it;
+            continue;
+        }
+        cudaFree(it->second.p);
+        it = c->free_blocks.erase(it);
+    }
 }
 
 cudaError_t malloc_or_trim(void **p, size_t nbytes) {
@@ -175,12 +250,73 @@ cudaError_t malloc_or_trim(void **p, size_t nbytes) {
     return e;
 }
 
-BlockCacheScope::BlockCacheScope() : prev(g_block_cache), cache(new BlockCache()) { g_block_cache = cache; }
+BlockCacheScope::BlockCacheScope(size_t slab_bytes) : prev(g_block_cache), cache(new BlockCache()) {
+    cache->slab_bytes = align_up(slab_bytes);
+    g_block_cache = cache;
+}
 
 BlockCacheScope::~BlockCacheScope() {
     g_block_cache = prev;
-    for (auto &kv : cache->free_blocks) cudaFree(kv.second);  // cudaFree waits for the device
+    block_cache_trim(cache);  // cudaFree waits for the device
+    for (void *p : cache->slabs) cudaFree(p);
     delete cache;
+}
+
+int pack_buffers(DevBuf *const *bufs, int n, DevBuf *const *fresh, int n_fresh, size_t fresh_bytes, DevBuf &block,
+                 cudaStream_t s) {
+    size_t total = 0, widest = 0;
+    int parts = 0;
+    for (int i = 0; i < n; ++i) {
+        if (!bufs[i]->p || !bufs[i]->slab) continue;
+        total += align_up(bufs[i]->used);
+        widest = std::max(widest, bufs[i]->used);
+        ++parts;
+    }
+    total += n_fresh * align_up(fresh_bytes);
+    if (parts > kMaxParts) return fail(EDFMM_ERR_ARG, "too many buffers to pack");
+    if (total > 0) {
+        void *q = nullptr;
+        cudaError_t e = malloc_or_trim(&q, total);
+        if (e != cudaSuccess)
+            return fail(EDFMM_ERR_ALLOC, std::string("cudaMalloc of ") + std::to_string(total) +
+                                             " bytes failed: " + cudaGetErrorString(e));
+        block.release();
+        block.p = q;
+        block.bytes = block.used = total;
+        char *at = static_cast<char *>(q);
+        PackArgs A;
+        int k = 0;
+        for (int i = 0; i < n; ++i) {
+            DevBuf &b = *bufs[i];
+            if (!b.p || !b.slab) continue;
+            const size_t used = b.used;
+            A.src[k] = static_cast<const uint4 *>(b.p);
+            A.dst[k] = reinterpret_cast<uint4 *>(at);
+            A.words[k] = (used + 15) / 16;  // slab blocks and parts both end on 256 bytes
+            ++k;
+            b.release();  // reused, if at all, later in the stream
+            b.p = at;
+            b.bytes = b.used = used;
+            b.part = true;
+            at += align_up(used);
+        }
+        if (k > 0) {
+            const unsigned gx = (unsigned)std::min<size_t>((widest + 4095) / 4096, 152 * 4);
+            k_pack<<<dim3(gx ? gx : 1, k), 256, 0, s>>>(A);
+            EDFMM_LAUNCH_CHECK("k_pack");
+        }
+        for (int i = 0; i < n_fresh; ++i) {
+            DevBuf &b = *fresh[i];
+            b.release();
+            b.p = at;
+            b.bytes = b.used = fresh_bytes;
+            b.part = true;
+            at += align_up(fresh_bytes);
+        }
+    }
+    for (int i = 0; i < n; ++i)
+        if (int rc = bufs[i]->shrink_to_fit(s)) return rc;
+    return EDFMM_OK;
 }
 
 void set_error(const std::string &msg) { g_last_error = msg; }
@@ -222,29 +358,10 @@ int edfmm_plan_create(const void *points_dev, int64_t n, int dtype, int leaf_siz
     p->leaf_size = leaf_size;
     p->max_depth = max_depth;
     cudaStream_t s = S(stream);
-    BlockCacheScope cache_scope;  // the build runs on `s` alone
+    BlockCacheScope cache_scope(setup_slab_bytes(n, dtype));  // the build runs on `s` alone
     rc = tree_build(points_dev, n, dtype, leaf_size, max_depth, p->tree, s);
     if (!rc) rc = lists_build(p->tree, mac_theta, p->lists, s);
-    if (!rc) rc = grid_prepare(p->tree, s);
-    if (!rc) rc = shrink_tree_lists(p->tree, p->lists, s);
-    if (!rc) {
-        p->fmm.p = expansion_order;
-        p->fmm.nc = num_coeffs(expansion_order);
-        p->fmm.nc_pad = (p->fmm.nc + 1) & ~1;
-        size_t esz = (dtype == EDFMM_F64 ? 16 : 8) * (size_t)p->fmm.nc_pad * (size_t)std::max<int64_t>(p->tree.n_nodes, 1);
-        rc = p->fmm.multipoles.reserve(esz);
-        if (!rc) rc = p->fmm.locals.reserve(esz);
-        if (!rc) rc = p->fmm.translated.reserve(esz);
-        if (!rc) rc = p->fmm.multipoles.shrink_to_fit(s);
-        if (!rc) rc = p->fmm.locals.shrink_to_fit(s);
-        if (!rc) rc = p->fmm.translated.shrink_to_fit(s);
-        if (!rc) {
-            cudaError_t e = cudaMemsetAsync(p->fmm.multipoles.p, 0, esz, s);
-            if (e == cudaSuccess) e = cudaMemsetAsync(p->fmm.locals.p, 0, esz, s);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-            if (e != cudaSuccess) rc = fail(EDFMM_ERR_CUDA, std::string("plan set-up: ") + cudaGetErrorString(e));
-        }
-    }
+    if (!rc) rc = finish_plan(p, dtype, expansion_order, s);
     if (rc) {
         delete p;
         return rc;
@@ -271,7 +388,7 @@ int edfmm_plan_create_batch(const void *points_dev, const int64_t *offsets, int 
     if (rc) return rc;
     cudaStream_t s = S(stream);
     // every build below runs on `s`: temporaries are recycled in stream order
-    BlockCacheScope cache_scope;
+    BlockCacheScope cache_scope(setup_slab_bytes(offsets[n_instances], dtype));
     // one forest over all instances, level by level (each instance's tree and
     // lists equal what edfmm_plan_create builds for it alone)
     edfmm_plan *p = new edfmm_plan();
@@ -285,26 +402,7 @@ int edfmm_plan_create_batch(const void *points_dev, const int64_t *offsets, int 
     }
     rc = tree_build_forest(points_dev, offsets, n_instances, dtype, leaf_size, max_depth, p->tree, s);
     if (!rc) rc = lists_build(p->tree, mac_theta, p->lists, s);
-    if (!rc) rc = grid_prepare(p->tree, s);
-    if (!rc) rc = shrink_tree_lists(p->tree, p->lists, s);
-    if (!rc) {
-        p->fmm.p = expansion_order;
-        p->fmm.nc = num_coeffs(expansion_order);
-        p->fmm.nc_pad = (p->fmm.nc + 1) & ~1;
-        size_t esz = (dtype == EDFMM_F64 ? 16 : 8) * (size_t)p->fmm.nc_pad * (size_t)std::max<int64_t>(p->tree.n_nodes, 1);
-        rc = p->fmm.multipoles.reserve(esz);
-        if (!rc) rc = p->fmm.locals.reserve(esz);
-        if (!rc) rc = p->fmm.translated.reserve(esz);
-        if (!rc) rc = p->fmm.multipoles.shrink_to_fit(s);
-        if (!rc) rc = p->fmm.locals.shrink_to_fit(s);
-        if (!rc) rc = p->fmm.translated.shrink_to_fit(s);
-        if (!rc) {
-            cudaError_t e = cudaMemsetAsync(p->fmm.multipoles.p, 0, esz, s);
-            if (e == cudaSuccess) e = cudaMemsetAsync(p->fmm.locals.p, 0, esz, s);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-            if (e != cudaSuccess) rc = fail(EDFMM_ERR_CUDA, std::string("plan set-up: ") + cudaGetErrorString(e));
-        }
-    }
+    if (!rc) rc = finish_plan(p, dtype, expansion_order, s);
     if (rc) {
         delete p;
         return rc;
@@ -705,7 +803,26 @@ struct edfmm_targets {
     DevLists lists;              // rows: target nodes; sources: source-plan nodes
     FmmBuffers buf;              // target locals
     DevBuf near_sum;             // near sums at the targets, tree order
+    DevBuf block;                // the set-up's small buffers (pack_buffers)
 };
+
+// tree and lists are built: the rest of a target set-up (synchronises the stream)
+static int finish_targets(edfmm_targets *t, cudaStream_t s) {
+    const edfmm_plan *p = t->plan;
+    t->buf.p = p->fmm.p;
+    t->buf.nc = p->fmm.nc;
+    t->buf.nc_pad = p->fmm.nc_pad;
+    const size_t esz = (p->tree.dtype == EDFMM_F64 ? 16 : 8) * (size_t)t->buf.nc_pad *
+                       (size_t)std::max<int64_t>(t->tree.n_nodes, 1);
+    DevBuf *exp[] = {&t->buf.locals};
+    int rc = settle_buffers(t->tree, t->lists, exp, 1, esz, t->block, s);
+    if (!rc) {
+        cudaError_t e = cudaMemsetAsync(t->buf.locals.p, 0, esz, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) rc = fail(EDFMM_ERR_CUDA, std::string("target set-up: ") + cudaGetErrorString(e));
+    }
+    return rc;
+}
 
 int edfmm_targets_create(edfmm_plan *p, const void *targets_dev, int64_t m, void *stream, edfmm_targets **out) {
     if (!out) return fail(EDFMM_ERR_ARG, "out is NULL");
@@ -716,21 +833,10 @@ int edfmm_targets_create(edfmm_plan *p, const void *targets_dev, int64_t m, void
     cudaStream_t s = S(stream);
     edfmm_targets *t = new edfmm_targets();
     t->plan = p;
+    BlockCacheScope cache_scope(setup_slab_bytes(m, p->tree.dtype));  // the build runs on `s` alone
     int rc = tree_build(targets_dev, m, p->tree.dtype, p->leaf_size, p->max_depth, t->tree, s);
     if (!rc) rc = lists_build_two(p->tree, t->tree, p->mac_theta, t->lists, s);
-    if (!rc) {
-        t->buf.p = p->fmm.p;
-        t->buf.nc = p->fmm.nc;
-        t->buf.nc_pad = p->fmm.nc_pad;
-        const size_t esz = (p->tree.dtype == EDFMM_F64 ? 16 : 8) * (size_t)t->buf.nc_pad *
-                           (size_t)std::max<int64_t>(t->tree.n_nodes, 1);
-        rc = t->buf.locals.reserve(esz);
-        if (!rc) {
-            cudaError_t e = cudaMemsetAsync(t->buf.locals.p, 0, esz, s);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-            if (e != cudaSuccess) rc = fail(EDFMM_ERR_CUDA, std::string("target set-up: ") + cudaGetErrorString(e));
-        }
-    }
+    if (!rc) rc = finish_targets(t, s);
     if (rc) {
         delete t;
         return rc;
@@ -750,6 +856,7 @@ int edfmm_targets_create_from_plan(edfmm_plan *p, const edfmm_plan *tp, double m
         return fail(EDFMM_ERR_UNSUPPORTED, "batched plans have no two-tree lists");
     if (!(mac_theta > 0.0 && mac_theta < 1.0)) return fail(EDFMM_ERR_ARG, "mac_theta must be in (0, 1)");
     cudaStream_t s = S(stream);
+    BlockCacheScope cache_scope(setup_slab_bytes(tp->tree.n_points, p->tree.dtype));  // the build runs on `s` alone
     std::unique_ptr<edfmm_targets> t(new edfmm_targets());
     t->plan = p;
     const DevTree &a = tp->tree;
@@ -768,19 +875,7 @@ int edfmm_targets_create_from_plan(edfmm_plan *p, const edfmm_plan *tp, double m
     int rc = EDFMM_OK;
     for (size_t i = 0; !rc && i < sizeof(from) / sizeof(from[0]); ++i) rc = clone_buf(*from[i], *to[i], s);
     if (!rc) rc = lists_build_two(p->tree, tt, mac_theta, t->lists, s);
-    if (!rc) {
-        t->buf.p = p->fmm.p;
-        t->buf.nc = p->fmm.nc;
-        t->buf.nc_pad = p->fmm.nc_pad;
-        const size_t esz = (tt.dtype == EDFMM_F64 ? 16 : 8) * (size_t)t->buf.nc_pad *
-                           (size_t)std::max<int64_t>(tt.n_nodes, 1);
-        rc = t->buf.locals.reserve(esz);
-        if (!rc) {
-            cudaError_t e = cudaMemsetAsync(t->buf.locals.p, 0, esz, s);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-            if (e != cudaSuccess) rc = fail(EDFMM_ERR_CUDA, std::string("target set-up: ") + cudaGetErrorString(e));
-        }
-    }
+    if (!rc) rc = finish_targets(t.get(), s);
     if (rc) return rc;
     *out = t.release();
     return EDFMM_OK;

@@ -19,6 +19,15 @@
 //     each node by (range start, level): nodes sharing a start form a chain
 //     of first children, so dfs = #nodes with smaller start + depth inside
 //     the chain.
+// Points move between two buffers level by level; a leaf's points go to their
+// final place in the level that finds the leaf.  The set-up is bound by
+// launches and by the host's one read a level (the number of children): a
+// level whose nodes all hold at most 1024 points, which is every level but
+// the first two or three, is a single kernel with a block per node.  A whole
+// plan (tree, lists, buffers), created and destroyed: 100,003 points in a
+// cube 4.9 -> 0.90 ms, 2,003 points 1.17 -> 0.58 ms, 1,048,576 points 14.4 ->
+// 3.9 ms against two reads a level, 13 launches a level and a copy of the
+// points back into place.
 #include <algorithm>
 #include <cfloat>
 
@@ -78,17 +87,27 @@ __device__ __forceinline__ double radius_of(double hx, double hy, double hz) {
     return rn_mul(r, 1.0 + 1e-12);
 }
 
-template <typename T> struct LevelNode {
-    int32_t start, end;
-};
-
 // ---------------------------------------------------------------------------
 // kernels
 // ---------------------------------------------------------------------------
 
+// what the host reads back after each level
+struct BuildState {
+    int64_t next;          // nodes of the next level
+    int32_t leaves, warn;  // leaves so far, leaves above leaf_size at max_depth
+    int32_t max_child[66]; // points of the largest node of each level
+};
+
+// points into tree layout, and the roots (one, or one per instance)
 template <typename T>
-__global__ void k_init_points(const T *__restrict__ pts, int64_t n, typename Vec4<T>::type *xyz, int32_t *perm) {
+__global__ void k_init_points(const T *__restrict__ pts, int64_t n, typename Vec4<T>::type *xyz, int32_t *perm,
+                              const int64_t *inst_off, int K0, int2 *rng, int32_t *parent, int32_t *root) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < K0) {
+        rng[i] = inst_off ? make_int2((int)inst_off[i], (int)inst_off[i + 1]) : make_int2(0, (int)n);
+        parent[i] = -1;
+        root[i] = (int32_t)i;
+    }
     if (i >= n) return;
     typename Vec4<T>::type v;
     v.x = pts[3 * i];
@@ -99,12 +118,17 @@ __global__ void k_init_points(const T *__restrict__ pts, int64_t n, typename Vec
     perm[i] = (int32_t)i;
 }
 
-// chunk counts per node of the level
-__global__ void k_chunk_counts(const int2 *rng, int K, int32_t *cnt) {
+// chunk counts per node of the level; empty bounding boxes
+template <typename T>
+__global__ void k_chunk_counts(const int2 *rng, int K, int32_t *cnt, typename OrdT<T>::type *bb) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= K) return;
     int n = rng[i].y - rng[i].x;
     cnt[i] = (n + kChunk - 1) / kChunk;
+    for (int a = 0; a < 3; ++a) {
+        bb[6 * i + a] = OrdT<T>::hi;      // min
+        bb[6 * i + 3 + a] = OrdT<T>::lo;  // max
+    }
 }
 
 __global__ void k_chunk_fill(const int2 *rng, int K, const int32_t *chunk_off, int32_t *chunk_node) {
@@ -117,21 +141,12 @@ __global__ void k_chunk_fill(const int2 *rng, int K, const int32_t *chunk_off, i
 }
 
 template <typename T>
-__global__ void k_bbox_init(typename OrdT<T>::type *bb, int K) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= K) return;
-    for (int a = 0; a < 3; ++a) {
-        bb[6 * i + a] = OrdT<T>::hi;      // min
-        bb[6 * i + 3 + a] = OrdT<T>::lo;  // max
-    }
-}
-
-template <typename T>
 __global__ void __launch_bounds__(kChunk) k_bbox(const typename Vec4<T>::type *__restrict__ xyz, const int2 *rng,
                                                  const int32_t *chunk_node, const int32_t *chunk_off,
-                                                 typename OrdT<T>::type *bb) {
+                                                 const int64_t *n_chunks, typename OrdT<T>::type *bb) {
     using O = typename OrdT<T>::type;
     int q = blockIdx.x;
+    if (q >= *n_chunks) return;  // the grid is a bound on the level's chunks
     int node = chunk_node[q];
     int k = q - chunk_off[node];
     int s = rng[node].x + k * kChunk;
@@ -174,41 +189,54 @@ __global__ void __launch_bounds__(kChunk) k_bbox(const typename Vec4<T>::type *_
     }
 }
 
-// centre / half / radius / leaf decision for every node of the level
+// centre / half / radius of a node from its bounding box; true if it is a leaf
 template <typename T>
-__global__ void k_finalize(const typename OrdT<T>::type *bb, const int2 *rng, int K, int level, int leaf_size,
-                           int max_depth, typename Vec4<T>::type *center, typename Vec4<T>::type *half,
-                           uint8_t *is_leaf, int *warn) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= K) return;
+__device__ __forceinline__ bool node_geometry(const T *mn, const T *mx, int n, int level, int leaf_size, int max_depth,
+                                              typename Vec4<T>::type &cv, typename Vec4<T>::type &hv, bool &too_deep) {
     T c[3], h[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        T mn = from_ord(bb[6 * i + a]);
-        T mx = from_ord(bb[6 * i + 3 + a]);
-        c[a] = rn_mul((T)0.5, rn_add(mn, mx));
-        T hh = rn_mul((T)0.5, rn_sub(mx, mn));
+        c[a] = rn_mul((T)0.5, rn_add(mn[a], mx[a]));
+        T hh = rn_mul((T)0.5, rn_sub(mx[a], mn[a]));
         h[a] = hh < (T)0 ? (T)0 : hh;
     }
-    T r = radius_of(h[0], h[1], h[2]);
-    typename Vec4<T>::type cv, hv;
     cv.x = c[0];
     cv.y = c[1];
     cv.z = c[2];
-    cv.w = r;
+    cv.w = radius_of(h[0], h[1], h[2]);
     hv.x = h[0];
     hv.y = h[1];
     hv.z = h[2];
     hv.w = 0;  // expansion scale, filled after the root radius is known
-    center[i] = cv;
-    half[i] = hv;
-    int n = rng[i].y - rng[i].x;
     T hmax = h[0] > h[1] ? h[0] : h[1];
     hmax = hmax > h[2] ? hmax : h[2];
-    bool degenerate = (double)hmax < 1e-7;
-    bool leaf = n <= leaf_size || level >= max_depth || degenerate;
+    const bool degenerate = (double)hmax < 1e-7;
+    too_deep = level >= max_depth && n > leaf_size && !degenerate;
+    return n <= leaf_size || level >= max_depth || degenerate;
+}
+
+// centre / half / radius / leaf decision for every node of the level
+template <typename T>
+__global__ void k_finalize(const typename OrdT<T>::type *bb, const int2 *rng, int K, int level, int leaf_size,
+                           int max_depth, typename Vec4<T>::type *center, typename Vec4<T>::type *half,
+                           uint8_t *is_leaf, int32_t *lev, BuildState *st) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= K) return;
+    T mn[3], mx[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        mn[a] = from_ord(bb[6 * i + a]);
+        mx[a] = from_ord(bb[6 * i + 3 + a]);
+    }
+    typename Vec4<T>::type cv, hv;
+    bool deep;
+    const bool leaf = node_geometry<T>(mn, mx, rng[i].y - rng[i].x, level, leaf_size, max_depth, cv, hv, deep);
+    center[i] = cv;
+    half[i] = hv;
     is_leaf[i] = leaf ? 1 : 0;
-    if (level >= max_depth && n > leaf_size && !degenerate) atomicAdd(warn, 1);
+    lev[i] = level;
+    if (leaf) atomicAdd(&st->leaves, 1);
+    if (deep) atomicAdd(&st->warn, 1);
 }
 
 template <typename T>
@@ -220,10 +248,11 @@ __device__ __forceinline__ int octant_of(const typename Vec4<T>::type &p, const 
 template <typename T>
 __global__ void __launch_bounds__(kChunk) k_octant_counts(const typename Vec4<T>::type *__restrict__ xyz,
                                                           const int2 *rng, const int32_t *chunk_node,
-                                                          const int32_t *chunk_off,
+                                                          const int32_t *chunk_off, const int64_t *n_chunks,
                                                           const typename Vec4<T>::type *center,
                                                           const uint8_t *is_leaf, int32_t *ccnt) {
     int q = blockIdx.x;
+    if (q >= *n_chunks) return;
     int node = chunk_node[q];
     if (is_leaf[node]) return;
     __shared__ int cnt[8];
@@ -240,7 +269,8 @@ __global__ void __launch_bounds__(kChunk) k_octant_counts(const typename Vec4<T>
 
 // per split node: exclusive prefix of octant counts over its chunks, totals
 __global__ void k_node_octants(const int2 *rng, int K, const int32_t *chunk_off, const uint8_t *is_leaf,
-                               int32_t *ccnt, int32_t *oct_start, int32_t *oct_cnt, int32_t *n_children) {
+                               int32_t *ccnt, int32_t *oct_start, int32_t *oct_cnt, int32_t *n_children,
+                               int32_t *max_child) {
     // all 32 lanes stay to the end: the shuffles below use the full mask
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     int i = t >> 3, o = t & 7;
@@ -268,25 +298,35 @@ __global__ void k_node_octants(const int2 *rng, int K, const int32_t *chunk_off,
     oct_cnt[8 * i + o] = run;
     oct_start[8 * i + o] = rng[i].x + base;
     if (o == 0) n_children[i] = nz;
+    if (run > 0) atomicMax(max_child, run);
 }
 
-// stable scatter of the chunk's points into their octant slots
+// a leaf's points to their final place (the buffer's positions are the tree's)
+// or stable scatter of the chunk's points into their octant slots
 template <typename T>
 __global__ void __launch_bounds__(kChunk) k_scatter(const typename Vec4<T>::type *__restrict__ xyz,
                                                     const int32_t *__restrict__ perm, const int2 *rng,
                                                     const int32_t *chunk_node, const int32_t *chunk_off,
-                                                    const typename Vec4<T>::type *center, const uint8_t *is_leaf,
-                                                    const int32_t *ccnt, const int32_t *oct_start,
-                                                    typename Vec4<T>::type *xyz_out, int32_t *perm_out) {
+                                                    const int64_t *n_chunks, const typename Vec4<T>::type *center,
+                                                    const uint8_t *is_leaf, const int32_t *ccnt,
+                                                    const int32_t *oct_start, typename Vec4<T>::type *xyz_out,
+                                                    int32_t *perm_out, typename Vec4<T>::type *pts, int32_t *index_map) {
     int q = blockIdx.x;
+    if (q >= *n_chunks) return;
     int node = chunk_node[q];
-    if (is_leaf[node]) return;
     __shared__ int wcnt[32][8];
     int k = q - chunk_off[node];
     int s = rng[node].x + k * kChunk;
     int e = min(rng[node].y, s + kChunk);
     int i = s + threadIdx.x;
     bool valid = i < e;
+    if (is_leaf[node]) {
+        if (valid) {
+            pts[i] = xyz[i];
+            index_map[i] = perm[i];
+        }
+        return;
+    }
     int o = -1;
     typename Vec4<T>::type v;
     if (valid) {
@@ -321,21 +361,139 @@ __global__ void __launch_bounds__(kChunk) k_scatter(const typename Vec4<T>::type
     }
 }
 
+// A whole level whose nodes hold at most kChunk points each: one block per
+// node does the bounding box, the node's geometry, its octants and the stable
+// scatter with the points in registers (4 a thread).  Replaces 8 launches and
+// three passes over the points.
+constexpr int kSmallThreads = 256;
+constexpr int kSmallTiles = kChunk / kSmallThreads;
+
 template <typename T>
-__global__ void __launch_bounds__(kChunk) k_copy_back(const int2 *rng, const int32_t *chunk_node,
-                                                      const int32_t *chunk_off, const uint8_t *is_leaf,
-                                                      const typename Vec4<T>::type *xyz_tmp, const int32_t *perm_tmp,
-                                                      typename Vec4<T>::type *xyz, int32_t *perm) {
-    int q = blockIdx.x;
-    int node = chunk_node[q];
-    if (is_leaf[node]) return;
-    int k = q - chunk_off[node];
-    int s = rng[node].x + k * kChunk;
-    int e = min(rng[node].y, s + kChunk);
-    int i = s + threadIdx.x;
-    if (i < e) {
-        xyz[i] = xyz_tmp[i];
-        perm[i] = perm_tmp[i];
+__global__ void __launch_bounds__(kSmallThreads) k_small_level(
+    const typename Vec4<T>::type *__restrict__ xyz, const int32_t *__restrict__ perm, const int2 *rng, int level,
+    int leaf_size, int max_depth, typename Vec4<T>::type *center, typename Vec4<T>::type *half, uint8_t *is_leaf,
+    int32_t *lev, int32_t *oct_start, int32_t *oct_cnt, int32_t *n_children, typename Vec4<T>::type *xyz_out,
+    int32_t *perm_out, typename Vec4<T>::type *pts, int32_t *index_map, BuildState *st) {
+    using T4 = typename Vec4<T>::type;
+    using O = typename OrdT<T>::type;
+    constexpr int kWarps = kSmallThreads / 32;
+    __shared__ O smn[kWarps][3], smx[kWarps][3];
+    __shared__ T4 sc;
+    __shared__ int sleaf;
+    __shared__ int wcnt[kSmallTiles * kWarps][8], ostart[8];
+    const int node = blockIdx.x;
+    const int s = rng[node].x, e = rng[node].y;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    T4 v[kSmallTiles];
+    O mn[3] = {OrdT<T>::hi, OrdT<T>::hi, OrdT<T>::hi}, mx[3] = {OrdT<T>::lo, OrdT<T>::lo, OrdT<T>::lo};
+#pragma unroll
+    for (int t = 0; t < kSmallTiles; ++t) {
+        const int i = s + t * kSmallThreads + threadIdx.x;
+        if (i >= e) continue;
+        v[t] = xyz[i];
+        const O x = ord_of(v[t].x), y = ord_of(v[t].y), z = ord_of(v[t].z);
+        mn[0] = x < mn[0] ? x : mn[0];
+        mn[1] = y < mn[1] ? y : mn[1];
+        mn[2] = z < mn[2] ? z : mn[2];
+        mx[0] = x > mx[0] ? x : mx[0];
+        mx[1] = y > mx[1] ? y : mx[1];
+        mx[2] = z > mx[2] ? z : mx[2];
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const O y = __shfl_xor_sync(0xffffffffu, mn[a], o);
+            mn[a] = y < mn[a] ? y : mn[a];
+            const O z = __shfl_xor_sync(0xffffffffu, mx[a], o);
+            mx[a] = z > mx[a] ? z : mx[a];
+        }
+    }
+    if (lane == 0)
+        for (int a = 0; a < 3; ++a) {
+            smn[w][a] = mn[a];
+            smx[w][a] = mx[a];
+        }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        T lo[3], hi[3];
+        for (int a = 0; a < 3; ++a) {
+            O m0 = smn[0][a], m1 = smx[0][a];
+            for (int ww = 1; ww < kWarps; ++ww) {
+                m0 = smn[ww][a] < m0 ? smn[ww][a] : m0;
+                m1 = smx[ww][a] > m1 ? smx[ww][a] : m1;
+            }
+            lo[a] = from_ord(m0);
+            hi[a] = from_ord(m1);
+        }
+        T4 cv, hv;
+        bool deep;
+        const bool leaf = node_geometry<T>(lo, hi, e - s, level, leaf_size, max_depth, cv, hv, deep);
+        center[node] = cv;
+        half[node] = hv;
+        is_leaf[node] = leaf ? 1 : 0;
+        lev[node] = level;
+        if (leaf) {
+            n_children[node] = 0;
+            atomicAdd(&st->leaves, 1);
+        }
+        if (deep) atomicAdd(&st->warn, 1);
+        sc = cv;
+        sleaf = leaf ? 1 : 0;
+    }
+    __syncthreads();
+    if (sleaf) {
+#pragma unroll
+        for (int t = 0; t < kSmallTiles; ++t) {
+            const int i = s + t * kSmallThreads + threadIdx.x;
+            if (i >= e) continue;
+            pts[i] = v[t];
+            index_map[i] = perm[i];
+        }
+        if (threadIdx.x < 8) oct_cnt[8 * node + threadIdx.x] = 0;
+        return;
+    }
+    const T4 c = sc;
+    const unsigned lt = (1u << lane) - 1u;
+    int oct[kSmallTiles], rank[kSmallTiles];
+#pragma unroll
+    for (int t = 0; t < kSmallTiles; ++t) {
+        const int i = s + t * kSmallThreads + threadIdx.x;
+        oct[t] = i < e ? octant_of<T>(v[t], c) : -1;
+        rank[t] = 0;
+#pragma unroll
+        for (int oo = 0; oo < 8; ++oo) {
+            const unsigned m = __ballot_sync(0xffffffffu, oct[t] == oo);
+            if (oct[t] == oo) rank[t] = __popc(m & lt);
+            if (lane == 0) wcnt[t * kWarps + w][oo] = __popc(m);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        int run = 0;
+        for (int ww = 0; ww < kSmallTiles * kWarps; ++ww) {
+            const int q = wcnt[ww][threadIdx.x];
+            wcnt[ww][threadIdx.x] = run;
+            run += q;
+        }
+        int base = 0, nz = 0;
+        for (int oo = 0; oo < 8; ++oo) {
+            const int q = __shfl_sync(0xffu, run, oo);
+            if (oo < (int)threadIdx.x) base += q;
+            nz += q > 0 ? 1 : 0;
+        }
+        oct_cnt[8 * node + threadIdx.x] = run;
+        oct_start[8 * node + threadIdx.x] = s + base;
+        ostart[threadIdx.x] = s + base;
+        if (threadIdx.x == 0) n_children[node] = nz;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < kSmallTiles; ++t) {
+        if (oct[t] < 0) continue;
+        const int dest = ostart[oct[t]] + wcnt[t * kWarps + w][oct[t]] + rank[t];
+        xyz_out[dest] = v[t];
+        perm_out[dest] = perm[s + t * kSmallThreads + threadIdx.x];
     }
 }
 
@@ -378,24 +536,28 @@ __global__ void k_dfs_ids(const int2 *rng, const int32_t *lev, int64_t M, const 
     dfs[b] = base_at[s] + lev[b] - minlev_at[s];
 }
 
-// Floor of the expansion scale of each tree of the forest: 2^-40 of its
-// root's radius (1 for a root of radius 0); level 0 holds the roots.
-template <typename T>
-__global__ void k_root_floors(const typename Vec4<T>::type *root_cen, int K, T *floors) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= K) return;
-    const T r = root_cen[k].w;
-    floors[k] = r > (T)0 ? (T)(r * (T)9.094947017729282e-13) : (T)1;
+// Floor of the expansion scale of a tree: 2^-40 of its root's radius (1 for a
+// root of radius 0).
+template <typename T> __device__ __forceinline__ T scale_floor(T r) {
+    return r > (T)0 ? (T)(r * (T)9.094947017729282e-13) : (T)1;
 }
 
+// Nodes into DFS order.  The expansion scale is the node's radius, but not
+// below its tree's floor nor below 1/8 of the parent's scale: a node whose
+// points coincide (radius 0, e.g. a single-point leaf) would otherwise get the
+// global floor, and every M2L pair into it would have a source/target scale
+// ratio far above the fast kernel's range.  Any positive scale is exact
+// algebra; this one keeps the ratios O(10).  Multiplying by 1/8 rounds
+// monotonically, so the largest of the ancestors' radii, each multiplied
+// level by level, is what passing the scale down the levels gives.
 template <typename T>
 __global__ void k_permute_nodes(int64_t M, const int32_t *dfs, const int2 *rng, const int32_t *lev,
                                 const int32_t *par_bfs, const int32_t *ch_bfs,
                                 const typename Vec4<T>::type *cen, const typename Vec4<T>::type *hal,
-                                const uint8_t *leaf, const int32_t *root, const T *floors, int2 *o_rng,
+                                const uint8_t *leaf, const int32_t *root, int2 *o_rng,
                                 int32_t *o_lev, int32_t *o_par,
                                 int32_t *o_ch, typename Vec4<T>::type *o_cen, typename Vec4<T>::type *o_hal,
-                                uint8_t *o_leaf, int32_t *level_nodes) {
+                                uint8_t *o_leaf, int32_t *level_nodes, int32_t *flag) {
     int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= M) return;
     int d = dfs[b];
@@ -408,34 +570,24 @@ __global__ void k_permute_nodes(int64_t M, const int32_t *dfs, const int2 *rng, 
     }
     o_cen[d] = cen[b];
     typename Vec4<T>::type h = hal[b];
-    const T r = cen[b].w, scale_floor = floors[root[b]];
-    h.w = r > scale_floor ? r : scale_floor;
+    const T lo = scale_floor<T>(cen[root[b]].w);
+    T a = cen[b].w;
+    a = a > lo ? a : lo;
+    int up = 0;  // levels between the node and the ancestor
+    for (int q = par_bfs[b]; q >= 0; q = par_bfs[q]) {
+        ++up;
+        T r = cen[q].w;
+        r = r > lo ? r : lo;
+        for (int k = 0; k < up; ++k) r = rn_mul(r, (T)0.125);
+        a = a > r ? a : r;
+    }
+    h.w = a;
     o_hal[d] = h;
     o_leaf[d] = leaf[b];
     level_nodes[b] = d;
+    flag[d] = leaf[b];
 }
 
-// Expansion scale of one level's nodes: at least 1/8 of the parent's scale.
-// A node whose points coincide (radius 0, e.g. a single-point leaf) would
-// otherwise get the global floor, and every M2L pair into it would have a
-// source/target scale ratio far above the fast kernel's range.  Any positive
-// scale is exact algebra; this one keeps the ratios O(10).
-template <typename T>
-__global__ void k_scale_from_parent(const int32_t *__restrict__ nodes, int count, const int32_t *__restrict__ parent,
-                                    typename Vec4<T>::type *half) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const int d = nodes[i];
-    const int p = parent[d];
-    if (p < 0) return;
-    const T lo = half[p].w * (T)0.125;
-    if (half[d].w < lo) half[d].w = lo;
-}
-
-__global__ void k_leaf_flags(const uint8_t *leaf, int64_t M, int32_t *flag) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < M) flag[i] = leaf[i];
-}
 __global__ void k_leaf_compact(const uint8_t *leaf, int64_t M, const int32_t *off, int32_t *leaves) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < M && leaf[i]) leaves[off[i]] = (int32_t)i;
@@ -443,11 +595,27 @@ __global__ void k_leaf_compact(const uint8_t *leaf, int64_t M, const int32_t *of
 
 inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
-// One level's working set.
-template <typename T> struct Level {
-    int K = 0;
-    int base = 0;  // BFS id of the level's first node
-    DevBuf rng, parent, center, half, leaf, children, root;
+// The nodes of all levels so far, in BFS order.
+template <typename T> struct BfsNodes {
+    using T4 = typename Vec4<T>::type;
+    DevBuf rng, parent, root, lev, center, half, leaf, children;
+    int64_t cap = 0;
+    // room for `want` nodes, at least doubled; the first `keep` nodes stay
+    int ensure(int64_t want, int64_t keep, cudaStream_t s) {
+        if (want <= cap) return EDFMM_OK;
+        const int64_t nc = std::max<int64_t>(want, 2 * cap);
+        DevBuf *bufs[] = {&rng, &parent, &root, &lev, &center, &half, &leaf, &children};
+        const size_t sz[] = {sizeof(int2), 4, 4, 4, sizeof(T4), sizeof(T4), 1, 32};
+        for (int i = 0; i < 8; ++i) {
+            DevBuf nb;
+            if (int rc = nb.reserve(sz[i] * (size_t)nc)) return rc;
+            if (keep > 0)
+                EDFMM_CUDA_TRY(cudaMemcpyAsync(nb.p, bufs[i]->p, sz[i] * (size_t)keep, cudaMemcpyDeviceToDevice, s));
+            *bufs[i] = std::move(nb);  // the old block is reused in stream order, or freed behind the copy
+        }
+        cap = nc;
+        return EDFMM_OK;
+    }
 };
 
 __global__ void k_inst_node_off(const int32_t *level_nodes, int K, int32_t M, int32_t *off) {
@@ -478,136 +646,107 @@ int build_impl(const void *points_dev, int64_t n, int leaf_size, int max_depth, 
     }
     if (n >= (int64_t)INT32_MAX) return fail(EDFMM_ERR_ARG, "n_points must be < 2^31");
 
-    DevBuf xyz, xyz_tmp, perm, perm_tmp, warn, scan_tmp, total;
-    if ((rc = xyz.reserve(sizeof(T4) * n)) || (rc = xyz_tmp.reserve(sizeof(T4) * n)) ||
-        (rc = perm.reserve(sizeof(int32_t) * n)) || (rc = perm_tmp.reserve(sizeof(int32_t) * n)) ||
-        (rc = warn.reserve(sizeof(int))) || (rc = total.reserve(sizeof(int64_t))))
+    const int K0 = inst_off ? n_inst : 1;
+    DevBuf xyz[2], perm[2], state, scan_tmp, chunks, d_off;
+    BfsNodes<T> B;
+    if ((rc = xyz[0].reserve(sizeof(T4) * n)) || (rc = xyz[1].reserve(sizeof(T4) * n)) ||
+        (rc = perm[0].reserve(sizeof(int32_t) * n)) || (rc = perm[1].reserve(sizeof(int32_t) * n)) ||
+        (rc = state.reserve(sizeof(BuildState))) || (rc = chunks.reserve(sizeof(int64_t))) ||
+        (rc = tree.pts.reserve(sizeof(T4) * n)) || (rc = tree.index_map.reserve(sizeof(int32_t) * n)) ||
+        (rc = B.ensure(std::max<int64_t>(1024, K0 + 4 * n / std::max(leaf_size, 2)), 0, s)))
         return rc;
-    EDFMM_CUDA_TRY(cudaMemsetAsync(warn.p, 0, sizeof(int), s));
-    k_init_points<T><<<nblk(n, 256), 256, 0, s>>>(static_cast<const T *>(points_dev), n, dptr<T4>(xyz), dptr<int32_t>(perm));
+    BuildState *st = dptr<BuildState>(state);
+    EDFMM_CUDA_TRY(cudaMemsetAsync(st, 0, sizeof(BuildState), s));
+    int64_t largest = n;  // points of the level's largest node
+    if (inst_off) {
+        if ((rc = d_off.reserve(sizeof(int64_t) * (K0 + 1)))) return rc;
+        EDFMM_CUDA_TRY(cudaMemcpyAsync(d_off.p, inst_off, sizeof(int64_t) * (K0 + 1), cudaMemcpyHostToDevice, s));
+        largest = 0;
+        for (int k = 0; k < K0; ++k) largest = std::max(largest, inst_off[k + 1] - inst_off[k]);
+    }
+    k_init_points<T><<<nblk(std::max<int64_t>(n, K0), 256), 256, 0, s>>>(
+        static_cast<const T *>(points_dev), n, dptr<T4>(xyz[0]), dptr<int32_t>(perm[0]), dptr<int64_t>(d_off), K0,
+        dptr<int2>(B.rng), dptr<int32_t>(B.parent), dptr<int32_t>(B.root));
     EDFMM_LAUNCH_CHECK("k_init_points");
 
-    std::vector<Level<T>> levels;
-    levels.emplace_back();
-    const int K0 = inst_off ? n_inst : 1;
-    std::vector<int2> h_r0(K0);
-    std::vector<int32_t> h_p0(K0, -1), h_root0(K0);
-    {
-        Level<T> &L0 = levels.back();
-        L0.K = K0;
-        L0.base = 0;
-        if ((rc = L0.rng.reserve(sizeof(int2) * K0)) || (rc = L0.parent.reserve(sizeof(int32_t) * K0)) ||
-            (rc = L0.root.reserve(sizeof(int32_t) * K0)))
-            return rc;
-        for (int k = 0; k < K0; ++k) {
-            h_r0[k] = inst_off ? make_int2((int)inst_off[k], (int)inst_off[k + 1]) : make_int2(0, (int)n);
-            h_root0[k] = k;
-        }
-        EDFMM_CUDA_TRY(cudaMemcpyAsync(L0.rng.p, h_r0.data(), sizeof(int2) * K0, cudaMemcpyHostToDevice, s));
-        EDFMM_CUDA_TRY(cudaMemcpyAsync(L0.parent.p, h_p0.data(), sizeof(int32_t) * K0, cudaMemcpyHostToDevice, s));
-        EDFMM_CUDA_TRY(cudaMemcpyAsync(L0.root.p, h_root0.data(), sizeof(int32_t) * K0, cudaMemcpyHostToDevice, s));
-    }
     DevBuf cnt, off, chunk_node, bb, ccnt, oct_start, oct_cnt, nchild, child_off;
-    int64_t total_nodes = K0;  // the roots
+    std::vector<int32_t> level_off(1, 0);  // BFS id of each level's first node
+    int64_t total_nodes = K0;              // the roots
+    BuildState h{};
     for (int lev = 0;; ++lev) {
-        Level<T> &L = levels[lev];
-        const int K = L.K;
-        if ((rc = L.center.reserve(sizeof(T4) * K)) || (rc = L.half.reserve(sizeof(T4) * K)) ||
-            (rc = L.leaf.reserve(K)) || (rc = L.children.reserve(sizeof(int32_t) * 8 * K)) ||
-            (rc = cnt.reserve(sizeof(int32_t) * K)) || (rc = off.reserve(sizeof(int32_t) * K)) ||
-            (rc = bb.reserve(sizeof(O) * 6 * K)) || (rc = oct_start.reserve(sizeof(int32_t) * 8 * K)) ||
-            (rc = oct_cnt.reserve(sizeof(int32_t) * 8 * K)) || (rc = nchild.reserve(sizeof(int32_t) * K)) ||
-            (rc = child_off.reserve(sizeof(int32_t) * K)) || (rc = scan_tmp.reserve(scan_tmp_bytes(K))))
+        const int base = level_off[lev], K = (int)(total_nodes - base);
+        level_off.push_back((int32_t)total_nodes);
+        if ((rc = oct_start.reserve(sizeof(int32_t) * 8 * K)) || (rc = oct_cnt.reserve(sizeof(int32_t) * 8 * K)) ||
+            (rc = nchild.reserve(sizeof(int32_t) * K)) || (rc = child_off.reserve(sizeof(int32_t) * K)) ||
+            (rc = scan_tmp.reserve(scan_tmp_bytes(K))))
             return rc;
-        const int2 *rng = dptr<int2>(L.rng);
-        // chunks
-        k_chunk_counts<<<nblk(K, 256), 256, 0, s>>>(rng, K, dptr<int32_t>(cnt));
-        EDFMM_LAUNCH_CHECK("k_chunk_counts");
-        if ((rc = scan_exclusive(dptr<int32_t>(cnt), dptr<int32_t>(off), K, dptr<int64_t>(total), scan_tmp.p, s))) return rc;
-        int64_t Q = 0;
-        EDFMM_CUDA_TRY(cudaMemcpyAsync(&Q, total.p, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        EDFMM_CUDA_TRY(cudaStreamSynchronize(s));
-        if ((rc = chunk_node.reserve(sizeof(int32_t) * Q)) || (rc = ccnt.reserve(sizeof(int32_t) * 8 * Q))) return rc;
-        k_chunk_fill<<<nblk(K, 256), 256, 0, s>>>(rng, K, dptr<int32_t>(off), dptr<int32_t>(chunk_node));
-        EDFMM_LAUNCH_CHECK("k_chunk_fill");
-        // bounding boxes and node geometry
-        k_bbox_init<T><<<nblk(K, 256), 256, 0, s>>>(dptr<O>(bb), K);
-        EDFMM_LAUNCH_CHECK("k_bbox_init");
-        k_bbox<T><<<(unsigned)Q, kChunk, 0, s>>>(dptr<T4>(xyz), rng, dptr<int32_t>(chunk_node), dptr<int32_t>(off), dptr<O>(bb));
-        EDFMM_LAUNCH_CHECK("k_bbox");
-        k_finalize<T><<<nblk(K, 256), 256, 0, s>>>(dptr<O>(bb), rng, K, lev, leaf_size, max_depth, dptr<T4>(L.center),
-                                                     dptr<T4>(L.half), dptr<uint8_t>(L.leaf), dptr<int>(warn));
-        EDFMM_LAUNCH_CHECK("k_finalize");
-        // partition the points of split nodes
-        k_octant_counts<T><<<(unsigned)Q, kChunk, 0, s>>>(dptr<T4>(xyz), rng, dptr<int32_t>(chunk_node), dptr<int32_t>(off),
-                                                          dptr<T4>(L.center), dptr<uint8_t>(L.leaf), dptr<int32_t>(ccnt));
-        EDFMM_LAUNCH_CHECK("k_octant_counts");
-        k_node_octants<<<nblk((int64_t)K * 8, 256), 256, 0, s>>>(rng, K, dptr<int32_t>(off), dptr<uint8_t>(L.leaf),
-                                                                 dptr<int32_t>(ccnt), dptr<int32_t>(oct_start),
-                                                                 dptr<int32_t>(oct_cnt), dptr<int32_t>(nchild));
-        EDFMM_LAUNCH_CHECK("k_node_octants");
-        k_scatter<T><<<(unsigned)Q, kChunk, 0, s>>>(dptr<T4>(xyz), dptr<int32_t>(perm), rng, dptr<int32_t>(chunk_node),
-                                                    dptr<int32_t>(off), dptr<T4>(L.center), dptr<uint8_t>(L.leaf),
-                                                    dptr<int32_t>(ccnt), dptr<int32_t>(oct_start), dptr<T4>(xyz_tmp),
-                                                    dptr<int32_t>(perm_tmp));
-        EDFMM_LAUNCH_CHECK("k_scatter");
-        k_copy_back<T><<<(unsigned)Q, kChunk, 0, s>>>(rng, dptr<int32_t>(chunk_node), dptr<int32_t>(off),
-                                                      dptr<uint8_t>(L.leaf), dptr<T4>(xyz_tmp), dptr<int32_t>(perm_tmp),
-                                                      dptr<T4>(xyz), dptr<int32_t>(perm));
-        EDFMM_LAUNCH_CHECK("k_copy_back");
-        // next level
-        if ((rc = scan_exclusive(dptr<int32_t>(nchild), dptr<int32_t>(child_off), K, dptr<int64_t>(total), scan_tmp.p, s)))
-            return rc;
-        int64_t Kn = 0;
-        EDFMM_CUDA_TRY(cudaMemcpyAsync(&Kn, total.p, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        EDFMM_CUDA_TRY(cudaStreamSynchronize(s));
-        int next_base = L.base + K;
-        Level<T> next;
-        next.K = (int)Kn;
-        next.base = next_base;
-        if (Kn > 0) {
-            if ((rc = next.rng.reserve(sizeof(int2) * Kn)) || (rc = next.parent.reserve(sizeof(int32_t) * Kn)) ||
-                (rc = next.root.reserve(sizeof(int32_t) * Kn)))
+        const int2 *rng = dptr<int2>(B.rng) + base;
+        T4 *center = dptr<T4>(B.center) + base, *half = dptr<T4>(B.half) + base;
+        uint8_t *leaf = dptr<uint8_t>(B.leaf) + base;
+        int32_t *blev = dptr<int32_t>(B.lev) + base;
+        const T4 *in = dptr<T4>(xyz[lev & 1]);
+        const int32_t *pin = dptr<int32_t>(perm[lev & 1]);
+        T4 *out = dptr<T4>(xyz[(lev + 1) & 1]);
+        int32_t *pout = dptr<int32_t>(perm[(lev + 1) & 1]);
+        if (largest <= kChunk) {
+            k_small_level<T><<<(unsigned)K, kSmallThreads, 0, s>>>(
+                in, pin, rng, lev, leaf_size, max_depth, center, half, leaf, blev, dptr<int32_t>(oct_start),
+                dptr<int32_t>(oct_cnt), dptr<int32_t>(nchild), out, pout, dptr<T4>(tree.pts),
+                dptr<int32_t>(tree.index_map), st);
+            EDFMM_LAUNCH_CHECK("k_small_level");
+        } else {
+            // chunks of the level's nodes: at most one short chunk a node
+            const int64_t Q = n / kChunk + K;
+            if ((rc = cnt.reserve(sizeof(int32_t) * K)) || (rc = off.reserve(sizeof(int32_t) * K)) ||
+                (rc = bb.reserve(sizeof(O) * 6 * K)) || (rc = chunk_node.reserve(sizeof(int32_t) * Q)) ||
+                (rc = ccnt.reserve(sizeof(int32_t) * 8 * Q)))
                 return rc;
+            const int64_t *nq = dptr<int64_t>(chunks);
+            k_chunk_counts<T><<<nblk(K, 256), 256, 0, s>>>(rng, K, dptr<int32_t>(cnt), dptr<O>(bb));
+            EDFMM_LAUNCH_CHECK("k_chunk_counts");
+            if ((rc = scan_exclusive(dptr<int32_t>(cnt), dptr<int32_t>(off), K, dptr<int64_t>(chunks), scan_tmp.p, s)))
+                return rc;
+            k_chunk_fill<<<nblk(K, 256), 256, 0, s>>>(rng, K, dptr<int32_t>(off), dptr<int32_t>(chunk_node));
+            EDFMM_LAUNCH_CHECK("k_chunk_fill");
+            // bounding boxes and node geometry
+            k_bbox<T><<<(unsigned)Q, kChunk, 0, s>>>(in, rng, dptr<int32_t>(chunk_node), dptr<int32_t>(off), nq, dptr<O>(bb));
+            EDFMM_LAUNCH_CHECK("k_bbox");
+            k_finalize<T><<<nblk(K, 256), 256, 0, s>>>(dptr<O>(bb), rng, K, lev, leaf_size, max_depth, center, half,
+                                                         leaf, blev, st);
+            EDFMM_LAUNCH_CHECK("k_finalize");
+            // partition the points of split nodes
+            k_octant_counts<T><<<(unsigned)Q, kChunk, 0, s>>>(in, rng, dptr<int32_t>(chunk_node), dptr<int32_t>(off), nq,
+                                                              center, leaf, dptr<int32_t>(ccnt));
+            EDFMM_LAUNCH_CHECK("k_octant_counts");
+            k_node_octants<<<nblk((int64_t)K * 8, 256), 256, 0, s>>>(
+                rng, K, dptr<int32_t>(off), leaf, dptr<int32_t>(ccnt), dptr<int32_t>(oct_start), dptr<int32_t>(oct_cnt),
+                dptr<int32_t>(nchild), &st->max_child[lev + 1]);
+            EDFMM_LAUNCH_CHECK("k_node_octants");
+            k_scatter<T><<<(unsigned)Q, kChunk, 0, s>>>(in, pin, rng, dptr<int32_t>(chunk_node), dptr<int32_t>(off), nq,
+                                                        center, leaf, dptr<int32_t>(ccnt), dptr<int32_t>(oct_start), out,
+                                                        pout, dptr<T4>(tree.pts), dptr<int32_t>(tree.index_map));
+            EDFMM_LAUNCH_CHECK("k_scatter");
         }
-        k_make_children<<<nblk(K, 256), 256, 0, s>>>(K, dptr<uint8_t>(L.leaf), dptr<int32_t>(oct_start),
-                                                     dptr<int32_t>(oct_cnt), dptr<int32_t>(child_off), L.base, next_base,
-                                                     dptr<int2>(next.rng), dptr<int32_t>(next.parent),
-                                                     dptr<int32_t>(L.children), dptr<int32_t>(L.root),
-                                                     dptr<int32_t>(next.root));
+        // next level
+        if ((rc = scan_exclusive(dptr<int32_t>(nchild), dptr<int32_t>(child_off), K, &st->next, scan_tmp.p, s))) return rc;
+        EDFMM_CUDA_TRY(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, s));
+        EDFMM_CUDA_TRY(cudaStreamSynchronize(s));
+        const int64_t Kn = h.next;
+        if (total_nodes + Kn >= (int64_t)INT32_MAX / 8) return fail(EDFMM_ERR_ARG, "octree too large");
+        if ((rc = B.ensure(total_nodes + Kn, total_nodes, s))) return rc;
+        const int next_base = (int)total_nodes;
+        k_make_children<<<nblk(K, 256), 256, 0, s>>>(
+            K, dptr<uint8_t>(B.leaf) + base, dptr<int32_t>(oct_start), dptr<int32_t>(oct_cnt), dptr<int32_t>(child_off),
+            base, next_base, dptr<int2>(B.rng) + next_base, dptr<int32_t>(B.parent) + next_base,
+            dptr<int32_t>(B.children) + 8 * (int64_t)base, dptr<int32_t>(B.root) + base, dptr<int32_t>(B.root) + next_base);
         EDFMM_LAUNCH_CHECK("k_make_children");
         if (Kn == 0) break;
+        if (largest > kChunk) largest = h.max_child[lev + 1];
         total_nodes += Kn;
-        if (total_nodes >= (int64_t)INT32_MAX / 8) return fail(EDFMM_ERR_ARG, "octree too large");
-        levels.push_back(std::move(next));
     }
-    const int64_t M = total_nodes;
-    const int nlev = (int)levels.size();
-    // concatenate the levels (BFS order)
-    DevBuf b_rng, b_lev, b_par, b_ch, b_cen, b_hal, b_leaf, b_root;
-    if ((rc = b_rng.reserve(sizeof(int2) * M)) || (rc = b_lev.reserve(sizeof(int32_t) * M)) ||
-        (rc = b_par.reserve(sizeof(int32_t) * M)) || (rc = b_ch.reserve(sizeof(int32_t) * 8 * M)) ||
-        (rc = b_cen.reserve(sizeof(T4) * M)) || (rc = b_hal.reserve(sizeof(T4) * M)) || (rc = b_leaf.reserve(M)) ||
-        (rc = b_root.reserve(sizeof(int32_t) * M)))
-        return rc;
-    std::vector<int32_t> hlev(M);
-    tree.level_offsets.assign(nlev + 1, 0);
-    for (int l = 0; l < nlev; ++l) {
-        Level<T> &L = levels[l];
-        size_t b = L.base;
-        EDFMM_CUDA_TRY(cudaMemcpyAsync(dptr<int2>(b_rng) + b, L.rng.p, sizeof(int2) * L.K, cudaMemcpyDeviceToDevice, s));
-        EDFMM_CUDA_TRY(cudaMemcpyAsync(dptr<int32_t>(b_par) + b, L.parent.p, sizeof(int32_t) * L.K, cudaMemcpyDeviceToDevice, s));
-        EDFMM_CUDA_TRY(cudaMemcpyAsync(dptr<int32_t>(b_ch) + 8 * b, L.children.p, sizeof(int32_t) * 8 * L.K,
-                                       cudaMemcpyDeviceToDevice, s));
-        EDFMM_CUDA_TRY(cudaMemcpyAsync(dptr<T4>(b_cen) + b, L.center.p, sizeof(T4) * L.K, cudaMemcpyDeviceToDevice, s));
-        EDFMM_CUDA_TRY(cudaMemcpyAsync(dptr<T4>(b_hal) + b, L.half.p, sizeof(T4) * L.K, cudaMemcpyDeviceToDevice, s));
-        EDFMM_CUDA_TRY(cudaMemcpyAsync(dptr<uint8_t>(b_leaf) + b, L.leaf.p, L.K, cudaMemcpyDeviceToDevice, s));
-        EDFMM_CUDA_TRY(cudaMemcpyAsync(dptr<int32_t>(b_root) + b, L.root.p, sizeof(int32_t) * L.K,
-                                       cudaMemcpyDeviceToDevice, s));
-        for (int i = 0; i < L.K; ++i) hlev[b + i] = l;
-        tree.level_offsets[l + 1] = L.base + L.K;
-    }
-    EDFMM_CUDA_TRY(cudaMemcpyAsync(b_lev.p, hlev.data(), sizeof(int32_t) * M, cudaMemcpyHostToDevice, s));
+    const int64_t M = total_nodes, nleaves = h.leaves;
+    const int nlev = (int)level_off.size() - 1;
+    tree.level_offsets = level_off;
     // DFS numbering
     DevBuf cnt_at, minlev_at, base_at, dfs;
     if ((rc = cnt_at.reserve(sizeof(int32_t) * n)) || (rc = minlev_at.reserve(sizeof(int32_t) * n)) ||
@@ -616,60 +755,36 @@ int build_impl(const void *points_dev, int64_t n, int leaf_size, int max_depth, 
         return rc;
     EDFMM_CUDA_TRY(cudaMemsetAsync(cnt_at.p, 0, sizeof(int32_t) * n, s));
     EDFMM_CUDA_TRY(cudaMemsetAsync(minlev_at.p, 0x7f, sizeof(int32_t) * n, s));
-    k_dfs_marks<<<nblk(M, 256), 256, 0, s>>>(dptr<int2>(b_rng), dptr<int32_t>(b_lev), M, dptr<int32_t>(cnt_at),
+    k_dfs_marks<<<nblk(M, 256), 256, 0, s>>>(dptr<int2>(B.rng), dptr<int32_t>(B.lev), M, dptr<int32_t>(cnt_at),
                                              dptr<int32_t>(minlev_at));
     EDFMM_LAUNCH_CHECK("k_dfs_marks");
     if ((rc = scan_exclusive(dptr<int32_t>(cnt_at), dptr<int32_t>(base_at), n, nullptr, scan_tmp.p, s))) return rc;
-    k_dfs_ids<<<nblk(M, 256), 256, 0, s>>>(dptr<int2>(b_rng), dptr<int32_t>(b_lev), M, dptr<int32_t>(base_at),
+    k_dfs_ids<<<nblk(M, 256), 256, 0, s>>>(dptr<int2>(B.rng), dptr<int32_t>(B.lev), M, dptr<int32_t>(base_at),
                                            dptr<int32_t>(minlev_at), dptr<int32_t>(dfs));
     EDFMM_LAUNCH_CHECK("k_dfs_ids");
-    // each root's radius sets the floor of its tree's expansion scales
-    DevBuf floors;
-    if ((rc = floors.reserve(sizeof(T) * K0))) return rc;
-    k_root_floors<T><<<nblk(K0, 256), 256, 0, s>>>(dptr<T4>(b_cen), K0, dptr<T>(floors));
-    EDFMM_LAUNCH_CHECK("k_root_floors");
+    DevBuf flag, loff;
     if ((rc = tree.range.reserve(sizeof(int2) * M)) || (rc = tree.level.reserve(sizeof(int32_t) * M)) ||
         (rc = tree.parent.reserve(sizeof(int32_t) * M)) || (rc = tree.children.reserve(sizeof(int32_t) * 8 * M)) ||
         (rc = tree.center.reserve(sizeof(T4) * M)) || (rc = tree.half.reserve(sizeof(T4) * M)) ||
-        (rc = tree.is_leaf.reserve(M)) || (rc = tree.level_nodes.reserve(sizeof(int32_t) * M)))
+        (rc = tree.is_leaf.reserve(M)) || (rc = tree.level_nodes.reserve(sizeof(int32_t) * M)) ||
+        (rc = tree.leaves.reserve(sizeof(int32_t) * nleaves)) || (rc = flag.reserve(sizeof(int32_t) * M)) ||
+        (rc = loff.reserve(sizeof(int32_t) * M)))
         return rc;
     k_permute_nodes<T><<<nblk(M, 256), 256, 0, s>>>(
-        M, dptr<int32_t>(dfs), dptr<int2>(b_rng), dptr<int32_t>(b_lev), dptr<int32_t>(b_par), dptr<int32_t>(b_ch),
-        dptr<T4>(b_cen), dptr<T4>(b_hal), dptr<uint8_t>(b_leaf), dptr<int32_t>(b_root), dptr<T>(floors),
+        M, dptr<int32_t>(dfs), dptr<int2>(B.rng), dptr<int32_t>(B.lev), dptr<int32_t>(B.parent),
+        dptr<int32_t>(B.children), dptr<T4>(B.center), dptr<T4>(B.half), dptr<uint8_t>(B.leaf), dptr<int32_t>(B.root),
         dptr<int2>(tree.range), dptr<int32_t>(tree.level),
         dptr<int32_t>(tree.parent), dptr<int32_t>(tree.children), dptr<T4>(tree.center), dptr<T4>(tree.half),
-        dptr<uint8_t>(tree.is_leaf), dptr<int32_t>(tree.level_nodes));
+        dptr<uint8_t>(tree.is_leaf), dptr<int32_t>(tree.level_nodes), dptr<int32_t>(flag));
     EDFMM_LAUNCH_CHECK("k_permute_nodes");
-    for (size_t l = 1; l + 1 < tree.level_offsets.size(); ++l) {
-        const int a = tree.level_offsets[l], b = tree.level_offsets[l + 1];
-        if (b <= a) continue;
-        k_scale_from_parent<T><<<nblk(b - a, 256), 256, 0, s>>>(dptr<int32_t>(tree.level_nodes) + a, b - a,
-                                                                 dptr<int32_t>(tree.parent), dptr<T4>(tree.half));
-        EDFMM_LAUNCH_CHECK("k_scale_from_parent");
-    }
     // leaves
-    DevBuf flag, loff;
-    if ((rc = flag.reserve(sizeof(int32_t) * M)) || (rc = loff.reserve(sizeof(int32_t) * M))) return rc;
-    k_leaf_flags<<<nblk(M, 256), 256, 0, s>>>(dptr<uint8_t>(tree.is_leaf), M, dptr<int32_t>(flag));
-    EDFMM_LAUNCH_CHECK("k_leaf_flags");
-    if ((rc = scan_exclusive(dptr<int32_t>(flag), dptr<int32_t>(loff), M, dptr<int64_t>(total), scan_tmp.p, s))) return rc;
-    int64_t nleaves = 0;
-    int hwarn = 0;
-    EDFMM_CUDA_TRY(cudaMemcpyAsync(&nleaves, total.p, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    EDFMM_CUDA_TRY(cudaMemcpyAsync(&hwarn, warn.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    EDFMM_CUDA_TRY(cudaStreamSynchronize(s));
-    if ((rc = tree.leaves.reserve(sizeof(int32_t) * nleaves))) return rc;
+    if ((rc = scan_exclusive(dptr<int32_t>(flag), dptr<int32_t>(loff), M, nullptr, scan_tmp.p, s))) return rc;
     k_leaf_compact<<<nblk(M, 256), 256, 0, s>>>(dptr<uint8_t>(tree.is_leaf), M, dptr<int32_t>(loff), dptr<int32_t>(tree.leaves));
     EDFMM_LAUNCH_CHECK("k_leaf_compact");
-    // points in tree order: keep xyz (charges filled per matvec), permutation
-    if ((rc = tree.pts.reserve(sizeof(T4) * n)) || (rc = tree.index_map.reserve(sizeof(int32_t) * n))) return rc;
-    EDFMM_CUDA_TRY(cudaMemcpyAsync(tree.pts.p, xyz.p, sizeof(T4) * n, cudaMemcpyDeviceToDevice, s));
-    EDFMM_CUDA_TRY(cudaMemcpyAsync(tree.index_map.p, perm.p, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s));
-    EDFMM_CUDA_TRY(cudaStreamSynchronize(s));
     tree.n_nodes = M;
     tree.n_leaves = nleaves;
     tree.max_level = nlev - 1;
-    tree.depth_warnings = hwarn;
+    tree.depth_warnings = h.warn;
     tree.n_inst = 0;
     if (inst_off) {
         // instance k owns the DFS range [root_k, root_{k+1}) (roots are BFS 0..K0-1)
