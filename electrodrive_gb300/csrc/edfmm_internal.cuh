@@ -1,6 +1,8 @@
 // Internal declarations shared by the libedfmm translation units.
 #pragma once
 
+#include <algorithm>
+
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -317,6 +319,20 @@ int lists_build_two(const DevTree &src_tree, const DevTree &tgt_tree, double the
 // ---------------------------------------------------------------------------
 inline int num_coeffs(int p) { return (p + 1) * (p + 2) / 2; }
 
+// The FP32 and two-float kernels read the multipoles by columns: groups of 32
+// nodes, word w (16 bytes) of node s at [(s / 32) * words * 32 + w * 32 + s % 32].
+// The lanes of a warp hold consecutive sources of one target's row, which come
+// in runs of siblings with consecutive node ids, so that a load takes a few
+// 128-byte lines where rows take one line per lane.
+constexpr int kColNodes = 32;
+#ifdef __CUDACC__
+__host__ __device__ __forceinline__ int64_t col_of(int64_t s, int words) {
+    return (s / kColNodes) * ((int64_t)words * kColNodes) + s % kColNodes;
+}
+#endif
+// nodes of an expansion buffer: whole groups
+inline int64_t padded_nodes(int64_t n) { return (std::max<int64_t>(n, 1) + kColNodes - 1) / kColNodes * kColNodes; }
+
 // M2L pairs whose source radius exceeds 256x the target radius, as CSR rows
 // by target (FP32 plans only; empty for uniform trees).
 struct ExtremeRows {
@@ -329,14 +345,17 @@ struct FmmBuffers {
     int p = 8;
     int nc = 45;
     int nc_pad = 46;  // per-node stride in complex numbers (even: 16-byte rows for float)
+    // rows of padded_nodes(n_nodes) nodes
     DevBuf multipoles;  // complex T, n_nodes x nc_pad
     DevBuf locals;      // complex T, n_nodes x nc_pad
-    DevBuf translated;  // complex T, n_nodes x nc_pad: each node's multipole moved to its parent's centre
+    // complex T, n_nodes x nc_pad: each node's multipole moved to its parent's
+    // centre (M2M), then, in FP32, the multipoles by columns (M2L)
+    DevBuf translated;
     ExtremeRows extreme, extreme_swapped;
     InstMask mask;  // set around the steps of a batched solve
     // FP64 plans: EDFMM_ARITH_TWO_FLOAT runs M2L and the near field in
     // two-float arithmetic on the FP32 pipe (twofloat.cuh); mult_tf holds
-    // the multipoles split into (hi, lo) pairs for the two-float M2L
+    // the multipoles split into (hi, lo) pairs, by columns, for the two-float M2L
     int arith = EDFMM_ARITH_NATIVE;
     DevBuf mult_tf;
     // launch shapes the autotuner may change (edfmm_plan_set_launch)

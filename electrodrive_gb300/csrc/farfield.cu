@@ -84,12 +84,39 @@ __global__ void k_split_nodes(const double4 *__restrict__ center, const double4 
     out[2 * i] = make_float4(x.hi, x.lo, y.hi, y.lo);
     out[2 * i + 1] = make_float4(z.hi, z.lo, a.hi, a.lo);
 }
-__global__ void k_split_coeffs(const double2 *__restrict__ in, int64_t n, float4 *__restrict__ out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double2 c = in[i];
-    const tf32x2 re = tf_from_double(c.x), im = tf_from_double(c.y);
-    out[i] = make_float4(re.hi, re.lo, im.hi, im.lo);
+// Multipoles into the column layout that the M2L kernels read (m2l_rot.cuh):
+// 16-byte words of 32 nodes' rows through shared memory, coalesced on both
+// sides.  FP32: a word is two coefficients; SPLIT: an FP64 coefficient becomes
+// (re hi, re lo, im hi, im lo).
+template <bool SPLIT>
+__global__ void __launch_bounds__(256) k_mult_columns(const float4 *__restrict__ in, int64_t n_nodes, int words,
+                                                      float4 *__restrict__ out) {
+    extern __shared__ float4 col_tile[];  // [32][words + 1]
+    const int64_t n0 = (int64_t)blockIdx.x * kColNodes;
+    const int nodes = (int)min((int64_t)kColNodes, n_nodes - n0);
+    for (int k = threadIdx.x; k < nodes * words; k += blockDim.x) {
+        float4 x = in[n0 * words + k];
+        if constexpr (SPLIT) {
+            const double2 c = *reinterpret_cast<const double2 *>(&x);
+            const tf32x2 re = tf_from_double(c.x), im = tf_from_double(c.y);
+            x = make_float4(re.hi, re.lo, im.hi, im.lo);
+        }
+        col_tile[(k / words) * (words + 1) + k % words] = x;
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < words * kColNodes; k += blockDim.x) {
+        const int s = k % kColNodes, w = k / kColNodes;
+        if (s < nodes) out[n0 * words + k] = col_tile[s * (words + 1) + w];
+    }
+}
+template <bool SPLIT>
+int mult_columns(const FmmBuffers &buf, int64_t n_nodes, const DevBuf &out, cudaStream_t s) {
+    const int words = SPLIT ? buf.nc_pad : buf.nc_pad / 2;
+    const size_t smem = sizeof(float4) * kColNodes * (size_t)(words + 1);
+    k_mult_columns<SPLIT><<<nblk(n_nodes, kColNodes), 256, smem, s>>>(dptr<float4>(buf.multipoles), n_nodes, words,
+                                                                      dptr<float4>(out));
+    EDFMM_LAUNCH_CHECK("k_mult_columns");
+    return EDFMM_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -1171,9 +1198,7 @@ int m2l_impl(const DevTree &tree, const DevTree &stree, const DevLists &lists, c
     if (sizeof(T) == 8 && buf.arith == EDFMM_ARITH_TWO_FLOAT && buf.p >= 6 && buf.p <= 8 && tree.nodes_tf.p &&
         stree.nodes_tf.p && sbuf.mult_tf.p) {
         // the source multipoles split once per node, then the pairs
-        const int64_t nq = stree.n_nodes * (int64_t)sbuf.nc_pad;
-        k_split_coeffs<<<nblk(nq, 256), 256, 0, s>>>(dptr<double2>(sbuf.multipoles), nq, dptr<float4>(sbuf.mult_tf));
-        EDFMM_LAUNCH_CHECK("k_split_coeffs");
+        if (int rc = mult_columns<true>(sbuf, stree.n_nodes, sbuf.mult_tf, s)) return rc;
         int rc = launch_m2l_rot_tf(buf.p, M, off, src, rows, tree.nodes_tf.p, tree.half.p, stree.nodes_tf.p, stree.half.p,
                                    sbuf.mult_tf.p, buf.locals.p, buf.nc_pad, buf.mask, buf.m2l_tf_block,
                                    buf.m2l_packed != 0, s);
@@ -1181,8 +1206,13 @@ int m2l_impl(const DevTree &tree, const DevTree &stree, const DevLists &lists, c
         else if (rc != EDFMM_ERR_UNSUPPORTED) return rc;
     }
     if (!two_float) {
+        // FP32 reads the multipoles by columns; `translated` is free once M2M has run
+        if constexpr (sizeof(T) == 4) {
+            if (int rc = mult_columns<false>(sbuf, stree.n_nodes, sbuf.translated, s)) return rc;
+        }
         if (int rc = launch_m2l_rot(sizeof(T) == 8 ? EDFMM_F64 : EDFMM_F32, buf.p, M, off, src, rows, tree.center.p,
-                                    tree.half.p, stree.center.p, stree.half.p, sbuf.multipoles.p, buf.locals.p,
+                                    tree.half.p, stree.center.p, stree.half.p,
+                                    sizeof(T) == 8 ? sbuf.multipoles.p : sbuf.translated.p, buf.locals.p,
                                     buf.nc_pad, buf.mask, s))
             return rc;
         if (sizeof(T) == 8) return EDFMM_OK;  // FP64 has the range for any scale ratio the tree produces
@@ -1241,7 +1271,7 @@ int prepare_two_float(DevTree &tree, FmmBuffers &buf, cudaStream_t s) {
     const int64_t M = std::max<int64_t>(tree.n_nodes, 1);
     int rc;
     if ((rc = tree.nodes_tf.reserve(sizeof(float4) * 2 * (size_t)M))) return rc;
-    if ((rc = buf.mult_tf.reserve(sizeof(float4) * (size_t)buf.nc_pad * (size_t)M))) return rc;
+    if ((rc = buf.mult_tf.reserve(sizeof(float4) * (size_t)buf.nc_pad * (size_t)padded_nodes(tree.n_nodes)))) return rc;
     if (tree.n_nodes > 0) {
         k_split_nodes<<<nblk(tree.n_nodes, 256), 256, 0, s>>>(dptr<double4>(tree.center), dptr<double4>(tree.half),
                                                               tree.n_nodes, dptr<float4>(tree.nodes_tf));

@@ -297,19 +297,17 @@ __device__ __forceinline__ void axial(V &v, const T (&h)[P + 1]) {
 // 3.82 ms at p = 8)
 template <typename T, int P> __host__ __device__ constexpr bool rot_binomial() { return !(sizeof(T) == 4 && P >= 8); }
 
-// One pair (FP32): translated locals of source row Mrow added to acc.
+// One pair (FP32): translated locals of the source with column Mcol added to acc.
 template <int P, typename V, typename A>
-__device__ __forceinline__ void rot_pair(V &v, A &acc, const float2 *__restrict__ Mrow, float c, float dx, float dy,
+__device__ __forceinline__ void rot_pair(V &v, A &acc, const float4 *__restrict__ Mcol, float c, float dx, float dy,
                                          float dz) {
-    // rows are read two coefficients per 16-byte load (rows of an even number
-    // of coefficients, 16-byte aligned): half the scattered loads
     float4 x4{};
 #pragma unroll
     for (int n = 0; n <= P; ++n) {
 #pragma unroll
         for (int m = 0; m <= n; ++m) {
             const int q = tri(n, m);
-            if ((q & 1) == 0) x4 = reinterpret_cast<const float4 *>(Mrow)[q >> 1];
+            if ((q & 1) == 0) x4 = __ldg(Mcol + (q >> 1) * kColNodes);  // two coefficients
             const float2 x = (q & 1) == 0 ? make_float2(x4.x, x4.y) : make_float2(x4.z, x4.w);
             if (m == 0) {
                 v.set(n * n, x.x);
@@ -388,12 +386,19 @@ __host__ __device__ constexpr bool pk_started(int I) {
 // One warp per target row, one lane per (target, source) pair.  The warps of
 // a block run the same number of rounds of pairs, with a barrier between
 // rounds, so that the warps of an SM walk the long straight-line pair code
-// close together and share its instruction fetches.
+// close together and share its instruction fetches.  Three warps a scheduler
+// (168 registers, 46 KB of accumulators a block) must cover every latency:
+// sources are read by columns and a round's source ids one round ahead.  30.6 M
+// pairs of order 8: 3,178 us with rows (L1 at 64% of its wavefronts, a line
+// per lane and load), 2,769 with columns (their copy, 8 us, included), 2,637
+// with the ids ahead (1,620 us at the FP32 pipe's full rate; issue slots 64%
+// used).  Reading the sources' centres ahead too: 2,766; four blocks (128
+// registers, spills): 3,130.
 template <int P>
 __global__ void __launch_bounds__(kRotThreads, rot_binomial<float, P>() ? 4 : 3)
     k_m2l_rot(int64_t n_nodes, const int32_t *__restrict__ off, const int32_t *__restrict__ src,
               const int32_t *__restrict__ rows, const float4 *__restrict__ tcenter, const float4 *__restrict__ thalf,
-              const float4 *__restrict__ center, const float4 *__restrict__ half, const float2 *__restrict__ Mexp,
+              const float4 *__restrict__ center, const float4 *__restrict__ half, const float4 *__restrict__ Mcols,
               float2 *__restrict__ Lexp, int nc_pad, const InstMask mask) {
     using T = float;
     using T2 = float2;
@@ -423,16 +428,18 @@ __global__ void __launch_bounds__(kRotThreads, rot_binomial<float, P>() ? 4 : 3)
     if (lane == 0) atomicMax(&max_rounds, (e - b + 31) >> 5);
     __syncthreads();
     const int rounds = max_rounds;
+    int sn = b + lane < e ? __ldg(src + b + lane) : 0;  // the next round's source
     for (int r = 0; r < rounds; ++r) {
         __syncthreads();
         const int k = b + r * 32 + lane;
         if (k >= e) continue;
-        const int s = __ldg(src + k);
+        const int s = sn;
+        if (k + 32 < e) sn = __ldg(src + k + 32);
         const float4 cs = center[s];
         const T c = half[s].w * iaL;
         if (c > kRotExtremeRatio) continue;  // translated by k_m2l_generic
         RegV<T, NV> v;
-        rot_pair<P>(v, acc, Mexp + (int64_t)s * nc_pad, c, (ct.x - cs.x) * iaL, (ct.y - cs.y) * iaL,
+        rot_pair<P>(v, acc, Mcols + col_of(s, nc_pad >> 1), c, (ct.x - cs.x) * iaL, (ct.y - cs.y) * iaL,
                     (ct.z - cs.z) * iaL);
     }
     if (!live) return;
@@ -787,17 +794,17 @@ template <int STRIDE> struct SmemSplit {
     }
 };
 
-// One pair: v <- the translated locals (real block basis) of source row Mrow
-// (split multipoles: (re hi, re lo, im hi, im lo) per coefficient).
+// One pair: v <- the translated locals (real block basis) of the source with
+// column Mcol (split multipoles: (re hi, re lo, im hi, im lo) per coefficient).
 template <int P, bool PK, typename V>
-__device__ __forceinline__ void rot_pair_tf(V &v, const float4 *__restrict__ Mrow, tf32x2 c, tf32x2 dx, tf32x2 dy,
+__device__ __forceinline__ void rot_pair_tf(V &v, const float4 *__restrict__ Mcol, tf32x2 c, tf32x2 dx, tf32x2 dy,
                                             tf32x2 dz) {
     using T = tf32x2;
 #pragma unroll
     for (int n = 0; n <= P; ++n) {
 #pragma unroll
         for (int m = 0; m <= n; ++m) {
-            const float4 x = Mrow[tri(n, m)];
+            const float4 x = __ldg(Mcol + tri(n, m) * kColNodes);
             if (m == 0) {
                 v.set(n * n, T(x.x, x.y));
             } else {
@@ -841,7 +848,7 @@ __global__ void __launch_bounds__(NT, 256 / NT)
                  const int32_t *__restrict__ rows,
                  const float4 *__restrict__ tnodes, const double4 *__restrict__ thalf,
                  const float4 *__restrict__ snodes, const double4 *__restrict__ half,
-                 const float4 *__restrict__ Mexp, double2 *__restrict__ Lexp, int nc_pad, const InstMask mask) {
+                 const float4 *__restrict__ Mcols, double2 *__restrict__ Lexp, int nc_pad, const InstMask mask) {
     using T = tf32x2;
     constexpr int NV = (P + 1) * (P + 1), NR = (NV + 31) / 32;
     extern __shared__ __align__(16) unsigned char rot_smem[];
@@ -890,7 +897,7 @@ __global__ void __launch_bounds__(NT, 256 / NT)
             if (!(half[s].w * iaL > (double)kRotExtremeRatio)) {
                 have = true;
                 const float4 u = snodes[2 * s], w = snodes[2 * s + 1];
-                rot_pair_tf<P, PK>(v, Mexp + (int64_t)s * nc_pad, T(w.z, w.w) * iaT, (ctx - T(u.x, u.y)) * iaT,
+                rot_pair_tf<P, PK>(v, Mcols + col_of(s, nc_pad), T(w.z, w.w) * iaT, (ctx - T(u.x, u.y)) * iaT,
                                    (cty - T(u.z, u.w)) * iaT, (ctz - T(w.x, w.y)) * iaT);
             }
         }
@@ -1109,7 +1116,7 @@ int launch_rot(int64_t M, const int32_t *off, const int32_t *src, const int32_t 
         return fail(EDFMM_ERR_CUDA, std::string("k_m2l_rot shared memory attribute: ") + cudaGetErrorString(attr));
     k_m2l_rot<P><<<nblk(M * 32, NT), NT, smem, s>>>(
         M, off, src, rows, static_cast<const float4 *>(tcen), static_cast<const float4 *>(thal),
-        static_cast<const float4 *>(cen), static_cast<const float4 *>(hal), static_cast<const float2 *>(Mx),
+        static_cast<const float4 *>(cen), static_cast<const float4 *>(hal), static_cast<const float4 *>(Mx),
         static_cast<float2 *>(Lx), nc_pad, mask);
     EDFMM_LAUNCH_CHECK("k_m2l_rot");
     return EDFMM_OK;

@@ -104,7 +104,7 @@ int alloc_expansions(edfmm_plan *p, int dtype, int expansion_order, cudaStream_t
     p->fmm.p = expansion_order;
     p->fmm.nc = num_coeffs(expansion_order);
     p->fmm.nc_pad = (p->fmm.nc + 1) & ~1;
-    size_t esz = (dtype == EDFMM_F64 ? 16 : 8) * (size_t)p->fmm.nc_pad * (size_t)std::max<int64_t>(p->tree.n_nodes, 1);
+    size_t esz = (dtype == EDFMM_F64 ? 16 : 8) * (size_t)p->fmm.nc_pad * (size_t)padded_nodes(p->tree.n_nodes);
     int rc = p->fmm.multipoles.reserve(esz);
     if (!rc) rc = p->fmm.locals.reserve(esz);
     if (!rc) rc = p->fmm.translated.reserve(esz);
@@ -151,7 +151,7 @@ int finish_plan(edfmm_plan *p, int dtype, int expansion_order, cudaStream_t s) {
     p->fmm.nc = num_coeffs(expansion_order);
     p->fmm.nc_pad = (p->fmm.nc + 1) & ~1;
     const size_t esz = (dtype == EDFMM_F64 ? 16 : 8) * (size_t)p->fmm.nc_pad *
-                       (size_t)std::max<int64_t>(p->tree.n_nodes, 1);
+                       (size_t)padded_nodes(p->tree.n_nodes);
     DevBuf *exp[] = {&p->fmm.multipoles, &p->fmm.locals, &p->fmm.translated};
     int rc = grid_prepare(p->tree, s);
     if (!rc) rc = settle_buffers(p->tree, p->lists, exp, 3, esz, p->block, s);
@@ -597,7 +597,7 @@ int edfmm_plan_set_order(edfmm_plan *p, int expansion_order, void *stream) {
     p->fmm.nc = num_coeffs(expansion_order);
     p->fmm.nc_pad = (p->fmm.nc + 1) & ~1;
     size_t esz = (p->tree.dtype == EDFMM_F64 ? 16 : 8) * (size_t)p->fmm.nc_pad *
-                 (size_t)std::max<int64_t>(p->tree.n_nodes, 1);
+                 (size_t)padded_nodes(p->tree.n_nodes);
     p->fmm.multipoles.release();
     p->fmm.locals.release();
     p->fmm.translated.release();
