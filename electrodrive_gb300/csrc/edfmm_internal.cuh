@@ -252,6 +252,11 @@ struct DevTree {
     DevBuf pts_grid;
     DevBuf grid_info;
     bool grid_tf = false;
+    // levels whose translations run a block per node (farfield.cu): what each
+    // node's translation to and from its parent needs, level l's nodes from
+    // frame_off[l] (-1: none)
+    DevBuf shift_frames;
+    std::vector<int64_t> frame_off;
     // batched plans: instance k owns nodes inst_node_off[k] .. inst_node_off[k+1]-1
     int n_inst = 0;
     DevBuf inst_node_off;  // int32 x (n_inst + 1)
@@ -409,6 +414,8 @@ int run_p2p(const DevTree &tree, const DevLists &lists, const FmmBuffers &buf, c
             cudaStream_t s);
 int run_l2p(const DevTree &tree, const FmmBuffers &buf, const L2pArgs &args, cudaStream_t s);
 int grid_prepare(DevTree &tree, cudaStream_t s);
+// the tree's shift_frames (once per tree)
+int shift_prepare(DevTree &tree, cudaStream_t s);
 int upload_tables();
 
 }  // namespace edfmm

@@ -282,7 +282,7 @@ __device__ __forceinline__ void fma2_into(float &sr, float &si, float xr, float 
 // ---------------------------------------------------------------------------
 // M2M / L2L fast paths (compile-time order), one launch per level.  Two forms:
 // one thread per node (FP32, levels of many nodes: registers, packed FMAs),
-// and one warp per node (FP64, and small FP32 levels; below).  Both
+// and one block per node (FP64, and small FP32 levels; below).  Both
 // translations factor the azimuth out like the M2L.  With
 // d = (c_C - c_P) / a_P = (s cos phi, s sin phi, z) and the real regular
 // harmonics rho_k^l := R_k^l(s, 0, z) (R_k^l(d) = e^{i l phi} rho_k^l,
@@ -567,18 +567,21 @@ __global__ void __launch_bounds__(kFastThreads) k_l2l_fast(const int32_t *__rest
 }
 
 // ---------------------------------------------------------------------------
-// The same translations with one warp per node, lanes over output
-// coefficients.  A thread that owns a node walks about 2,600 dependent
-// operations: 10 us however few nodes a level has in FP32, and 130 to 280 us in
-// FP64, whose pipe issues a warp's operation in 64 cycles whether one lane is
-// active or all (two FP64 lanes per SM and clock).  Spread over the lanes a
-// node takes about 45 multiply-adds per lane.  The lanes' outputs are paired
-// long with short, so that the warp's longest chain (the number of (k, l)
-// terms of its outputs) is within a few terms of the mean.  FP64, 50k-panel
-// torus, six levels: M2M 1,060 -> 127 us, L2L 640 -> 119 us.
+// The same translations with one block per node, its threads over the terms.
+// A thread that owns a node walks about 2,600 dependent operations: 10 us
+// however few nodes a level has in FP32, and 130 to 280 us in FP64, whose pipe
+// issues a warp's operation in 64 cycles whether one lane is active or all (two
+// FP64 lanes per SM and clock).  So what counts is the number of warp
+// operations, along the chain and in all.  The terms (k, l) of all outputs are
+// dealt to the threads in equal runs (12 at order 8 with 128 threads), each
+// within one output, whose partial sums its first thread adds; the azimuth
+// phases, harmonics and powers of the scale ratio of a node are laid out with
+// the plan (ShiftFrame).  A warp per node that formed them itself and took whole
+// outputs per lane (chains of 101 terms) needed 300 FP64 operations a node.
+// FP64, 50k-panel torus, six levels: M2M 1,060 (a thread per node), 136 (a
+// warp), 64 us; L2L 640, 138, 57.  FP32, 2,003 points, three and two levels:
+// M2M 29 -> 24, L2L 24 -> 18 us, launches included.
 // ---------------------------------------------------------------------------
-constexpr int kWarpNodes = 4;  // nodes (warps) per block
-
 // number of terms (k, l) of output (n, m): |l| <= k and |m - l| <= n - k (M2M),
 // or k <= P - n, |l| <= k (L2L)
 __host__ __device__ constexpr int shift_terms(int P, bool l2l, int n, int m) {
@@ -590,39 +593,68 @@ __host__ __device__ constexpr int shift_terms(int P, bool l2l, int n, int m) {
         }
     return t;
 }
-// the outputs of each lane, (n, m) packed as n * 16 + m, 255 for none: the
-// outputs by decreasing term count take the lanes in turn, back and forth
-template <int P, bool L2L> struct ShiftPlan {
-    static constexpr int NR = (ncoef(P) + 31) / 32;
-    unsigned char out[NR][32];
-    __host__ __device__ constexpr ShiftPlan() : out() {
-        int key[ncoef(P)] = {}, nm[ncoef(P)] = {};
-        int c = 0;
-        for (int n = 0; n <= P; ++n)
-            for (int m = 0; m <= n; ++m, ++c) {
-                const int t = shift_terms(P, L2L, n, m);
-                int i = c;
-                for (; i > 0 && key[i - 1] < t; --i) {
-                    key[i] = key[i - 1];
-                    nm[i] = nm[i - 1];
-                }
-                key[i] = t;
-                nm[i] = n * 16 + m;
-            }
-        for (int r = 0; r < NR; ++r)
-            for (int l = 0; l < 32; ++l) {
-                const int q = r * 32 + l;
-                out[r][(r & 1) ? 31 - l : l] = q < ncoef(P) ? (unsigned char)nm[q] : 255;
+// threads of a block: about 12 terms each
+template <int P> __host__ __device__ constexpr int shift_threads() { return P >= 7 ? 128 : (P >= 5 ? 64 : 32); }
+
+// The terms of each thread: output (n, m), first term (k, l) and the number of
+// terms; and for each output its first thread and the number of its threads.
+template <int P, bool L2L> struct ShiftSplit {
+    static constexpr int NT = shift_threads<P>();
+    unsigned char n[NT], m[NT], k[NT], cnt[NT];
+    signed char l[NT];
+    unsigned char first[ncoef(P)], parts[ncoef(P)];
+    __host__ __device__ constexpr ShiftSplit() : n(), m(), k(), cnt(), l(), first(), parts() {
+        int cap = 1;  // the smallest run that fits the threads
+        for (;; ++cap) {
+            int used = 0;
+            for (int n_ = 0; n_ <= P; ++n_)
+                for (int m_ = 0; m_ <= n_; ++m_) used += (shift_terms(P, L2L, n_, m_) + cap - 1) / cap;
+            if (used <= NT) break;
+        }
+        int t = 0, q = 0;
+        for (int n_ = 0; n_ <= P; ++n_)
+            for (int m_ = 0; m_ <= n_; ++m_, ++q) {
+                const int terms = shift_terms(P, L2L, n_, m_), np = (terms + cap - 1) / cap;
+                first[q] = (unsigned char)t;
+                parts[q] = (unsigned char)np;
+                int at = 0, part = 0;
+                for (int kk = 0; kk <= (L2L ? P - n_ : n_); ++kk)
+                    for (int ll = -kk; ll <= kk; ++ll) {
+                        const int u = L2L ? m_ + ll : m_ - ll, j = L2L ? n_ + kk : n_ - kk;
+                        if (u < -j || u > j) continue;
+                        if (part < np && at == part * terms / np) {  // equal runs
+                            n[t] = (unsigned char)n_;
+                            m[t] = (unsigned char)m_;
+                            k[t] = (unsigned char)kk;
+                            l[t] = (signed char)ll;
+                            cnt[t] = (unsigned char)((part + 1) * terms / np - at);
+                            ++t;
+                            ++part;
+                        }
+                        ++at;
+                    }
             }
     }
 };
-template <int P, bool L2L> __device__ const ShiftPlan<P, L2L> d_shift_plan{};
+template <int P, bool L2L> __device__ const ShiftSplit<P, L2L> d_shift_split{};
+
+// What a node's translation from or to its parent needs, for any order up to
+// 8: rho_k^l at k^2 + k + l, e^{i m phi}, (a_C / a_P)^n
+constexpr int kFrameP = 8, kFramePh = (kFrameP + 1) * (kFrameP + 1), kFrameFr = kFramePh + 2 * (kFrameP + 1),
+              kFrameSize = kFrameFr + kFrameP + 1;  // 108 values
+
+template <typename T, int P> struct ShiftSmem {
+    typename Pair<T>::type x[(P + 1) * (P + 1)];  // rotated input, all orders: (n, m) at n^2 + n + m
+    typename Pair<T>::type part[shift_threads<P>()];
+    T rho[(P + 1) * (P + 1)];
+    T ph[2 * (P + 1)];
+    T fr[P + 1];
+};
 
 template <typename T, int P> struct WarpShift {
-    typename Pair<T>::type x[(P + 1) * (P + 1)];  // rotated input, all orders: (n, m) at n^2 + n + m
-    T rho[(P + 1) * (P + 1)];                     // rho_k^l at k^2 + k + l
-    typename Pair<T>::type ph[P + 1];             // e^{i m phi}
-    T fr[P + 1];                                  // (a_C / a_P)^n
+    typename Pair<T>::type ph[P + 1];  // e^{i m phi}
+    T rho[(P + 1) * (P + 1)];          // rho_k^l at k^2 + k + l
+    T fr[P + 1];                       // (a_C / a_P)^n
 };
 
 // lanes 0..P: e^{i m phi}, ratio^m and column m of rho
@@ -667,33 +699,69 @@ __device__ __forceinline__ void warp_shift_frame(WarpShift<T, P> &S, const Shift
     }
 }
 
+// the frames of a level's nodes (a warp each)
+template <typename T>
+__global__ void __launch_bounds__(128) k_shift_frames(const int32_t *__restrict__ nodes, int count,
+                                                      const int32_t *__restrict__ parent,
+                                                      const typename Vec4<T>::type *__restrict__ center,
+                                                      const typename Vec4<T>::type *__restrict__ half,
+                                                      T *__restrict__ frames) {
+    constexpr int P = kFrameP;
+    __shared__ WarpShift<T, P> shifts[4];
+    const int lane = threadIdx.x & 31, i = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (i >= count) return;
+    WarpShift<T, P> &S = shifts[threadIdx.x >> 5];
+    const int node = nodes[i], par = parent[node];
+    if (par < 0) return;  // roots have no frame
+    warp_shift_frame<T, P>(S, shift_of<T>(center[node], center[par], half[node].w, half[par].w), lane);
+    __syncwarp();
+    T *o = frames + (int64_t)i * kFrameSize;
+    for (int q = lane; q < kFramePh; q += 32) o[q] = S.rho[q];
+    if (lane <= P) {
+        o[kFramePh + 2 * lane] = S.ph[lane].x;
+        o[kFramePh + 2 * lane + 1] = S.ph[lane].y;
+        o[kFrameFr + lane] = S.fr[lane];
+    }
+}
+
+template <typename T, int P>
+__device__ __forceinline__ void load_frame(ShiftSmem<T, P> &S, const T *__restrict__ fr) {
+    constexpr int NT = shift_threads<P>(), NH = (P + 1) * (P + 1);
+#pragma unroll
+    for (int q = threadIdx.x; q < NH + 3 * (P + 1); q += NT) {
+        if (q < NH) S.rho[q] = fr[q];
+        else if (q < NH + 2 * (P + 1)) S.ph[q - NH] = fr[kFramePh + q - NH];
+        else S.fr[q - NH - 2 * (P + 1)] = fr[kFrameFr + q - NH - 2 * (P + 1)];
+    }
+}
+
 // x_n^m e^{i m phi} g, stored for orders m and -m (X^{-m} = (-1)^m conj X^m)
 template <typename T, int P>
-__device__ __forceinline__ void warp_shift_put(WarpShift<T, P> &S, int n, int m, T xr, T xi, T g) {
-    const auto w = S.ph[m];
-    const T fr = w.x * g, fi = w.y * g;
-    const T yr = xr * fr - xi * fi, yi = xr * fi + xi * fr;
-    const T sg = (m & 1) ? (T)-1 : (T)1;
-    S.x[n * n + n - m] = mk2(sg * yr, -sg * yi);
+__device__ __forceinline__ void shift_put(ShiftSmem<T, P> &S, int n, int m, typename Pair<T>::type x, T g) {
+    const T fr = S.ph[2 * m] * g, fi = S.ph[2 * m + 1] * g;
+    const T yr = x.x * fr - x.y * fi, yi = x.x * fi + x.y * fr;
+    const bool odd = m & 1;
+    S.x[n * n + n - m] = mk2(odd ? -yr : yr, odd ? yi : -yi);
     S.x[n * n + n + m] = mk2(yr, yi);
 }
 
-// sum over the terms of output (n, m)
+// this thread's run of terms into its partial sum
 template <typename T, int P, bool L2L>
-__device__ __forceinline__ typename Pair<T>::type warp_shift_sum(const WarpShift<T, P> &S, int n, int m) {
-    T sr = 0, si = 0;
-    const int kmax = L2L ? P - n : n;
-    int k = 0, ri = 0, xi = n * n + n + m, left = 1;  // k = 0: the single term l = 0
-    while (true) {
+__device__ __forceinline__ void shift_terms_sum(ShiftSmem<T, P> &S, int n, int m, int k, int l, int cnt) {
+    typename Pair<T>::type s = mk2((T)0, (T)0);
+    int j = L2L ? n + k : n - k;
+    int ri = k * k + k + l, xi = j * j + j + (L2L ? m + l : m - l);
+    int left = (L2L ? min(k, j - m) : min(k, m + j)) - l + 1;  // of degree k
+    for (int t = 0; t < cnt; ++t) {
         const auto x = S.x[xi];
         const T r = S.rho[ri];
-        sr = fma(r, x.x, sr);
-        si = fma(r, x.y, si);
+        s.x = fma(r, x.x, s.x);
+        s.y = fma(r, x.y, s.y);
         ++ri;
         xi += L2L ? 1 : -1;
         if (--left == 0) {
-            if (++k > kmax) break;
-            const int j = L2L ? n + k : n - k;
+            ++k;
+            j = L2L ? n + k : n - k;
             // l from max(-k, m - j) (M2M) or max(-k, -j - m) (L2L) to min(k, m + j) or min(k, j - m)
             const int lo = max(-k, L2L ? -j - m : m - j), hi = min(k, L2L ? j - m : m + j);
             left = hi - lo + 1;
@@ -701,96 +769,123 @@ __device__ __forceinline__ typename Pair<T>::type warp_shift_sum(const WarpShift
             xi = j * j + j + (L2L ? m + lo : m - lo);
         }
     }
-    return mk2(sr, si);
+    S.part[threadIdx.x] = s;
+}
+template <typename T, int P>
+__device__ __forceinline__ typename Pair<T>::type shift_total(const ShiftSmem<T, P> &S, int first, int parts) {
+    typename Pair<T>::type v = S.part[first];
+    for (int p = 1; p < parts; ++p) {
+        v.x += S.part[first + p].x;
+        v.y += S.part[first + p].y;
+    }
+    return v;
 }
 
 template <typename T, int P>
-__global__ void __launch_bounds__(32 * kWarpNodes) k_m2m_warp(
-    const int32_t *__restrict__ nodes, int count, const uint8_t *__restrict__ is_leaf,
-    const int32_t *__restrict__ children, const int32_t *__restrict__ parent,
-    const typename Vec4<T>::type *__restrict__ center, const typename Vec4<T>::type *__restrict__ half,
-    typename Pair<T>::type *__restrict__ Mexp, typename Pair<T>::type *__restrict__ moved, int nc_pad) {
+__global__ void __launch_bounds__(shift_threads<P>()) k_m2m_node(
+    const int32_t *__restrict__ nodes, const uint8_t *__restrict__ is_leaf, const int32_t *__restrict__ children,
+    const T *__restrict__ frames, typename Pair<T>::type *__restrict__ Mexp, typename Pair<T>::type *__restrict__ moved,
+    int nc_pad) {
     using T2 = typename Pair<T>::type;
-    constexpr int NR = ShiftPlan<P, false>::NR;
-    __shared__ WarpShift<T, P> shifts[kWarpNodes];
-    const int lane = threadIdx.x & 31, i = blockIdx.x * kWarpNodes + (threadIdx.x >> 5);
-    if (i >= count) return;
-    WarpShift<T, P> &S = shifts[threadIdx.x >> 5];
-    const int node = nodes[i], par = parent[node];
-    T2 x[NR];
-    int nm[NR];
+    constexpr int NT = shift_threads<P>(), NC = ncoef(P);
+    __shared__ ShiftSmem<T, P> S;
+    const int tid = threadIdx.x, node = nodes[blockIdx.x];
+    const ShiftSplit<P, false> &D = d_shift_split<P, false>;
+    const int tn = D.n[tid], tm = D.m[tid], tk = D.k[tid], tl = D.l[tid], tc = D.cnt[tid];
+    if (frames) load_frame<T, P>(S, frames + (int64_t)blockIdx.x * kFrameSize);
+    const bool leaf = is_leaf[node];
+    T2 x[(NC + NT - 1) / NT];
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
-        nm[r] = d_shift_plan<P, false>.out[r][lane];
-        x[r] = mk2((T)0, (T)0);
-        if (nm[r] == 255) continue;
-        const int q = tri(nm[r] >> 4, nm[r] & 15);
-        if (is_leaf[node]) {
+    for (int r = 0; r < (NC + NT - 1) / NT; ++r) {
+        const int q = tid + r * NT;
+        if (q >= NC) continue;
+        if (leaf) {
             x[r] = Mexp[(int64_t)node * nc_pad + q];
         } else {
+            T2 v[8];
+#pragma unroll
             for (int o = 0; o < 8; ++o) {
                 const int ch = children[8 * node + o];
-                if (ch < 0) continue;
-                const T2 v = moved[(int64_t)ch * nc_pad + q];
-                x[r].x += v.x;
-                x[r].y += v.y;
+                v[o] = ch >= 0 ? moved[(int64_t)ch * nc_pad + q] : mk2((T)0, (T)0);
+            }
+            x[r] = v[0];
+#pragma unroll
+            for (int o = 1; o < 8; ++o) {
+                x[r].x += v[o].x;
+                x[r].y += v[o].y;
             }
             Mexp[(int64_t)node * nc_pad + q] = x[r];
         }
     }
-    if (par < 0) return;
-    const Shift<T> f = shift_of<T>(center[node], center[par], half[node].w, half[par].w);
-    warp_shift_frame<T, P>(S, f, lane);
-    __syncwarp();
+    if (!frames) return;  // the roots
+    __syncthreads();
 #pragma unroll
-    for (int r = 0; r < NR; ++r)
-        if (nm[r] != 255) warp_shift_put<T, P>(S, nm[r] >> 4, nm[r] & 15, x[r].x, x[r].y, S.fr[nm[r] >> 4]);
-    __syncwarp();
+    for (int r = 0; r < (NC + NT - 1) / NT; ++r) {
+        const int q = tid + r * NT;
+        if (q >= NC) continue;
+        int n = 0;
+        while (tri(n + 1, 0) <= q) ++n;
+        shift_put<T, P>(S, n, q - tri(n, 0), x[r], S.fr[n]);
+    }
+    __syncthreads();
+    shift_terms_sum<T, P, false>(S, tn, tm, tk, tl, tc);
+    __syncthreads();
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
-        if (nm[r] == 255) continue;
-        const int n = nm[r] >> 4, m = nm[r] & 15;
-        const T2 v = warp_shift_sum<T, P, false>(S, n, m), w = S.ph[m];
-        moved[(int64_t)node * nc_pad + tri(n, m)] = mk2(v.x * w.x + v.y * w.y, v.y * w.x - v.x * w.y);  // e^{-i m phi}
+    for (int r = 0; r < (NC + NT - 1) / NT; ++r) {
+        const int q = tid + r * NT;
+        if (q >= NC) continue;
+        int n = 0;
+        while (tri(n + 1, 0) <= q) ++n;
+        const int m = q - tri(n, 0);
+        const T2 v = shift_total<T, P>(S, D.first[q], D.parts[q]);
+        const T wx = S.ph[2 * m], wy = S.ph[2 * m + 1];
+        moved[(int64_t)node * nc_pad + q] = mk2(v.x * wx + v.y * wy, v.y * wx - v.x * wy);  // e^{-i m phi}
     }
 }
 
 template <typename T, int P>
-__global__ void __launch_bounds__(32 * kWarpNodes) k_l2l_warp(
-    const int32_t *__restrict__ nodes, int count, const int32_t *__restrict__ parent,
-    const typename Vec4<T>::type *__restrict__ center, const typename Vec4<T>::type *__restrict__ half,
-    typename Pair<T>::type *__restrict__ Lexp, int nc_pad) {
+__global__ void __launch_bounds__(shift_threads<P>()) k_l2l_node(const int32_t *__restrict__ nodes,
+                                                                 const int32_t *__restrict__ parent,
+                                                                 const T *__restrict__ frames,
+                                                                 typename Pair<T>::type *__restrict__ Lexp, int nc_pad) {
     using T2 = typename Pair<T>::type;
-    constexpr int NR = ShiftPlan<P, true>::NR;
-    __shared__ WarpShift<T, P> shifts[kWarpNodes];
-    const int lane = threadIdx.x & 31, i = blockIdx.x * kWarpNodes + (threadIdx.x >> 5);
-    if (i >= count) return;
-    WarpShift<T, P> &S = shifts[threadIdx.x >> 5];
-    const int node = nodes[i], par = parent[node];
-    if (par < 0) return;
-    T2 x[NR];
-    int nm[NR];
+    constexpr int NT = shift_threads<P>(), NC = ncoef(P);
+    __shared__ ShiftSmem<T, P> S;
+    const int tid = threadIdx.x, node = nodes[blockIdx.x], par = parent[node];
+    const ShiftSplit<P, true> &D = d_shift_split<P, true>;
+    const int tn = D.n[tid], tm = D.m[tid], tk = D.k[tid], tl = D.l[tid], tc = D.cnt[tid];
+    load_frame<T, P>(S, frames + (int64_t)blockIdx.x * kFrameSize);
+    T2 x[(NC + NT - 1) / NT], old[(NC + NT - 1) / NT];
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
-        nm[r] = d_shift_plan<P, true>.out[r][lane];
-        if (nm[r] != 255) x[r] = Lexp[(int64_t)par * nc_pad + tri(nm[r] >> 4, nm[r] & 15)];
+    for (int r = 0; r < (NC + NT - 1) / NT; ++r) {
+        const int q = tid + r * NT;
+        if (q >= NC) continue;
+        x[r] = Lexp[(int64_t)par * nc_pad + q];
+        old[r] = Lexp[(int64_t)node * nc_pad + q];
     }
-    const Shift<T> f = shift_of<T>(center[node], center[par], half[node].w, half[par].w);
-    warp_shift_frame<T, P>(S, f, lane);
-    __syncwarp();
+    __syncthreads();
 #pragma unroll
-    for (int r = 0; r < NR; ++r)
-        if (nm[r] != 255) warp_shift_put<T, P>(S, nm[r] >> 4, nm[r] & 15, x[r].x, x[r].y, (T)1);
-    __syncwarp();
+    for (int r = 0; r < (NC + NT - 1) / NT; ++r) {
+        const int q = tid + r * NT;
+        if (q >= NC) continue;
+        int n = 0;
+        while (tri(n + 1, 0) <= q) ++n;
+        shift_put<T, P>(S, n, q - tri(n, 0), x[r], (T)1);
+    }
+    __syncthreads();
+    shift_terms_sum<T, P, true>(S, tn, tm, tk, tl, tc);
+    __syncthreads();
 #pragma unroll
-    for (int r = 0; r < NR; ++r) {
-        if (nm[r] == 255) continue;
-        const int n = nm[r] >> 4, m = nm[r] & 15;
-        const T2 v = warp_shift_sum<T, P, true>(S, n, m), w = S.ph[m];
-        const T g = S.fr[n];  // (a_C / a_P)^j e^{-i u phi}
-        T2 *o = Lexp + (int64_t)node * nc_pad + tri(n, m);
-        const T2 old = *o;
-        *o = mk2(old.x + g * (v.x * w.x + v.y * w.y), old.y + g * (v.y * w.x - v.x * w.y));
+    for (int r = 0; r < (NC + NT - 1) / NT; ++r) {
+        const int q = tid + r * NT;
+        if (q >= NC) continue;
+        int n = 0;
+        while (tri(n + 1, 0) <= q) ++n;
+        const int m = q - tri(n, 0);
+        const T2 v = shift_total<T, P>(S, D.first[q], D.parts[q]);
+        const T wx = S.ph[2 * m], wy = S.ph[2 * m + 1], g = S.fr[n];  // (a_C / a_P)^j e^{-i u phi}
+        Lexp[(int64_t)node * nc_pad + q] =
+            mk2(old[r].x + g * (v.x * wx + v.y * wy), old[r].y + g * (v.y * wx - v.x * wy));
     }
 }
 
@@ -1018,56 +1113,85 @@ template <typename T> int p2m_impl(const DevTree &tree, FmmBuffers &buf, cudaStr
     return EDFMM_OK;
 }
 
-// FP32 levels up to this many nodes take a warp per node.  At order 6 a level
-// of about 3,000 nodes takes 5.3 us with a warp per node and 10.8 with a
-// thread, one of about 7,000 nodes 9.3 us with a thread; a warp's work per node
-// is ten times a thread's share, so the forms meet between the two.
-constexpr int kWarpLevel = 6144;
+// FP32 levels up to this many nodes take a block per node (FP64 all levels).
+// M2M and L2L of the 200k-panel torus (levels of 2,344 and 6,968 nodes at order
+// 6) take 62 and 43 us with the line at 2,048, 58 and 44 at 6,144, 58 and 49 at
+// 12,288; of 1,048,576 points (4,096 and 32,768 nodes at order 8) 60 and 48, 56
+// and 51, and 95 and 86 us with every level a block per node.
+constexpr int kNodeLevel = 6144;
 
 template <typename T, int P> int launch_m2m_fast(const DevTree &tree, FmmBuffers &buf, cudaStream_t s) {
-    using T4 = typename Vec4<T>::type;
     using T2 = typename Pair<T>::type;
     for (int lev = tree.max_level; lev >= 0; --lev) {
         const int lo = tree.level_offsets[lev], hi = tree.level_offsets[lev + 1];
         if (hi <= lo) continue;
         const int32_t *nodes = dptr<int32_t>(tree.level_nodes) + lo;
-        bool warp = sizeof(T) == 8 || hi - lo <= kWarpLevel;
-        if constexpr (sizeof(T) == 4) {
-            if (!warp)
-                k_m2m_fast<P><<<nblk(hi - lo, kFastThreads), kFastThreads, 0, s>>>(
-                    nodes, hi - lo, dptr<uint8_t>(tree.is_leaf), dptr<int32_t>(tree.children),
-                    dptr<int32_t>(tree.parent), dptr<float4>(tree.center), dptr<float4>(tree.half),
-                    dptr<float2>(buf.multipoles), dptr<float2>(buf.translated), buf.nc_pad);
-        }
-        if (warp)
-            k_m2m_warp<T, P><<<nblk(hi - lo, kWarpNodes), 32 * kWarpNodes, 0, s>>>(
+        const int64_t frames = tree.frame_off[lev];
+        if (frames >= 0 || lev == 0) {
+            k_m2m_node<T, P><<<(unsigned)(hi - lo), shift_threads<P>(), 0, s>>>(
+                nodes, dptr<uint8_t>(tree.is_leaf), dptr<int32_t>(tree.children),
+                lev == 0 ? nullptr : dptr<T>(tree.shift_frames) + frames * kFrameSize, dptr<T2>(buf.multipoles),
+                dptr<T2>(buf.translated), buf.nc_pad);
+        } else if constexpr (sizeof(T) == 4) {
+            k_m2m_fast<P><<<nblk(hi - lo, kFastThreads), kFastThreads, 0, s>>>(
                 nodes, hi - lo, dptr<uint8_t>(tree.is_leaf), dptr<int32_t>(tree.children), dptr<int32_t>(tree.parent),
-                dptr<T4>(tree.center), dptr<T4>(tree.half), dptr<T2>(buf.multipoles), dptr<T2>(buf.translated),
-                buf.nc_pad);
+                dptr<float4>(tree.center), dptr<float4>(tree.half), dptr<float2>(buf.multipoles),
+                dptr<float2>(buf.translated), buf.nc_pad);
+        }
         if (lev > 0) count_launch();
     }
     return EDFMM_OK;
 }
 
 template <typename T, int P> int launch_l2l_fast(const DevTree &tree, FmmBuffers &buf, cudaStream_t s) {
-    using T4 = typename Vec4<T>::type;
     using T2 = typename Pair<T>::type;
     for (int lev = 1; lev <= tree.max_level; ++lev) {
         const int lo = tree.level_offsets[lev], hi = tree.level_offsets[lev + 1];
         if (hi <= lo) continue;
         const int32_t *nodes = dptr<int32_t>(tree.level_nodes) + lo;
-        bool warp = sizeof(T) == 8 || hi - lo <= kWarpLevel;
-        if constexpr (sizeof(T) == 4) {
-            if (!warp)
-                k_l2l_fast<P><<<nblk(hi - lo, kFastThreads), kFastThreads, 0, s>>>(
-                    nodes, hi - lo, dptr<int32_t>(tree.parent), dptr<float4>(tree.center), dptr<float4>(tree.half),
-                    dptr<float2>(buf.locals), buf.nc_pad);
-        }
-        if (warp)
-            k_l2l_warp<T, P><<<nblk(hi - lo, kWarpNodes), 32 * kWarpNodes, 0, s>>>(
-                nodes, hi - lo, dptr<int32_t>(tree.parent), dptr<T4>(tree.center), dptr<T4>(tree.half),
+        const int64_t frames = tree.frame_off[lev];
+        if (frames >= 0) {
+            k_l2l_node<T, P><<<(unsigned)(hi - lo), shift_threads<P>(), 0, s>>>(
+                nodes, dptr<int32_t>(tree.parent), dptr<T>(tree.shift_frames) + frames * kFrameSize,
                 dptr<T2>(buf.locals), buf.nc_pad);
+        } else if constexpr (sizeof(T) == 4) {
+            k_l2l_fast<P><<<nblk(hi - lo, kFastThreads), kFastThreads, 0, s>>>(
+                nodes, hi - lo, dptr<int32_t>(tree.parent), dptr<float4>(tree.center), dptr<float4>(tree.half),
+                dptr<float2>(buf.locals), buf.nc_pad);
+        }
         if (lev < tree.max_level) count_launch();
+    }
+    return EDFMM_OK;
+}
+
+template <typename T> int shift_prepare_impl(DevTree &tree, cudaStream_t s) {
+    using T4 = typename Vec4<T>::type;
+    const int levels = (int)tree.level_offsets.size() - 1;
+    tree.frame_off.assign(std::max(levels, 0), -1);
+    int64_t n = 0;
+    for (int lev = 1; lev < levels; ++lev) {
+        const int count = tree.level_offsets[lev + 1] - tree.level_offsets[lev];
+        if (sizeof(T) == 4 && count > kNodeLevel) continue;
+        tree.frame_off[lev] = n;
+        n += count;
+    }
+    if (n == 0) return EDFMM_OK;
+    if (int rc = tree.shift_frames.reserve(sizeof(T) * kFrameSize * (size_t)n)) return rc;
+    for (int lev = 1; lev < levels;) {  // runs of levels that have frames lie one after another
+        if (tree.frame_off[lev] < 0) {
+            ++lev;
+            continue;
+        }
+        int end = lev + 1;
+        while (end < levels && tree.frame_off[end] >= 0) ++end;
+        const int lo = tree.level_offsets[lev], hi = tree.level_offsets[end];
+        if (hi > lo) {
+            k_shift_frames<T><<<nblk(hi - lo, 4), 128, 0, s>>>(
+                dptr<int32_t>(tree.level_nodes) + lo, hi - lo, dptr<int32_t>(tree.parent), dptr<T4>(tree.center),
+                dptr<T4>(tree.half), dptr<T>(tree.shift_frames) + tree.frame_off[lev] * kFrameSize);
+            EDFMM_LAUNCH_CHECK("k_shift_frames");
+        }
+        lev = end;
     }
     return EDFMM_OK;
 }
@@ -1249,6 +1373,10 @@ int set_charges(const DevTree &tree, const void *a, const void *b, cudaStream_t 
                                                   static_cast<const float *>(b));
     EDFMM_LAUNCH_CHECK("k_set_charges");
     return EDFMM_OK;
+}
+
+int shift_prepare(DevTree &tree, cudaStream_t s) {
+    return tree.dtype == EDFMM_F64 ? shift_prepare_impl<double>(tree, s) : shift_prepare_impl<float>(tree, s);
 }
 
 int run_p2m(const DevTree &tree, FmmBuffers &buf, cudaStream_t s) {

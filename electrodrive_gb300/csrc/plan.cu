@@ -134,7 +134,7 @@ int settle_buffers(DevTree &t, DevLists &l, DevBuf *const *exp, int n_exp, size_
                       &t.parent,   &t.children,      &t.level,       &t.is_leaf, &t.leaves,
                       &t.level_nodes, &t.inst_node_off, &l.p2p_off,  &l.p2p_src, &l.m2l_off,
                       &l.m2l_src,  &l.m2l_swapped_off, &l.m2l_swapped_src, &l.p2p_leaves, &l.m2l_rows,
-                      &t.pts_grid, &t.grid_info};
+                      &t.pts_grid, &t.grid_info,     &t.shift_frames};
     const int n = (int)(sizeof(bufs) / sizeof(bufs[0]));
     if (n_exp * esz <= ((size_t)16 << 20)) return pack_buffers(bufs, n, exp, n_exp, esz, block, s);
     int rc = pack_buffers(bufs, n, nullptr, 0, 0, block, s);
@@ -154,6 +154,7 @@ int finish_plan(edfmm_plan *p, int dtype, int expansion_order, cudaStream_t s) {
                        (size_t)padded_nodes(p->tree.n_nodes);
     DevBuf *exp[] = {&p->fmm.multipoles, &p->fmm.locals, &p->fmm.translated};
     int rc = grid_prepare(p->tree, s);
+    if (!rc) rc = shift_prepare(p->tree, s);
     if (!rc) rc = settle_buffers(p->tree, p->lists, exp, 3, esz, p->block, s);
     if (!rc) {
         cudaError_t e = cudaMemsetAsync(p->fmm.multipoles.p, 0, esz, s);
@@ -454,6 +455,7 @@ int edfmm_plan_convert(const edfmm_plan *src, int dtype, int expansion_order, vo
                     &l.m2l_swapped_off, &l.m2l_swapped_src, &l.p2p_leaves, &l.m2l_rows};
     for (size_t i = 0; !rc && i < sizeof(from) / sizeof(from[0]); ++i) rc = clone_buf(*from[i], *to[i], s);
     if (!rc) rc = grid_prepare(t, s);
+    if (!rc) rc = shift_prepare(t, s);
     if (!rc && dtype == EDFMM_F64) rc = set_charges(t, nullptr, nullptr, s);
     if (!rc) rc = alloc_expansions(p, dtype, expansion_order, s);  // synchronises the stream
     if (rc) {
@@ -815,7 +817,8 @@ static int finish_targets(edfmm_targets *t, cudaStream_t s) {
     const size_t esz = (p->tree.dtype == EDFMM_F64 ? 16 : 8) * (size_t)t->buf.nc_pad *
                        (size_t)std::max<int64_t>(t->tree.n_nodes, 1);
     DevBuf *exp[] = {&t->buf.locals};
-    int rc = settle_buffers(t->tree, t->lists, exp, 1, esz, t->block, s);
+    int rc = shift_prepare(t->tree, s);
+    if (!rc) rc = settle_buffers(t->tree, t->lists, exp, 1, esz, t->block, s);
     if (!rc) {
         cudaError_t e = cudaMemsetAsync(t->buf.locals.p, 0, esz, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
