@@ -17,13 +17,15 @@
 // one maximum and one MUFU.RSQ (16 per SM and clock: the bound).  19,997
 // panels, one matvec: 175 -> 123 us (5.03e12 rsqrt/s: 79 us).
 //
-// FP64 (k_dense_f64): the distances run on the FP32 pipe at FP64 accuracy
-// (gridpoint.cuh); two FP64 operations per interaction remain, beside 16 in
-// IEEE arithmetic, whose pipe bounded the kernel (15.8 operations at 2 per SM
-// and clock).  5,120 panels, one matvec: 770 -> 173 us.  A tile of sources
+// FP64 (k_dense_f64): the inverse distances run on the FP32 pipe at FP64
+// accuracy (gridpoint.cuh), two pairs in packed operations; one FP64 operation
+// per interaction remains, beside 16 in IEEE arithmetic, whose pipe bounded
+// the kernel (15.8 operations at 2 per SM and clock).  5,120 panels, one
+// matvec: 770 -> 160 us.  A tile of sources
 // whose coordinates are not finite, or all zero, and pairs too close for the
 // split run in IEEE FP64.
 #include <algorithm>
+#include <cmath>
 
 #include "edfmm_internal.cuh"
 #include "gridpoint.cuh"
@@ -232,15 +234,24 @@ __global__ void __launch_bounds__(kThreads) k_dense_f32(const DenseArgs<float> A
 
 // ---------------------------------------------------------------------------
 // FP64: 128 / GROUPS targets per block, one per thread; the groups of threads
-// take every GROUPS-th source of a tile
+// take every GROUPS-th pair of sources of a tile, two pairs at a time (packed
+// operations issue in half the slots, and two independent chains cover their
+// latency).  The FMA pipe is the bound, 141 cycles of a scheduler per 32
+// interactions: 5,120 panels 165 us scalar, one source at a time, with two FP64
+// operations an interaction; 154 packed (75% of the pipe's time; the rest is
+// the exact split of each tile's sources, again for every 64 targets, and the
+// uneven number of blocks per SM).
 // ---------------------------------------------------------------------------
-struct Src64 {
-    float4 u, v, w;  // (xa, xb, xc, ya), (yb, yc, za, zb), (zc, -, charge as two words)
-};
+// Sources lie in the tile in pairs, value by value (24 words a pair: the nine
+// parts of both, a gap, both charges), so that a load gives packed operands.
+constexpr int kPairWords = 24, kPairCharge = 10;  // the charges as doubles 10 and 11 of a pair
 struct Tgt64 {
     double x, y, z;
-    GridCoord gx, gy, gz;  // scaled
+    GridCoordT<float2> gx, gy, gz;  // scaled, in both halves
 };
+__device__ __forceinline__ GridCoordT<float2> grid_both(const GridCoord &g) {
+    return GridCoordT<float2>{make_float2(g.a, g.a), make_float2(g.b, g.b), make_float2(g.c, g.c)};
+}
 
 __device__ __forceinline__ unsigned high_abs(double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; }
 
@@ -265,7 +276,7 @@ __device__ __noinline__ void dense_pair_ieee(const double *c, int64_t j, int64_t
 template <int KIND, int GROUPS>
 __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> A) {
     constexpr int COMP = KIND == kField ? 3 : 1, ROWS = kThreads / GROUPS;
-    __shared__ Src64 src[kTile64];
+    __shared__ __align__(16) float src[kTile64 / 2 * kPairWords];
     __shared__ double xyz[KIND == kField ? 3 * kTile64 : 1];
     __shared__ double part[kThreads * COMP];
     __shared__ unsigned s_hi[4];
@@ -284,6 +295,9 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
     const unsigned thi = max(high_abs(T.x), max(high_abs(T.y), high_abs(T.z)));
     int kprev = INT32_MIN;
     double ex = 0, ey = 0, ez = 0;
+    auto charge = [&](int q) -> double & {
+        return reinterpret_cast<double *>(src)[(q >> 1) * (kPairWords / 2) + kPairCharge + (q & 1)];
+    };
     for (int64_t jb = j0; jb < j1; jb += kTile64) {
         const int cnt = (int)min((int64_t)kTile64, j1 - jb);
         double x = 0, y = 0, z = 0, w = 0;
@@ -302,12 +316,11 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
         int k;
         const bool split = grid_exponent(max(max(s_hi[0], s_hi[1]), max(s_hi[2], s_hi[3])), k);
         if (!split) {
-            if ((int)threadIdx.x < cnt) reinterpret_cast<double *>(&src[threadIdx.x])[0] = w;
+            if ((int)threadIdx.x < cnt) charge(threadIdx.x) = w;
             __syncthreads();
             for (int s = grp; s < cnt; s += GROUPS) {
                 double px, py, pz;
-                dense_pair_ieee<KIND>(A.c, jb + s, i, T.x, T.y, T.z, reinterpret_cast<double *>(&src[s])[0], A.k_e, px,
-                                      py, pz);
+                dense_pair_ieee<KIND>(A.c, jb + s, i, T.x, T.y, T.z, charge(s), A.k_e, px, py, pz);
                 ex += px;
                 ey += py;
                 ez += pz;
@@ -316,80 +329,94 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
         }
         const double down = grid_pow2(-k);
         if (k != kprev) {
-            T.gx = grid_split(T.x * down);
-            T.gy = grid_split(T.y * down);
-            T.gz = grid_split(T.z * down);
+            T.gx = grid_both(grid_split(T.x * down));
+            T.gy = grid_both(grid_split(T.y * down));
+            T.gz = grid_both(grid_split(T.z * down));
             kprev = k;
         }
-        if ((int)threadIdx.x < cnt) {
-            const GridCoord a = grid_split(x * down), b = grid_split(y * down), c = grid_split(z * down);
-            Src64 &S = src[threadIdx.x];
-            S.u = make_float4(a.a, a.b, a.c, b.a);
-            S.v = make_float4(b.b, b.c, c.a, c.b);
-            S.w = make_float4(c.c, 0.0f, __int_as_float(__double2loint(w)), __int_as_float(__double2hiint(w)));
+        if ((int)threadIdx.x < ((cnt + 4 * GROUPS - 1) & ~(4 * GROUPS - 1))) {
+            // padding: no charge, outside the scaled box
+            const bool real = (int)threadIdx.x < cnt;
+            const GridCoord out{3.0f, 0.0f, 0.0f};
+            const GridCoord a = real ? grid_split(x * down) : out, b = real ? grid_split(y * down) : out,
+                            c = real ? grid_split(z * down) : out;
+            float *q = src + (threadIdx.x >> 1) * kPairWords + (threadIdx.x & 1);
+            q[0] = a.a;
+            q[2] = a.b;
+            q[4] = a.c;
+            q[6] = b.a;
+            q[8] = b.b;
+            q[10] = b.c;
+            q[12] = c.a;
+            q[14] = c.b;
+            q[16] = c.c;
+            charge(threadIdx.x) = w;
             if (KIND == kField) {
                 xyz[3 * threadIdx.x] = x;
                 xyz[3 * threadIdx.x + 1] = y;
                 xyz[3 * threadIdx.x + 2] = z;
             }
-        } else if ((int)threadIdx.x < ((cnt + 2 * GROUPS - 1) & ~(2 * GROUPS - 1))) {  // padding: no charge, outside the scaled box
-            Src64 &S = src[threadIdx.x];
-            S.u = make_float4(3.0f, 0.0f, 0.0f, 3.0f);
-            S.v = make_float4(0.0f, 0.0f, 3.0f, 0.0f);
-            S.w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (KIND == kField) xyz[3 * threadIdx.x] = xyz[3 * threadIdx.x + 1] = xyz[3 * threadIdx.x + 2] = 0.0;
         }
         __syncthreads();
         // closer than the split resolves, or than the clamp: IEEE
         const float near2 = fmaxf(kGridNear2, (float)(1.0001e-24 * down * down));
         double tx = 0, ty = 0, tz = 0;  // two-level sum: tile, then chunk; the split pairs in scaled units
         double sx = 0, sy = 0, sz = 0;
-        auto load = [&](int s, GridDiff &dx, GridDiff &dy, GridDiff &dz, double &w) {
-            const float4 u = src[s].u, v = src[s].v, q = src[s].w;
-            w = __hiloint2double(__float_as_int(q.w), __float_as_int(q.z));
-            dx = grid_diff(T.gx, GridCoord{u.x, u.y, u.z});
-            dy = grid_diff(T.gy, GridCoord{u.w, v.x, v.y});
-            dz = grid_diff(T.gz, GridCoord{v.z, v.w, q.x});
-        };
-        auto add = [&](int s, const GridR2 &r2, double w) {
-            float y0;
-            unsigned ci;
-            grid_rsqrt(r2, y0, ci);
+        auto add = [&](int s, float y0, float eh, float v, double w) {
+            const double ir = grid_inv(y0, grid_ci(eh, v));
             if (KIND == kField) {
-                const double ir = grid_double(y0) * grid_one_plus(ci);
                 const double f = (A.k_e * (ir * ir * ir)) * w;
                 tx = fma(f, T.x - xyz[3 * s], tx);
                 ty = fma(f, T.y - xyz[3 * s + 1], ty);
                 tz = fma(f, T.z - xyz[3 * s + 2], tz);
             } else {
-                tx = fma(w * grid_double(y0), grid_one_plus(ci), tx);
+                tx = fma(w, ir, tx);
             }
         };
-        auto add_any = [&](int s, const GridR2 &r2, double w) {
-            if (r2.R1 < near2) {
-                if (s >= cnt) return;  // padding
-                double px, py, pz;
-                dense_pair_ieee<KIND>(A.c, jb + s, i, T.x, T.y, T.z, w, A.k_e, px, py, pz);
-                sx += px;
-                sy += py;
-                sz += pz;
-            } else {
-                add(s, r2, w);
-            }
+        auto ieee = [&](int s, double w) {
+            if (s >= cnt) return;  // padding
+            double px, py, pz;
+            dense_pair_ieee<KIND>(A.c, jb + s, i, T.x, T.y, T.z, w, A.k_e, px, py, pz);
+            sx += px;
+            sy += py;
+            sz += pz;
         };
-        for (int s = grp; s < cnt; s += 2 * GROUPS) {  // two sources side by side in the padded tile
-            GridDiff dx, dy, dz;
-            double w0, w1;
-            load(s, dx, dy, dz, w0);
-            const GridR2 r0 = grid_r2(dx, dy, dz);
-            load(s + GROUPS, dx, dy, dz, w1);
-            const GridR2 r1 = grid_r2(dx, dy, dz);
-            if (fminf(r0.R1, r1.R1) < near2) {
-                add_any(s, r0, w0);
-                add_any(s + GROUPS, r1, w1);
+        struct Pair2 {
+            float2 R1, y0, eh, v;
+            double2 w;
+        };
+        auto pair_of = [&](int s, Pair2 &p) {
+            const float4 *q = reinterpret_cast<const float4 *>(src + (s >> 1) * kPairWords);
+            const float4 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3];
+            const float2 q4 = *reinterpret_cast<const float2 *>(q + 4);
+            p.w = *reinterpret_cast<const double2 *>(q + 5);
+            const GridR2<float2> r2 = grid_r2(
+                grid_diff(T.gx, GridCoordT<float2>{make_float2(q0.x, q0.y), make_float2(q0.z, q0.w), make_float2(q1.x, q1.y)}),
+                grid_diff(T.gy, GridCoordT<float2>{make_float2(q1.z, q1.w), make_float2(q2.x, q2.y), make_float2(q2.z, q2.w)}),
+                grid_diff(T.gz, GridCoordT<float2>{make_float2(q3.x, q3.y), make_float2(q3.z, q3.w), q4}));
+            p.R1 = r2.R1;
+            grid_rsqrt(r2, p.y0, p.eh, p.v);
+        };
+        auto add_pair = [&](int s, const Pair2 &p) {
+            add(s, p.y0.x, p.eh.x, p.v.x, p.w.x);
+            add(s + 1, p.y0.y, p.eh.y, p.v.y, p.w.y);
+        };
+        auto add_close = [&](int s, const Pair2 &p) {
+            if (p.R1.x < near2) ieee(s, p.w.x);
+            else add(s, p.y0.x, p.eh.x, p.v.x, p.w.x);
+            if (p.R1.y < near2) ieee(s + 1, p.w.y);
+            else add(s + 1, p.y0.y, p.eh.y, p.v.y, p.w.y);
+        };
+        for (int s = 2 * grp; s < cnt; s += 4 * GROUPS) {  // two pairs of sources in the padded tile
+            Pair2 a, b;
+            pair_of(s, a);
+            pair_of(s + 2 * GROUPS, b);
+            if (fminf(fminf(a.R1.x, a.R1.y), fminf(b.R1.x, b.R1.y)) < near2) {
+                add_close(s, a);
+                add_close(s + 2 * GROUPS, b);
             } else {
-                add(s, r0, w0);
-                add(s + GROUPS, r1, w1);
+                add_pair(s, a);
+                add_pair(s + 2 * GROUPS, b);
             }
         }
         const double unscale = KIND == kField ? down * down * down : down;
@@ -419,18 +446,25 @@ int sm_count() {
     return sms;
 }
 
-// Cluster size: the number of blocks that share a target tile's sources.  An
-// SM's time is the blocks it gets times a block's (its sources, plus about 40
-// sources' worth of set-up and reduction), so the choice minimises
-// ceil(tiles * cs / SMs) * (n / cs + 40); from eight blocks per SM on, a
-// split gains nothing.
-int cluster_size(int64_t tiles, int64_t n) {
+// Cluster size: the number of blocks that share a target tile's sources.  A
+// block costs its sources plus about 40 sources' worth of set-up and
+// reduction, and the fullest SM decides.  FP64: up to four blocks per SM run at
+// once, beyond that blocks follow one another and the last one costs half its
+// time on average; and fewer than three blocks leave the pipes waiting, so an
+// SM takes the time of three.  3,000 panels: 142 us with clusters of 3 (one
+// block per SM), 92 with 8; 5,120: 207 with 6, 182 with 7, 189 with 8; 12,000:
+// 892 with 4, 796 with 8.  FP32 lanes hold several targets:
+// 1,000 targets, 5,120 sources take 34 us with clusters chosen for one block
+// per SM and 36 for three.
+int cluster_size(int64_t tiles, int64_t n, bool f64) {
     const int64_t sms = sm_count();
     if (tiles >= 8 * sms) return 1;
     int best = 1;
-    int64_t cost = INT64_MAX;
+    double cost = 1e300;
     for (int cs = 1; cs <= kMaxCluster; ++cs) {
-        const int64_t t = (tiles * cs + sms - 1) / sms * ((n + cs - 1) / cs + 40);
+        const double per_sm = (double)(tiles * cs) / (double)sms, whole = std::ceil(per_sm);
+        const double blocks = !f64 ? whole : per_sm <= 4.0 ? std::max(whole, 3.0) : per_sm + 0.5;
+        const double t = blocks * (std::ceil((double)n / cs) + 40.0);
         if (t < cost) {
             cost = t;
             best = cs;
@@ -449,7 +483,7 @@ int dense_launch(const T *tgt, int64_t m, const T *c, const T *sigma, const T *a
     const bool narrow = sizeof(T) == 8 && (m + 63) / 64 * kMaxCluster < 2 * sm_count();
     const int ROWS = sizeof(T) == 4 ? 32 * tpt32<KIND>() : narrow ? 32 : 64;
     const int64_t tiles = (m + ROWS - 1) / ROWS;
-    DenseArgs<T> A{tgt, m, c, sigma, areas, n, 0, cluster_size(tiles, n), k_e, self_int, out};
+    DenseArgs<T> A{tgt, m, c, sigma, areas, n, 0, cluster_size(tiles, n, sizeof(T) == 8), k_e, self_int, out};
     A.chunk = ((n + A.cs - 1) / A.cs + 1) & ~(int64_t)1;
     if (tiles * A.cs > INT32_MAX) return fail(EDFMM_ERR_ARG, "too many targets for one launch");
     cudaLaunchConfig_t cfg = {};

@@ -248,7 +248,7 @@ struct DevTree {
     DevBuf nodes_tf;
     // FP64 trees: per point the exact coordinate split of gridpoint.cuh and
     // the charge (three float4; the charge as a double, or as two floats in
-    // two-float mode), and the split's scale
+    // two-float mode), and the split's scale (batched plans: one per instance)
     DevBuf pts_grid;
     DevBuf grid_info;
     bool grid_tf = false;
@@ -273,14 +273,18 @@ struct InstMask {
     int stride = 0;
 };
 #ifdef __CUDACC__
-__device__ __forceinline__ bool inst_active(const InstMask &m, int node) {
-    if (!m.node_off) return true;
-    int lo = 0, hi = m.n_inst - 1;  // last instance whose first node <= node
+// the instance of a node (0 when there is one tree, node_off NULL)
+__device__ __forceinline__ int instance_of_node(const int32_t *node_off, int n_inst, int node) {
+    if (!node_off) return 0;
+    int lo = 0, hi = n_inst - 1;  // last instance whose first node <= node
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (m.node_off[mid] <= node) lo = mid; else hi = mid - 1;
+        if (node_off[mid] <= node) lo = mid; else hi = mid - 1;
     }
-    return m.flags[(int64_t)lo * m.stride] != 0.0;
+    return lo;
+}
+__device__ __forceinline__ bool inst_active(const InstMask &m, int node) {
+    return !m.node_off || m.flags[(int64_t)instance_of_node(m.node_off, m.n_inst, node) * m.stride] != 0.0;
 }
 #endif
 

@@ -23,8 +23,8 @@ namespace {
 __constant__ float2 c_rdiv_tf[kPMax + 1][kPMax + 1];  // (hi, lo) of 1 / ((n + m)(n - m)), 1 / n^2 at m = 0
 
 // ---------------------------------------------------------------------------
-// P2P.  One warp owns up to 64 targets of a leaf (a whole leaf at the usual
-// leaf sizes); with few leaves the four warps of a block share one leaf, each
+// P2P.  One warp owns up to 64 (split forms: 32) targets of a leaf (a whole
+// leaf at the usual leaf sizes); with few leaves the four warps of a block share one leaf, each
 // walking a quarter of its row.
 //
 // Lanes: the nt targets are held R per lane by L = ceil(nt / R) lanes, and
@@ -41,9 +41,11 @@ __constant__ float2 c_rdiv_tf[kPMax + 1][kPMax + 1];  // (hi, lo) of 1 / ((n + m
 // leaf at a time, the fixed work per leaf was about half of the kernel on
 // surface meshes.
 // Alone: FP32, 200k-panel torus 295 -> 143 us, a million points in a cube 2,352
-// -> 1,738 us (16 rsqrt per SM and clock: 58 and 935 us); FP64, 20,011 points
-// on a sphere 2,486 -> 277 us (gridpoint.cuh; 63 us at full issue); two-float,
-// 50k-panel torus 1,089 -> 327 us (140 us at full issue).
+// -> 1,738 us (16 rsqrt per SM and clock: 58 and 935 us).  The split forms
+// (gridpoint.cuh) take two sources in packed operations: FP64, 20,011 points on
+// a sphere 2,486 -> 277 scalar -> 246 us packed (the FMA pipe's time is 65 us:
+// leaves of about 16 points, three waves of blocks); two-float, 50k-panel torus
+// 1,089 -> 327 -> 261 us (the FMA pipe's time: 110 us).
 // ---------------------------------------------------------------------------
 enum NearMode {
     kF32,   // packed pairs of sources on the FP32 pipe
@@ -62,19 +64,23 @@ template <> struct NearCfg<kF32> {
     // but the warps of an SM then run six copies of the loop, and on surface
     // leaves (200k-panel torus 190 instead of 143 us, 24 dimers 427 instead of
     // 326) the instruction fetches cost more than the idle lanes.
-    static constexpr int CH = 128, REC = 1, RS = 0x1c, A = 5, B = 11;
+    static constexpr int W = 64, CH = 128, REC = 1, RS = 0x1c, A = 5, B = 11;
 };
+// The split forms take one target a lane, 32 a window: the packed coordinates
+// of a target are 18 registers, so that R = 2 and 3 spill at four blocks per SM
+// (R = 1, 2, 3: 261 and 279 us on the two shapes above; R = 1, 2: 255 and 261;
+// R = 1: 246 and 261; five blocks per SM 265 and 269).
 template <> struct NearCfg<kTF> {
     using T = double;
-    static constexpr int CH = 64, REC = 3, RS = 0xe, A = 6, B = 75;
+    static constexpr int W = 32, CH = 64, REC = 3, RS = 0x2, A = 6, B = 75;
 };
 template <> struct NearCfg<kGrid> {
     using T = double;
-    static constexpr int CH = 64, REC = 3, RS = 0xe, A = 6, B = 150;
+    static constexpr int W = 32, CH = 64, REC = 3, RS = 0x2, A = 6, B = 150;
 };
 template <> struct NearCfg<kIeee> {
     using T = double;
-    static constexpr int CH = 64, REC = 2, RS = 0xe, A = 5, B = 128;
+    static constexpr int W = 64, CH = 64, REC = 2, RS = 0xe, A = 5, B = 128;
 };
 
 // targets per lane for nt targets: the least (A + B R) / G with G = 32 / ceil(nt / R)
@@ -108,7 +114,9 @@ template <typename T> struct NearParams {
     const int2 *range;                   // target leaves' point ranges
     const typename Vec4<T>::type *spts;  // sources (== pts for one tree)
     const float4 *spts_split;            // kTF, kGrid: three float4 per point
-    const GridInfo *grid;                // kTF, kGrid
+    const GridInfo *grid;                // kTF, kGrid: one per instance
+    const int32_t *inst_off;             // batched plans: first node of each instance (NULL: one tree)
+    int n_inst;
     const int2 *srange;
     int same;  // one tree: drop i == j in self pairs
     T eps2;
@@ -172,13 +180,16 @@ template <int R> struct Targets<kF32, R> {
     float acc[R];
 };
 template <int R> struct Targets<kTF, R> {
-    GridCoord x[R], y[R], z[R];
+    GridCoordT<float2> x[R], y[R], z[R];  // in both halves
     double acc[R];
 };
 template <int R> struct Targets<kGrid, R> {
-    GridCoord x[R], y[R], z[R];
+    GridCoordT<float2> x[R], y[R], z[R];
     double acc[R];
 };
+__device__ __forceinline__ GridCoordT<float2> grid_both(const GridCoord &g) {
+    return GridCoordT<float2>{make_float2(g.a, g.a), make_float2(g.b, g.b), make_float2(g.c, g.c)};
+}
 template <int R> struct Targets<kIeee, R> {
     double x[R], y[R], z[R], acc[R];
 };
@@ -226,12 +237,17 @@ template <int MODE> __device__ __forceinline__ void stage(float4 *buf, int pair,
         d[2 * pair] = f.a;
         d[2 * pair + 1] = f.b;
     } else {
-        constexpr int N = NearCfg<MODE>::REC;
+        // value by value like the FP32 records: the nine parts of both sources,
+        // both indices and the charges (kGrid: two doubles; kTF: (hi, hi', lo, lo'))
+        float4 *d = buf + 6 * pair;
 #pragma unroll
-        for (int c = 0; c < N; ++c) {
-            buf[N * (2 * pair) + c] = f.a[c];
-            buf[N * (2 * pair + 1) + c] = f.b[c];
+        for (int c = 0; c < 2; ++c) {
+            d[2 * c] = make_float4(f.a[c].x, f.b[c].x, f.a[c].y, f.b[c].y);
+            d[2 * c + 1] = make_float4(f.a[c].z, f.b[c].z, f.a[c].w, f.b[c].w);
         }
+        d[4] = make_float4(f.a[2].x, f.b[2].x, f.a[2].y, f.b[2].y);
+        d[5] = MODE == kGrid ? make_float4(f.a[2].z, f.a[2].w, f.b[2].z, f.b[2].w)
+                             : make_float4(f.a[2].z, f.b[2].z, f.a[2].w, f.b[2].w);
     }
 }
 
@@ -244,9 +260,9 @@ __device__ __forceinline__ void load_target(const NearParams<T> &P, int ti, int 
         X.nz[r] = make_float2(-x.z, -x.z);
         X.acc[r] = 0.0f;
     } else if constexpr (MODE == kTF || MODE == kGrid) {
-        X.x[r] = grid_split(x.x * g.down);
-        X.y[r] = grid_split(x.y * g.down);
-        X.z[r] = grid_split(x.z * g.down);
+        X.x[r] = grid_both(grid_split(x.x * g.down));
+        X.y[r] = grid_both(grid_split(x.y * g.down));
+        X.z[r] = grid_both(grid_split(x.z * g.down));
         X.acc[r] = 0.0;
     } else {
         X.x[r] = x.x;
@@ -266,14 +282,29 @@ __device__ __noinline__ double grid_pair_ieee(const double4 *pts, int s, int t, 
     return b.w * inv_dist(dx * dx + dy * dy + dz * dz, eps2) * up;
 }
 
-// hi + lo += (qh + ql) (y0 + z)
-__device__ __forceinline__ void grid_add_tf(float qh, float ql, float y0, float z, float &hi, float &lo) {
-    const float p = g_mul(qh, y0);
-    const float e = g_fma(ql, y0, g_fma(qh, z, g_fma(qh, y0, -p)));
-    float s, f;
+// hi + lo -= (qh + ql) (y0 + z), both halves; nq = -qh
+__device__ __forceinline__ void grid_sub_tf(float2 qh, float2 nq, float2 ql, float2 y0, float2 z, float2 &hi, float2 &lo) {
+    const float2 p = g_mul(nq, y0);
+    const float2 e = g_fma(ql, y0, g_fma(qh, z, g_fma(qh, y0, p)));
+    float2 s, f;
     grid_two_sum(hi, p, s, f);
     hi = s;
-    lo = g_add(lo, g_add(f, e));
+    lo = g_add(lo, g_sub(f, e));
+}
+// a staged pair of split sources
+struct GridPair {
+    GridCoordT<float2> x, y, z;
+    float4 idx, q;  // (-, -, index, index'), charges
+};
+__device__ __forceinline__ GridPair grid_pair(const float4 *d) {
+    const float4 a = d[0], b = d[1], c = d[2], e = d[3];
+    GridPair p;
+    p.idx = d[4];
+    p.q = d[5];
+    p.x = GridCoordT<float2>{make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y)};
+    p.y = GridCoordT<float2>{make_float2(b.z, b.w), make_float2(c.x, c.y), make_float2(c.z, c.w)};
+    p.z = GridCoordT<float2>{make_float2(e.x, e.y), make_float2(e.z, e.w), make_float2(p.idx.x, p.idx.y)};
+    return p;
 }
 
 // sources part, part + G, ... of a staged chunk of cnt sources; SELF: the
@@ -309,80 +340,64 @@ __device__ __forceinline__ void accumulate(const NearParams<T> &P, const float4 
 #pragma unroll
         for (int r = 0; r < R; ++r) X.acc[r] += ps[r].x + ps[r].y;  // per-chunk partial, then one add
     } else if constexpr (MODE == kTF) {
-        float hi[R], lo[R];  // a chunk's sum, hi + lo, of at most 64 terms; then FP64
+        float2 hi[R], lo[R];  // minus a chunk's sums, hi + lo, of at most 32 terms each; then FP64
         double ps[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            hi[r] = lo[r] = 0.0f;
+            hi[r] = lo[r] = make_float2(0.0f, 0.0f);
             ps[r] = 0.0;
         }
-        for (int j = part; j < cnt; j += G) {
-            const float4 u = buf[3 * j], v = buf[3 * j + 1], q = buf[3 * j + 2];
-            float R1[R], M[R];
-            bool close = false;
+        const int np = (cnt + 1) >> 1;
+        for (int j = part; j < np; j += G) {
+            const GridPair s = grid_pair(buf + 6 * j);
+            const float2 qh = make_float2(s.q.x, s.q.y), ql = make_float2(s.q.z, s.q.w), nq = g_neg(qh);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                R1[r] = grid_r2_tf(grid_diff2(X.x[r], GridCoord{u.x, u.y, u.z}),
-                                   grid_diff2(X.y[r], GridCoord{u.w, v.x, v.y}),
-                                   grid_diff2(X.z[r], GridCoord{v.z, v.w, q.x}), M[r]);
-                close = close || !(R1[r] >= g.near2);
-            }
-            if (close) {
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    if (!(R1[r] >= g.near2)) {
-                        ps[r] += grid_pair_ieee(P.pts, __float_as_int(q.y), min(t0 + L * r, last), P.eps2, g.up);
-                    } else {
-                        float y0, z;
-                        grid_rsqrt_tf(R1[r], M[r], y0, z);
-                        grid_add_tf(q.z, q.w, y0, z, hi[r], lo[r]);
+                float2 N, y0, z;
+                const float2 R1 = grid_r2_tf(grid_diff2(X.x[r], s.x), grid_diff2(X.y[r], s.y), grid_diff2(X.z[r], s.z), N);
+                float2 h = qh, m = nq, l = ql;
+                grid_rsqrt_tf(R1, N, y0, z);
+                if (!(fminf(R1.x, R1.y) >= g.near2)) {  // the target itself, or a pair the split does not resolve
+                    const int t = min(t0 + L * r, last);
+                    if (!(R1.x >= g.near2)) {
+                        ps[r] += grid_pair_ieee(P.pts, __float_as_int(s.idx.z), t, P.eps2, g.up);
+                        h.x = m.x = l.x = y0.x = z.x = 0.0f;
+                    }
+                    if (!(R1.y >= g.near2)) {
+                        ps[r] += grid_pair_ieee(P.pts, __float_as_int(s.idx.w), t, P.eps2, g.up);
+                        h.y = m.y = l.y = y0.y = z.y = 0.0f;
                     }
                 }
-            } else {
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    float y0, z;
-                    grid_rsqrt_tf(R1[r], M[r], y0, z);
-                    grid_add_tf(q.z, q.w, y0, z, hi[r], lo[r]);
-                }
+                grid_sub_tf(h, m, l, y0, z, hi[r], lo[r]);
             }
         }
 #pragma unroll
-        for (int r = 0; r < R; ++r) X.acc[r] += ps[r] + ((double)hi[r] + (double)lo[r]);
+        for (int r = 0; r < R; ++r)
+            X.acc[r] += ps[r] - (((double)hi[r].x + (double)lo[r].x) + ((double)hi[r].y + (double)lo[r].y));
     } else if constexpr (MODE == kGrid) {
         double ps[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) ps[r] = 0.0;
-        for (int j = part; j < cnt; j += G) {
-            const float4 u = buf[3 * j], v = buf[3 * j + 1], q = buf[3 * j + 2];
-            const double w = __hiloint2double(__float_as_int(q.w), __float_as_int(q.z));
-            GridR2 r2[R];
-            bool close = false;
+        const int np = (cnt + 1) >> 1;
+        for (int j = part; j < np; j += G) {
+            const GridPair s = grid_pair(buf + 6 * j);
+            const double wa = __hiloint2double(__float_as_int(s.q.y), __float_as_int(s.q.x)),
+                         wb = __hiloint2double(__float_as_int(s.q.w), __float_as_int(s.q.z));
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                r2[r] = grid_r2(grid_diff(X.x[r], GridCoord{u.x, u.y, u.z}), grid_diff(X.y[r], GridCoord{u.w, v.x, v.y}),
-                                grid_diff(X.z[r], GridCoord{v.z, v.w, q.x}));
-                close = close || !(r2[r].R1 >= g.near2);
-            }
-            if (close) {  // the target itself, or a pair the split does not resolve
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    if (!(r2[r].R1 >= g.near2)) {
-                        ps[r] += grid_pair_ieee(P.pts, __float_as_int(q.y), min(t0 + L * r, last), P.eps2, g.up);
-                    } else {
-                        float y0;
-                        unsigned ci;
-                        grid_rsqrt(r2[r], y0, ci);
-                        ps[r] = fma(w * grid_double(y0), grid_one_plus(ci), ps[r]);
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    float y0;
-                    unsigned ci;
-                    grid_rsqrt(r2[r], y0, ci);
-                    ps[r] = fma(w * grid_double(y0), grid_one_plus(ci), ps[r]);
+                const GridR2<float2> r2 =
+                    grid_r2(grid_diff(X.x[r], s.x), grid_diff(X.y[r], s.y), grid_diff(X.z[r], s.z));
+                float2 y0, eh, v;
+                grid_rsqrt(r2, y0, eh, v);
+                if (!(fminf(r2.R1.x, r2.R1.y) >= g.near2)) {  // the target itself, or a pair the split does not resolve
+                    const int t = min(t0 + L * r, last);
+                    if (!(r2.R1.x >= g.near2)) ps[r] += grid_pair_ieee(P.pts, __float_as_int(s.idx.z), t, P.eps2, g.up);
+                    else ps[r] = fma(wa, grid_inv(y0.x, grid_ci(eh.x, v.x)), ps[r]);
+                    if (!(r2.R1.y >= g.near2)) ps[r] += grid_pair_ieee(P.pts, __float_as_int(s.idx.w), t, P.eps2, g.up);
+                    else ps[r] = fma(wb, grid_inv(y0.y, grid_ci(eh.y, v.y)), ps[r]);
+                } else {
+                    ps[r] = fma(wa, grid_inv(y0.x, grid_ci(eh.x, v.x)), ps[r]);
+                    ps[r] = fma(wb, grid_inv(y0.y, grid_ci(eh.y, v.y)), ps[r]);
                 }
             }
         }
@@ -524,9 +539,9 @@ __global__ void __launch_bounds__(32 * kNearWarps, near_blocks<MODE>())
     if (!inst_active(P.mask, t)) return;  // uniform over the warps that share a leaf
     const int2 rg = P.range[t];
     GridInfo g{};
-    if constexpr (MODE == kGrid || MODE == kTF) g = *P.grid;
-    for (int tb = rg.x; tb < rg.y; tb += 64) {
-        const int nt = min(64, rg.y - tb);
+    if constexpr (MODE == kGrid || MODE == kTF) g = P.grid[instance_of_node(P.inst_off, P.n_inst, t)];
+    for (int tb = rg.x; tb < rg.y; tb += C::W) {
+        const int nt = min(C::W, rg.y - tb);
         const int R = d_near_shape<MODE>.r[nt];
 #define EDFMM_NEAR_R(RR)                                                                                     \
     if constexpr ((C::RS >> RR) & 1) {                                                                           \
@@ -685,38 +700,68 @@ __global__ void __launch_bounds__(128) k_l2p(const L2pParams<T> P) {
 // ---------------------------------------------------------------------------
 // FP64 trees: the exact split of the points (gridpoint.cuh)
 // ---------------------------------------------------------------------------
-__global__ void k_grid_max(const double4 *__restrict__ pts, int64_t n, GridInfo *info) {
-    unsigned hi = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double4 p = pts[i];
-        hi = max(hi, (unsigned)__double2hiint(p.x) & 0x7fffffffu);
-        hi = max(hi, (unsigned)__double2hiint(p.y) & 0x7fffffffu);
-        hi = max(hi, (unsigned)__double2hiint(p.z) & 0x7fffffffu);
+// A batched plan has one scale per instance, so that each instance's results are
+// those of its own plan.  node_off NULL: one tree.
+__device__ __forceinline__ int instance_of_point(const int32_t *node_off, int n_inst, const int2 *range, int64_t i) {
+    if (!node_off) return 0;
+    int lo = 0, hi = n_inst - 1;  // last instance whose root's points start at or before i
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (range[node_off[mid]].x <= i) lo = mid; else hi = mid - 1;
     }
-    hi = __reduce_max_sync(0xffffffffu, hi);
-    if ((threadIdx.x & 31) == 0) atomicMax(&info->hi, hi);
+    return lo;
+}
+__global__ void k_grid_max(const double4 *__restrict__ pts, int64_t n, const int32_t *node_off, int n_inst,
+                           const int2 *__restrict__ range, GridInfo *info) {
+    // a block takes a run of points: mostly of one instance
+    const int64_t per = (n + gridDim.x - 1) / gridDim.x, b = blockIdx.x * per, e = min(n, b + per);
+    for (int64_t i0 = b; i0 < e; i0 += blockDim.x) {
+        const int64_t i = i0 + threadIdx.x;
+        unsigned hi = 0;
+        int k = -1;
+        if (i < e) {
+            k = instance_of_point(node_off, n_inst, range, i);
+            const double4 p = pts[i];
+            hi = max(hi, (unsigned)__double2hiint(p.x) & 0x7fffffffu);
+            hi = max(hi, (unsigned)__double2hiint(p.y) & 0x7fffffffu);
+            hi = max(hi, (unsigned)__double2hiint(p.z) & 0x7fffffffu);
+        }
+        const int k0 = __shfl_sync(0xffffffffu, k, 0);
+        if (__all_sync(0xffffffffu, k == k0 || k < 0)) {
+            hi = __reduce_max_sync(0xffffffffu, hi);
+            if ((threadIdx.x & 31) == 0 && k0 >= 0) atomicMax(&info[k0].hi, hi);
+        } else if (k >= 0) {
+            atomicMax(&info[k].hi, hi);
+        }
+    }
+}
+// each scale from its largest coordinate
+__global__ void k_grid_scales(int n_inst, GridInfo *info) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_inst) return;
+    int k;
+    const bool ok = grid_exponent(info[i].hi, k);
+    if (!ok) k = 0;
+    info[i].down = grid_pow2(-k);
+    info[i].up = grid_pow2(k);
+    // without a usable scale every pair is evaluated in IEEE FP64: no r^2 is >= NaN
+    info[i].near2 =
+        ok ? fmaxf(kGridNear2, (float)(1.0001 * DBL_EPSILON * DBL_EPSILON * info[i].down * info[i].down)) : NAN;
 }
 // three float4 per point: (xa, xb, xc, ya), (yb, yc, za, zb), (zc, -, charge);
 // set_charges writes the charge
-__global__ void k_grid_points(const double4 *__restrict__ pts, int64_t n, GridInfo *info, float4 *__restrict__ out) {
-    int k;
-    const bool ok = grid_exponent(info->hi, k);
-    if (!ok) k = 0;
-    const double down = grid_pow2(-k);
+__global__ void k_grid_points(const double4 *__restrict__ pts, int64_t n, const int32_t *node_off, int n_inst,
+                              const int2 *__restrict__ range, const GridInfo *__restrict__ info,
+                              float4 *__restrict__ out) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) {
-        info->down = down;
-        info->up = grid_pow2(k);
-        // without a usable scale every pair is evaluated in IEEE FP64: no r^2 is >= NaN
-        info->near2 = ok ? fmaxf(kGridNear2, (float)(1.0001 * DBL_EPSILON * DBL_EPSILON * down * down)) : NAN;
-    }
     if (i >= n) return;
+    const GridInfo g = info[instance_of_point(node_off, n_inst, range, i)];
     const double4 p = pts[i];
     GridCoord x{}, y{}, z{};
-    if (ok) {
-        x = grid_split(p.x * down);
-        y = grid_split(p.y * down);
-        z = grid_split(p.z * down);
+    if (g.near2 >= 0.0f) {  // not NaN
+        x = grid_split(p.x * g.down);
+        y = grid_split(p.y * g.down);
+        z = grid_split(p.z * g.down);
     }
     out[3 * i] = make_float4(x.a, x.b, x.c, y.a);
     out[3 * i + 1] = make_float4(y.b, y.c, z.a, z.b);
@@ -729,15 +774,22 @@ __global__ void k_grid_points(const double4 *__restrict__ pts, int64_t n, GridIn
 int grid_prepare(DevTree &tree, cudaStream_t s) {
     if (tree.dtype != EDFMM_F64 || tree.n_points == 0) return EDFMM_OK;
     int rc;
+    const int K = std::max(tree.n_inst, 1);
     if ((rc = tree.pts_grid.reserve(sizeof(float4) * 3 * (size_t)tree.n_points)) ||
-        (rc = tree.grid_info.reserve(sizeof(GridInfo))))
+        (rc = tree.grid_info.reserve(sizeof(GridInfo) * (size_t)K)))
         return rc;
     GridInfo *info = dptr<GridInfo>(tree.grid_info);
-    EDFMM_CUDA_TRY(cudaMemsetAsync(info, 0, sizeof(GridInfo), s));
+    const int32_t *node_off = tree.n_inst > 0 ? dptr<int32_t>(tree.inst_node_off) : nullptr;
+    const int2 *range = dptr<int2>(tree.range);
+    EDFMM_CUDA_TRY(cudaMemsetAsync(info, 0, sizeof(GridInfo) * (size_t)K, s));
     const int64_t nb = (tree.n_points + 255) / 256;
-    k_grid_max<<<(unsigned)(nb < 608 ? nb : 608), 256, 0, s>>>(dptr<double4>(tree.pts), tree.n_points, info);
+    k_grid_max<<<(unsigned)(nb < 608 ? nb : 608), 256, 0, s>>>(dptr<double4>(tree.pts), tree.n_points, node_off, K, range,
+                                                               info);
     EDFMM_LAUNCH_CHECK("k_grid_max");
-    k_grid_points<<<(unsigned)nb, 256, 0, s>>>(dptr<double4>(tree.pts), tree.n_points, info, dptr<float4>(tree.pts_grid));
+    k_grid_scales<<<(unsigned)((K + 127) / 128), 128, 0, s>>>(K, info);
+    EDFMM_LAUNCH_CHECK("k_grid_scales");
+    k_grid_points<<<(unsigned)nb, 256, 0, s>>>(dptr<double4>(tree.pts), tree.n_points, node_off, K, range, info,
+                                               dptr<float4>(tree.pts_grid));
     EDFMM_LAUNCH_CHECK("k_grid_points");
     return EDFMM_OK;
 }
@@ -801,6 +853,8 @@ int near_impl(const DevTree &tree, const DevLists &lists, const FmmBuffers &buf,
         if (src_tree) return near_launch<kIeee>(P, s);
         P.spts_split = dptr<float4>(tree.pts_grid);
         P.grid = dptr<GridInfo>(tree.grid_info);
+        P.inst_off = tree.n_inst > 0 ? dptr<int32_t>(tree.inst_node_off) : nullptr;
+        P.n_inst = tree.n_inst;
         return tree.grid_tf ? near_launch<kTF>(P, s) : near_launch<kGrid>(P, s);
     }
 }
