@@ -29,8 +29,8 @@ from torch import Tensor
 from .. import _lib
 from ..utils.config import K_E, BEMConfig
 from .bem_mesh import TriMesh, generate_mesh
-from .bem_near import (NearCorrection, add_point_charges, field_at_targets, near_potential_correction,
-                       point_charge_potential, potential_at_targets, self_integrals)
+from .bem_near import (NearCorrection, add_point_charges, near_potential_correction,
+                       point_charge_potential, potential_at_targets, potential_field_at_targets, self_integrals)
 from .bem_solver import gmres_batched, gmres_restart
 from .operators import DenseOperator, FmmOperator
 
@@ -155,25 +155,31 @@ class BEMSolution:
         """Total potential V_free + V_induced at points (N, 3): the dense induced
         part, corrected near the surface by the panels' quadrature when
         ``near_quadrature`` is on and panel vertices are known (bem.py:1461-1499)."""
-        pts = torch.as_tensor(points).to(self.sigma.device, self.sigma.dtype).reshape(-1, 3).contiguous()
-        v = potential_at_targets(pts, self.centroids, self.sigma, self.areas)
-        if self.near_quadrature and self.panel_vertices is not None and self.panel_vertices.numel() > 0:
-            v = near_potential_correction(v, pts, self.centroids, self.areas, self.sigma, self.panel_vertices,
-                                          distance_factor=self.near_quad_dist_factor,
-                                          quad_order=self.near_quad_order, max_depth=self.near_quad_max_depth)
+        pts = self._points(points)
+        v = self._near_corrected(potential_at_targets(pts, self.centroids, self.sigma, self.areas), pts)
         if self.charges:
             add_point_charges(pts, self.charges, V=v)
         return v
+
+    def _points(self, points: Tensor) -> Tensor:
+        return torch.as_tensor(points).to(self.sigma.device, self.sigma.dtype).reshape(-1, 3).contiguous()
+
+    def _near_corrected(self, v: Tensor, pts: Tensor) -> Tensor:
+        if not (self.near_quadrature and self.panel_vertices is not None and self.panel_vertices.numel() > 0):
+            return v
+        return near_potential_correction(v, pts, self.centroids, self.areas, self.sigma, self.panel_vertices,
+                                         distance_factor=self.near_quad_dist_factor,
+                                         quad_order=self.near_quad_order, max_depth=self.near_quad_max_depth)
 
     def eval_V_E_batched(self, points: Tensor) -> Tuple[Tensor, Tensor]:
         """Total potential (N,) and field (N, 3) at points: free-space point
         charges plus the panels' induced part (bem.py:1533-1542 with
         bem_E_field_targets, bem_kernel.py:914, for the field)."""
-        pts = torch.as_tensor(points).to(self.sigma.device, self.sigma.dtype).reshape(-1, 3).contiguous()
-        v = self.eval(pts)
-        e = field_at_targets(pts, self.centroids, self.sigma, self.areas)
+        pts = self._points(points)
+        v, e = potential_field_at_targets(pts, self.centroids, self.sigma, self.areas)
+        v = self._near_corrected(v, pts)
         if self.charges:
-            add_point_charges(pts, self.charges, E=e)
+            add_point_charges(pts, self.charges, V=v, E=e)
         return v, e
 
 

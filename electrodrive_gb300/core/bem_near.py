@@ -201,6 +201,24 @@ def potential_at_targets(targets: Tensor, centroids: Tensor, sigma: Tensor, area
     return out
 
 
+def potential_field_at_targets(targets: Tensor, centroids: Tensor, sigma: Tensor, areas: Tensor, *,
+                               k_e: float = K_E):
+    """:func:`potential_at_targets` and :func:`field_at_targets` in one pass
+    over the panels (the distances are formed once)."""
+    L = _lib.load_library()
+    dev, dt = sigma.device, sigma.dtype
+    T = lambda x: x.to(dev, dt).contiguous()
+    t = T(targets)
+    v = torch.empty(t.shape[0], dtype=dt, device=dev)
+    e = torch.empty(t.shape[0], 3, dtype=dt, device=dev)
+    with torch.cuda.device(dev):
+        _lib.check(L.edfmm_dense_potential_field_targets(
+            _lib.ptr(t), t.shape[0], _lib.ptr(T(centroids)), _lib.ptr(T(sigma)), _lib.ptr(T(areas)), sigma.shape[0],
+            _lib.dtype_code(dt), float(k_e), _lib.ptr(v), _lib.ptr(e), _lib.stream_handle(dev)),
+            "edfmm_dense_potential_field_targets")
+    return v, e
+
+
 def field_at_targets(targets: Tensor, centroids: Tensor, sigma: Tensor, areas: Tensor, *,
                      k_e: float = K_E) -> Tensor:
     """Induced field of panel charges at targets, (M, 3) (bem_E_field_targets,

@@ -34,7 +34,10 @@ namespace edfmm {
 
 namespace {
 
-enum DenseKind { kMatvec = 0, kPotential = 1, kField = 2 };
+enum DenseKind { kMatvec = 0, kPotential = 1, kField = 2, kBoth = 3 };  // kBoth: field and potential in one pass
+template <int KIND> __host__ __device__ constexpr bool has_field() { return KIND == kField || KIND == kBoth; }
+// sums per target: the field's three, the potential
+template <int KIND> __host__ __device__ constexpr int dense_comp() { return KIND == kField ? 3 : KIND == kBoth ? 4 : 1; }
 
 constexpr int kThreads = 128;     // 4 warps
 constexpr int kTile32 = 256;      // sources staged per shared-memory tile, FP32
@@ -54,6 +57,7 @@ template <typename T> struct DenseArgs {
     T k_e;
     const T *self_int;  // kMatvec only
     T *out;
+    T *out_v;  // kBoth: the potential
 };
 
 __device__ __forceinline__ void cluster_sync_all() {
@@ -79,7 +83,7 @@ __device__ __forceinline__ double dsm_load(const double *p, int rank) {
 // rows.  part[(g * ROWS + row) * COMP + comp]: group g's sums of this block.
 template <typename T, int KIND, int ROWS, int GROUPS>
 __device__ __forceinline__ void dense_finish(const DenseArgs<T> &A, T *part, int64_t row0, int rank) {
-    constexpr int COMP = KIND == kField ? 3 : 1, NV = ROWS * COMP;
+    constexpr int COMP = dense_comp<KIND>(), NV = ROWS * COMP;
     __syncthreads();
     for (int q = threadIdx.x; q < NV; q += kThreads) {
         T v = part[q];
@@ -101,8 +105,10 @@ __device__ __forceinline__ void dense_finish(const DenseArgs<T> &A, T *part, int
                 A.out[i] = isfinite(v) ? v : (T)0;
             } else if (KIND == kPotential) {
                 A.out[i] = v * A.k_e;
+            } else if (KIND == kBoth && q % COMP == 3) {
+                A.out_v[i] = v * A.k_e;
             } else {
-                A.out[row0 * 3 + q] = isfinite(v) ? v : (T)0;
+                A.out[i * 3 + q % COMP] = isfinite(v) ? v : (T)0;
             }
         }
     }
@@ -126,12 +132,13 @@ __device__ __forceinline__ void dense_ranges(const DenseArgs<T> &A, int rows, in
 // reference's does, and non-finite components become zero at the end
 // (bem_kernel.py:990-997).
 // ---------------------------------------------------------------------------
-template <int KIND> __host__ __device__ constexpr int tpt32() { return KIND == kField ? 2 : 4; }
+template <int KIND> __host__ __device__ constexpr int tpt32() { return has_field<KIND>() ? 2 : 4; }
 
 template <int KIND, bool SELF, int TPT>
 __device__ __forceinline__ void dense_tile_f32(const float4 *src, int npairs, int wid, float k_e, const float2 (&nx)[TPT],
                                                const float2 (&ny)[TPT], const float2 (&nz)[TPT], int self0,
-                                               float2 (&ax)[TPT], float2 (&ay)[TPT], float2 (&az)[TPT]) {
+                                               float2 (&ax)[TPT], float2 (&ay)[TPT], float2 (&az)[TPT],
+                                               float2 (&av)[TPT]) {
 #pragma unroll 2
     for (int k = wid; k < npairs; k += 4) {
         const float4 u = src[2 * k], v = src[2 * k + 1];  // (x, x', y, y'), (z, z', q, q')
@@ -146,22 +153,21 @@ __device__ __forceinline__ void dense_tile_f32(const float4 *src, int npairs, in
                 if (2 * k == self0 + 32 * t) ir.x = 0.0f;
                 if (2 * k + 1 == self0 + 32 * t) ir.y = 0.0f;
             }
-            if (KIND == kField) {
+            if (has_field<KIND>()) {
                 const float2 ke2 = make_float2(k_e, k_e);
                 const float2 w = __fmul2_rn(__fmul2_rn(ke2, __fmul2_rn(__fmul2_rn(ir, ir), ir)), qw);
                 ax[t] = __ffma2_rn(w, dx, ax[t]);  // source minus target: the sign is taken at the end
                 ay[t] = __ffma2_rn(w, dy, ay[t]);
                 az[t] = __ffma2_rn(w, dz, az[t]);
-            } else {
-                ax[t] = __ffma2_rn(qw, ir, ax[t]);
             }
+            if (KIND != kField) av[t] = __ffma2_rn(qw, ir, av[t]);
         }
     }
 }
 
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) k_dense_f32(const DenseArgs<float> A) {
-    constexpr int TPT = tpt32<KIND>(), ROWS = 32 * TPT, COMP = KIND == kField ? 3 : 1;
+    constexpr int TPT = tpt32<KIND>(), ROWS = 32 * TPT, COMP = dense_comp<KIND>();
     __shared__ float4 src[kTile32];
     __shared__ float part[4 * ROWS * COMP];
     int64_t row0, j0, j1;
@@ -169,14 +175,14 @@ __global__ void __launch_bounds__(kThreads) k_dense_f32(const DenseArgs<float> A
     dense_ranges(A, ROWS, row0, rank, j0, j1);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float2 nx[TPT], ny[TPT], nz[TPT];
-    float ex[TPT], ey[TPT], ez[TPT];
+    float ex[TPT], ey[TPT], ez[TPT], ev[TPT];
 #pragma unroll
     for (int t = 0; t < TPT; ++t) {
         const int64_t i = min(row0 + lane + 32 * t, A.m - 1);
         nx[t].x = nx[t].y = -A.tgt[3 * i];
         ny[t].x = ny[t].y = -A.tgt[3 * i + 1];
         nz[t].x = nz[t].y = -A.tgt[3 * i + 2];
-        ex[t] = ey[t] = ez[t] = 0.0f;
+        ex[t] = ey[t] = ez[t] = ev[t] = 0.0f;
     }
     float *sf = reinterpret_cast<float *>(src);
     for (int64_t jb = j0; jb < j1; jb += kTile32) {
@@ -201,33 +207,33 @@ __global__ void __launch_bounds__(kThreads) k_dense_f32(const DenseArgs<float> A
         }
         __syncthreads();
         // two-level sum (tile, then chunk) bounds FP32 rounding growth
-        float2 ax[TPT], ay[TPT], az[TPT];
+        float2 ax[TPT], ay[TPT], az[TPT], av[TPT];
 #pragma unroll
-        for (int t = 0; t < TPT; ++t) ax[t] = ay[t] = az[t] = make_float2(0.0f, 0.0f);
+        for (int t = 0; t < TPT; ++t) ax[t] = ay[t] = az[t] = av[t] = make_float2(0.0f, 0.0f);
         const int np = (cnt + 1) >> 1;
         if (KIND == kMatvec && jb < row0 + ROWS && row0 < jb + cnt)
-            dense_tile_f32<KIND, true>(src, np, wid, A.k_e, nx, ny, nz, (int)(row0 - jb) + lane, ax, ay, az);
+            dense_tile_f32<KIND, true>(src, np, wid, A.k_e, nx, ny, nz, (int)(row0 - jb) + lane, ax, ay, az, av);
         else
-            dense_tile_f32<KIND, false>(src, np, wid, A.k_e, nx, ny, nz, 0, ax, ay, az);
+            dense_tile_f32<KIND, false>(src, np, wid, A.k_e, nx, ny, nz, 0, ax, ay, az, av);
 #pragma unroll
         for (int t = 0; t < TPT; ++t) {
-            ex[t] += ax[t].x + ax[t].y;
-            if (KIND == kField) {
+            if (has_field<KIND>()) {
+                ex[t] += ax[t].x + ax[t].y;
                 ey[t] += ay[t].x + ay[t].y;
                 ez[t] += az[t].x + az[t].y;
             }
+            if (KIND != kField) ev[t] += av[t].x + av[t].y;
         }
     }
 #pragma unroll
     for (int t = 0; t < TPT; ++t) {
         float *p = part + (wid * ROWS + lane + 32 * t) * COMP;
-        if (KIND == kField) {
+        if (has_field<KIND>()) {
             p[0] = -ex[t];
             p[1] = -ey[t];
             p[2] = -ez[t];
-        } else {
-            p[0] = ex[t];
         }
+        if (KIND != kField) p[COMP - 1] = ev[t];
     }
     dense_finish<float, KIND, ROWS, 4>(A, part, row0, rank);
 }
@@ -258,26 +264,25 @@ __device__ __forceinline__ unsigned high_abs(double x) { return (unsigned)__doub
 // one source in IEEE FP64, from device memory (w: the charge)
 template <int KIND>
 __device__ __noinline__ void dense_pair_ieee(const double *c, int64_t j, int64_t self, double x, double y, double z,
-                                             double w, double k_e, double &ex, double &ey, double &ez) {
-    ex = ey = ez = 0.0;
+                                             double w, double k_e, double &ex, double &ey, double &ez, double &ev) {
+    ex = ey = ez = ev = 0.0;
     if (KIND == kMatvec && j == self) return;
     const double dx = x - c[3 * j], dy = y - c[3 * j + 1], dz = z - c[3 * j + 2];
     const double ir = inv_r(dx * dx + dy * dy + dz * dz);
-    if (KIND == kField) {
+    if (has_field<KIND>()) {
         const double f = (k_e * (ir * ir * ir)) * w;
         ex = f * dx;
         ey = f * dy;
         ez = f * dz;
-    } else {
-        ex = w * ir;
     }
+    ev = w * ir;
 }
 
 template <int KIND, int GROUPS>
 __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> A) {
-    constexpr int COMP = KIND == kField ? 3 : 1, ROWS = kThreads / GROUPS;
+    constexpr int COMP = dense_comp<KIND>(), ROWS = kThreads / GROUPS;
     __shared__ __align__(16) float src[kTile64 / 2 * kPairWords];
-    __shared__ double xyz[KIND == kField ? 3 * kTile64 : 1];
+    __shared__ double xyz[has_field<KIND>() ? 3 * kTile64 : 1];
     __shared__ double part[kThreads * COMP];
     __shared__ unsigned s_hi[4];
     int64_t row0, j0, j1;
@@ -294,7 +299,7 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
     }
     const unsigned thi = max(high_abs(T.x), max(high_abs(T.y), high_abs(T.z)));
     int kprev = INT32_MIN;
-    double ex = 0, ey = 0, ez = 0;
+    double ex = 0, ey = 0, ez = 0, ev = 0;
     auto charge = [&](int q) -> double & {
         return reinterpret_cast<double *>(src)[(q >> 1) * (kPairWords / 2) + kPairCharge + (q & 1)];
     };
@@ -319,11 +324,12 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
             if ((int)threadIdx.x < cnt) charge(threadIdx.x) = w;
             __syncthreads();
             for (int s = grp; s < cnt; s += GROUPS) {
-                double px, py, pz;
-                dense_pair_ieee<KIND>(A.c, jb + s, i, T.x, T.y, T.z, charge(s), A.k_e, px, py, pz);
+                double px, py, pz, pv;
+                dense_pair_ieee<KIND>(A.c, jb + s, i, T.x, T.y, T.z, charge(s), A.k_e, px, py, pz, pv);
                 ex += px;
                 ey += py;
                 ez += pz;
+                ev += pv;
             }
             continue;
         }
@@ -351,7 +357,7 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
             q[14] = c.b;
             q[16] = c.c;
             charge(threadIdx.x) = w;
-            if (KIND == kField) {
+            if (has_field<KIND>()) {
                 xyz[3 * threadIdx.x] = x;
                 xyz[3 * threadIdx.x + 1] = y;
                 xyz[3 * threadIdx.x + 2] = z;
@@ -360,26 +366,28 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
         __syncthreads();
         // closer than the split resolves, or than the clamp: IEEE
         const float near2 = fmaxf(kGridNear2, (float)(1.0001e-24 * down * down));
-        double tx = 0, ty = 0, tz = 0;  // two-level sum: tile, then chunk; the split pairs in scaled units
-        double sx = 0, sy = 0, sz = 0;
+        double tx = 0, ty = 0, tz = 0, tv = 0;  // two-level sum: tile, then chunk; the split pairs in scaled units
+        double sx = 0, sy = 0, sz = 0, sv = 0;
         auto add = [&](int s, float y0, float eh, float v, double w) {
             const double ir = grid_inv(y0, grid_ci(eh, v));
-            if (KIND == kField) {
-                const double f = (A.k_e * (ir * ir * ir)) * w;
+            if (has_field<KIND>()) {  // every FP64 operation is 64 cycles: k_e at the end, w / r shared
+                const double wr = w * ir, f = wr * (ir * ir);
                 tx = fma(f, T.x - xyz[3 * s], tx);
                 ty = fma(f, T.y - xyz[3 * s + 1], ty);
                 tz = fma(f, T.z - xyz[3 * s + 2], tz);
+                if (KIND == kBoth) tv += wr;
             } else {
-                tx = fma(w, ir, tx);
+                tv = fma(w, ir, tv);
             }
         };
         auto ieee = [&](int s, double w) {
             if (s >= cnt) return;  // padding
-            double px, py, pz;
-            dense_pair_ieee<KIND>(A.c, jb + s, i, T.x, T.y, T.z, w, A.k_e, px, py, pz);
+            double px, py, pz, pv;
+            dense_pair_ieee<KIND>(A.c, jb + s, i, T.x, T.y, T.z, w, A.k_e, px, py, pz, pv);
             sx += px;
             sy += py;
             sz += pz;
+            sv += pv;
         };
         struct Pair2 {
             float2 R1, y0, eh, v;
@@ -419,19 +427,21 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
                 add_pair(s + 2 * GROUPS, b);
             }
         }
-        const double unscale = KIND == kField ? down * down * down : down;
-        ex += tx * unscale + sx;
-        if (KIND == kField) {
-            ey += ty * unscale + sy;
-            ez += tz * unscale + sz;
+        if (has_field<KIND>()) {
+            const double unscale = down * down * down;
+            ex += A.k_e * (tx * unscale) + sx;
+            ey += A.k_e * (ty * unscale) + sy;
+            ez += A.k_e * (tz * unscale) + sz;
         }
+        if (KIND != kField) ev += tv * down + sv;
     }
     double *p = part + threadIdx.x * COMP;
-    p[0] = ex;
-    if (KIND == kField) {
+    if (has_field<KIND>()) {
+        p[0] = ex;
         p[1] = ey;
         p[2] = ez;
     }
+    if (KIND != kField) p[COMP - 1] = ev;
     dense_finish<double, KIND, ROWS, GROUPS>(A, part, row0, rank);
 }
 
@@ -475,7 +485,7 @@ int cluster_size(int64_t tiles, int64_t n, bool f64) {
 
 template <typename T, int KIND>
 int dense_launch(const T *tgt, int64_t m, const T *c, const T *sigma, const T *areas, int64_t n, T k_e,
-                 const T *self_int, T *out, cudaStream_t s) {
+                 const T *self_int, T *out, T *out_v, cudaStream_t s) {
     // FP64: 64 targets per block, or 32 when those would leave SMs without a block
     // even in clusters of eight; the smaller tile splits every source for half
     // the targets (1,000 targets, 5,120 sources: 89 and 290 us, potential and
@@ -483,7 +493,7 @@ int dense_launch(const T *tgt, int64_t m, const T *c, const T *sigma, const T *a
     const bool narrow = sizeof(T) == 8 && (m + 63) / 64 * kMaxCluster < 2 * sm_count();
     const int ROWS = sizeof(T) == 4 ? 32 * tpt32<KIND>() : narrow ? 32 : 64;
     const int64_t tiles = (m + ROWS - 1) / ROWS;
-    DenseArgs<T> A{tgt, m, c, sigma, areas, n, 0, cluster_size(tiles, n, sizeof(T) == 8), k_e, self_int, out};
+    DenseArgs<T> A{tgt, m, c, sigma, areas, n, 0, cluster_size(tiles, n, sizeof(T) == 8), k_e, self_int, out, out_v};
     A.chunk = ((n + A.cs - 1) / A.cs + 1) & ~(int64_t)1;
     if (tiles * A.cs > INT32_MAX) return fail(EDFMM_ERR_ARG, "too many targets for one launch");
     cudaLaunchConfig_t cfg = {};
@@ -506,12 +516,13 @@ int dense_launch(const T *tgt, int64_t m, const T *c, const T *sigma, const T *a
 
 template <int KIND>
 int dense_any(const void *tgt, int64_t m, const void *c, const void *sigma, const void *areas, int64_t n, int dtype,
-              double k_e, const void *self_int, void *out, cudaStream_t s) {
+              double k_e, const void *self_int, void *out, void *out_v, cudaStream_t s) {
     if (dtype == EDFMM_F64)
         return dense_launch<double, KIND>((const double *)tgt, m, (const double *)c, (const double *)sigma,
-                                          (const double *)areas, n, k_e, (const double *)self_int, (double *)out, s);
+                                          (const double *)areas, n, k_e, (const double *)self_int, (double *)out,
+                                          (double *)out_v, s);
     return dense_launch<float, KIND>((const float *)tgt, m, (const float *)c, (const float *)sigma, (const float *)areas,
-                                     n, (float)k_e, (const float *)self_int, (float *)out, s);
+                                     n, (float)k_e, (const float *)self_int, (float *)out, (float *)out_v, s);
 }
 
 }  // namespace
@@ -530,7 +541,7 @@ extern "C" EDFMM_API int edfmm_dense_matvec(const void *centroids, const void *s
     if (n == 0) return EDFMM_OK;
     if (!centroids || !sigma || !areas || !out) return fail(EDFMM_ERR_ARG, "centroids, sigma, areas, out must be non-NULL");
     return dense_any<kMatvec>(centroids, n, centroids, sigma, areas, n, dtype, k_e, self_integrals, out,
-                              static_cast<cudaStream_t>(stream));
+                              nullptr, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" EDFMM_API int edfmm_dense_matvec_noalloc(const void *centroids, const void *sigma, const void *areas,
@@ -562,7 +573,7 @@ extern "C" EDFMM_API int edfmm_dense_field_targets(const void *targets, int64_t 
         return EDFMM_OK;
     }
     if (!targets || !centroids || !sigma || !areas || !out) return fail(EDFMM_ERR_ARG, "NULL argument");
-    return dense_any<kField>(targets, m, centroids, sigma, areas, n, dtype, k_e, nullptr, out, s);
+    return dense_any<kField>(targets, m, centroids, sigma, areas, n, dtype, k_e, nullptr, out, nullptr, s);
 }
 
 extern "C" EDFMM_API int edfmm_dense_potential_targets(const void *targets, int64_t m, const void *centroids,
@@ -577,5 +588,23 @@ extern "C" EDFMM_API int edfmm_dense_potential_targets(const void *targets, int6
         return EDFMM_OK;
     }
     if (!targets || !centroids || !sigma || !areas || !out) return fail(EDFMM_ERR_ARG, "NULL argument");
-    return dense_any<kPotential>(targets, m, centroids, sigma, areas, n, dtype, k_e, nullptr, out, s);
+    return dense_any<kPotential>(targets, m, centroids, sigma, areas, n, dtype, k_e, nullptr, out, nullptr, s);
+}
+
+extern "C" EDFMM_API int edfmm_dense_potential_field_targets(const void *targets, int64_t m, const void *centroids,
+                                                             const void *sigma, const void *areas, int64_t n, int dtype,
+                                                             double k_e, void *potential, void *field, void *stream) {
+    if (m < 0 || n < 0) return fail(EDFMM_ERR_ARG, "sizes must be >= 0");
+    if (dtype != EDFMM_F32 && dtype != EDFMM_F64) return fail(EDFMM_ERR_ARG, "bad dtype");
+    if (m == 0) return EDFMM_OK;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (!targets || !potential || !field) return fail(EDFMM_ERR_ARG, "NULL argument");
+    if (n == 0) {
+        const size_t row = (size_t)m * (dtype == EDFMM_F64 ? 8 : 4);
+        EDFMM_CUDA_TRY(cudaMemsetAsync(potential, 0, row, s));
+        EDFMM_CUDA_TRY(cudaMemsetAsync(field, 0, 3 * row, s));
+        return EDFMM_OK;
+    }
+    if (!centroids || !sigma || !areas) return fail(EDFMM_ERR_ARG, "NULL argument");
+    return dense_any<kBoth>(targets, m, centroids, sigma, areas, n, dtype, k_e, nullptr, field, potential, s);
 }

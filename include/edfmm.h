@@ -282,6 +282,10 @@ EDFMM_API int edfmm_dense_potential_targets(const void *targets_dev, int64_t m, 
 EDFMM_API int edfmm_dense_field_targets(const void *targets_dev, int64_t m, const void *centroids_dev,
                                         const void *sigma_dev, const void *areas_dev, int64_t n, int dtype,
                                         double k_e, void *out_dev, void *stream);
+/* both in one pass over the panels: potential (m), field (m, 3) */
+EDFMM_API int edfmm_dense_potential_field_targets(const void *targets_dev, int64_t m, const void *centroids_dev,
+                                                  const void *sigma_dev, const void *areas_dev, int64_t n, int dtype,
+                                                  double k_e, void *potential_dev, void *field_dev, void *stream);
 
 /*
  * Dense operator with a caller-provided workspace of
