@@ -129,6 +129,9 @@ def _declare(L):
         "edfmm_dense_matvec_ws": (i32, [_vp, _vp, _vp, _vp, i64, i32, dbl, _vp, _vp, C.c_size_t, _vp]),
         "edfmm_dense_potential_targets": (i32, [_vp, i64, _vp, _vp, _vp, i64, i32, dbl, _vp, _vp]),
         "edfmm_dense_field_targets": (i32, [_vp, i64, _vp, _vp, _vp, i64, i32, dbl, _vp, _vp]),
+        "edfmm_dense_table_bytes": (C.c_size_t, [i64]),
+        "edfmm_dense_table_build": (i32, [_vp, i64, _vp, _vp]),
+        "edfmm_dense_table_matvec": (i32, [_vp, _vp, _vp, _vp, i64, dbl, _vp, _vp]),
         "edfmm_dense_potential_field_targets": (i32, [_vp, i64, _vp, _vp, _vp, i64, i32, dbl, _vp, _vp, _vp]),
         "edfmm_self_integrals": (i32, [_vp, _vp, i64, i32, i32, dbl, _vp, _vp]),
         "edfmm_near_targets_correct": (i32, [_vp, i64, _vp, _vp, _vp, _vp, i64, dbl, i32, i32, dbl, _vp, _vp]),

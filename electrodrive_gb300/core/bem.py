@@ -288,6 +288,8 @@ def _solve_pass(spec: Any, cfg: BEMConfig, mesh: TriMesh, h: float, *, dev, dtyp
                                        distance_factor=float(getattr(cfg, "near_quadrature_distance_factor", 1.5)),
                                        order=order, depth=depth_near, dtype=dtype)
     op = build_operator(C64, A64, self_corr, dtype=dtype, kind=operator, fmm_threshold=fmm_threshold, device=dev)
+    if isinstance(op.base, DenseOperator) and not mixed:  # a mixed solve applies the FP64 operator a few times only
+        op.base.tabulate()
     if near_job is not None:
         near = op.near = near_job()
     op32 = None

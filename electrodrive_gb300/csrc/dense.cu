@@ -34,7 +34,8 @@ namespace edfmm {
 
 namespace {
 
-enum DenseKind { kMatvec = 0, kPotential = 1, kField = 2, kBoth = 3 };  // kBoth: field and potential in one pass
+// kBoth: field and potential in one pass; kTable: every 1 / r of the operator written out
+enum DenseKind { kMatvec = 0, kPotential = 1, kField = 2, kBoth = 3, kTable = 4 };
 template <int KIND> __host__ __device__ constexpr bool has_field() { return KIND == kField || KIND == kBoth; }
 // sums per target: the field's three, the potential
 template <int KIND> __host__ __device__ constexpr int dense_comp() { return KIND == kField ? 3 : KIND == kBoth ? 4 : 1; }
@@ -58,6 +59,7 @@ template <typename T> struct DenseArgs {
     const T *self_int;  // kMatvec only
     T *out;
     T *out_v;  // kBoth: the potential
+    int64_t ld;  // kTable: distance of out's rows
 };
 
 __device__ __forceinline__ void cluster_sync_all() {
@@ -266,7 +268,7 @@ template <int KIND>
 __device__ __noinline__ void dense_pair_ieee(const double *c, int64_t j, int64_t self, double x, double y, double z,
                                              double w, double k_e, double &ex, double &ey, double &ez, double &ev) {
     ex = ey = ez = ev = 0.0;
-    if (KIND == kMatvec && j == self) return;
+    if ((KIND == kMatvec || KIND == kTable) && j == self) return;
     const double dx = x - c[3 * j], dy = y - c[3 * j + 1], dz = z - c[3 * j + 2];
     const double ir = inv_r(dx * dx + dy * dy + dz * dz);
     if (has_field<KIND>()) {
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
             x = A.c[3 * j];
             y = A.c[3 * j + 1];
             z = A.c[3 * j + 2];
-            w = A.sigma[j] * A.areas[j];
+            w = KIND == kTable ? 1.0 : A.sigma[j] * A.areas[j];
         }
         // the tile's scale: a power of two above every |coordinate| of its sources and targets
         const unsigned hi = __reduce_max_sync(0xffffffffu, max(max(thi, high_abs(x)), max(high_abs(y), high_abs(z))));
@@ -326,6 +328,7 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
             for (int s = grp; s < cnt; s += GROUPS) {
                 double px, py, pz, pv;
                 dense_pair_ieee<KIND>(A.c, jb + s, i, T.x, T.y, T.z, charge(s), A.k_e, px, py, pz, pv);
+                if (KIND == kTable && i < A.m) A.out[(jb + s) * A.ld + i] = pv;
                 ex += px;
                 ey += py;
                 ez += pz;
@@ -376,6 +379,8 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
                 ty = fma(f, T.y - xyz[3 * s + 1], ty);
                 tz = fma(f, T.z - xyz[3 * s + 2], tz);
                 if (KIND == kBoth) tv += wr;
+            } else if (KIND == kTable) {
+                if (s < cnt && i < A.m) A.out[(jb + s) * A.ld + i] = ir * down;
             } else {
                 tv = fma(w, ir, tv);
             }
@@ -388,6 +393,7 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
             sy += py;
             sz += pz;
             sv += pv;
+            if (KIND == kTable && i < A.m) A.out[(jb + s) * A.ld + i] = pv;
         };
         struct Pair2 {
             float2 R1, y0, eh, v;
@@ -435,6 +441,7 @@ __global__ void __launch_bounds__(kThreads) k_dense_f64(const DenseArgs<double> 
         }
         if (KIND != kField) ev += tv * down + sv;
     }
+    if (KIND == kTable) return;
     double *p = part + threadIdx.x * COMP;
     if (has_field<KIND>()) {
         p[0] = ex;
@@ -485,15 +492,15 @@ int cluster_size(int64_t tiles, int64_t n, bool f64) {
 
 template <typename T, int KIND>
 int dense_launch(const T *tgt, int64_t m, const T *c, const T *sigma, const T *areas, int64_t n, T k_e,
-                 const T *self_int, T *out, T *out_v, cudaStream_t s) {
+                 const T *self_int, T *out, T *out_v, cudaStream_t s, int64_t ld = 0) {
     // FP64: 64 targets per block, or 32 when those would leave SMs without a block
     // even in clusters of eight; the smaller tile splits every source for half
     // the targets (1,000 targets, 5,120 sources: 89 and 290 us, potential and
     // field, with 64, 76 and 180 with 32)
-    const bool narrow = sizeof(T) == 8 && (m + 63) / 64 * kMaxCluster < 2 * sm_count();
+    const bool narrow = sizeof(T) == 8 && KIND != kTable && (m + 63) / 64 * kMaxCluster < 2 * sm_count();
     const int ROWS = sizeof(T) == 4 ? 32 * tpt32<KIND>() : narrow ? 32 : 64;
     const int64_t tiles = (m + ROWS - 1) / ROWS;
-    DenseArgs<T> A{tgt, m, c, sigma, areas, n, 0, cluster_size(tiles, n, sizeof(T) == 8), k_e, self_int, out, out_v};
+    DenseArgs<T> A{tgt, m, c, sigma, areas, n, 0, cluster_size(tiles, n, sizeof(T) == 8), k_e, self_int, out, out_v, ld};
     A.chunk = ((n + A.cs - 1) / A.cs + 1) & ~(int64_t)1;
     if (tiles * A.cs > INT32_MAX) return fail(EDFMM_ERR_ARG, "too many targets for one launch");
     cudaLaunchConfig_t cfg = {};
@@ -513,6 +520,75 @@ int dense_launch(const T *tgt, int64_t m, const T *c, const T *sigma, const T *a
     EDFMM_LAUNCH_CHECK("k_dense");
     return EDFMM_OK;
 }
+
+// ---------------------------------------------------------------------------
+// The FP64 operator of repeated applications: its 1 / r as a table (symmetric,
+// so row j serves source j's column), and their matrix-vector product.  A pair
+// then costs 8 bytes and one FP64 multiply-add in place of 136 FP32 operations.
+// A lane owns two targets, a warp 64; the eight warps of a block and the blocks
+// of a cluster of eight take every 64th source, and their sums are added in
+// a fixed order as in the kernels above.  5,120 panels: 162 us an application
+// from the coordinates, 63 with the table (210 MB; the FP64 pipe's time is 45 us),
+// 180 once to fill it; 20,000 panels (3.2 GB) 2,035 and 734 us.
+// ---------------------------------------------------------------------------
+constexpr size_t kTableCharges = 32768;  // bytes of a block's charges
+constexpr int kTableThreads = 256, kTableRows = 64, kTableWarps = kTableThreads / 32;
+
+__global__ void __launch_bounds__(kTableThreads) k_dense_table(const double *__restrict__ table, int64_t ld,
+                                                               const DenseArgs<double> A) {
+    __shared__ double part[kTableWarps * kTableRows];
+    extern __shared__ double charge[];  // this block's sources: a product a warp would otherwise form again
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int64_t row0 = (int64_t)(blockIdx.x / (unsigned)A.cs) * kTableRows;
+    const int rank = (int)(blockIdx.x % (unsigned)A.cs);
+    const int64_t j0 = min(A.n, rank * A.chunk);
+    const int cnt = (int)(min(A.n, j0 + A.chunk) - j0);
+    for (int q = threadIdx.x; q < cnt; q += kTableThreads) charge[q] = A.sigma[j0 + q] * A.areas[j0 + q];
+    __syncthreads();
+    const double *col = table + j0 * ld + row0 + 2 * lane;
+    double ax = 0, ay = 0;
+    int j = wid;
+    constexpr int U = 8;  // loads in flight
+    for (; j + (U - 1) * kTableWarps < cnt; j += U * kTableWarps) {
+        double2 k[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            k[u] = __ldg(reinterpret_cast<const double2 *>(col + (int64_t)(j + u * kTableWarps) * ld));
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const double w = charge[j + u * kTableWarps];
+            ax = fma(k[u].x, w, ax);
+            ay = fma(k[u].y, w, ay);
+        }
+    }
+    for (; j < cnt; j += kTableWarps) {
+        const double2 k = __ldg(reinterpret_cast<const double2 *>(col + (int64_t)j * ld));
+        ax = fma(k.x, charge[j], ax);
+        ay = fma(k.y, charge[j], ay);
+    }
+    part[wid * kTableRows + 2 * lane] = ax;
+    part[wid * kTableRows + 2 * lane + 1] = ay;
+    __syncthreads();
+    if (threadIdx.x < kTableRows) {
+        double v = part[threadIdx.x];
+#pragma unroll
+        for (int g = 1; g < kTableWarps; ++g) v += part[g * kTableRows + threadIdx.x];
+        part[threadIdx.x] = v;
+    }
+    if (A.cs > 1) cluster_sync_all();
+    else __syncthreads();
+    const int64_t i = row0 + threadIdx.x;
+    if (rank == 0 && threadIdx.x < kTableRows && i < A.m) {
+        double v = part[threadIdx.x];
+        for (int r = 1; r < A.cs; ++r) v += dsm_load(part + threadIdx.x, r);
+        v *= A.k_e;
+        if (A.self_int) v += A.self_int[i] * A.sigma[i] * A.areas[i];
+        A.out[i] = isfinite(v) ? v : 0.0;
+    }
+    if (A.cs > 1) cluster_sync_all();  // the other blocks' shared memory stays until it has been read
+}
+
+inline int64_t table_ld(int64_t n) { return (n + kTableRows - 1) / kTableRows * kTableRows; }
 
 template <int KIND>
 int dense_any(const void *tgt, int64_t m, const void *c, const void *sigma, const void *areas, int64_t n, int dtype,
@@ -607,4 +683,48 @@ extern "C" EDFMM_API int edfmm_dense_potential_field_targets(const void *targets
     }
     if (!centroids || !sigma || !areas) return fail(EDFMM_ERR_ARG, "NULL argument");
     return dense_any<kBoth>(targets, m, centroids, sigma, areas, n, dtype, k_e, nullptr, field, potential, s);
+}
+
+extern "C" EDFMM_API size_t edfmm_dense_table_bytes(int64_t n) {
+    return n > 0 && n <= (int64_t)(kTableCharges / sizeof(double)) * kMaxCluster ? (size_t)n * (size_t)table_ld(n) * sizeof(double) : 0;
+}
+
+extern "C" EDFMM_API int edfmm_dense_table_build(const void *centroids, int64_t n, void *table, void *stream) {
+    if (n < 0) return fail(EDFMM_ERR_ARG, "n must be >= 0");
+    if (n == 0) return EDFMM_OK;
+    if (!centroids || !table) return fail(EDFMM_ERR_ARG, "NULL argument");
+    if (edfmm_dense_table_bytes(n) == 0) return fail(EDFMM_ERR_ARG, "edfmm_dense_table_build: too many panels");
+    const double *c = static_cast<const double *>(centroids);
+    return dense_launch<double, kTable>(c, n, c, nullptr, nullptr, n, 1.0, nullptr, static_cast<double *>(table),
+                                        nullptr, static_cast<cudaStream_t>(stream), table_ld(n));
+}
+
+extern "C" EDFMM_API int edfmm_dense_table_matvec(const void *table, const void *sigma, const void *areas,
+                                                  const void *self_integrals, int64_t n, double k_e, void *out,
+                                                  void *stream) {
+    if (n < 0) return fail(EDFMM_ERR_ARG, "n must be >= 0");
+    if (n == 0) return EDFMM_OK;
+    if (!table || !sigma || !areas || !out) return fail(EDFMM_ERR_ARG, "table, sigma, areas, out must be non-NULL");
+    const int64_t tiles = (n + kTableRows - 1) / kTableRows;
+    const int64_t chunk = (n + kMaxCluster - 1) / kMaxCluster;
+    if (chunk * sizeof(double) > kTableCharges)
+        return fail(EDFMM_ERR_ARG, "edfmm_dense_table_matvec: at most " +
+                                       std::to_string(kTableCharges / sizeof(double) * kMaxCluster) + " panels");
+    DenseArgs<double> A{nullptr, n, nullptr, (const double *)sigma, (const double *)areas, n, chunk, kMaxCluster, k_e,
+                        (const double *)self_integrals, (double *)out, nullptr, 0};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles * A.cs));
+    cfg.blockDim = dim3(kTableThreads);
+    cfg.dynamicSmemBytes = (size_t)chunk * sizeof(double);
+    cfg.stream = static_cast<cudaStream_t>(stream);
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)A.cs;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_dense_table, static_cast<const double *>(table), table_ld(n), A);
+    if (e != cudaSuccess) return fail(EDFMM_ERR_CUDA, std::string("launch of k_dense_table failed: ") + cudaGetErrorString(e));
+    EDFMM_LAUNCH_CHECK("k_dense_table");
+    return EDFMM_OK;
 }

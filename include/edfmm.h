@@ -282,6 +282,16 @@ EDFMM_API int edfmm_dense_potential_targets(const void *targets_dev, int64_t m, 
 EDFMM_API int edfmm_dense_field_targets(const void *targets_dev, int64_t m, const void *centroids_dev,
                                         const void *sigma_dev, const void *areas_dev, int64_t n, int dtype,
                                         double k_e, void *out_dev, void *stream);
+/*
+ * The FP64 dense operator for repeated applications: every 1 / |c_i - c_j| (0 on
+ * the diagonal) in a table of edfmm_dense_table_bytes(n) bytes (0: n is above
+ * 32,768), 16-byte aligned, and edfmm_dense_matvec's result from it.
+ */
+EDFMM_API size_t edfmm_dense_table_bytes(int64_t n);
+EDFMM_API int edfmm_dense_table_build(const void *centroids_dev, int64_t n, void *table_dev, void *stream);
+EDFMM_API int edfmm_dense_table_matvec(const void *table_dev, const void *sigma_dev, const void *areas_dev,
+                                       const void *self_integrals_dev, int64_t n, double k_e, void *out_dev,
+                                       void *stream);
 /* both in one pass over the panels: potential (m), field (m, 3) */
 EDFMM_API int edfmm_dense_potential_field_targets(const void *targets_dev, int64_t m, const void *centroids_dev,
                                                   const void *sigma_dev, const void *areas_dev, int64_t n, int dtype,
