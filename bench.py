@@ -70,17 +70,20 @@ def m2l_flops_per_pair(p):
 M2L_FLOPS_PER_PAIR = m2l_flops_per_pair(8)
 # DRAM bytes one M2L launch moves per pair: the source index (4 B) and one read
 # of the source's multipole row (the rows stay in L2 across a target's pairs);
-# taken from an ncu capture of k_m2l_rot<float, 8> at N = 262,144 (44.54 MB read
-# for 9,091,877 pairs)
-M2L_DRAM_BYTES_PER_PAIR = 44.54e6 / 9_091_877
-# DRAM bytes (read + write) per M2L pair of k_m2l_rot<float, p> on the
+# taken from an ncu capture of k_m2l_rot<8> at N = 262,144 (44.64 MB moved for
+# 9,017,270 pairs)
+M2L_DRAM_BYTES_PER_PAIR = 44.64e6 / 9_017_270
+# DRAM bytes (read + write) per M2L pair of k_m2l_rot<p> on the
 # 200,000-panel torus (FP32 inner operator), from ncu captures of that kernel
 # on that mesh (median over the profile run's launches)
 M2L_DRAM_BYTES_PER_PAIR_TORUS = {(8, 64): 14_461_269 / 2_315_072, (6, 64): 12_600_576 / 2_315_072}  # (p, leaf)
 # the same for the 256-dimer batch (FP32 inner operator, autotuned order)
 M2L_DRAM_BYTES_PER_PAIR_BATCH = {(6, 64): (244_023_808 + 55_725_312) / 39_011_439}  # (p, leaf)
-# DRAM bytes of one k_dense_partial<double> launch at n = 5,120 (ncu capture)
-DENSE_DRAM_BYTES_PER_MATVEC_5120 = 293_120
+# DRAM bytes of one k_dense_f64 launch at n = 5,120 (ncu capture)
+DENSE_DRAM_BYTES_PER_MATVEC_5120 = 196_608
+# the FP64 dense kernel forms 1 / r on the FP32 pipe: 136 operations a pair there
+# (a multiply-add counts two), one FP64 multiply-add beside them
+DENSE_FP32_FLOPS_PER_INTERACTION = 2 * 136
 # near field: 3 sub + 3 fma (r^2) + max + rsqrt + fma per interaction, counted
 # as the reference FLOP model's 20 flops (autotune.py:622-667)
 P2P_FLOPS_PER_INTERACTION = 20
@@ -565,14 +568,14 @@ def run_solve_workload(args, rank, world, local, emit=True):
             mv[key] = statistics.median(_time_cuda(lambda: op(s_dt), dev, stream, flush, 3, 10))
     extra = {}
     if name == "sphere_solve":
-        peak = _lib.measure_fp64_peak()
-        flops = 20.0 * n * n
+        peak = _lib.measure_fp32_peak()
+        flops = float(DENSE_FP32_FLOPS_PER_INTERACTION) * n * n
         achieved = flops / (mv["float64"] * 1e-3) / 1e12
-        roof = {"kernel": "k_dense_partial<double> (dense FP64 operator)", "bound": "fp64", "achieved": achieved,
+        roof = {"kernel": "k_dense_f64 (dense FP64 operator)", "bound": "fp32", "achieved": achieved,
                 "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
                 "traffic": DENSE_DRAM_BYTES_PER_MATVEC_5120,
-                "traffic_note": "DRAM bytes of one k_dense_partial<double> launch at n = 5,120 (ncu)",
-                "peak_source": "FP64 FMA probe measured in this run (edfmm_measure_fp64_peak)",
+                "traffic_note": "DRAM bytes of one k_dense_f64 launch at n = 5,120 (ncu)",
+                "peak_source": "FP32 FMA probe measured in this run (edfmm_measure_fp32_peak)",
                 "flops_per_matvec": flops}
         # Kelvin image and exterior potential
         from electrodrive_gb300.core.bem import BEMSolution
@@ -676,7 +679,7 @@ def run_solve_workload(args, rank, world, local, emit=True):
         order32 = int(p32.info.expansion_order)
         achieved = p32.info.n_m2l_pairs * m2l_flops_per_pair(order32) / (m2l_ms * 1e-3) / 1e12
         per_pair = M2L_DRAM_BYTES_PER_PAIR_TORUS.get((order32, int(p32.info.leaf_size)))
-        roof = {"kernel": f"k_m2l_rot<float, {order32}> (M2L of the FP32 inner operator)", "bound": "fp32",
+        roof = {"kernel": f"k_m2l_rot<{order32}> (M2L of the FP32 inner operator)", "bound": "fp32",
                 "achieved": achieved,
                 "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak if fp32_peak else None,
                 "traffic": per_pair * p32.info.n_m2l_pairs if per_pair else None,
@@ -957,7 +960,7 @@ def run_batch_workload(args, rank, world, local, emit=True):
                                                            "self integrals, rhs), the solve and the read-back",
                        "setup_phases_ms": setup_phases},
                "gpu_launches": int(launches), "clocks": clk.summary(),
-               "roofline": {"kernel": f"k_m2l_rot<float, {order}> (M2L of the FP32 inner operator)", "bound": "fp32",
+               "roofline": {"kernel": f"k_m2l_rot<{order}> (M2L of the FP32 inner operator)", "bound": "fp32",
                             "achieved": ach, "peak": fp32_peak, "unit": "TFLOP/s",
                             "frac": ach / fp32_peak if ach else None,
                             "traffic": per_pair * p32.info.n_m2l_pairs if per_pair else None,
@@ -1295,7 +1298,7 @@ def main():
                     "ms_per_step": e2e_ms},
             "gpu_launches": int(launches),
             "clocks": clk.summary(),
-            "roofline": {"kernel": "k_m2l_rot<float, 8> (rotation-based M2L stage)", "bound": "fp32",
+            "roofline": {"kernel": "k_m2l_rot<8> (rotation-based M2L stage)", "bound": "fp32",
                          "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                          "frac": achieved / fp32_peak if fp32_peak else None,
                          "traffic": M2L_DRAM_BYTES_PER_PAIR * info.n_m2l_pairs,
