@@ -560,44 +560,47 @@ __global__ void __launch_bounds__(32 * kNearWarps, near_blocks<MODE>())
 // ---------------------------------------------------------------------------
 // L2P and epilogue: one warp per leaf, one lane per target
 // ---------------------------------------------------------------------------
-// Re sum_{n,m} L_n^m R_n^m(x, y, z) over m in [-n, n]
+// Re sum_{n,m} L_n^m R_n^m(x, y, z) over m in [-n, n].  R_n^m = R_m^m rho_n with a
+// real rho (rho_m = 1), so that a term takes five operations (three of the
+// recursion, two sums) and a column one complex product at its end, where the
+// complex recursion took nine a term.  FP64, 1,254 leaves 69 -> 47 us; two-float,
+// 2,468 leaves 52 -> 41; FP32, 29,158 leaves at order 6 32 -> 26.
+template <typename T, int P, int M>
+__device__ __forceinline__ T l2p_columns(const Cplx<T> *L, T x, T y, T r2, const T (&zc)[P + 1], T dr, T di, T acc) {
+    Cplx<T> lv = L[tri(M, M)];
+    T re = lv.re, im = lv.im, rho = (T)1, last = (T)0;
+#pragma unroll
+    for (int n = M + 1; n <= P; ++n) {
+        const T d = (T)(1.0 / ((n + M) * (n - M)));
+        const T next = (n == M + 1 ? zc[n] : zc[n] * rho - r2 * last) * d;
+        last = rho;
+        rho = next;
+        lv = L[tri(n, M)];
+        re += lv.re * rho;
+        if (M > 0) im += lv.im * rho;
+    }
+    acc += M == 0 ? re : (T)2 * (re * dr - im * di);
+    if constexpr (M < P) {
+        constexpr double c = -0.5 / (M + 1);
+        const T sx = (T)c * x, sy = (T)c * y;
+        return l2p_columns<T, P, M + 1>(L, x, y, r2, zc, M == 0 ? sx : sx * dr - sy * di,
+                                        M == 0 ? sy : sx * di + sy * dr, acc);
+    } else {
+        return acc;
+    }
+}
 template <typename T, int P>
 __device__ __forceinline__ T l2p_point(const Cplx<T> *L, T x, T y, T z) {
-    const T r2 = x * x + y * y + z * z;
-    T acc = (T)0, dr = (T)1, di = (T)0;
+    T zc[P + 1];
 #pragma unroll
-    for (int m = 0; m <= P; ++m) {
-        if (m > 0) {
-            const T s = (T)(-0.5 / (m > 0 ? m : 1));
-            const T nr = s * (x * dr - y * di), ni = s * (x * di + y * dr);
-            dr = nr;
-            di = ni;
-        }
-        const T w = m == 0 ? (T)1 : (T)2;
-        T pr = dr, pi = di, qr = (T)0, qi = (T)0;
-        Cplx<T> lv = L[tri(m, m)];
-        T col = lv.re * pr - lv.im * pi;
-#pragma unroll
-        for (int n = m + 1; n <= P; ++n) {
-            const T d = (T)(1.0 / ((n + m) * (n - m)));
-            const T c1 = (T)(2 * n - 1) * z;
-            const T nr = (c1 * pr - r2 * qr) * d, ni = (c1 * pi - r2 * qi) * d;
-            lv = L[tri(n, m)];
-            col += lv.re * nr - lv.im * ni;
-            qr = pr;
-            qi = pi;
-            pr = nr;
-            pi = ni;
-        }
-        acc += w * col;
-    }
-    return acc;
+    for (int n = 1; n <= P; ++n) zc[n] = (T)(2 * n - 1) * z;
+    return l2p_columns<T, P, 0>(L, x, y, x * x + y * y + z * z, zc, (T)1, (T)0, (T)0);
 }
 
 // l2p_point in two-float arithmetic, on two-float locals
 __device__ __forceinline__ tf32x2 l2p_point_tf(const tf32x2c *L, int p, tf32x2 x, tf32x2 y, tf32x2 z) {
     using T = tf32x2;
-    const T r2 = fma(z, z, fma(y, y, x * x));
+    const T r2 = fma(z, z, fma(y, y, x * x)), n2 = -r2;
     T acc = T(0), dr = T(1), di = T(0);
     for (int m = 0; m <= p; ++m) {
         if (m > 0) {
@@ -607,21 +610,18 @@ __device__ __forceinline__ tf32x2 l2p_point_tf(const tf32x2c *L, int p, tf32x2 x
             dr = nr;
             di = ni;
         }
-        T pr = dr, pi = di, qr = T(0), qi = T(0);
         tf32x2c lv = L[tri(m, m)];
-        T col = lv.x * pr - lv.y * pi;
+        T re = lv.x, im = lv.y, rho = T(1), last = T(0);
         for (int n = m + 1; n <= p; ++n) {
             const float2 rd = c_rdiv_tf[n][m];
-            const T d(rd.x, rd.y);
-            const T c1 = T(2 * n - 1) * z;
-            const T nr = (c1 * pr - r2 * qr) * d, ni = (c1 * pi - r2 * qi) * d;
+            const T next = fma(T(2 * n - 1) * z, rho, n2 * last) * T(rd.x, rd.y);
+            last = rho;
+            rho = next;
             lv = L[tri(n, m)];
-            col = col + (lv.x * nr - lv.y * ni);
-            qr = pr;
-            qi = pi;
-            pr = nr;
-            pi = ni;
+            re = fma(lv.x, rho, re);
+            im = fma(lv.y, rho, im);
         }
+        const T col = re * dr - im * di;
         acc = m == 0 ? acc + col : acc + T(2) * col;
     }
     return acc;
