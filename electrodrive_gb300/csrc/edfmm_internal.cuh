@@ -288,6 +288,33 @@ __device__ __forceinline__ bool inst_active(const InstMask &m, int node) {
 }
 #endif
 
+// Chains of small kernels (the far field of a small tree): a kernel launched by
+// chain_launch may start while its predecessor in the stream still runs.  It
+// reads what the plan holds, calls chain_wait (all threads, before any return),
+// and only then reads or writes what other kernels of the chain do; chain_next
+// lets its own successor start.  Without the launch attribute both do nothing.
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... K, typename... A>
+cudaError_t chain_launch(bool chained, void (*kernel)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                         A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+#endif
+// small trees, outside a capture (a graph has its own order)
+bool chain_tree(int64_t n_nodes, int dtype, cudaStream_t s);
+
 int tree_build(const void *points_dev, int64_t n, int dtype, int leaf_size, int max_depth,
                DevTree &tree, cudaStream_t s);
 // One tree per instance (rows inst_off[k] .. inst_off[k+1]-1, host offsets),

@@ -92,6 +92,8 @@ template <bool SPLIT>
 __global__ void __launch_bounds__(256) k_mult_columns(const float4 *__restrict__ in, int64_t n_nodes, int words,
                                                       float4 *__restrict__ out) {
     extern __shared__ float4 col_tile[];  // [32][words + 1]
+    chain_next();
+    chain_wait();
     const int64_t n0 = (int64_t)blockIdx.x * kColNodes;
     const int nodes = (int)min((int64_t)kColNodes, n_nodes - n0);
     for (int k = threadIdx.x; k < nodes * words; k += blockDim.x) {
@@ -110,11 +112,11 @@ __global__ void __launch_bounds__(256) k_mult_columns(const float4 *__restrict__
     }
 }
 template <bool SPLIT>
-int mult_columns(const FmmBuffers &buf, int64_t n_nodes, const DevBuf &out, cudaStream_t s) {
+int mult_columns(const FmmBuffers &buf, int64_t n_nodes, const DevBuf &out, bool chained, cudaStream_t s) {
     const int words = SPLIT ? buf.nc_pad : buf.nc_pad / 2;
     const size_t smem = sizeof(float4) * kColNodes * (size_t)(words + 1);
-    k_mult_columns<SPLIT><<<nblk(n_nodes, kColNodes), 256, smem, s>>>(dptr<float4>(buf.multipoles), n_nodes, words,
-                                                                      dptr<float4>(out));
+    EDFMM_CUDA_TRY(chain_launch(chained, k_mult_columns<SPLIT>, nblk(n_nodes, kColNodes), 256, smem, s,
+                                dptr<float4>(buf.multipoles), n_nodes, words, dptr<float4>(out)));
     EDFMM_LAUNCH_CHECK("k_mult_columns");
     return EDFMM_OK;
 }
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(32 * p2m_warps<T>())
           const int2 *__restrict__ range, Cplx<T> *__restrict__ Mexp, int nc_pad) {
     constexpr int NV = 2 * ncoef(P), NR = (NV + 31) / 32;
     extern __shared__ __align__(16) unsigned char p2m_smem[];
+    chain_next();
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= n_leaves) return;
@@ -796,6 +799,11 @@ __global__ void __launch_bounds__(shift_threads<P>()) k_m2m_node(
     const int tn = D.n[tid], tm = D.m[tid], tk = D.k[tid], tl = D.l[tid], tc = D.cnt[tid];
     if (frames) load_frame<T, P>(S, frames + (int64_t)blockIdx.x * kFrameSize);
     const bool leaf = is_leaf[node];
+    int child[8];
+#pragma unroll
+    for (int o = 0; o < 8; ++o) child[o] = leaf ? -1 : children[8 * node + o];
+    chain_next();
+    chain_wait();
     T2 x[(NC + NT - 1) / NT];
 #pragma unroll
     for (int r = 0; r < (NC + NT - 1) / NT; ++r) {
@@ -807,8 +815,7 @@ __global__ void __launch_bounds__(shift_threads<P>()) k_m2m_node(
             T2 v[8];
 #pragma unroll
             for (int o = 0; o < 8; ++o) {
-                const int ch = children[8 * node + o];
-                v[o] = ch >= 0 ? moved[(int64_t)ch * nc_pad + q] : mk2((T)0, (T)0);
+                v[o] = child[o] >= 0 ? moved[(int64_t)child[o] * nc_pad + q] : mk2((T)0, (T)0);
             }
             x[r] = v[0];
 #pragma unroll
@@ -857,6 +864,8 @@ __global__ void __launch_bounds__(shift_threads<P>()) k_l2l_node(const int32_t *
     const ShiftSplit<P, true> &D = d_shift_split<P, true>;
     const int tn = D.n[tid], tm = D.m[tid], tk = D.k[tid], tl = D.l[tid], tc = D.cnt[tid];
     load_frame<T, P>(S, frames + (int64_t)blockIdx.x * kFrameSize);
+    chain_next();
+    chain_wait();
     T2 x[(NC + NT - 1) / NT], old[(NC + NT - 1) / NT];
 #pragma unroll
     for (int r = 0; r < (NC + NT - 1) / NT; ++r) {
@@ -1115,6 +1124,15 @@ template <typename T> int p2m_impl(const DevTree &tree, FmmBuffers &buf, cudaStr
     return EDFMM_OK;
 }
 
+// Far-field chains of trees up to these sizes overlap their launches
+// (chain_launch).  FP32 matvecs of 2,003 points (73 nodes) take 60 us without and
+// 43 with, 16,000 points (585 nodes) 125 and 102, the 200k-panel torus (11,705)
+// 339 and 331, a million points (37,449) 4,600 and 4,624; FP64 2,000 points (65)
+// 177 and 164, 20,011 points (1,500) 1,291 and 1,296, the 50k-panel torus in
+// two-float (2,937) 1,602 and 1,655: blocks that wait for their predecessor hold
+// places the near field would use.
+constexpr int64_t kChainNodes32 = 16384, kChainNodes64 = 512;
+
 // FP32 levels up to this many nodes take a block per node (FP64 all levels).
 // M2M and L2L of the 200k-panel torus (levels of 2,344 and 6,968 nodes at order
 // 6) take 62 and 43 us with the line at 2,048, 58 and 44 at 6,144, 58 and 49 at
@@ -1124,16 +1142,18 @@ constexpr int kNodeLevel = 6144;
 
 template <typename T, int P> int launch_m2m_fast(const DevTree &tree, FmmBuffers &buf, cudaStream_t s) {
     using T2 = typename Pair<T>::type;
+    const bool chained = chain_tree(tree.n_nodes, tree.dtype, s);
     for (int lev = tree.max_level; lev >= 0; --lev) {
         const int lo = tree.level_offsets[lev], hi = tree.level_offsets[lev + 1];
         if (hi <= lo) continue;
         const int32_t *nodes = dptr<int32_t>(tree.level_nodes) + lo;
         const int64_t frames = tree.frame_off[lev];
         if (frames >= 0 || lev == 0) {
-            k_m2m_node<T, P><<<(unsigned)(hi - lo), shift_threads<P>(), 0, s>>>(
-                nodes, dptr<uint8_t>(tree.is_leaf), dptr<int32_t>(tree.children),
-                lev == 0 ? nullptr : dptr<T>(tree.shift_frames) + frames * kFrameSize, dptr<T2>(buf.multipoles),
-                dptr<T2>(buf.translated), buf.nc_pad);
+            EDFMM_CUDA_TRY(chain_launch(
+                chained, k_m2m_node<T, P>, (unsigned)(hi - lo), shift_threads<P>(), 0, s, nodes,
+                dptr<uint8_t>(tree.is_leaf), dptr<int32_t>(tree.children),
+                lev == 0 ? (T *)nullptr : dptr<T>(tree.shift_frames) + frames * kFrameSize, dptr<T2>(buf.multipoles),
+                dptr<T2>(buf.translated), buf.nc_pad));
         } else if constexpr (sizeof(T) == 4) {
             k_m2m_fast<P><<<nblk(hi - lo, kFastThreads), kFastThreads, 0, s>>>(
                 nodes, hi - lo, dptr<uint8_t>(tree.is_leaf), dptr<int32_t>(tree.children), dptr<int32_t>(tree.parent),
@@ -1147,15 +1167,16 @@ template <typename T, int P> int launch_m2m_fast(const DevTree &tree, FmmBuffers
 
 template <typename T, int P> int launch_l2l_fast(const DevTree &tree, FmmBuffers &buf, cudaStream_t s) {
     using T2 = typename Pair<T>::type;
+    const bool chained = chain_tree(tree.n_nodes, tree.dtype, s);
     for (int lev = 1; lev <= tree.max_level; ++lev) {
         const int lo = tree.level_offsets[lev], hi = tree.level_offsets[lev + 1];
         if (hi <= lo) continue;
         const int32_t *nodes = dptr<int32_t>(tree.level_nodes) + lo;
         const int64_t frames = tree.frame_off[lev];
         if (frames >= 0) {
-            k_l2l_node<T, P><<<(unsigned)(hi - lo), shift_threads<P>(), 0, s>>>(
-                nodes, dptr<int32_t>(tree.parent), dptr<T>(tree.shift_frames) + frames * kFrameSize,
-                dptr<T2>(buf.locals), buf.nc_pad);
+            EDFMM_CUDA_TRY(chain_launch(chained, k_l2l_node<T, P>, (unsigned)(hi - lo), shift_threads<P>(), 0, s, nodes,
+                                        dptr<int32_t>(tree.parent), dptr<T>(tree.shift_frames) + frames * kFrameSize,
+                                        dptr<T2>(buf.locals), buf.nc_pad));
         } else if constexpr (sizeof(T) == 4) {
             k_l2l_fast<P><<<nblk(hi - lo, kFastThreads), kFastThreads, 0, s>>>(
                 nodes, hi - lo, dptr<int32_t>(tree.parent), dptr<float4>(tree.center), dptr<float4>(tree.half),
@@ -1324,7 +1345,7 @@ int m2l_impl(const DevTree &tree, const DevTree &stree, const DevLists &lists, c
     if (sizeof(T) == 8 && buf.arith == EDFMM_ARITH_TWO_FLOAT && buf.p >= 6 && buf.p <= 8 && tree.nodes_tf.p &&
         stree.nodes_tf.p && sbuf.mult_tf.p) {
         // the source multipoles split once per node, then the pairs
-        if (int rc = mult_columns<true>(sbuf, stree.n_nodes, sbuf.mult_tf, s)) return rc;
+        if (int rc = mult_columns<true>(sbuf, stree.n_nodes, sbuf.mult_tf, chain_tree(stree.n_nodes, stree.dtype, s), s)) return rc;
         int rc = launch_m2l_rot_tf(buf.p, M, off, src, rows, tree.nodes_tf.p, tree.half.p, stree.nodes_tf.p, stree.half.p,
                                    sbuf.mult_tf.p, buf.locals.p, buf.nc_pad, buf.mask, buf.m2l_tf_block,
                                    buf.m2l_packed != 0, s);
@@ -1334,7 +1355,7 @@ int m2l_impl(const DevTree &tree, const DevTree &stree, const DevLists &lists, c
     if (!two_float) {
         // FP32 reads the multipoles by columns; `translated` is free once M2M has run
         if constexpr (sizeof(T) == 4) {
-            if (int rc = mult_columns<false>(sbuf, stree.n_nodes, sbuf.translated, s)) return rc;
+            if (int rc = mult_columns<false>(sbuf, stree.n_nodes, sbuf.translated, chain_tree(stree.n_nodes, stree.dtype, s), s)) return rc;
         }
         if (int rc = launch_m2l_rot(sizeof(T) == 8 ? EDFMM_F64 : EDFMM_F32, buf.p, M, off, src, rows, tree.center.p,
                                     tree.half.p, stree.center.p, stree.half.p,
@@ -1375,6 +1396,12 @@ int set_charges(const DevTree &tree, const void *a, const void *b, cudaStream_t 
                                                   static_cast<const float *>(b));
     EDFMM_LAUNCH_CHECK("k_set_charges");
     return EDFMM_OK;
+}
+
+bool chain_tree(int64_t n_nodes, int dtype, cudaStream_t s) {
+    if (n_nodes > (dtype == EDFMM_F64 ? kChainNodes64 : kChainNodes32)) return false;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
 }
 
 int shift_prepare(DevTree &tree, cudaStream_t s) {

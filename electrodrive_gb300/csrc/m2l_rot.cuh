@@ -405,6 +405,7 @@ __global__ void __launch_bounds__(kRotThreads, rot_binomial<float, P>() ? 4 : 3)
     constexpr int NV = (P + 1) * (P + 1), NQ = (P + 1) * (P + 2) / 2, NT = kRotThreads;
     extern __shared__ __align__(16) unsigned char rot_smem[];
     __shared__ int max_rounds;
+    chain_next();
     T2 *sq = reinterpret_cast<T2 *>(rot_smem);
     AccC<NT> acc{sq + threadIdx.x};
     // warp w takes target row rows[w] (rows by decreasing pair count), or row w
@@ -428,6 +429,7 @@ __global__ void __launch_bounds__(kRotThreads, rot_binomial<float, P>() ? 4 : 3)
     if (lane == 0) atomicMax(&max_rounds, (e - b + 31) >> 5);
     __syncthreads();
     const int rounds = max_rounds;
+    chain_wait();
     int sn = b + lane < e ? __ldg(src + b + lane) : 0;  // the next round's source
     for (int r = 0; r < rounds; ++r) {
         __syncthreads();
@@ -853,6 +855,7 @@ __global__ void __launch_bounds__(NT, 256 / NT)
     constexpr int NV = (P + 1) * (P + 1), NR = (NV + 31) / 32;
     extern __shared__ __align__(16) unsigned char rot_smem[];
     __shared__ int max_rounds;
+    chain_next();
     T *slots = reinterpret_cast<T *>(rot_smem);  // slot i of thread u at slots[i * NT + u]
     float *slots_hi = reinterpret_cast<float *>(rot_smem), *slots_lo = slots_hi + NV * NT;  // PK
     using VS = typename std::conditional<PK, SmemSplit<NT>, SmemV<T, NT>>::type;
@@ -886,6 +889,7 @@ __global__ void __launch_bounds__(NT, 256 / NT)
     if (lane == 0) atomicMax(&max_rounds, (e - b + 31) >> 5);
     __syncthreads();
     const int rounds = max_rounds;
+    chain_wait();
     for (int r = 0; r < rounds; ++r) {
         // the block's warps walk the (long, straight-line) pair code together
         // and share its instruction fetches; every thread runs `rounds` rounds
@@ -974,6 +978,8 @@ __global__ void __launch_bounds__(kRotThreads, 2)
     constexpr int NV = (P + 1) * (P + 1), NR = (NV + 31) / 32, NT = kRotThreads, NW = NT / 32;
     extern __shared__ __align__(16) unsigned char rot_smem[];
     double *slots = reinterpret_cast<double *>(rot_smem);  // slot i of thread u at slots[i * NT + u]
+    chain_next();
+    chain_wait();
     const int64_t t = rows ? (int64_t)rows[blockIdx.x] : (int64_t)blockIdx.x;
     if (t >= n_nodes || !inst_active(mask, (int)t)) return;
     const int lane = threadIdx.x & 31, wbase = threadIdx.x & ~31;
@@ -1079,10 +1085,10 @@ int launch_rot_tf(int64_t M, const int32_t *off, const int32_t *src, const int32
         cudaFuncSetAttribute(k_m2l_rot_tf<P, NT, PK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (attr != cudaSuccess)
         return fail(EDFMM_ERR_CUDA, std::string("k_m2l_rot_tf shared memory attribute: ") + cudaGetErrorString(attr));
-    k_m2l_rot_tf<P, NT, PK><<<nblk(M * 32, NT), NT, smem, s>>>(
-        M, off, src, rows, static_cast<const float4 *>(tnodes), static_cast<const double4 *>(thal),
-        static_cast<const float4 *>(snodes), static_cast<const double4 *>(hal), static_cast<const float4 *>(Mx),
-        static_cast<double2 *>(Lx), nc_pad, mask);
+    EDFMM_CUDA_TRY(chain_launch(chain_tree(M, EDFMM_F64, s), k_m2l_rot_tf<P, NT, PK>, nblk(M * 32, NT), NT, smem, s, M, off, src,
+                                rows, static_cast<const float4 *>(tnodes), static_cast<const double4 *>(thal),
+                                static_cast<const float4 *>(snodes), static_cast<const double4 *>(hal),
+                                static_cast<const float4 *>(Mx), static_cast<double2 *>(Lx), nc_pad, mask));
     EDFMM_LAUNCH_CHECK("k_m2l_rot_tf");
     return EDFMM_OK;
 }
@@ -1096,10 +1102,10 @@ int launch_rot_f64(int64_t M, const int32_t *off, const int32_t *src, const int3
         cudaFuncSetAttribute(k_m2l_rot_f64<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (attr != cudaSuccess)
         return fail(EDFMM_ERR_CUDA, std::string("k_m2l_rot_f64 shared memory attribute: ") + cudaGetErrorString(attr));
-    k_m2l_rot_f64<P><<<(unsigned)M, kRotThreads, smem, s>>>(
-        M, off, src, rows, static_cast<const double4 *>(tcen), static_cast<const double4 *>(thal),
-        static_cast<const double4 *>(cen), static_cast<const double4 *>(hal), static_cast<const double2 *>(Mx),
-        static_cast<double2 *>(Lx), nc_pad, mask);
+    EDFMM_CUDA_TRY(chain_launch(chain_tree(M, EDFMM_F64, s), k_m2l_rot_f64<P>, (unsigned)M, kRotThreads, smem, s, M, off, src, rows,
+                                static_cast<const double4 *>(tcen), static_cast<const double4 *>(thal),
+                                static_cast<const double4 *>(cen), static_cast<const double4 *>(hal),
+                                static_cast<const double2 *>(Mx), static_cast<double2 *>(Lx), nc_pad, mask));
     EDFMM_LAUNCH_CHECK("k_m2l_rot_f64");
     return EDFMM_OK;
 }
@@ -1114,10 +1120,10 @@ int launch_rot(int64_t M, const int32_t *off, const int32_t *src, const int32_t 
         cudaFuncSetAttribute(k_m2l_rot<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (attr != cudaSuccess)
         return fail(EDFMM_ERR_CUDA, std::string("k_m2l_rot shared memory attribute: ") + cudaGetErrorString(attr));
-    k_m2l_rot<P><<<nblk(M * 32, NT), NT, smem, s>>>(
-        M, off, src, rows, static_cast<const float4 *>(tcen), static_cast<const float4 *>(thal),
-        static_cast<const float4 *>(cen), static_cast<const float4 *>(hal), static_cast<const float4 *>(Mx),
-        static_cast<float2 *>(Lx), nc_pad, mask);
+    EDFMM_CUDA_TRY(chain_launch(chain_tree(M, EDFMM_F32, s), k_m2l_rot<P>, nblk(M * 32, NT), NT, smem, s, M, off, src, rows,
+                                static_cast<const float4 *>(tcen), static_cast<const float4 *>(thal),
+                                static_cast<const float4 *>(cen), static_cast<const float4 *>(hal),
+                                static_cast<const float4 *>(Mx), static_cast<float2 *>(Lx), nc_pad, mask));
     EDFMM_LAUNCH_CHECK("k_m2l_rot");
     return EDFMM_OK;
 }
