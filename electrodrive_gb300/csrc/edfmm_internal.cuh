@@ -293,6 +293,9 @@ __device__ __forceinline__ bool inst_active(const InstMask &m, int node) {
 // reads what the plan holds, calls chain_wait (all threads, before any return),
 // and only then reads or writes what other kernels of the chain do; chain_next
 // lets its own successor start.  Without the launch attribute both do nothing.
+// What the chain writes is read through pointers that are neither const
+// __restrict__ nor __ldg: those loads assume data that stay as they are for the
+// kernel's whole life, which here begins before its predecessor's end.
 #ifdef __CUDACC__
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -89,8 +89,7 @@ __global__ void k_split_nodes(const double4 *__restrict__ center, const double4 
 // sides.  FP32: a word is two coefficients; SPLIT: an FP64 coefficient becomes
 // (re hi, re lo, im hi, im lo).
 template <bool SPLIT>
-__global__ void __launch_bounds__(256) k_mult_columns(const float4 *__restrict__ in, int64_t n_nodes, int words,
-                                                      float4 *__restrict__ out) {
+__global__ void __launch_bounds__(256) k_mult_columns(const float4 *in, int64_t n_nodes, int words, float4 *out) {
     extern __shared__ float4 col_tile[];  // [32][words + 1]
     chain_next();
     chain_wait();

@@ -299,7 +299,7 @@ template <typename T, int P> __host__ __device__ constexpr bool rot_binomial() {
 
 // One pair (FP32): translated locals of the source with column Mcol added to acc.
 template <int P, typename V, typename A>
-__device__ __forceinline__ void rot_pair(V &v, A &acc, const float4 *__restrict__ Mcol, float c, float dx, float dy,
+__device__ __forceinline__ void rot_pair(V &v, A &acc, const float4 *Mcol, float c, float dx, float dy,
                                          float dz) {
     float4 x4{};
 #pragma unroll
@@ -307,7 +307,7 @@ __device__ __forceinline__ void rot_pair(V &v, A &acc, const float4 *__restrict_
 #pragma unroll
         for (int m = 0; m <= n; ++m) {
             const int q = tri(n, m);
-            if ((q & 1) == 0) x4 = __ldg(Mcol + (q >> 1) * kColNodes);  // two coefficients
+            if ((q & 1) == 0) x4 = Mcol[(q >> 1) * kColNodes];  // two coefficients
             const float2 x = (q & 1) == 0 ? make_float2(x4.x, x4.y) : make_float2(x4.z, x4.w);
             if (m == 0) {
                 v.set(n * n, x.x);
@@ -398,7 +398,7 @@ template <int P>
 __global__ void __launch_bounds__(kRotThreads, rot_binomial<float, P>() ? 4 : 3)
     k_m2l_rot(int64_t n_nodes, const int32_t *__restrict__ off, const int32_t *__restrict__ src,
               const int32_t *__restrict__ rows, const float4 *__restrict__ tcenter, const float4 *__restrict__ thalf,
-              const float4 *__restrict__ center, const float4 *__restrict__ half, const float4 *__restrict__ Mcols,
+              const float4 *__restrict__ center, const float4 *__restrict__ half, const float4 *Mcols,
               float2 *__restrict__ Lexp, int nc_pad, const InstMask mask) {
     using T = float;
     using T2 = float2;
@@ -799,14 +799,14 @@ template <int STRIDE> struct SmemSplit {
 // One pair: v <- the translated locals (real block basis) of the source with
 // column Mcol (split multipoles: (re hi, re lo, im hi, im lo) per coefficient).
 template <int P, bool PK, typename V>
-__device__ __forceinline__ void rot_pair_tf(V &v, const float4 *__restrict__ Mcol, tf32x2 c, tf32x2 dx, tf32x2 dy,
+__device__ __forceinline__ void rot_pair_tf(V &v, const float4 *Mcol, tf32x2 c, tf32x2 dx, tf32x2 dy,
                                             tf32x2 dz) {
     using T = tf32x2;
 #pragma unroll
     for (int n = 0; n <= P; ++n) {
 #pragma unroll
         for (int m = 0; m <= n; ++m) {
-            const float4 x = __ldg(Mcol + tri(n, m) * kColNodes);
+            const float4 x = Mcol[tri(n, m) * kColNodes];
             if (m == 0) {
                 v.set(n * n, T(x.x, x.y));
             } else {
@@ -850,7 +850,7 @@ __global__ void __launch_bounds__(NT, 256 / NT)
                  const int32_t *__restrict__ rows,
                  const float4 *__restrict__ tnodes, const double4 *__restrict__ thalf,
                  const float4 *__restrict__ snodes, const double4 *__restrict__ half,
-                 const float4 *__restrict__ Mcols, double2 *__restrict__ Lexp, int nc_pad, const InstMask mask) {
+                 const float4 *Mcols, double2 *__restrict__ Lexp, int nc_pad, const InstMask mask) {
     using T = tf32x2;
     constexpr int NV = (P + 1) * (P + 1), NR = (NV + 31) / 32;
     extern __shared__ __align__(16) unsigned char rot_smem[];
@@ -973,7 +973,7 @@ __global__ void __launch_bounds__(kRotThreads, 2)
     k_m2l_rot_f64(int64_t n_nodes, const int32_t *__restrict__ off, const int32_t *__restrict__ src,
                   const int32_t *__restrict__ rows, const double4 *__restrict__ tcenter,
                   const double4 *__restrict__ thalf, const double4 *__restrict__ center,
-                  const double4 *__restrict__ half, const double2 *__restrict__ Mexp, double2 *__restrict__ Lexp,
+                  const double4 *__restrict__ half, const double2 *Mexp, double2 *__restrict__ Lexp,
                   int nc_pad, const InstMask mask) {
     constexpr int NV = (P + 1) * (P + 1), NR = (NV + 31) / 32, NT = kRotThreads, NW = NT / 32;
     extern __shared__ __align__(16) unsigned char rot_smem[];
