@@ -357,29 +357,42 @@ int launch_linear(const __nv_bfloat16 *X, const __nv_bfloat16 *Wt, const float *
 // same as over device memory, without a load's latency in every few links
 // (30,000 rows: 36 -> 12 us).
 constexpr int kColStage = 128;
+constexpr size_t kColSmem = 2 * kColStage * W * sizeof(__nv_bfloat16);
 __global__ void __launch_bounds__(512) k_pcn_colsum_part(const __nv_bfloat16 *__restrict__ h, const float *__restrict__ w,
                                                          int64_t n, float *__restrict__ part) {
-    __shared__ __align__(16) __nv_bfloat16 t[kColStage * W];
-    __shared__ float tw[kColStage];
+    extern __shared__ __align__(16) __nv_bfloat16 stage[];  // two stages of kColStage rows
+    __shared__ float tw[2][kColStage];
     const int c = threadIdx.x;
     const int64_t r0 = (int64_t)blockIdx.x * kColRows, r1 = (n < r0 + kColRows) ? n : r0 + kColRows;
+    auto fetch = [&](int64_t rt, int buf) {  // the next stage's rows come while one is added
+        if (rt < r1) {
+            const int rows = (int)(r1 - rt < kColStage ? r1 - rt : kColStage);
+            for (int i = threadIdx.x; i < rows * (W / 8); i += 512)
+                cp16(stage + buf * kColStage * W + 8 * i, h + rt * W + 8 * i, true);
+            if (w)
+                for (int i = threadIdx.x; i < rows; i += 512) tw[buf][i] = w[rt + i];
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
     float s = 0.0f;
-    for (int64_t rt = r0; rt < r1; rt += kColStage) {
+    fetch(r0, 0);
+    int buf = 0;
+    for (int64_t rt = r0; rt < r1; rt += kColStage, buf ^= 1) {
         const int rows = (int)(r1 - rt < kColStage ? r1 - rt : kColStage);
-        __syncthreads();
-        for (int i = threadIdx.x; i < rows * (W / 8); i += 512) cp16(t + 8 * i, h + rt * W + 8 * i, true);
-        if (w)
-            for (int i = threadIdx.x; i < rows; i += 512) tw[i] = w[rt + i];
-        cp_wait();
+        fetch(rt + kColStage, buf ^ 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
         if (c < W) {
+            const __nv_bfloat16 *t = stage + buf * kColStage * W;
 #pragma unroll 16
             for (int r = 0; r < rows; ++r) {
                 const float v = __bfloat162float(t[r * W + c]);
-                s += w ? tw[r] * v : v;
+                s += w ? tw[buf][r] * v : v;
             }
         }
+        __syncthreads();
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     if (c < W) part[(int64_t)blockIdx.x * W + c] = s;
 }
 
@@ -392,12 +405,25 @@ __global__ void __launch_bounds__(W) k_pcn_reduce_cols(const float *__restrict__
     out[c] = s * scale;
 }
 
-__global__ void __launch_bounds__(W) k_pcn_context(const float *__restrict__ prm, const float *__restrict__ g,
-                                                   float *__restrict__ c2) {
+// the matrix is staged by all threads (a thread per row that read its own words
+// from memory took 10 us); one thread a row then adds in column order
+constexpr int kCtxLd = W + 1;
+constexpr size_t kCtxSmem = (W * kCtxLd + W) * sizeof(float);
+__global__ void __launch_bounds__(8 * W) k_pcn_context(const float *__restrict__ prm, const float *__restrict__ g,
+                                                       float *__restrict__ c2) {
+    extern __shared__ float ctx[];  // [W][W + 1], then g
+#pragma unroll
+    for (int i = 0; i < W / 8; ++i) {
+        const int q = threadIdx.x + 8 * W * i;
+        ctx[(q / W) * kCtxLd + q % W] = prm[O_V2 + q];
+    }
+    if (threadIdx.x < W) ctx[W * kCtxLd + threadIdx.x] = g[threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x >= W) return;
     const int r = threadIdx.x;
     float s = prm[O_B2 + r];
 #pragma unroll 32
-    for (int k = 0; k < W; ++k) s += prm[O_V2 + r * W + k] * g[k];
+    for (int k = 0; k < W; ++k) s += ctx[r * kCtxLd + k] * ctx[W * kCtxLd + k];
     c2[r] = s;
 }
 
@@ -533,25 +559,40 @@ __global__ void __launch_bounds__(W) k_pcn_context_grad(const float *__restrict_
     dg[k] = s / (float)(n > 0 ? n : 1);
 }
 
+int staged_smem() {  // dynamic shared memory above 48 KB
+    static const cudaError_t attr[2] = {
+        cudaFuncSetAttribute(k_pcn_context, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtxSmem),
+        cudaFuncSetAttribute(k_pcn_colsum_part, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColSmem)};
+    for (cudaError_t e : attr)
+        if (e != cudaSuccess)
+            return fail(EDFMM_ERR_CUDA, std::string("warm-start kernels' shared memory: ") + cudaGetErrorString(e));
+    return EDFMM_OK;
+}
+
 // ---------------------------------------------------------------------------
 // loss: L = sum A (s (1 + y) - sigma)^2 / sum A sigma^2, dL/dy.  One cluster of
 // eight blocks: dL/dy needs the whole denominator, and the blocks exchange
 // their sums through distributed shared memory (added in block order), so the
 // call needs no scratch.  30,000 panels: one block took 189 us, the cluster
-// 24.
+// 24, 18 with the products of a thread's first elements kept for dL/dy (about
+// 13 FP64 operations an element on eight SMs' pipes).
 // ---------------------------------------------------------------------------
-constexpr int kLossBlocks = 8;
+constexpr int kLossBlocks = 8, kLossKept = 4;
 __global__ void __cluster_dims__(kLossBlocks, 1, 1) __launch_bounds__(1024)
     k_pcn_loss(const float *__restrict__ y, const double *__restrict__ s, const double *__restrict__ sigma,
                const double *__restrict__ a, int64_t n, float *__restrict__ dy, double *__restrict__ loss) {
     __shared__ double red[2][32];
     __shared__ double sums[2], inv_s;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, rank = blockIdx.x;
-    double num = 0, den = 0;
-    for (int64_t i = rank * 1024 + tid; i < n; i += kLossBlocks * 1024) {
-        const double e = s[i] * (1.0 + (double)y[i]) - sigma[i];
-        num += a[i] * e * e;
-        den += a[i] * sigma[i] * sigma[i];
+    double num = 0, den = 0, kept[kLossKept];  // a e s of the thread's first elements
+    int k = 0;
+    for (int64_t i = rank * 1024 + tid; i < n; i += kLossBlocks * 1024, ++k) {
+        const double si = s[i], gi = sigma[i], e = si * (1.0 + (double)y[i]) - gi, ae = a[i] * e;
+        num += ae * e;
+        den += a[i] * gi * gi;
+#pragma unroll
+        for (int q = 0; q < kLossKept; ++q)
+            if (q == k) kept[q] = ae * si;
     }
     for (int o = 16; o > 0; o >>= 1) {
         num += __shfl_xor_sync(0xffffffffu, num, o);
@@ -590,7 +631,11 @@ __global__ void __cluster_dims__(kLossBlocks, 1, 1) __launch_bounds__(1024)
     }
     cluster_sync();  // the sums have been read (and the block sees inv_s)
     const double f = inv_s;
-    for (int64_t i = rank * 1024 + tid; i < n; i += kLossBlocks * 1024) {
+    int64_t i = rank * 1024 + tid;
+#pragma unroll
+    for (int q = 0; q < kLossKept; ++q, i += kLossBlocks * 1024)
+        if (i < n) dy[i] = (float)(kept[q] * f);
+    for (; i < n; i += kLossBlocks * 1024) {
         const double e = s[i] * (1.0 + (double)y[i]) - sigma[i];
         dy[i] = (float)(a[i] * e * s[i] * f);
     }
@@ -650,6 +695,7 @@ extern "C" EDFMM_API int edfmm_pcn_forward(const float *params_dev, const float 
     Ws w = carve(ws_dev, n);
     if (ws_bytes < w.bytes) return fail(EDFMM_ERR_ARG, "edfmm_pcn_forward: workspace too small");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (int rc = staged_smem()) return rc;
     const int64_t np = n_col_parts(n);
     k_pcn_cast<<<nblk(W * W, 256), 256, 0, s>>>(params_dev, w.w1b, w.w2b, w.w3b, w.w2t, w.w3t);
     EDFMM_LAUNCH_CHECK("k_pcn_cast");
@@ -657,11 +703,11 @@ extern "C" EDFMM_API int edfmm_pcn_forward(const float *params_dev, const float 
     EDFMM_LAUNCH_CHECK("k_pcn_cast_x");
     if (int rc = launch_linear<NIN, EPI_RELU, false>(w.x0, w.w1b, params_dev + O_B1, nullptr, n, w.h1, params_dev, nullptr, s))
         return rc;
-    k_pcn_colsum_part<<<(unsigned)np, 512, 0, s>>>(w.h1, nullptr, n, w.part);
+    k_pcn_colsum_part<<<(unsigned)np, 512, kColSmem, s>>>(w.h1, nullptr, n, w.part);
     EDFMM_LAUNCH_CHECK("k_pcn_colsum_part");
     k_pcn_reduce_cols<<<1, W, 0, s>>>(w.part, np, 1.0f / (float)n, w.g);
     EDFMM_LAUNCH_CHECK("k_pcn_reduce_cols");
-    k_pcn_context<<<1, W, 0, s>>>(params_dev, w.g, w.c2);
+    k_pcn_context<<<1, 8 * W, kCtxSmem, s>>>(params_dev, w.g, w.c2);
     EDFMM_LAUNCH_CHECK("k_pcn_context");
     if (int rc = launch_linear<W, EPI_RELU, false>(w.h1, w.w2b, w.c2, nullptr, n, w.h2, params_dev, nullptr, s)) return rc;
     return launch_linear<W, EPI_RELU, true>(w.h2, w.w3b, params_dev + O_B3, nullptr, n, w.h3, params_dev, y_dev, s);
@@ -674,10 +720,11 @@ extern "C" EDFMM_API int edfmm_pcn_backward(const float *params_dev, int64_t n, 
     Ws w = carve(ws_dev, n);
     if (ws_bytes < w.bytes) return fail(EDFMM_ERR_ARG, "edfmm_pcn_backward: workspace too small");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (int rc = staged_smem()) return rc;
     const int64_t np = n_parts(n), nc = n_col_parts(n);
     const int pr = part_rows(n);
     // head: dw4 = sum_r dy_r h3_r, db4 = sum dy
-    k_pcn_colsum_part<<<(unsigned)nc, 512, 0, s>>>(w.h3, dy_dev, n, w.part);
+    k_pcn_colsum_part<<<(unsigned)nc, 512, kColSmem, s>>>(w.h3, dy_dev, n, w.part);
     EDFMM_LAUNCH_CHECK("k_pcn_colsum_part");
     k_pcn_reduce_cols<<<1, W, 0, s>>>(w.part, nc, 1.0f, grads_dev + O_W4);
     EDFMM_LAUNCH_CHECK("k_pcn_reduce_cols");
