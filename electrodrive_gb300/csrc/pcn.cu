@@ -53,14 +53,13 @@ constexpr int kColRows = 1024;  // rows per partial column sum
 
 inline int64_t n_col_parts(int64_t n) { return std::max<int64_t>(1, (n + kColRows - 1) / kColRows); }
 
-// Rows per weight-gradient partial: about one partial per SM, at most 1,024
-// rows (a multiple of the 64-row stage).  30,000 panels in 30 partials of 1,024
-// rows left most SMs idle: 83 us per 128-wide layer, 10 in 157 of 192.
-inline int part_rows(int64_t n) {
-    const int64_t r = (n + 151) / 152;
-    return (int)std::min<int64_t>(1024, std::max<int64_t>(64, (r + 63) / 64 * 64));
-}
-inline int64_t n_parts(int64_t n) { return std::max<int64_t>(1, (n + part_rows(n) - 1) / part_rows(n)); }
+// Rows per weight-gradient partial.  It sets the order of the FP32 additions, and
+// training amplifies a change of it (Adam scales gradients near zero up to the
+// step size, and the weights are rounded to BF16), so the work is split over
+// output rows instead of shorter partials: a training step of 30,000 panels takes
+// 221 us (212 with partials of 256 rows, whose gradients had other last bits).
+constexpr int kPartRows = 1024;
+inline int64_t n_parts(int64_t n) { return std::max<int64_t>(1, (n + kPartRows - 1) / kPartRows); }
 
 Ws carve(void *base, int64_t n) {
     Ws w{};
@@ -453,64 +452,94 @@ __global__ void k_pcn_head_grad(const __nv_bfloat16 *__restrict__ h3, const floa
 // The product D^T X has the rows r as its reduction dimension: stages of 64
 // rows are copied to shared memory as they are (16 bytes at a time, padded
 // rows, rows past the end zero) and ldmatrix transposes the fragments of both
-// operands.  Warp w computes output rows 16w..16w+15 against all K columns
-// (mma.sync m16n8k16, BF16 in, FP32 accumulate; fixed order).  The bias sums
-// run on the FP32 pipe in row order.
-constexpr int kWgStage = 64;
+// operands.  A block computes 32 of the 128 output rows (blockIdx.y): a warp 16
+// of them against up to 32 columns (mma.sync m16n8k16, BF16 in, FP32
+// accumulate; fixed order), and one more warp the bias sums, in row order on
+// the FP32 pipe.  Bound by the latency of the copies (a partial is a chain of
+// 16 stages), so three stages are in flight; X is read four times, from L2.
+constexpr int kWgStage = 64, kWgDepth = 4, kWgSlice = 32, kWgLdd = kWgSlice + 8;
 template <int K>
-__global__ void __launch_bounds__(256) k_pcn_wgrad_part(const __nv_bfloat16 *__restrict__ D,
-                                                        const __nv_bfloat16 *__restrict__ X, int64_t n, int rows_part,
-                                                        float *__restrict__ part) {
-    constexpr int LDD = W + 8, LDX = K + 8;  // padded row strides (bf16 elements)
-    constexpr int NT = K / 8;                // n-tiles of 8 columns
-    __shared__ __align__(16) __nv_bfloat16 Dt[kWgStage * LDD];
-    __shared__ __align__(16) __nv_bfloat16 Xt[kWgStage * LDX];
+struct Wg {
+    static constexpr int groups = K > 32 ? K / 32 : 1, cols = K / groups, threads = (2 * groups + 1) * 32;
+    static constexpr int ldx = K + 8;  // padded row strides (bf16 elements): odd multiples of 16 bytes
+    static constexpr int stage = kWgStage * (kWgLdd + ldx);
+    static constexpr size_t smem = kWgDepth * stage * sizeof(__nv_bfloat16);
+};
+template <int K>
+__global__ void __launch_bounds__(Wg<K>::threads) k_pcn_wgrad_part(const __nv_bfloat16 *__restrict__ D,
+                                                                   const __nv_bfloat16 *__restrict__ X, int64_t n,
+                                                                   float *__restrict__ part) {
+    using G = Wg<K>;
+    constexpr int LDX = G::ldx, NT = G::cols / 8;  // NT: n-tiles of 8 columns per warp
+    extern __shared__ __align__(16) __nv_bfloat16 wg_smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3, lr = lane & 7, lm = lane >> 3;
-    const int o0 = 16 * warp;
+    const int slice = blockIdx.y * kWgSlice, o0 = 16 * (warp & 1), c0 = G::cols * (warp >> 1);
+    const bool bias = warp == 2 * G::groups;
     float acc[NT][4];
 #pragma unroll
     for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
     float bsum = 0.0f;
-    const int64_t r0 = (int64_t)blockIdx.x * rows_part, r1 = (n < r0 + rows_part) ? n : r0 + rows_part;
-    for (int64_t rt = r0; rt < r1; rt += kWgStage) {
-        const int rows = (int)((r1 - rt < kWgStage) ? r1 - rt : kWgStage);
-        __syncthreads();
-        for (int i = tid; i < kWgStage * (W / 8); i += 256) {
-            const int r = i / (W / 8), c = (i % (W / 8)) * 8;
-            cp16(Dt + r * LDD + c, D + (r < rows ? (rt + r) * W + c : 0), r < rows);
-        }
-        for (int i = tid; i < kWgStage * (K / 8); i += 256) {
-            const int r = i / (K / 8), c = (i % (K / 8)) * 8;
-            cp16(Xt + r * LDX + c, X + (r < rows ? (rt + r) * K + c : 0), r < rows);
-        }
-        cp_wait();
-        __syncthreads();
-#pragma unroll
-        for (int k0 = 0; k0 < kWgStage; k0 += 16) {
-            uint32_t a[4];  // (o 0-7, r 0-7), (o 8-15, r 0-7), (o 0-7, r 8-15), (o 8-15, r 8-15)
-            ldsm4t(a, Dt + (k0 + (lm >> 1) * 8 + lr) * LDD + o0 + (lm & 1) * 8);
-#pragma unroll
-            for (int j = 0; j < NT; j += 2) {
-                uint32_t b[4];  // column tiles j, j + 1, row halves 0, 1 of each
-                ldsm4t(b, Xt + (k0 + (lm & 1) * 8 + lr) * LDX + 8 * (j + (lm >> 1)));
-                mma_bf16(acc[j], a, b[0], b[1]);
-                mma_bf16(acc[j + 1], a, b[2], b[3]);
+    const int64_t r0 = (int64_t)blockIdx.x * kPartRows;
+    const int rows = (int)((n - r0 < kPartRows) ? n - r0 : kPartRows), stages = (rows + kWgStage - 1) / kWgStage;
+    auto fetch = [&](int q) {  // one group of copies per call, empty past the end
+        if (q < stages) {
+            __nv_bfloat16 *Dt = wg_smem + (q % kWgDepth) * G::stage, *Xt = Dt + kWgStage * kWgLdd;
+            const int left = rows - q * kWgStage;
+            const int64_t rq = r0 + q * kWgStage;
+            for (int i = tid; i < kWgStage * (kWgSlice / 8); i += G::threads) {
+                const int r = i / (kWgSlice / 8), c = (i % (kWgSlice / 8)) * 8;
+                cp16(Dt + r * kWgLdd + c, D + (r < left ? (rq + r) * W + slice + c : 0), r < left);
+            }
+            for (int i = tid; i < kWgStage * (K / 8); i += G::threads) {
+                const int r = i / (K / 8), c = (i % (K / 8)) * 8;
+                cp16(Xt + r * LDX + c, X + (r < left ? (rq + r) * K + c : 0), r < left);
             }
         }
-        if (tid < W) {
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int q = 0; q < kWgDepth - 1; ++q) fetch(q);
+    for (int q = 0; q < stages; ++q) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kWgDepth - 2) : "memory");
+        __syncthreads();  // stage q is there, and stage q - 1 has been read
+        fetch(q + kWgDepth - 1);
+        const __nv_bfloat16 *Dt = wg_smem + (q % kWgDepth) * G::stage, *Xt = Dt + kWgStage * kWgLdd;
+        if (bias) {
+            const int left = rows - q * kWgStage, m = left < kWgStage ? left : kWgStage;
 #pragma unroll 16
-            for (int r = 0; r < rows; ++r) bsum += __bfloat162float(Dt[r * LDD + tid]);
+            for (int r = 0; r < m; ++r) bsum += __bfloat162float(Dt[r * kWgLdd + lane]);
+        } else {
+#pragma unroll
+            for (int k0 = 0; k0 < kWgStage; k0 += 16) {
+                uint32_t a[4];  // (o 0-7, r 0-7), (o 8-15, r 0-7), (o 0-7, r 8-15), (o 8-15, r 8-15)
+                ldsm4t(a, Dt + (k0 + (lm >> 1) * 8 + lr) * kWgLdd + o0 + (lm & 1) * 8);
+#pragma unroll
+                for (int j = 0; j < NT; j += 2) {
+                    uint32_t b[4];  // column tiles j, j + 1, row halves 0, 1 of each
+                    ldsm4t(b, Xt + (k0 + (lm & 1) * 8 + lr) * LDX + c0 + 8 * (j + (lm >> 1)));
+                    mma_bf16(acc[j], a, b[0], b[1]);
+                    mma_bf16(acc[j + 1], a, b[2], b[3]);
+                }
+            }
         }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     float *pp = part + (int64_t)blockIdx.x * (W * K + W);
+    if (bias) {
+        pp[W * K + slice + lane] = bsum;
+        return;
+    }
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
-        const int col = 8 * j + 2 * t;
-        *reinterpret_cast<float2 *>(pp + (o0 + g) * K + col) = make_float2(acc[j][0], acc[j][1]);
-        *reinterpret_cast<float2 *>(pp + (o0 + g + 8) * K + col) = make_float2(acc[j][2], acc[j][3]);
+        const int col = c0 + 8 * j + 2 * t;
+        *reinterpret_cast<float2 *>(pp + (slice + o0 + g) * K + col) = make_float2(acc[j][0], acc[j][1]);
+        *reinterpret_cast<float2 *>(pp + (slice + o0 + g + 8) * K + col) = make_float2(acc[j][2], acc[j][3]);
     }
-    if (tid < W) pp[W * K + tid] = bsum;
+}
+template <int K>
+void launch_wgrad(const __nv_bfloat16 *D, const __nv_bfloat16 *X, int64_t n, float *part, cudaStream_t s) {
+    k_pcn_wgrad_part<K><<<dim3((unsigned)n_parts(n), W / kWgSlice), Wg<K>::threads, Wg<K>::smem, s>>>(D, X, n, part);
 }
 
 // grads[off + i] = sum_p part[p][i] (i < W*K), grads[boff + o] = sum_p part[p][W*K + o]
@@ -560,7 +589,8 @@ __global__ void __launch_bounds__(W) k_pcn_context_grad(const float *__restrict_
 }
 
 int staged_smem() {  // dynamic shared memory above 48 KB
-    static const cudaError_t attr[2] = {
+    static const cudaError_t attr[3] = {
+        cudaFuncSetAttribute(k_pcn_wgrad_part<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Wg<W>::smem),
         cudaFuncSetAttribute(k_pcn_context, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtxSmem),
         cudaFuncSetAttribute(k_pcn_colsum_part, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColSmem)};
     for (cudaError_t e : attr)
@@ -722,7 +752,6 @@ extern "C" EDFMM_API int edfmm_pcn_backward(const float *params_dev, int64_t n, 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (int rc = staged_smem()) return rc;
     const int64_t np = n_parts(n), nc = n_col_parts(n);
-    const int pr = part_rows(n);
     // head: dw4 = sum_r dy_r h3_r, db4 = sum dy
     k_pcn_colsum_part<<<(unsigned)nc, 512, kColSmem, s>>>(w.h3, dy_dev, n, w.part);
     EDFMM_LAUNCH_CHECK("k_pcn_colsum_part");
@@ -733,13 +762,13 @@ extern "C" EDFMM_API int edfmm_pcn_backward(const float *params_dev, int64_t n, 
     // layer 3: dz3 = (h3 > 0) dy w4;  dW3 = dz3^T h2;  dz2 = (h2 > 0) dz3 W3
     k_pcn_head_grad<<<nblk(n * (W / 8), 256), 256, 0, s>>>(w.h3, dy_dev, params_dev, n, w.dz);
     EDFMM_LAUNCH_CHECK("k_pcn_head_grad");
-    k_pcn_wgrad_part<W><<<(unsigned)np, 256, 0, s>>>(w.dz, w.h2, n, pr, w.part);
+    launch_wgrad<W>(w.dz, w.h2, n, w.part, s);
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_part");
     k_pcn_wgrad_reduce<<<nblk(W * W + W, 256), 256, 0, s>>>(w.part, np, W, grads_dev, O_W3, O_B3);
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_reduce");
     if (int rc = launch_linear<W, EPI_MASK, false>(w.dz, w.w3t, nullptr, w.h2, n, w.dz2, params_dev, nullptr, s)) return rc;
     // layer 2: dW2 = dz2^T h1, dc2 = colsum(dz2) -> dV2, db2, dg
-    k_pcn_wgrad_part<W><<<(unsigned)np, 256, 0, s>>>(w.dz2, w.h1, n, pr, w.part);
+    launch_wgrad<W>(w.dz2, w.h1, n, w.part, s);
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_part");
     k_pcn_wgrad_reduce<<<nblk(W * W + W, 256), 256, 0, s>>>(w.part, np, W, grads_dev, O_W2, O_B2);
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_reduce");
@@ -747,7 +776,7 @@ extern "C" EDFMM_API int edfmm_pcn_backward(const float *params_dev, int64_t n, 
     EDFMM_LAUNCH_CHECK("k_pcn_context_grad");
     // layer 1: dz1 = (h1 > 0) (dz2 W2 + dg / n);  dW1 = dz1^T x0
     if (int rc = launch_linear<W, EPI_MASK, false>(w.dz2, w.w2t, w.dg, w.h1, n, w.dz, params_dev, nullptr, s)) return rc;
-    k_pcn_wgrad_part<NIN><<<(unsigned)np, 256, 0, s>>>(w.dz, w.x0, n, pr, w.part);
+    launch_wgrad<NIN>(w.dz, w.x0, n, w.part, s);
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_part");
     k_pcn_wgrad_reduce<<<nblk(W * NIN + W, 256), 256, 0, s>>>(w.part, np, NIN, grads_dev, O_W1, O_B1);
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_reduce");
