@@ -56,8 +56,9 @@ inline int64_t n_col_parts(int64_t n) { return std::max<int64_t>(1, (n + kColRow
 // Rows per weight-gradient partial.  It sets the order of the FP32 additions, and
 // training amplifies a change of it (Adam scales gradients near zero up to the
 // step size, and the weights are rounded to BF16), so the work is split over
-// output rows instead of shorter partials: a training step of 30,000 panels takes
-// 221 us (212 with partials of 256 rows, whose gradients had other last bits).
+// output rows instead of shorter partials: a training step of 30,000 panels took
+// 221 us with it and 212 with partials of 256 rows, whose gradients had other
+// last bits.
 constexpr int kPartRows = 1024;
 inline int64_t n_parts(int64_t n) { return std::max<int64_t>(1, (n + kPartRows - 1) / kPartRows); }
 
@@ -173,25 +174,23 @@ __global__ void k_pcn_features(const double *__restrict__ c, const double *__res
 }
 
 // ---------------------------------------------------------------------------
-// weights: FP32 master -> BF16 (and transposed BF16 for the data gradients)
+// weights: FP32 master -> BF16 (and transposed BF16 for the data gradients),
+// and the features of all rows
 // ---------------------------------------------------------------------------
 __global__ void k_pcn_cast(const float *__restrict__ prm, __nv_bfloat16 *w1b, __nv_bfloat16 *w2b,
-                           __nv_bfloat16 *w3b, __nv_bfloat16 *w2t, __nv_bfloat16 *w3t) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+                           __nv_bfloat16 *w3b, __nv_bfloat16 *w2t, __nv_bfloat16 *w3t,
+                           const float *__restrict__ f, int64_t nf, __nv_bfloat16 *__restrict__ x0) {
+    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < nf) x0[j] = __float2bfloat16_rn(f[j]);
+    if (j >= W * W) return;
+    const int i = (int)j;
     if (i < W * NIN) w1b[i] = __float2bfloat16_rn(prm[O_W1 + i]);
-    if (i < W * W) {
-        const int r = i / W, c = i % W;
-        const __nv_bfloat16 x2 = __float2bfloat16_rn(prm[O_W2 + i]), x3 = __float2bfloat16_rn(prm[O_W3 + i]);
-        w2b[i] = x2;
-        w3b[i] = x3;
-        w2t[c * W + r] = x2;
-        w3t[c * W + r] = x3;
-    }
-}
-
-__global__ void k_pcn_cast_x(const float *__restrict__ f, int64_t n, __nv_bfloat16 *__restrict__ x0) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n * NIN) x0[i] = __float2bfloat16_rn(f[i]);
+    const int r = i / W, c = i % W;
+    const __nv_bfloat16 x2 = __float2bfloat16_rn(prm[O_W2 + i]), x3 = __float2bfloat16_rn(prm[O_W3 + i]);
+    w2b[i] = x2;
+    w3b[i] = x3;
+    w2t[c * W + r] = x2;
+    w3t[c * W + r] = x3;
 }
 
 // ---------------------------------------------------------------------------
@@ -396,19 +395,21 @@ __global__ void __launch_bounds__(512) k_pcn_colsum_part(const __nv_bfloat16 *__
 }
 
 // out[c] = scale * sum_p part[p][c]  (fixed order)
-__global__ void __launch_bounds__(W) k_pcn_reduce_cols(const float *__restrict__ part, int64_t np, float scale,
-                                                       float *__restrict__ out) {
-    const int c = threadIdx.x;
+__device__ __forceinline__ float reduce_cols(const float *__restrict__ part, int64_t np, int c) {
     float s = 0.0f;
+#pragma unroll 16
     for (int64_t p = 0; p < np; ++p) s += part[p * W + c];
-    out[c] = s * scale;
+    return s;
 }
 
-// the matrix is staged by all threads (a thread per row that read its own words
-// from memory took 10 us); one thread a row then adds in column order
+// g = scale * column sums of h1, and the context c2 = b2 + V2 g: one block,
+// since each is a chain of W adds that no second block shortens.  The matrix is staged by all threads (a thread per row that read its own words
+// from memory took 10 us) while the first W add the sums; one thread a row then
+// adds in column order
 constexpr int kCtxLd = W + 1;
 constexpr size_t kCtxSmem = (W * kCtxLd + W) * sizeof(float);
-__global__ void __launch_bounds__(8 * W) k_pcn_context(const float *__restrict__ prm, const float *__restrict__ g,
+__global__ void __launch_bounds__(8 * W) k_pcn_context(const float *__restrict__ prm, const float *__restrict__ part,
+                                                       int64_t np, float scale, float *__restrict__ g,
                                                        float *__restrict__ c2) {
     extern __shared__ float ctx[];  // [W][W + 1], then g
 #pragma unroll
@@ -416,7 +417,7 @@ __global__ void __launch_bounds__(8 * W) k_pcn_context(const float *__restrict__
         const int q = threadIdx.x + 8 * W * i;
         ctx[(q / W) * kCtxLd + q % W] = prm[O_V2 + q];
     }
-    if (threadIdx.x < W) ctx[W * kCtxLd + threadIdx.x] = g[threadIdx.x];
+    if (threadIdx.x < W) g[threadIdx.x] = ctx[W * kCtxLd + threadIdx.x] = reduce_cols(part, np, threadIdx.x) * scale;
     __syncthreads();
     if (threadIdx.x >= W) return;
     const int r = threadIdx.x;
@@ -429,10 +430,38 @@ __global__ void __launch_bounds__(8 * W) k_pcn_context(const float *__restrict__
 // ---------------------------------------------------------------------------
 // backward
 // ---------------------------------------------------------------------------
-// dz3[r][c] = (h3 > 0) ? dy[r] w4[c] : 0, eight columns (16 bytes) per thread
-__global__ void k_pcn_head_grad(const __nv_bfloat16 *__restrict__ h3, const float *__restrict__ dy,
-                                const float *__restrict__ prm, int64_t n, __nv_bfloat16 *__restrict__ dz) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Head of the network, three results of dy and h3 that need nothing of one
+// another.  Block 0: db4 = sum dy; block 1: dw4 = sums of the column parts; the
+// others: dz3[r][c] = (h3 > 0) ? dy[r] w4[c] : 0, eight columns (16 bytes) per
+// thread.  The two reductions are latency chains of one block each, and run
+// beside the rows instead of before them (with the casts in one launch and the
+// context's sums in its kernel, a training step of 30,000 panels went from 221
+// to 209 us).
+constexpr int kHeadSums = 2;
+__global__ void __launch_bounds__(256) k_pcn_head_grad(const __nv_bfloat16 *__restrict__ h3, const float *__restrict__ dy,
+                                                       const float *__restrict__ prm, int64_t n,
+                                                       const float *__restrict__ part, int64_t np,
+                                                       float *__restrict__ grads, __nv_bfloat16 *__restrict__ dz) {
+    if (blockIdx.x == 0) {
+        __shared__ float red[8];
+        float s = 0.0f;
+#pragma unroll 16
+        for (int64_t i = threadIdx.x; i < n; i += 256) s += dy[i];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float t = 0.0f;
+            for (int w = 0; w < 8; ++w) t += red[w];
+            grads[O_B4] = t;
+        }
+        return;
+    }
+    if (blockIdx.x == 1) {
+        if (threadIdx.x < W) grads[O_W4 + threadIdx.x] = reduce_cols(part, np, threadIdx.x);
+        return;
+    }
+    const int64_t i = (int64_t)(blockIdx.x - kHeadSums) * blockDim.x + threadIdx.x;
     if (i >= n * (W / 8)) return;
     const int c = (int)(i % (W / 8)) * 8;
     const float d = dy[i / (W / 8)];
@@ -555,21 +584,6 @@ __global__ void k_pcn_wgrad_reduce(const float *__restrict__ part, int64_t np, i
         grads[off + i] = s;
     else
         grads[boff + (i - W * K)] = s;
-}
-
-// head: dw4[c] = sum_r dy[r] h3[r][c] (from colsum partials), db4 = sum dy
-__global__ void __launch_bounds__(256) k_pcn_sum(const float *__restrict__ v, int64_t n, float *__restrict__ out) {
-    __shared__ float red[8];
-    float s = 0.0f;
-    for (int64_t i = threadIdx.x; i < n; i += 256) s += v[i];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.0f;
-        for (int w = 0; w < 8; ++w) t += red[w];
-        *out = t;
-    }
 }
 
 // context backward: dV2 = dc2 g^T, db2 = dc2, dg = V2^T dc2 / n  (dc2 = column
@@ -727,17 +741,15 @@ extern "C" EDFMM_API int edfmm_pcn_forward(const float *params_dev, const float 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (int rc = staged_smem()) return rc;
     const int64_t np = n_col_parts(n);
-    k_pcn_cast<<<nblk(W * W, 256), 256, 0, s>>>(params_dev, w.w1b, w.w2b, w.w3b, w.w2t, w.w3t);
+    const int64_t nf = n * NIN;
+    k_pcn_cast<<<nblk(nf > W * W ? nf : W * W, 256), 256, 0, s>>>(params_dev, w.w1b, w.w2b, w.w3b, w.w2t, w.w3t, features_dev,
+                                                                  nf, w.x0);
     EDFMM_LAUNCH_CHECK("k_pcn_cast");
-    k_pcn_cast_x<<<nblk(n * NIN, 256), 256, 0, s>>>(features_dev, n, w.x0);
-    EDFMM_LAUNCH_CHECK("k_pcn_cast_x");
     if (int rc = launch_linear<NIN, EPI_RELU, false>(w.x0, w.w1b, params_dev + O_B1, nullptr, n, w.h1, params_dev, nullptr, s))
         return rc;
     k_pcn_colsum_part<<<(unsigned)np, 512, kColSmem, s>>>(w.h1, nullptr, n, w.part);
     EDFMM_LAUNCH_CHECK("k_pcn_colsum_part");
-    k_pcn_reduce_cols<<<1, W, 0, s>>>(w.part, np, 1.0f / (float)n, w.g);
-    EDFMM_LAUNCH_CHECK("k_pcn_reduce_cols");
-    k_pcn_context<<<1, 8 * W, kCtxSmem, s>>>(params_dev, w.g, w.c2);
+    k_pcn_context<<<1, 8 * W, kCtxSmem, s>>>(params_dev, w.part, np, 1.0f / (float)n, w.g, w.c2);
     EDFMM_LAUNCH_CHECK("k_pcn_context");
     if (int rc = launch_linear<W, EPI_RELU, false>(w.h1, w.w2b, w.c2, nullptr, n, w.h2, params_dev, nullptr, s)) return rc;
     return launch_linear<W, EPI_RELU, true>(w.h2, w.w3b, params_dev + O_B3, nullptr, n, w.h3, params_dev, y_dev, s);
@@ -752,16 +764,12 @@ extern "C" EDFMM_API int edfmm_pcn_backward(const float *params_dev, int64_t n, 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (int rc = staged_smem()) return rc;
     const int64_t np = n_parts(n), nc = n_col_parts(n);
-    // head: dw4 = sum_r dy_r h3_r, db4 = sum dy
+    // head: dw4 = sum_r dy_r h3_r, db4 = sum dy, dz3 = (h3 > 0) dy w4
     k_pcn_colsum_part<<<(unsigned)nc, 512, kColSmem, s>>>(w.h3, dy_dev, n, w.part);
     EDFMM_LAUNCH_CHECK("k_pcn_colsum_part");
-    k_pcn_reduce_cols<<<1, W, 0, s>>>(w.part, nc, 1.0f, grads_dev + O_W4);
-    EDFMM_LAUNCH_CHECK("k_pcn_reduce_cols");
-    k_pcn_sum<<<1, 256, 0, s>>>(dy_dev, n, grads_dev + O_B4);
-    EDFMM_LAUNCH_CHECK("k_pcn_sum");
-    // layer 3: dz3 = (h3 > 0) dy w4;  dW3 = dz3^T h2;  dz2 = (h2 > 0) dz3 W3
-    k_pcn_head_grad<<<nblk(n * (W / 8), 256), 256, 0, s>>>(w.h3, dy_dev, params_dev, n, w.dz);
+    k_pcn_head_grad<<<kHeadSums + nblk(n * (W / 8), 256), 256, 0, s>>>(w.h3, dy_dev, params_dev, n, w.part, nc, grads_dev, w.dz);
     EDFMM_LAUNCH_CHECK("k_pcn_head_grad");
+    // layer 3: dW3 = dz3^T h2;  dz2 = (h2 > 0) dz3 W3
     launch_wgrad<W>(w.dz, w.h2, n, w.part, s);
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_part");
     k_pcn_wgrad_reduce<<<nblk(W * W + W, 256), 256, 0, s>>>(w.part, np, W, grads_dev, O_W3, O_B3);
