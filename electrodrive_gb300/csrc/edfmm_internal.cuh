@@ -288,7 +288,8 @@ __device__ __forceinline__ bool inst_active(const InstMask &m, int node) {
 }
 #endif
 
-// Chains of small kernels (the far field of a small tree): a kernel launched by
+// Chains of small kernels (the far field of a small tree, the warm-start
+// network): a kernel launched by
 // chain_launch may start while its predecessor in the stream still runs.  It
 // reads what the plan holds, calls chain_wait (all threads, before any return),
 // and only then reads or writes what other kernels of the chain do; chain_next
@@ -315,7 +316,8 @@ cudaError_t chain_launch(bool chained, void (*kernel)(K...), unsigned grid, unsi
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
 }
 #endif
-// small trees, outside a capture (a graph has its own order)
+// outside a capture (a graph has its own order); small trees there
+bool chain_stream(cudaStream_t s);
 bool chain_tree(int64_t n_nodes, int dtype, cudaStream_t s);
 
 int tree_build(const void *points_dev, int64_t n, int dtype, int leaf_size, int max_depth,

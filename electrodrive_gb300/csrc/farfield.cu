@@ -1398,7 +1398,9 @@ int set_charges(const DevTree &tree, const void *a, const void *b, cudaStream_t 
 }
 
 bool chain_tree(int64_t n_nodes, int dtype, cudaStream_t s) {
-    if (n_nodes > (dtype == EDFMM_F64 ? kChainNodes64 : kChainNodes32)) return false;
+    return n_nodes <= (dtype == EDFMM_F64 ? kChainNodes64 : kChainNodes32) && chain_stream(s);
+}
+bool chain_stream(cudaStream_t s) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
 }

@@ -173,13 +173,21 @@ __global__ void k_pcn_features(const double *__restrict__ c, const double *__res
     for (int q = 8; q < NIN; ++q) o[q] = 0.0f;
 }
 
+// From here on all kernels but the loss are a chain of overlapped launches: they
+// wait before their first access, and read through plain pointers (a step's
+// parameters are written by the kernel before).  What it saves is the start of
+// some 17 short kernels: a training step of 140 / 4,026 / 30,000 / 123,000 panels
+// went from 117 / 170 / 208 / 424 to 92 / 148 / 194 / 409 us.
+
 // ---------------------------------------------------------------------------
 // weights: FP32 master -> BF16 (and transposed BF16 for the data gradients),
 // and the features of all rows
 // ---------------------------------------------------------------------------
-__global__ void k_pcn_cast(const float *__restrict__ prm, __nv_bfloat16 *w1b, __nv_bfloat16 *w2b,
+__global__ void k_pcn_cast(const float *prm, __nv_bfloat16 *w1b, __nv_bfloat16 *w2b,
                            __nv_bfloat16 *w3b, __nv_bfloat16 *w2t, __nv_bfloat16 *w3t,
-                           const float *__restrict__ f, int64_t nf, __nv_bfloat16 *__restrict__ x0) {
+                           const float *f, int64_t nf, __nv_bfloat16 *x0) {
+    chain_next();
+    chain_wait();
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j < nf) x0[j] = __float2bfloat16_rn(f[j]);
     if (j >= W * W) return;
@@ -243,10 +251,12 @@ template <int K> constexpr size_t lin_smem_out() {  // the output rows take over
 }
 
 template <int K, int EPI, bool HEAD>
-__global__ void __launch_bounds__(256) k_pcn_linear(const __nv_bfloat16 *__restrict__ X, const __nv_bfloat16 *__restrict__ Wt,
-                                                    const float *__restrict__ bias, const __nv_bfloat16 *__restrict__ mask,
-                                                    int64_t n, __nv_bfloat16 *__restrict__ out,
-                                                    const float *__restrict__ prm, float *__restrict__ y) {
+__global__ void __launch_bounds__(256) k_pcn_linear(const __nv_bfloat16 *X, const __nv_bfloat16 *Wt,
+                                                    const float *bias, const __nv_bfloat16 *mask,
+                                                    int64_t n, __nv_bfloat16 *out,
+                                                    const float *prm, float *y) {
+    chain_next();
+    chain_wait();
     constexpr int LD = K + 8, LO = W + 8;  // padded row strides (bf16 elements)
     extern __shared__ __align__(16) __nv_bfloat16 lin_sm[];
     __nv_bfloat16 *sw = lin_sm, *sx = lin_sm + W * LD;
@@ -334,14 +344,15 @@ __global__ void __launch_bounds__(256) k_pcn_linear(const __nv_bfloat16 *__restr
 }
 
 template <int K, int EPI, bool HEAD>
-int launch_linear(const __nv_bfloat16 *X, const __nv_bfloat16 *Wt, const float *bias, const __nv_bfloat16 *mask,
+int launch_linear(bool chained, const __nv_bfloat16 *X, const __nv_bfloat16 *Wt, const float *bias, const __nv_bfloat16 *mask,
                   int64_t n, __nv_bfloat16 *out, const float *prm, float *y, cudaStream_t s) {
     constexpr size_t smem = lin_smem_out<K>();
     static const cudaError_t attr =
         cudaFuncSetAttribute(k_pcn_linear<K, EPI, HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (attr != cudaSuccess)
         return fail(EDFMM_ERR_CUDA, std::string("k_pcn_linear shared memory: ") + cudaGetErrorString(attr));
-    k_pcn_linear<K, EPI, HEAD><<<nblk(n, kLinRows), 256, smem, s>>>(X, Wt, bias, mask, n, out, prm, y);
+    EDFMM_CUDA_TRY(chain_launch(chained, k_pcn_linear<K, EPI, HEAD>, nblk(n, kLinRows), 256, smem, s, X, Wt, bias, mask, n,
+                                out, prm, y));
     EDFMM_LAUNCH_CHECK("k_pcn_linear");
     return EDFMM_OK;
 }
@@ -356,8 +367,10 @@ int launch_linear(const __nv_bfloat16 *X, const __nv_bfloat16 *Wt, const float *
 // (30,000 rows: 36 -> 12 us).
 constexpr int kColStage = 128;
 constexpr size_t kColSmem = 2 * kColStage * W * sizeof(__nv_bfloat16);
-__global__ void __launch_bounds__(512) k_pcn_colsum_part(const __nv_bfloat16 *__restrict__ h, const float *__restrict__ w,
-                                                         int64_t n, float *__restrict__ part) {
+__global__ void __launch_bounds__(512) k_pcn_colsum_part(const __nv_bfloat16 *h, const float *w,
+                                                         int64_t n, float *part) {
+    chain_next();
+    chain_wait();
     extern __shared__ __align__(16) __nv_bfloat16 stage[];  // two stages of kColStage rows
     __shared__ float tw[2][kColStage];
     const int c = threadIdx.x;
@@ -395,7 +408,7 @@ __global__ void __launch_bounds__(512) k_pcn_colsum_part(const __nv_bfloat16 *__
 }
 
 // out[c] = scale * sum_p part[p][c]  (fixed order)
-__device__ __forceinline__ float reduce_cols(const float *__restrict__ part, int64_t np, int c) {
+__device__ __forceinline__ float reduce_cols(const float *part, int64_t np, int c) {
     float s = 0.0f;
 #pragma unroll 16
     for (int64_t p = 0; p < np; ++p) s += part[p * W + c];
@@ -408,9 +421,11 @@ __device__ __forceinline__ float reduce_cols(const float *__restrict__ part, int
 // adds in column order
 constexpr int kCtxLd = W + 1;
 constexpr size_t kCtxSmem = (W * kCtxLd + W) * sizeof(float);
-__global__ void __launch_bounds__(8 * W) k_pcn_context(const float *__restrict__ prm, const float *__restrict__ part,
-                                                       int64_t np, float scale, float *__restrict__ g,
-                                                       float *__restrict__ c2) {
+__global__ void __launch_bounds__(8 * W) k_pcn_context(const float *prm, const float *part,
+                                                       int64_t np, float scale, float *g,
+                                                       float *c2) {
+    chain_next();
+    chain_wait();
     extern __shared__ float ctx[];  // [W][W + 1], then g
 #pragma unroll
     for (int i = 0; i < W / 8; ++i) {
@@ -438,10 +453,12 @@ __global__ void __launch_bounds__(8 * W) k_pcn_context(const float *__restrict__
 // context's sums in its kernel, a training step of 30,000 panels went from 221
 // to 209 us).
 constexpr int kHeadSums = 2;
-__global__ void __launch_bounds__(256) k_pcn_head_grad(const __nv_bfloat16 *__restrict__ h3, const float *__restrict__ dy,
-                                                       const float *__restrict__ prm, int64_t n,
-                                                       const float *__restrict__ part, int64_t np,
-                                                       float *__restrict__ grads, __nv_bfloat16 *__restrict__ dz) {
+__global__ void __launch_bounds__(256) k_pcn_head_grad(const __nv_bfloat16 *h3, const float *dy,
+                                                       const float *prm, int64_t n,
+                                                       const float *part, int64_t np,
+                                                       float *grads, __nv_bfloat16 *dz) {
+    chain_next();
+    chain_wait();
     if (blockIdx.x == 0) {
         __shared__ float red[8];
         float s = 0.0f;
@@ -481,12 +498,12 @@ __global__ void __launch_bounds__(256) k_pcn_head_grad(const __nv_bfloat16 *__re
 // The product D^T X has the rows r as its reduction dimension: stages of 64
 // rows are copied to shared memory as they are (16 bytes at a time, padded
 // rows, rows past the end zero) and ldmatrix transposes the fragments of both
-// operands.  A block computes 32 of the 128 output rows (blockIdx.y): a warp 16
+// operands.  A block computes 32 of the 128 output rows (blockIdx.x % 4): a warp 16
 // of them against up to 32 columns (mma.sync m16n8k16, BF16 in, FP32
 // accumulate; fixed order), and one more warp the bias sums, in row order on
 // the FP32 pipe.  Bound by the latency of the copies (a partial is a chain of
 // 16 stages), so three stages are in flight; X is read four times, from L2.
-constexpr int kWgStage = 64, kWgDepth = 4, kWgSlice = 32, kWgLdd = kWgSlice + 8;
+constexpr int kWgStage = 64, kWgDepth = 4, kWgSlice = 32, kWgSlices = W / kWgSlice, kWgLdd = kWgSlice + 8;
 template <int K>
 struct Wg {
     static constexpr int groups = K > 32 ? K / 32 : 1, cols = K / groups, threads = (2 * groups + 1) * 32;
@@ -495,21 +512,23 @@ struct Wg {
     static constexpr size_t smem = kWgDepth * stage * sizeof(__nv_bfloat16);
 };
 template <int K>
-__global__ void __launch_bounds__(Wg<K>::threads) k_pcn_wgrad_part(const __nv_bfloat16 *__restrict__ D,
-                                                                   const __nv_bfloat16 *__restrict__ X, int64_t n,
-                                                                   float *__restrict__ part) {
+__global__ void __launch_bounds__(Wg<K>::threads) k_pcn_wgrad_part(const __nv_bfloat16 *D,
+                                                                   const __nv_bfloat16 *X, int64_t n,
+                                                                   float *part) {
+    chain_next();
+    chain_wait();
     using G = Wg<K>;
     constexpr int LDX = G::ldx, NT = G::cols / 8;  // NT: n-tiles of 8 columns per warp
     extern __shared__ __align__(16) __nv_bfloat16 wg_smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3, lr = lane & 7, lm = lane >> 3;
-    const int slice = blockIdx.y * kWgSlice, o0 = 16 * (warp & 1), c0 = G::cols * (warp >> 1);
+    const int slice = (int)(blockIdx.x % kWgSlices) * kWgSlice, o0 = 16 * (warp & 1), c0 = G::cols * (warp >> 1);
     const bool bias = warp == 2 * G::groups;
     float acc[NT][4];
 #pragma unroll
     for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
     float bsum = 0.0f;
-    const int64_t r0 = (int64_t)blockIdx.x * kPartRows;
+    const int64_t p = blockIdx.x / kWgSlices, r0 = p * kPartRows;
     const int rows = (int)((n - r0 < kPartRows) ? n - r0 : kPartRows), stages = (rows + kWgStage - 1) / kWgStage;
     auto fetch = [&](int q) {  // one group of copies per call, empty past the end
         if (q < stages) {
@@ -554,7 +573,7 @@ __global__ void __launch_bounds__(Wg<K>::threads) k_pcn_wgrad_part(const __nv_bf
         }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-    float *pp = part + (int64_t)blockIdx.x * (W * K + W);
+    float *pp = part + p * (W * K + W);
     if (bias) {
         pp[W * K + slice + lane] = bsum;
         return;
@@ -567,13 +586,16 @@ __global__ void __launch_bounds__(Wg<K>::threads) k_pcn_wgrad_part(const __nv_bf
     }
 }
 template <int K>
-void launch_wgrad(const __nv_bfloat16 *D, const __nv_bfloat16 *X, int64_t n, float *part, cudaStream_t s) {
-    k_pcn_wgrad_part<K><<<dim3((unsigned)n_parts(n), W / kWgSlice), Wg<K>::threads, Wg<K>::smem, s>>>(D, X, n, part);
+cudaError_t launch_wgrad(bool chained, const __nv_bfloat16 *D, const __nv_bfloat16 *X, int64_t n, float *part, cudaStream_t s) {
+    return chain_launch(chained, k_pcn_wgrad_part<K>, (unsigned)(n_parts(n) * kWgSlices), Wg<K>::threads, Wg<K>::smem, s, D, X,
+                        n, part);
 }
 
 // grads[off + i] = sum_p part[p][i] (i < W*K), grads[boff + o] = sum_p part[p][W*K + o]
-__global__ void k_pcn_wgrad_reduce(const float *__restrict__ part, int64_t np, int K, float *__restrict__ grads,
+__global__ void k_pcn_wgrad_reduce(const float *part, int64_t np, int K, float *grads,
                                    int64_t off, int64_t boff) {
+    chain_next();
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int stride = W * K + W;
     if (i >= stride) return;
@@ -588,9 +610,11 @@ __global__ void k_pcn_wgrad_reduce(const float *__restrict__ part, int64_t np, i
 
 // context backward: dV2 = dc2 g^T, db2 = dc2, dg = V2^T dc2 / n  (dc2 = column
 // sum of dz2); block r < 128 writes row r of dV2, block 128 dg
-__global__ void __launch_bounds__(W) k_pcn_context_grad(const float *__restrict__ prm, const float *__restrict__ g,
-                                                        const float *__restrict__ dc, int64_t n, float *__restrict__ grads,
-                                                        float *__restrict__ dg) {
+__global__ void __launch_bounds__(W) k_pcn_context_grad(const float *prm, const float *g,
+                                                        const float *dc, int64_t n, float *grads,
+                                                        float *dg) {
+    chain_next();
+    chain_wait();
     const int k = threadIdx.x, r = blockIdx.x;
     if (r < W) {
         grads[O_V2 + r * W + k] = dc[r] * g[k];
@@ -685,9 +709,11 @@ __global__ void __cluster_dims__(kLossBlocks, 1, 1) __launch_bounds__(1024)
     }
 }
 
-__global__ void k_pcn_adam(float *__restrict__ p, const float *__restrict__ gr, float *__restrict__ m,
-                           float *__restrict__ v, int64_t count, float lr, float b1, float b2, float eps, float c1,
+__global__ void k_pcn_adam(float *p, const float *gr, float *m,
+                           float *v, int64_t count, float lr, float b1, float b2, float eps, float c1,
                            float c2) {
+    chain_next();
+    chain_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const float gi = gr[i];
@@ -740,19 +766,21 @@ extern "C" EDFMM_API int edfmm_pcn_forward(const float *params_dev, const float 
     if (ws_bytes < w.bytes) return fail(EDFMM_ERR_ARG, "edfmm_pcn_forward: workspace too small");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (int rc = staged_smem()) return rc;
+    const bool chained = chain_stream(s);
     const int64_t np = n_col_parts(n);
     const int64_t nf = n * NIN;
-    k_pcn_cast<<<nblk(nf > W * W ? nf : W * W, 256), 256, 0, s>>>(params_dev, w.w1b, w.w2b, w.w3b, w.w2t, w.w3t, features_dev,
-                                                                  nf, w.x0);
+    EDFMM_CUDA_TRY(chain_launch(chained, k_pcn_cast, nblk(nf > W * W ? nf : W * W, 256), 256, 0, s, params_dev, w.w1b,
+                                w.w2b, w.w3b, w.w2t, w.w3t, features_dev, nf, w.x0));
     EDFMM_LAUNCH_CHECK("k_pcn_cast");
-    if (int rc = launch_linear<NIN, EPI_RELU, false>(w.x0, w.w1b, params_dev + O_B1, nullptr, n, w.h1, params_dev, nullptr, s))
+    if (int rc = launch_linear<NIN, EPI_RELU, false>(chained, w.x0, w.w1b, params_dev + O_B1, nullptr, n, w.h1, params_dev, nullptr, s))
         return rc;
-    k_pcn_colsum_part<<<(unsigned)np, 512, kColSmem, s>>>(w.h1, nullptr, n, w.part);
+    EDFMM_CUDA_TRY(chain_launch(chained, k_pcn_colsum_part, (unsigned)np, 512, kColSmem, s, w.h1, nullptr, n, w.part));
     EDFMM_LAUNCH_CHECK("k_pcn_colsum_part");
-    k_pcn_context<<<1, 8 * W, kCtxSmem, s>>>(params_dev, w.part, np, 1.0f / (float)n, w.g, w.c2);
+    EDFMM_CUDA_TRY(chain_launch(chained, k_pcn_context, 1, 8 * W, kCtxSmem, s, params_dev, w.part, np, 1.0f / (float)n,
+                                w.g, w.c2));
     EDFMM_LAUNCH_CHECK("k_pcn_context");
-    if (int rc = launch_linear<W, EPI_RELU, false>(w.h1, w.w2b, w.c2, nullptr, n, w.h2, params_dev, nullptr, s)) return rc;
-    return launch_linear<W, EPI_RELU, true>(w.h2, w.w3b, params_dev + O_B3, nullptr, n, w.h3, params_dev, y_dev, s);
+    if (int rc = launch_linear<W, EPI_RELU, false>(chained, w.h1, w.w2b, w.c2, nullptr, n, w.h2, params_dev, nullptr, s)) return rc;
+    return launch_linear<W, EPI_RELU, true>(chained, w.h2, w.w3b, params_dev + O_B3, nullptr, n, w.h3, params_dev, y_dev, s);
 }
 
 extern "C" EDFMM_API int edfmm_pcn_backward(const float *params_dev, int64_t n, const float *dy_dev, float *grads_dev,
@@ -763,30 +791,36 @@ extern "C" EDFMM_API int edfmm_pcn_backward(const float *params_dev, int64_t n, 
     if (ws_bytes < w.bytes) return fail(EDFMM_ERR_ARG, "edfmm_pcn_backward: workspace too small");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (int rc = staged_smem()) return rc;
+    const bool chained = chain_stream(s);
     const int64_t np = n_parts(n), nc = n_col_parts(n);
     // head: dw4 = sum_r dy_r h3_r, db4 = sum dy, dz3 = (h3 > 0) dy w4
-    k_pcn_colsum_part<<<(unsigned)nc, 512, kColSmem, s>>>(w.h3, dy_dev, n, w.part);
+    EDFMM_CUDA_TRY(chain_launch(chained, k_pcn_colsum_part, (unsigned)nc, 512, kColSmem, s, w.h3, dy_dev, n, w.part));
     EDFMM_LAUNCH_CHECK("k_pcn_colsum_part");
-    k_pcn_head_grad<<<kHeadSums + nblk(n * (W / 8), 256), 256, 0, s>>>(w.h3, dy_dev, params_dev, n, w.part, nc, grads_dev, w.dz);
+    EDFMM_CUDA_TRY(chain_launch(chained, k_pcn_head_grad, kHeadSums + nblk(n * (W / 8), 256), 256, 0, s, w.h3, dy_dev,
+                                params_dev, n, w.part, nc, grads_dev, w.dz));
     EDFMM_LAUNCH_CHECK("k_pcn_head_grad");
     // layer 3: dW3 = dz3^T h2;  dz2 = (h2 > 0) dz3 W3
-    launch_wgrad<W>(w.dz, w.h2, n, w.part, s);
+    EDFMM_CUDA_TRY(launch_wgrad<W>(chained, w.dz, w.h2, n, w.part, s));
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_part");
-    k_pcn_wgrad_reduce<<<nblk(W * W + W, 256), 256, 0, s>>>(w.part, np, W, grads_dev, O_W3, O_B3);
+    EDFMM_CUDA_TRY(chain_launch(chained, k_pcn_wgrad_reduce, nblk(W * W + W, 256), 256, 0, s, w.part, np, W, grads_dev,
+                                O_W3, O_B3));
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_reduce");
-    if (int rc = launch_linear<W, EPI_MASK, false>(w.dz, w.w3t, nullptr, w.h2, n, w.dz2, params_dev, nullptr, s)) return rc;
+    if (int rc = launch_linear<W, EPI_MASK, false>(chained, w.dz, w.w3t, nullptr, w.h2, n, w.dz2, params_dev, nullptr, s)) return rc;
     // layer 2: dW2 = dz2^T h1, dc2 = colsum(dz2) -> dV2, db2, dg
-    launch_wgrad<W>(w.dz2, w.h1, n, w.part, s);
+    EDFMM_CUDA_TRY(launch_wgrad<W>(chained, w.dz2, w.h1, n, w.part, s));
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_part");
-    k_pcn_wgrad_reduce<<<nblk(W * W + W, 256), 256, 0, s>>>(w.part, np, W, grads_dev, O_W2, O_B2);
+    EDFMM_CUDA_TRY(chain_launch(chained, k_pcn_wgrad_reduce, nblk(W * W + W, 256), 256, 0, s, w.part, np, W, grads_dev,
+                                O_W2, O_B2));
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_reduce");
-    k_pcn_context_grad<<<W + 1, W, 0, s>>>(params_dev, w.g, grads_dev + O_B2, n, grads_dev, w.dg);
+    EDFMM_CUDA_TRY(chain_launch(chained, k_pcn_context_grad, W + 1, W, 0, s, params_dev, w.g, grads_dev + O_B2, n,
+                                grads_dev, w.dg));
     EDFMM_LAUNCH_CHECK("k_pcn_context_grad");
     // layer 1: dz1 = (h1 > 0) (dz2 W2 + dg / n);  dW1 = dz1^T x0
-    if (int rc = launch_linear<W, EPI_MASK, false>(w.dz2, w.w2t, w.dg, w.h1, n, w.dz, params_dev, nullptr, s)) return rc;
-    launch_wgrad<NIN>(w.dz, w.x0, n, w.part, s);
+    if (int rc = launch_linear<W, EPI_MASK, false>(chained, w.dz2, w.w2t, w.dg, w.h1, n, w.dz, params_dev, nullptr, s)) return rc;
+    EDFMM_CUDA_TRY(launch_wgrad<NIN>(chained, w.dz, w.x0, n, w.part, s));
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_part");
-    k_pcn_wgrad_reduce<<<nblk(W * NIN + W, 256), 256, 0, s>>>(w.part, np, NIN, grads_dev, O_W1, O_B1);
+    EDFMM_CUDA_TRY(chain_launch(chained, k_pcn_wgrad_reduce, nblk(W * NIN + W, 256), 256, 0, s, w.part, np, NIN, grads_dev,
+                                O_W1, O_B1));
     EDFMM_LAUNCH_CHECK("k_pcn_wgrad_reduce");
     return EDFMM_OK;
 }
@@ -808,8 +842,9 @@ extern "C" EDFMM_API int edfmm_pcn_adam(float *params_dev, const float *grads_de
     if (count <= 0 || step <= 0 || !params_dev || !grads_dev || !m_dev || !v_dev)
         return fail(EDFMM_ERR_ARG, "edfmm_pcn_adam: bad arguments");
     const float c1 = 1.0f - powf(beta1, (float)step), c2 = 1.0f - powf(beta2, (float)step);
-    k_pcn_adam<<<nblk(count, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(params_dev, grads_dev, m_dev, v_dev,
-                                                                                 count, lr, beta1, beta2, eps, c1, c2);
+    const bool chained = chain_stream(static_cast<cudaStream_t>(stream));
+    EDFMM_CUDA_TRY(chain_launch(chained, k_pcn_adam, nblk(count, 256), 256, 0, static_cast<cudaStream_t>(stream),
+                                params_dev, grads_dev, m_dev, v_dev, count, lr, beta1, beta2, eps, c1, c2));
     EDFMM_LAUNCH_CHECK("k_pcn_adam");
     return EDFMM_OK;
 }
