@@ -193,13 +193,16 @@ __global__ void __launch_bounds__(kThreads) k_dense_f32(const DenseArgs<float> A
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int q = threadIdx.x + h * kThreads;
-            float x = 0, y = 0, z = 0, w = 0;  // an odd tile ends with a source of no charge
-            if (q < cnt) {
-                const int64_t j = jb + q;
+            float x = 0, y = 0, z = 0, w = 0;
+            if (q < ((cnt + 1) & ~1)) {
+                // an odd tile ends with its last source again, without charge: a
+                // point of its own could meet a target, whose weight k_e / r^3
+                // then overflows and is NaN times no charge
+                const int64_t j = jb + min(q, cnt - 1);
                 x = A.c[3 * j];
                 y = A.c[3 * j + 1];
                 z = A.c[3 * j + 2];
-                w = A.sigma[j] * A.areas[j];
+                if (q < cnt) w = A.sigma[j] * A.areas[j];
             }
             float *o = sf + (q >> 1) * 8 + (q & 1);
             o[0] = x;

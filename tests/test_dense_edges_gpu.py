@@ -1,0 +1,32 @@
+"""The dense kernels where a tile is padded and where a charge is not finite.
+
+FP32 tolerance: a term rounds about 16 times and a target adds n of them, so
+(n + 32) 2^-23 of the sum of the terms' sizes."""
+import numpy as np
+import pytest
+import torch
+
+from electrodrive_gb300.utils.config import K_E
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m", [1, 65])
+@pytest.mark.parametrize("n", [1, 2, 129, 256, 257, 1025])
+def test_fp32_field_at_the_origin(cuda_lib, m, n):
+    """Targets at and next to the coordinate origin, odd and even numbers of panels, with
+    the physical constant (K_E / r^3 overflows FP32 below r = 3e-10)."""
+    from electrodrive_gb300.core.bem_near import field_at_targets, potential_field_at_targets
+
+    rng = np.random.default_rng(n)
+    T = lambda x: torch.as_tensor(x, dtype=torch.float32, device="cuda")
+    p = rng.normal(size=(n, 3)) + 0.3
+    c = T(p / np.linalg.norm(p, axis=1, keepdims=True))
+    s, a = T(1e-11 * rng.uniform(0.5, 1.5, n)), T(rng.uniform(0.5, 1.5, n))
+    t = torch.zeros(m, 3, device="cuda")
+    t[1:] = T(10.0 ** rng.uniform(-14, -6, (m - 1, 1)) * rng.normal(size=(m - 1, 3)))
+    d = t.double()[:, None] - c.double()[None]
+    term = (K_E * (s.double() * a.double()) / d.norm(dim=2) ** 3)[..., None] * d
+    tol = (n + 32) * 2.0 ** -23 * term.norm(dim=2).sum(1, keepdim=True)
+    for e in (field_at_targets(t, c, s, a), potential_field_at_targets(t, c, s, a)[1]):
+        assert bool(((e.double() - term.sum(1)).abs() <= tol).all())
