@@ -150,11 +150,7 @@ __device__ __forceinline__ void dense_tile_f32(const float4 *src, int npairs, in
             const float2 dx = __fadd2_rn(make_float2(u.x, u.y), nx[t]), dy = __fadd2_rn(make_float2(u.z, u.w), ny[t]),
                          dz = __fadd2_rn(make_float2(v.x, v.y), nz[t]);
             const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-            float2 ir = make_float2(inv_r(r2.x), inv_r(r2.y));
-            if (SELF) {  // self0 + 32 t: the target's position in this tile
-                if (2 * k == self0 + 32 * t) ir.x = 0.0f;
-                if (2 * k + 1 == self0 + 32 * t) ir.y = 0.0f;
-            }
+            const float2 ir = make_float2(inv_r(r2.x), inv_r(r2.y));
             if (has_field<KIND>()) {
                 const float2 ke2 = make_float2(k_e, k_e);
                 const float2 w = __fmul2_rn(__fmul2_rn(ke2, __fmul2_rn(__fmul2_rn(ir, ir), ir)), qw);
@@ -162,7 +158,14 @@ __device__ __forceinline__ void dense_tile_f32(const float4 *src, int npairs, in
                 ay[t] = __ffma2_rn(w, dy, ay[t]);
                 az[t] = __ffma2_rn(w, dz, az[t]);
             }
-            if (KIND != kField) av[t] = __ffma2_rn(qw, ir, av[t]);
+            if (KIND != kField) {
+                float2 v = __ffma2_rn(qw, ir, av[t]);
+                if (SELF) {  // not the target itself, at self0 + 32 t of this tile (its charge may be infinite)
+                    if (2 * k == self0 + 32 * t) v.x = av[t].x;
+                    if (2 * k + 1 == self0 + 32 * t) v.y = av[t].y;
+                }
+                av[t] = v;
+            }
         }
     }
 }
@@ -193,22 +196,16 @@ __global__ void __launch_bounds__(kThreads) k_dense_f32(const DenseArgs<float> A
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int q = threadIdx.x + h * kThreads;
-            float x = 0, y = 0, z = 0, w = 0;
-            if (q < ((cnt + 1) & ~1)) {
-                // an odd tile ends with its last source again, without charge: a
-                // point of its own could meet a target, whose weight k_e / r^3
-                // then overflows and is NaN times no charge
-                const int64_t j = jb + min(q, cnt - 1);
-                x = A.c[3 * j];
-                y = A.c[3 * j + 1];
-                z = A.c[3 * j + 2];
-                if (q < cnt) w = A.sigma[j] * A.areas[j];
-            }
+            // past its end a tile holds its last source, without charge: a point of
+            // its own there could meet a target, whose weight k_e / r^3 then
+            // overflows and is NaN times no charge
+            const int64_t j = jb + min(q, cnt - 1);
+            const float x = A.c[3 * j], y = A.c[3 * j + 1], z = A.c[3 * j + 2], w = A.sigma[j] * A.areas[j];
             float *o = sf + (q >> 1) * 8 + (q & 1);
             o[0] = x;
             o[2] = y;
             o[4] = z;
-            o[6] = w;
+            o[6] = q < cnt ? w : 0.0f;
         }
         __syncthreads();
         // two-level sum (tile, then chunk) bounds FP32 rounding growth
@@ -584,6 +581,11 @@ __global__ void __launch_bounds__(kTableThreads) k_dense_table(const double *__r
     if (rank == 0 && threadIdx.x < kTableRows && i < A.m) {
         double v = part[threadIdx.x];
         for (int r = 1; r < A.cs; ++r) v += dsm_load(part + threadIdx.x, r);
+        if (!isfinite(v) && !isfinite(A.sigma[i] * A.areas[i])) {  // its own charge times the diagonal's 0: the sum without it
+            v = 0.0;
+            for (int64_t j = 0; j < A.n; ++j)
+                if (j != i) v = fma(table[j * ld + i], A.sigma[j] * A.areas[j], v);
+        }
         v *= A.k_e;
         if (A.self_int) v += A.self_int[i] * A.sigma[i] * A.areas[i];
         A.out[i] = isfinite(v) ? v : 0.0;

@@ -30,3 +30,28 @@ def test_fp32_field_at_the_origin(cuda_lib, m, n):
     tol = (n + 32) * 2.0 ** -23 * term.norm(dim=2).sum(1, keepdim=True)
     for e in (field_at_targets(t, c, s, a), potential_field_at_targets(t, c, s, a)[1]):
         assert bool(((e.double() - term.sum(1)).abs() <= tol).all())
+
+
+@pytest.mark.parametrize("kernel", ["float32", "float64", "table"])
+@pytest.mark.parametrize("n,i", [(1, 0), (2, 1), (129, 128), (300, 5), (2049, 700)])
+def test_a_charge_that_is_not_finite_stays_out_of_its_own_row(cuda_lib, kernel, n, i):
+    """The sum over j != i without a self term: row i is that of the other panels, and
+    every other row is not finite, which the operator returns as 0."""
+    from electrodrive_gb300 import _lib
+    from electrodrive_gb300.core.operators import DenseOperator
+
+    rng = np.random.default_rng(n)
+    dt = torch.float32 if kernel == "float32" else torch.float64
+    T = lambda x: torch.as_tensor(x, dtype=dt, device="cuda")
+    c, s, a = T(rng.random((n, 3))), T(rng.uniform(0.5, 1.5, n)), T(rng.uniform(0.5, 1.5, n))
+    s[i] = float("inf")
+    if kernel == "table":
+        op = DenseOperator(c, a, None, k_e=1.0)
+        assert op.tabulate()
+        v = op(s)
+    else:
+        v = _lib.dense_matvec(c, s, a, None, k_e=1.0)
+    keep = torch.arange(n, device="cuda") != i
+    term = (s * a).double()[keep] / (c.double()[keep] - c.double()[i]).norm(dim=1)
+    assert abs(float(v[i]) - float(term.sum())) <= (n + 32) * torch.finfo(dt).eps * float(term.sum())
+    assert not bool(v[keep].any())
