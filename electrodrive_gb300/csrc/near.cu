@@ -863,21 +863,25 @@ struct HostCharges {
     int count;
 };
 
-// V += potential (summed in FP64), E += field (in T); FIRST: V is written, not added to
+// V += potential, E += field (in T).  A point's potential is one FP64 sum, rounded
+// to T once: with more charges than a launch takes, `sums` carries it from launch
+// to launch, and the LAST one gives it to V (OVERWRITE: written, not added).
 template <typename T>
-__global__ void k_point_charges_add(const T *pts, int64_t n, const HostCharges ch, double ke, int first, T *V, T *E) {
+__global__ void k_point_charges_add(const T *pts, int64_t n, const HostCharges ch, double ke, double *sums, int begin,
+                                    int last, int overwrite, T *V, T *E) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const T px = pts[3 * i], py = pts[3 * i + 1], pz = pts[3 * i + 2];
     if (V) {
-        double acc = 0.0;
+        double acc = begin ? 0.0 : sums[i];
         for (int k = 0; k < ch.count; ++k) {
             const double dx = (double)px - ch.q[k][1], dy = (double)py - ch.q[k][2], dz = (double)pz - ch.q[k][3];
             double r = sqrt(dx * dx + dy * dy + dz * dz);
             r = r < 1e-12 ? 1e-12 : r;
             acc += ke * ch.q[k][0] / r;
         }
-        V[i] = first ? (T)acc : V[i] + (T)acc;
+        if (!last) sums[i] = acc;
+        else V[i] = overwrite ? (T)acc : V[i] + (T)acc;
     }
     if (E) {
         T ex = 0, ey = 0, ez = 0;
@@ -923,19 +927,26 @@ extern "C" EDFMM_API int edfmm_point_charges_add(const void *points_dev, int64_t
     if (n == 0) return EDFMM_OK;
     if (!points_dev || (n_charges > 0 && !charges_host)) return fail(EDFMM_ERR_ARG, "NULL argument");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    for (int k0 = 0; k0 == 0 || k0 < n_charges; k0 += kChargesPerLaunch) {
+    double *sums = nullptr;
+    if (V_dev && n_charges > kChargesPerLaunch) EDFMM_CUDA_TRY(cudaMallocAsync((void **)&sums, sizeof(double) * (size_t)n, s));
+    cudaError_t e = cudaSuccess;
+    for (int k0 = 0; e == cudaSuccess && (k0 == 0 || k0 < n_charges); k0 += kChargesPerLaunch) {
         HostCharges ch;
-        ch.count = n_charges - k0 < kChargesPerLaunch ? n_charges - k0 : kChargesPerLaunch;
+        ch.count = std::min(n_charges - k0, kChargesPerLaunch);
         for (int k = 0; k < ch.count; ++k)
             for (int q = 0; q < 4; ++q) ch.q[k][q] = charges_host[4 * (k0 + k) + q];
-        const int first = overwrite && k0 == 0;
+        const int begin = k0 == 0, last = k0 + kChargesPerLaunch >= n_charges;
         if (dtype == EDFMM_F64)
-            k_point_charges_add<double><<<nb(n, 128), 128, 0, s>>>((const double *)points_dev, n, ch, k_e, first,
-                                                                   (double *)V_dev, (double *)E_dev);
+            k_point_charges_add<double><<<nb(n, 128), 128, 0, s>>>((const double *)points_dev, n, ch, k_e, sums, begin,
+                                                                   last, overwrite, (double *)V_dev, (double *)E_dev);
         else
-            k_point_charges_add<float><<<nb(n, 128), 128, 0, s>>>((const float *)points_dev, n, ch, k_e, first,
-                                                                  (float *)V_dev, (float *)E_dev);
-        EDFMM_LAUNCH_CHECK("k_point_charges_add");
+            k_point_charges_add<float><<<nb(n, 128), 128, 0, s>>>((const float *)points_dev, n, ch, k_e, sums, begin,
+                                                                  last, overwrite, (float *)V_dev, (float *)E_dev);
+        count_launch();
+        e = cudaGetLastError();
     }
+    if (sums) cudaFreeAsync(sums, s);
+    if (e != cudaSuccess)
+        return fail(EDFMM_ERR_CUDA, std::string("launch of k_point_charges_add failed: ") + cudaGetErrorString(e));
     return EDFMM_OK;
 }

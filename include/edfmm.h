@@ -434,7 +434,9 @@ EDFMM_API int edfmm_point_charge_potential(const void *points_dev, int64_t n, co
  * The same potential, and the charges' field (core/bem.py:340-370), added to
  * what V (n) and E (n, 3) hold (either may be NULL; `overwrite` writes V instead
  * of adding to it).  charges_host: (n_charges, 4) FP64 rows (q, x, y, z) in host
- * memory, passed as kernel parameters.
+ * memory, passed as kernel parameters, 32 to a launch.  The potential is one FP64
+ * sum, rounded once; above 32 charges it is carried in 8 n bytes of
+ * stream-ordered scratch.
  */
 EDFMM_API int edfmm_point_charges_add(const void *points_dev, int64_t n, const double *charges_host, int n_charges,
                                       double k_e, int dtype, int overwrite, void *V_dev, void *E_dev, void *stream);
