@@ -167,9 +167,9 @@ def add_point_charges(points: Tensor, charges, *, V: Optional[Tensor] = None, E:
     """V += sum_k k_e q_k / max(|x - r_k|, 1e-12) and E += the charges' field at
     CUDA points, in place (``overwrite``: V is written instead)."""
     L = _lib.load_library()
-    rows = [float(v) for q, pos in charges for v in (q, *pos)]
-    n_ch = len(rows) // 4
-    ch = (C.c_double * max(len(rows), 1))(*rows)
+    rows = np.asarray([[float(q), *map(float, pos)] for q, pos in charges], dtype=np.float64).reshape(-1, 4)
+    n_ch = rows.shape[0]
+    ch = rows.ctypes.data_as(C.POINTER(C.c_double))
     pts = points.contiguous()
     with torch.cuda.device(points.device):
         _lib.check(L.edfmm_point_charges_add(_lib.ptr(pts), points.shape[0], ch, n_ch, float(k_e),

@@ -37,3 +37,21 @@ def test_potential_of_many_charges_is_rounded_once(cuda_lib, dtype, n, k):
     w = torch.full((n,), 3.0, dtype=dtype, device="cuda")
     add_point_charges(pts, ch, V=w)
     assert bool(((w.double() - 3.0 - ref).abs() <= u * (2 * ref.abs() + 3.0) + size + 3.0 * 2.0 ** -52).all())
+
+
+@pytest.mark.parametrize("charges", [[(1.0, (0.0, 2.0))], [(1.0, (0.0, 2.0, 0.0, 1.0))], [(1.0, ())],
+                                     [(1.0, (0.0, 0.0, 2.0)), (1.0, (0.0, 2.0))]])
+def test_positions_without_three_coordinates_are_refused(cuda_lib, charges):
+    from electrodrive_gb300.core.bem import BEMSolution
+    from electrodrive_gb300.core.bem_near import add_point_charges, point_charge_potential
+
+    pts = torch.rand(5, 3, device="cuda", dtype=torch.float64)
+    with pytest.raises(ValueError):
+        point_charge_potential(pts, charges)
+    with pytest.raises(ValueError):
+        add_point_charges(pts, charges, V=torch.zeros(5, device="cuda", dtype=torch.float64))
+    one = torch.ones(1, device="cuda", dtype=torch.float64)
+    sol = BEMSolution(centroids=torch.zeros(1, 3, device="cuda", dtype=torch.float64), areas=one, sigma=one,
+                      charges=charges)
+    with pytest.raises(ValueError):
+        sol.eval_V_E_batched(pts)
