@@ -29,8 +29,9 @@ from torch import Tensor
 from .. import _lib
 from ..utils.config import K_E, BEMConfig
 from .bem_mesh import TriMesh, generate_mesh
-from .bem_near import (NearCorrection, add_point_charges, near_potential_correction,
-                       point_charge_potential, potential_at_targets, potential_field_at_targets, self_integrals)
+from .bem_near import (NearCorrection, add_point_charges, differentiated, near_potential_correction,
+                       point_charge_field, point_charge_potential, potential_at_targets, potential_field_at_targets,
+                       self_integrals)
 from .bem_solver import gmres_batched, gmres_restart
 from .operators import DenseOperator, FmmOperator
 
@@ -178,7 +179,10 @@ class BEMSolution:
         pts = self._points(points)
         v, e = potential_field_at_targets(pts, self.centroids, self.sigma, self.areas)
         v = self._near_corrected(v, pts)
-        if self.charges:
+        if self.charges and differentiated(pts, self.charges):
+            add_point_charges(pts, self.charges, V=v)
+            e = e + point_charge_field(pts, self.charges)
+        elif self.charges:
             add_point_charges(pts, self.charges, V=v, E=e)
         return v, e
 

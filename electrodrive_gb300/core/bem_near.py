@@ -185,6 +185,14 @@ def point_charge_potential(points: Tensor, charges, *, k_e: float = K_E) -> Tens
     return out
 
 
+def differentiated(points: Tensor, charges) -> bool:
+    """Whether a derivative is asked for with respect to the points or a charge's
+    position: the field is then :func:`point_charge_field`'s torch expression."""
+    ts = [points, *(pos for _, pos in charges if isinstance(pos, Tensor))]
+    return any((torch.is_grad_enabled() and t.requires_grad) or torch.autograd.forward_ad.unpack_dual(t).tangent is not None
+               for t in ts)
+
+
 def potential_at_targets(targets: Tensor, centroids: Tensor, sigma: Tensor, areas: Tensor, *,
                          k_e: float = K_E) -> Tensor:
     """Induced potential of panel charges at targets (bem_potential_targets, bem_kernel.py:233-270)."""
@@ -265,10 +273,6 @@ def point_charge_field(points: Tensor, charges) -> Tensor:
     (_free_space_E_field_at_points, bem.py:340-370), (M, 3) in the points' dtype."""
     P = points.reshape(-1, 3)
     E = torch.zeros_like(P)
-    if P.is_cuda and P.dtype in (torch.float32, torch.float64) and not P.requires_grad:
-        E = E.contiguous()
-        add_point_charges(P, charges, E=E)
-        return E
     for q, pos in charges:
         R = P - torch.as_tensor(pos, dtype=P.dtype, device=P.device)[None, :]
         r = torch.linalg.norm(R, dim=1, keepdim=True).clamp_min(1e-12)

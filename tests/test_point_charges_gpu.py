@@ -55,3 +55,66 @@ def test_positions_without_three_coordinates_are_refused(cuda_lib, charges):
                       charges=charges)
     with pytest.raises(ValueError):
         sol.eval_V_E_batched(pts)
+
+
+def _field(points, charges):
+    """K_E sum q (x - r) / |x - r|^3 in torch."""
+    d = points[:, None] - torch.stack([torch.as_tensor(r, dtype=points.dtype, device=points.device)
+                                       for _, r in charges])[None]
+    q = torch.tensor([float(c) for c, _ in charges], dtype=points.dtype, device=points.device)
+    return (K_E * q[:, None] * d / d.norm(dim=2, keepdim=True) ** 3).sum(1)
+
+
+def _case():
+    rng = np.random.default_rng(3)
+    pts = torch.as_tensor(rng.normal(size=(7, 3)), device="cuda")
+    pos = [torch.as_tensor(2.0 + rng.random(3), device="cuda") for _ in range(2)]
+    return pts, [(0.5, pos[0]), (-1.5, pos[1])]
+
+
+def _close(a, b):
+    return float((a - b).norm()) <= 1e-13 * float(b.norm())
+
+
+def test_field_has_derivatives_to_points_and_positions(cuda_lib):
+    from electrodrive_gb300.core.bem_near import point_charge_field
+
+    pts, ch = _case()
+    assert _close(point_charge_field(pts, ch), _field(pts, ch))
+    for leaf in (pts, ch[0][1]):
+        leaf.requires_grad_(True)
+        e = point_charge_field(pts, ch)
+        assert e.requires_grad
+        got, = torch.autograd.grad(e.square().sum(), leaf)
+        assert _close(got, torch.autograd.grad(_field(pts, ch).square().sum(), leaf)[0])
+        leaf.requires_grad_(False)
+
+
+def test_field_under_vmap_and_forward_mode(cuda_lib):
+    from electrodrive_gb300.core.bem_near import point_charge_field
+
+    pts, ch = _case()
+    batch = torch.stack([pts, 2.0 * pts])
+    got = torch.func.vmap(lambda p: point_charge_field(p, ch))(batch)
+    assert _close(got[0], _field(pts, ch)) and _close(got[1], _field(2.0 * pts, ch))
+    t = torch.ones_like(pts)
+    got = torch.func.jvp(lambda p: point_charge_field(p, ch), (pts,), (t,))[1]
+    assert _close(got, torch.func.jvp(lambda p: _field(p, ch), (pts,), (t,))[1])
+
+
+def test_evaluation_keeps_the_charges_part_of_the_fields_gradient(cuda_lib):
+    """eval_V_E_batched: the induced part has no graph, the point charges' part has one."""
+    from electrodrive_gb300.core.bem import BEMSolution
+
+    pts, ch = _case()
+    one = torch.ones(1, device="cuda", dtype=torch.float64)
+    sol = BEMSolution(centroids=torch.zeros(1, 3, device="cuda", dtype=torch.float64), areas=one, sigma=one, charges=ch)
+    plain = sol.eval_V_E_batched(pts)
+    for leaf in (pts, ch[1][1]):
+        leaf.requires_grad_(True)
+        v, e = sol.eval_V_E_batched(pts)
+        got, = torch.autograd.grad(e.sum(), leaf)
+        assert _close(got, torch.autograd.grad(_field(pts, ch).sum(), leaf)[0])
+        leaf.requires_grad_(False)
+        assert _close(v.detach(), plain[0]) and _close(e.detach(), plain[1])
+    assert not plain[1].requires_grad
