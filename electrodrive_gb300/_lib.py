@@ -82,6 +82,7 @@ def _declare(L):
         "edfmm_version": (C.c_char_p, []),
         "edfmm_launch_count": (i64, []),
         "edfmm_block_cache_selfcheck": (i32, [C.POINTER(i64)]),
+        "edfmm_device_once_selfcheck": (i32, [C.POINTER(i64)]),
         "edfmm_plan_create": (i32, [_vp, i64, i32, i32, i32, dbl, i32, _vp, C.POINTER(_vp)]),
         "edfmm_plan_create_batch": (i32, [_vp, C.POINTER(i64), i32, i32, i32, i32, dbl, i32, _vp, C.POINTER(_vp)]),
         "edfmm_plan_convert": (i32, [_vp, i32, i32, _vp, C.POINTER(_vp)]),

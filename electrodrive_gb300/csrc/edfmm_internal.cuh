@@ -2,6 +2,7 @@
 #pragma once
 
 #include <algorithm>
+#include <atomic>
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -36,6 +37,32 @@ void count_launch(int n = 1);
             return ::edfmm::fail(EDFMM_ERR_CUDA, std::string("launch of " name " failed: ") + \
                                                      cudaGetErrorString(_e));                 \
     } while (0)
+
+// ---------------------------------------------------------------------------
+// settings that belong to a device
+// ---------------------------------------------------------------------------
+// Runs `set` the first time it is asked for device `dev`: a kernel's attribute
+// holds on the device that was current when it was set, and a process may use
+// several.  A failure is not remembered; ordinals past the mask are set each time.
+struct DeviceOnce {
+    std::atomic<unsigned long long> done{0};
+};
+template <typename F> cudaError_t once_per_device(DeviceOnce &once, int dev, F &&set) {
+    const unsigned long long bit = dev >= 0 && dev < 64 ? 1ull << dev : 0ull;
+    if (once.done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    const cudaError_t e = set();
+    if (e == cudaSuccess && bit) once.done.fetch_or(bit, std::memory_order_release);
+    return e;
+}
+// opt-in of a kernel to more than 48 KB of dynamic shared memory on the current device
+template <typename K> cudaError_t allow_smem(DeviceOnce &once, K *kernel, size_t bytes) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return once_per_device(once, dev, [&] {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    });
+}
 
 // ---------------------------------------------------------------------------
 // device buffer (owning)

@@ -1094,11 +1094,8 @@ template <typename T> int p2m_impl(const DevTree &tree, FmmBuffers &buf, cudaStr
     const size_t smem = sizeof(T) * 33 * 2 * (size_t)ncoef(buf.p) * p2m_warps<T>();
 #define EDFMM_P2M_CASE(PP)                                                                                          \
     case PP: {                                                                                                      \
-        static const cudaError_t attr =                                                                             \
-            cudaFuncSetAttribute(k_p2m<T, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize,                         \
-                                 (int)(sizeof(T) * 33 * 2 * ncoef(PP) * p2m_warps<T>()));                            \
-        if (attr != cudaSuccess)                                                                                    \
-            return fail(EDFMM_ERR_CUDA, std::string("k_p2m shared memory: ") + cudaGetErrorString(attr));           \
+        static DeviceOnce once;                                                                                     \
+        EDFMM_CUDA_TRY(allow_smem(once, k_p2m<T, PP>, sizeof(T) * 33 * 2 * ncoef(PP) * p2m_warps<T>()));            \
         k_p2m<T, PP><<<grid, NT, smem, s>>>(dptr<int32_t>(tree.leaves), tree.n_leaves, dptr<T4>(tree.pts),           \
                                             dptr<T4>(tree.center), dptr<T4>(tree.half), dptr<int2>(tree.range),       \
                                             dptr<Cplx<T>>(buf.multipoles), buf.nc_pad);                              \

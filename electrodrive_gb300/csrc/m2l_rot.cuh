@@ -1081,10 +1081,8 @@ int launch_rot_tf(int64_t M, const int32_t *off, const int32_t *src, const int32
                   cudaStream_t s) {
     constexpr int NV = (P + 1) * (P + 1);
     constexpr size_t smem = (size_t)NV * NT * sizeof(tf32x2);
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_m2l_rot_tf<P, NT, PK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (attr != cudaSuccess)
-        return fail(EDFMM_ERR_CUDA, std::string("k_m2l_rot_tf shared memory attribute: ") + cudaGetErrorString(attr));
+    static DeviceOnce once;
+    EDFMM_CUDA_TRY(allow_smem(once, k_m2l_rot_tf<P, NT, PK>, smem));
     EDFMM_CUDA_TRY(chain_launch(chain_tree(M, EDFMM_F64, s), k_m2l_rot_tf<P, NT, PK>, nblk(M * 32, NT), NT, smem, s, M, off, src,
                                 rows, static_cast<const float4 *>(tnodes), static_cast<const double4 *>(thal),
                                 static_cast<const float4 *>(snodes), static_cast<const double4 *>(hal),
@@ -1098,10 +1096,8 @@ int launch_rot_f64(int64_t M, const int32_t *off, const int32_t *src, const int3
                    const void *thal, const void *cen, const void *hal, const void *Mx, void *Lx, int nc_pad,
                    const InstMask &mask, cudaStream_t s) {
     constexpr size_t smem = (size_t)(P + 1) * (P + 1) * kRotThreads * sizeof(double);
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_m2l_rot_f64<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (attr != cudaSuccess)
-        return fail(EDFMM_ERR_CUDA, std::string("k_m2l_rot_f64 shared memory attribute: ") + cudaGetErrorString(attr));
+    static DeviceOnce once;
+    EDFMM_CUDA_TRY(allow_smem(once, k_m2l_rot_f64<P>, smem));
     EDFMM_CUDA_TRY(chain_launch(chain_tree(M, EDFMM_F64, s), k_m2l_rot_f64<P>, (unsigned)M, kRotThreads, smem, s, M, off, src, rows,
                                 static_cast<const double4 *>(tcen), static_cast<const double4 *>(thal),
                                 static_cast<const double4 *>(cen), static_cast<const double4 *>(hal),
@@ -1116,10 +1112,8 @@ int launch_rot(int64_t M, const int32_t *off, const int32_t *src, const int32_t 
                const InstMask &mask, cudaStream_t s) {
     constexpr int NQ = (P + 1) * (P + 2) / 2, NT = kRotThreads;
     constexpr size_t smem = (size_t)NQ * NT * sizeof(float2);
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_m2l_rot<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (attr != cudaSuccess)
-        return fail(EDFMM_ERR_CUDA, std::string("k_m2l_rot shared memory attribute: ") + cudaGetErrorString(attr));
+    static DeviceOnce once;
+    EDFMM_CUDA_TRY(allow_smem(once, k_m2l_rot<P>, smem));
     EDFMM_CUDA_TRY(chain_launch(chain_tree(M, EDFMM_F32, s), k_m2l_rot<P>, nblk(M * 32, NT), NT, smem, s, M, off, src, rows,
                                 static_cast<const float4 *>(tcen), static_cast<const float4 *>(thal),
                                 static_cast<const float4 *>(cen), static_cast<const float4 *>(hal),

@@ -347,10 +347,8 @@ template <int K, int EPI, bool HEAD>
 int launch_linear(bool chained, const __nv_bfloat16 *X, const __nv_bfloat16 *Wt, const float *bias, const __nv_bfloat16 *mask,
                   int64_t n, __nv_bfloat16 *out, const float *prm, float *y, cudaStream_t s) {
     constexpr size_t smem = lin_smem_out<K>();
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_pcn_linear<K, EPI, HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (attr != cudaSuccess)
-        return fail(EDFMM_ERR_CUDA, std::string("k_pcn_linear shared memory: ") + cudaGetErrorString(attr));
+    static DeviceOnce once;
+    EDFMM_CUDA_TRY(allow_smem(once, k_pcn_linear<K, EPI, HEAD>, smem));
     EDFMM_CUDA_TRY(chain_launch(chained, k_pcn_linear<K, EPI, HEAD>, nblk(n, kLinRows), 256, smem, s, X, Wt, bias, mask, n,
                                 out, prm, y));
     EDFMM_LAUNCH_CHECK("k_pcn_linear");
@@ -627,13 +625,10 @@ __global__ void __launch_bounds__(W) k_pcn_context_grad(const float *prm, const 
 }
 
 int staged_smem() {  // dynamic shared memory above 48 KB
-    static const cudaError_t attr[3] = {
-        cudaFuncSetAttribute(k_pcn_wgrad_part<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Wg<W>::smem),
-        cudaFuncSetAttribute(k_pcn_context, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtxSmem),
-        cudaFuncSetAttribute(k_pcn_colsum_part, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColSmem)};
-    for (cudaError_t e : attr)
-        if (e != cudaSuccess)
-            return fail(EDFMM_ERR_CUDA, std::string("warm-start kernels' shared memory: ") + cudaGetErrorString(e));
+    static DeviceOnce once[3];
+    EDFMM_CUDA_TRY(allow_smem(once[0], k_pcn_wgrad_part<W>, Wg<W>::smem));
+    EDFMM_CUDA_TRY(allow_smem(once[1], k_pcn_context, kCtxSmem));
+    EDFMM_CUDA_TRY(allow_smem(once[2], k_pcn_colsum_part, kColSmem));
     return EDFMM_OK;
 }
 

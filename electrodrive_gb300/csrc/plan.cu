@@ -495,6 +495,30 @@ int edfmm_block_cache_selfcheck(int64_t *results_host) {
     return EDFMM_OK;
 }
 
+int edfmm_device_once_selfcheck(int64_t *results_host) {
+    if (!results_host) return fail(EDFMM_ERR_ARG, "results_host is NULL");
+    DeviceOnce once;
+    int calls[71] = {0};
+    auto run = [&](int dev, cudaError_t e) {
+        return once_per_device(once, dev, [&] {
+            ++calls[dev];
+            return e;
+        });
+    };
+    // set once on each of two devices, in any order of use
+    for (int k = 0; k < 3; ++k)
+        for (int dev = 0; dev < 2; ++dev) run(dev, cudaSuccess);
+    results_host[0] = calls[0] == 1 && calls[1] == 1;
+    // a failure is returned, and tried again
+    results_host[1] = run(63, cudaErrorInvalidValue) == cudaErrorInvalidValue && run(63, cudaSuccess) == cudaSuccess &&
+                      run(63, cudaErrorInvalidValue) == cudaSuccess && calls[63] == 2;
+    // past the mask: every time
+    run(70, cudaSuccess);
+    run(70, cudaSuccess);
+    results_host[2] = calls[70] == 2;
+    return EDFMM_OK;
+}
+
 int edfmm_plan_destroy(edfmm_plan *plan) {
     delete plan;
     return EDFMM_OK;

@@ -81,6 +81,15 @@ typedef struct {
  */
 EDFMM_API int edfmm_block_cache_selfcheck(int64_t *results_host);
 
+/*
+ * Self-check of the library's once-per-device settings (kernel attributes hold
+ * on the device they were set on; no counterpart in the reference), with made-up
+ * device ordinals and settings; needs no GPU.  results_host[0..2] are set to 1
+ * for each rule that held: once on each device, a failure is returned and tried
+ * again, ordinals above 63 are set every time.
+ */
+EDFMM_API int edfmm_device_once_selfcheck(int64_t *results_host);
+
 /* Thread-local description of the most recent failure. */
 EDFMM_API const char *edfmm_last_error(void);
 
