@@ -128,9 +128,9 @@ size_t setup_slab_bytes(int64_t n, int dtype) {
 // leaves in slabs or in cached blocks larger than they need move to exact
 // blocks before the plan is handed out; expansions of up to 16 MB (three
 // buffers of esz bytes) share the block of the small ones.
-int settle_buffers(DevTree &t, DevLists &l, DevBuf *const *exp, int n_exp, size_t esz, DevBuf &block,
+int settle_buffers(DevTree &t, DevLists &l, DevBuf &near_sum, DevBuf *const *exp, int n_exp, size_t esz, DevBuf &block,
                    cudaStream_t s) {
-    DevBuf *bufs[] = {&t.pts,      &t.index_map,     &t.center,      &t.half,    &t.range,
+    DevBuf *bufs[] = {&near_sum,   &t.pts,      &t.index_map,     &t.center,      &t.half,    &t.range,
                       &t.parent,   &t.children,      &t.level,       &t.is_leaf, &t.leaves,
                       &t.level_nodes, &t.inst_node_off, &l.p2p_off,  &l.p2p_src, &l.m2l_off,
                       &l.m2l_src,  &l.m2l_swapped_off, &l.m2l_swapped_src, &l.p2p_leaves, &l.m2l_rows,
@@ -155,7 +155,7 @@ int finish_plan(edfmm_plan *p, int dtype, int expansion_order, cudaStream_t s) {
     DevBuf *exp[] = {&p->fmm.multipoles, &p->fmm.locals, &p->fmm.translated};
     int rc = grid_prepare(p->tree, s);
     if (!rc) rc = shift_prepare(p->tree, s);
-    if (!rc) rc = settle_buffers(p->tree, p->lists, exp, 3, esz, p->block, s);
+    if (!rc) rc = settle_buffers(p->tree, p->lists, p->near_sum, exp, 3, esz, p->block, s);
     if (!rc) {
         cudaError_t e = cudaMemsetAsync(p->fmm.multipoles.p, 0, esz, s);
         if (e == cudaSuccess) e = cudaMemsetAsync(p->fmm.locals.p, 0, esz, s);
@@ -842,7 +842,9 @@ static int finish_targets(edfmm_targets *t, cudaStream_t s) {
                        (size_t)std::max<int64_t>(t->tree.n_nodes, 1);
     DevBuf *exp[] = {&t->buf.locals};
     int rc = shift_prepare(t->tree, s);
-    if (!rc) rc = settle_buffers(t->tree, t->lists, exp, 1, esz, t->block, s);
+    // here and not on first use: an evaluation allocates nothing, so its first may be captured
+    if (!rc) rc = t->near_sum.reserve((p->tree.dtype == EDFMM_F64 ? sizeof(double) : sizeof(float)) * (size_t)t->tree.n_points);
+    if (!rc) rc = settle_buffers(t->tree, t->lists, t->near_sum, exp, 1, esz, t->block, s);
     if (!rc) {
         cudaError_t e = cudaMemsetAsync(t->buf.locals.p, 0, esz, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -1000,12 +1002,7 @@ int edfmm_targets_potential(edfmm_targets *t, const void *sigma, const void *are
             (rc = run_m2l_two(t->tree, p->tree, t->lists, p->fmm, t->buf, s)) || (rc = run_l2l(t->tree, t->buf, s)))
             return rc;
     }
-    if (near) {
-        const size_t elt = t->tree.dtype == EDFMM_F64 ? sizeof(double) : sizeof(float);
-        if ((rc = t->near_sum.reserve(elt * (size_t)t->tree.n_points)) ||
-            (rc = run_p2p(t->tree, t->lists, t->buf, &p->tree, t->near_sum.p, s)))
-            return rc;
-    }
+    if (near && (rc = run_p2p(t->tree, t->lists, t->buf, &p->tree, t->near_sum.p, s))) return rc;
     L2pArgs a;
     a.k_e = k_e;
     a.out = out;
