@@ -241,16 +241,17 @@ __device__ __forceinline__ float rsqrt_normal(float x) {
 }
 #endif
 
-// Device-resident tree in DFS pre-order (the reference's node numbering).
-// Scale of an FP64 tree's split coordinates (gridpoint.cuh): 2^-k, 2^k, the
-// scaled r^2 below which a pair is evaluated in IEEE FP64, and the high word
-// of the largest |coordinate|.
+// Frame of an FP64 tree's split coordinates (gridpoint.cuh): the centre, 2^-k,
+// 2^k, and the scaled r^2 below which a pair is evaluated in IEEE FP64; the
+// largest x, y, z, -x, -y, -z while it is laid out (order-preserving integers).
 struct GridInfo {
     double down, up;
+    double center[3];
     float near2;
-    unsigned hi;
+    long long ext[6];
 };
 
+// Device-resident tree in DFS pre-order (the reference's node numbering).
 struct DevTree {
     int dtype = EDFMM_F32;
     int64_t n_points = 0;

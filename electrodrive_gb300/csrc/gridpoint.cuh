@@ -8,7 +8,8 @@
 // slots; packed operands cannot be negated for free, so the middle terms
 // carry the sign that needs the fewest negations).
 //
-// Coordinates are scaled by a power of two to |x| <= 1 and split exactly
+// Coordinates (the FMM's less a centre, where that difference is exact) are
+// scaled by a power of two to |x| <= 1 and split exactly
 // into x = a + b + c, a a multiple of 2^-23, b of 2^-47 with |b| <= 2^-24
 // and c the rest (a float, |c| <= 2^-48).  On these common grids the
 // differences of two points' a and b parts are exact, so a coordinate
@@ -24,7 +25,7 @@
 // adds to the bits of the double y0.
 // Every quantity is carried to about 2^-58 relative; the roundings to 2^-52
 // units make the error of an IEEE rounding.  Pairs closer than
-// 2^-19 of the largest |coordinate| (where the parts no longer hold all bits)
+// 2^-19 of the scale (where the parts no longer hold all bits)
 // are left to the caller's IEEE form.
 #pragma once
 

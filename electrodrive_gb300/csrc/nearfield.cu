@@ -9,6 +9,7 @@
 // bem_fmm.py:718-749 (K_E, original order, self term, non-finite -> 0), so
 // each output is written exactly once.
 #include <cfloat>
+#include <climits>
 #include <type_traits>
 
 #include "edfmm_internal.cuh"
@@ -260,9 +261,9 @@ __device__ __forceinline__ void load_target(const NearParams<T> &P, int ti, int 
         X.nz[r] = make_float2(-x.z, -x.z);
         X.acc[r] = 0.0f;
     } else if constexpr (MODE == kTF || MODE == kGrid) {
-        X.x[r] = grid_both(grid_split(x.x * g.down));
-        X.y[r] = grid_both(grid_split(x.y * g.down));
-        X.z[r] = grid_both(grid_split(x.z * g.down));
+        X.x[r] = grid_both(grid_split((x.x - g.center[0]) * g.down));
+        X.y[r] = grid_both(grid_split((x.y - g.center[1]) * g.down));
+        X.z[r] = grid_both(grid_split((x.z - g.center[2]) * g.down));
         X.acc[r] = 0.0;
     } else {
         X.x[r] = x.x;
@@ -711,36 +712,80 @@ __device__ __forceinline__ int instance_of_point(const int32_t *node_off, int n_
     }
     return lo;
 }
-__global__ void k_grid_max(const double4 *__restrict__ pts, int64_t n, const int32_t *node_off, int n_inst,
-                           const int2 *__restrict__ range, GridInfo *info) {
-    // a block takes a run of points: mostly of one instance
+// doubles to integers of the same order (NaN beyond the infinity of its sign)
+__device__ __forceinline__ long long ord_of(double x) {
+    const long long i = __double_as_longlong(x);
+    return i >= 0 ? i : i ^ 0x7fffffffffffffffLL;
+}
+__device__ __forceinline__ double from_ord(long long i) {
+    return __longlong_as_double(i >= 0 ? i : i ^ 0x7fffffffffffffffLL);
+}
+// memset's pattern for "no point yet": below every number of a usable scale
+constexpr int kNoExtent = 0x80;
+
+__global__ void k_grid_extent(const double4 *__restrict__ pts, int64_t n, const int32_t *node_off, int n_inst,
+                              const int2 *__restrict__ range, GridInfo *info) {
+    // a block takes a run of points, mostly of one instance; a thread adds its
+    // points up as long as the instance stays the same
     const int64_t per = (n + gridDim.x - 1) / gridDim.x, b = blockIdx.x * per, e = min(n, b + per);
+    long long m[6] = {LLONG_MIN, LLONG_MIN, LLONG_MIN, LLONG_MIN, LLONG_MIN, LLONG_MIN};
+    int k = -1;  // none yet, or past the end
+    auto flush = [&] {  // the warp's extents of its instance, or a lane's own
+        const int k0 = __shfl_sync(0xffffffffu, k, 0);
+        const bool one = __all_sync(0xffffffffu, k == k0 || k < 0);
+#pragma unroll
+        for (int a = 0; a < 6; ++a) {
+            long long v = m[a];
+            if (one) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v = max(v, (long long)__shfl_xor_sync(0xffffffffu, v, o));
+            }
+            if (k >= 0 && (!one || (threadIdx.x & 31) == 0)) atomicMax(&info[k].ext[a], v);
+        }
+    };
     for (int64_t i0 = b; i0 < e; i0 += blockDim.x) {
         const int64_t i = i0 + threadIdx.x;
-        unsigned hi = 0;
-        int k = -1;
-        if (i < e) {
-            k = instance_of_point(node_off, n_inst, range, i);
-            const double4 p = pts[i];
-            hi = max(hi, (unsigned)__double2hiint(p.x) & 0x7fffffffu);
-            hi = max(hi, (unsigned)__double2hiint(p.y) & 0x7fffffffu);
-            hi = max(hi, (unsigned)__double2hiint(p.z) & 0x7fffffffu);
+        const int ki = i < e ? instance_of_point(node_off, n_inst, range, i) : k;
+        if (__any_sync(0xffffffffu, ki != k)) {
+            flush();
+            k = ki;
+#pragma unroll
+            for (int a = 0; a < 6; ++a) m[a] = LLONG_MIN;
         }
-        const int k0 = __shfl_sync(0xffffffffu, k, 0);
-        if (__all_sync(0xffffffffu, k == k0 || k < 0)) {
-            hi = __reduce_max_sync(0xffffffffu, hi);
-            if ((threadIdx.x & 31) == 0 && k0 >= 0) atomicMax(&info[k0].hi, hi);
-        } else if (k >= 0) {
-            atomicMax(&info[k].hi, hi);
+        if (i < e) {
+            const double4 p = pts[i];
+            const double x[3] = {p.x, p.y, p.z};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                m[a] = max(m[a], ord_of(x[a]));
+                m[3 + a] = max(m[3 + a], ord_of(-x[a]));
+            }
         }
     }
+    flush();
 }
-// each scale from its largest coordinate
-__global__ void k_grid_scales(int n_inst, GridInfo *info) {
+// Each frame from its points' extents.  An axis on which the points lie within a
+// sixteenth of their distance from the origin has its centre at the nearest of
+// them: a coordinate and the centre are then within a factor of two of one
+// another, so that their difference is exact, and the scale is that of the
+// extent.  Without it a geometry far from the origin has all its near pairs
+// closer than the split resolves, each formed a second time in IEEE FP64 (20,011
+// points on a sphere at x = 1e6, two-float: 1,590 us against 148 at the origin).
+// The scale of an axis without a centre is at most 2^4 times its extent.
+__global__ void k_grid_frames(int n_inst, GridInfo *info) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_inst) return;
+    unsigned reach = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double hi = from_ord(info[i].ext[a]), lo = -from_ord(info[i].ext[3 + a]);
+        const double c = lo > 0.0 && hi <= 1.0625 * lo ? lo : hi < 0.0 && lo >= 1.0625 * hi ? hi : 0.0;
+        info[i].center[a] = c;
+        reach = max(reach, (unsigned)__double2hiint(hi - c) & 0x7fffffffu);
+        reach = max(reach, (unsigned)__double2hiint(lo - c) & 0x7fffffffu);
+    }
     int k;
-    const bool ok = grid_exponent(info[i].hi, k);
+    const bool ok = grid_exponent(reach, k);
     if (!ok) k = 0;
     info[i].down = grid_pow2(-k);
     info[i].up = grid_pow2(k);
@@ -759,9 +804,9 @@ __global__ void k_grid_points(const double4 *__restrict__ pts, int64_t n, const 
     const double4 p = pts[i];
     GridCoord x{}, y{}, z{};
     if (g.near2 >= 0.0f) {  // not NaN
-        x = grid_split(p.x * g.down);
-        y = grid_split(p.y * g.down);
-        z = grid_split(p.z * g.down);
+        x = grid_split((p.x - g.center[0]) * g.down);
+        y = grid_split((p.y - g.center[1]) * g.down);
+        z = grid_split((p.z - g.center[2]) * g.down);
     }
     out[3 * i] = make_float4(x.a, x.b, x.c, y.a);
     out[3 * i + 1] = make_float4(y.b, y.c, z.a, z.b);
@@ -781,13 +826,13 @@ int grid_prepare(DevTree &tree, cudaStream_t s) {
     GridInfo *info = dptr<GridInfo>(tree.grid_info);
     const int32_t *node_off = tree.n_inst > 0 ? dptr<int32_t>(tree.inst_node_off) : nullptr;
     const int2 *range = dptr<int2>(tree.range);
-    EDFMM_CUDA_TRY(cudaMemsetAsync(info, 0, sizeof(GridInfo) * (size_t)K, s));
+    EDFMM_CUDA_TRY(cudaMemsetAsync(info, kNoExtent, sizeof(GridInfo) * (size_t)K, s));
     const int64_t nb = (tree.n_points + 255) / 256;
-    k_grid_max<<<(unsigned)(nb < 608 ? nb : 608), 256, 0, s>>>(dptr<double4>(tree.pts), tree.n_points, node_off, K, range,
-                                                               info);
-    EDFMM_LAUNCH_CHECK("k_grid_max");
-    k_grid_scales<<<(unsigned)((K + 127) / 128), 128, 0, s>>>(K, info);
-    EDFMM_LAUNCH_CHECK("k_grid_scales");
+    k_grid_extent<<<(unsigned)(nb < 608 ? nb : 608), 256, 0, s>>>(dptr<double4>(tree.pts), tree.n_points, node_off, K,
+                                                                  range, info);
+    EDFMM_LAUNCH_CHECK("k_grid_extent");
+    k_grid_frames<<<(unsigned)((K + 127) / 128), 128, 0, s>>>(K, info);
+    EDFMM_LAUNCH_CHECK("k_grid_frames");
     k_grid_points<<<(unsigned)nb, 256, 0, s>>>(dptr<double4>(tree.pts), tree.n_points, node_off, K, range, info,
                                                dptr<float4>(tree.pts_grid));
     EDFMM_LAUNCH_CHECK("k_grid_points");
