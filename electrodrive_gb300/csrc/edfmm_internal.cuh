@@ -321,7 +321,9 @@ __device__ __forceinline__ bool inst_active(const InstMask &m, int node) {
 // chain_launch may start while its predecessor in the stream still runs.  It
 // reads what the plan holds, calls chain_wait (all threads, before any return),
 // and only then reads or writes what other kernels of the chain do; chain_next
-// lets its own successor start.  Without the launch attribute both do nothing.
+// lets its own successor start.  A chain begins with an ordinary launch, so that
+// all that came before it is complete.  Without the launch attribute both do
+// nothing.
 // What the chain writes is read through pointers that are neither const
 // __restrict__ nor __ldg: those loads assume data that stay as they are for the
 // kernel's whole life, which here begins before its predecessor's end.
@@ -436,7 +438,10 @@ struct FmmBuffers {
 int set_charges(const DevTree &tree, const void *sigma, const void *areas, cudaStream_t s);
 int run_p2m(const DevTree &tree, FmmBuffers &buf, cudaStream_t s);
 int run_m2m(const DevTree &tree, FmmBuffers &buf, cudaStream_t s);
-int run_m2l(const DevTree &tree, const DevLists &lists, FmmBuffers &buf, bool swapped, cudaStream_t s);
+// alone: a stage of its own, not after this tree's M2M in a chain of launches.  The
+// M2L reads its lists and the instances' flags ahead of its wait for its
+// predecessor, and another kernel may have written them just before.
+int run_m2l(const DevTree &tree, const DevLists &lists, FmmBuffers &buf, bool swapped, bool alone, cudaStream_t s);
 // rotation-based M2L (m2l_rot.cu, kernels in m2l_rot.cuh), orders 1..8, FP32 and FP64
 int launch_m2l_rot(int dtype, int p, int64_t M, const int32_t *off, const int32_t *src, const int32_t *rows,
                    const void *tcen,
@@ -451,7 +456,7 @@ int launch_m2l_rot_tf(int p, int64_t M, const int32_t *off, const int32_t *src, 
                       const void *snodes, const void *hal, const void *Mx, void *Lx, int nc_pad, const InstMask &mask,
                       int block, bool packed, cudaStream_t s);
 int run_m2l_two(const DevTree &tgt_tree, const DevTree &src_tree, const DevLists &lists, const FmmBuffers &src_buf,
-                FmmBuffers &tgt_buf, cudaStream_t s);
+                FmmBuffers &tgt_buf, bool alone, cudaStream_t s);
 int run_l2l(const DevTree &tree, FmmBuffers &buf, cudaStream_t s);
 // the same-tree extreme-pair rows of buf (built once; synchronises s)
 int prepare_extreme_rows(const DevTree &tree, const DevLists &lists, FmmBuffers &buf, cudaStream_t s);

@@ -1319,13 +1319,15 @@ int build_extreme(const DevTree &tree, const DevTree &stree, const int32_t *off,
 // (tbuf); for one tree, tree == stree and sbuf == tbuf.
 template <typename T>
 int m2l_impl(const DevTree &tree, const DevTree &stree, const DevLists &lists, const FmmBuffers &sbuf,
-             FmmBuffers &buf, bool swapped, cudaStream_t s) {
+             FmmBuffers &buf, bool swapped, bool alone, cudaStream_t s) {
     using T4 = typename Vec4<T>::type;
     const int64_t M = tree.n_nodes;
     if (M == 0 || stree.n_nodes == 0) return EDFMM_OK;
     const int32_t *off = swapped ? dptr<int32_t>(lists.m2l_swapped_off) : dptr<int32_t>(lists.m2l_off);
     const int32_t *src = swapped ? dptr<int32_t>(lists.m2l_swapped_src) : dptr<int32_t>(lists.m2l_src);
     const int32_t *rows = swapped ? nullptr : dptr<int32_t>(lists.m2l_rows);
+    // alone, the column copy begins the chain, with an ordinary launch
+    const bool chained = !alone && chain_tree(stree.n_nodes, stree.dtype, s);
     if (buf.p > kRotPMaxUsed) {
         // orders above 8: the shared-memory kernel (scales by the larger radius)
         k_m2l_generic<T><<<nblk(M, 4), 128, 0, s>>>(M, nullptr, off, src, dptr<T4>(tree.center), dptr<T4>(tree.half),
@@ -1341,7 +1343,7 @@ int m2l_impl(const DevTree &tree, const DevTree &stree, const DevLists &lists, c
     if (sizeof(T) == 8 && buf.arith == EDFMM_ARITH_TWO_FLOAT && buf.p >= 6 && buf.p <= 8 && tree.nodes_tf.p &&
         stree.nodes_tf.p && sbuf.mult_tf.p) {
         // the source multipoles split once per node, then the pairs
-        if (int rc = mult_columns<true>(sbuf, stree.n_nodes, sbuf.mult_tf, chain_tree(stree.n_nodes, stree.dtype, s), s)) return rc;
+        if (int rc = mult_columns<true>(sbuf, stree.n_nodes, sbuf.mult_tf, chained, s)) return rc;
         int rc = launch_m2l_rot_tf(buf.p, M, off, src, rows, tree.nodes_tf.p, tree.half.p, stree.nodes_tf.p, stree.half.p,
                                    sbuf.mult_tf.p, buf.locals.p, buf.nc_pad, buf.mask, buf.m2l_tf_block,
                                    buf.m2l_packed != 0, s);
@@ -1351,7 +1353,7 @@ int m2l_impl(const DevTree &tree, const DevTree &stree, const DevLists &lists, c
     if (!two_float) {
         // FP32 reads the multipoles by columns; `translated` is free once M2M has run
         if constexpr (sizeof(T) == 4) {
-            if (int rc = mult_columns<false>(sbuf, stree.n_nodes, sbuf.translated, chain_tree(stree.n_nodes, stree.dtype, s), s)) return rc;
+            if (int rc = mult_columns<false>(sbuf, stree.n_nodes, sbuf.translated, chained, s)) return rc;
         }
         if (int rc = launch_m2l_rot(sizeof(T) == 8 ? EDFMM_F64 : EDFMM_F32, buf.p, M, off, src, rows, tree.center.p,
                                     tree.half.p, stree.center.p, stree.half.p,
@@ -1412,14 +1414,15 @@ int run_p2m(const DevTree &tree, FmmBuffers &buf, cudaStream_t s) {
 int run_m2m(const DevTree &tree, FmmBuffers &buf, cudaStream_t s) {
     return tree.dtype == EDFMM_F64 ? m2m_impl<double>(tree, buf, s) : m2m_impl<float>(tree, buf, s);
 }
-int run_m2l(const DevTree &tree, const DevLists &lists, FmmBuffers &buf, bool swapped, cudaStream_t s) {
-    return tree.dtype == EDFMM_F64 ? m2l_impl<double>(tree, tree, lists, buf, buf, swapped, s)
-                                   : m2l_impl<float>(tree, tree, lists, buf, buf, swapped, s);
+int run_m2l(const DevTree &tree, const DevLists &lists, FmmBuffers &buf, bool swapped, bool alone, cudaStream_t s) {
+    return tree.dtype == EDFMM_F64 ? m2l_impl<double>(tree, tree, lists, buf, buf, swapped, alone, s)
+                                   : m2l_impl<float>(tree, tree, lists, buf, buf, swapped, alone, s);
 }
 int run_m2l_two(const DevTree &tgt_tree, const DevTree &src_tree, const DevLists &lists, const FmmBuffers &src_buf,
-                FmmBuffers &tgt_buf, cudaStream_t s) {
-    return tgt_tree.dtype == EDFMM_F64 ? m2l_impl<double>(tgt_tree, src_tree, lists, src_buf, tgt_buf, false, s)
-                                       : m2l_impl<float>(tgt_tree, src_tree, lists, src_buf, tgt_buf, false, s);
+                FmmBuffers &tgt_buf, bool alone, cudaStream_t s) {
+    return tgt_tree.dtype == EDFMM_F64
+               ? m2l_impl<double>(tgt_tree, src_tree, lists, src_buf, tgt_buf, false, alone, s)
+               : m2l_impl<float>(tgt_tree, src_tree, lists, src_buf, tgt_buf, false, alone, s);
 }
 int prepare_two_float(DevTree &tree, FmmBuffers &buf, cudaStream_t s) {
     if (tree.dtype != EDFMM_F64) return EDFMM_OK;

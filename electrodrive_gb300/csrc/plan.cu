@@ -742,7 +742,7 @@ int edfmm_plan_m2l(edfmm_plan *p, int flags, void *stream) {
     if (swapped) {
         if (int rc = lists_build_swapped(p->tree, p->lists, S(stream))) return rc;
     }
-    return run_m2l(p->tree, p->lists, p->fmm, swapped, S(stream));
+    return run_m2l(p->tree, p->lists, p->fmm, swapped, true, S(stream));
 }
 
 int edfmm_plan_l2l(edfmm_plan *p, void *stream) {
@@ -804,7 +804,7 @@ int edfmm_plan_matvec(edfmm_plan *p, const void *sigma, const void *areas, const
     }
     if (far && (rc = run_p2m(p->tree, p->fmm, f))) return rc;
     if (near && (rc = run_p2p(p->tree, p->lists, p->fmm, nullptr, p->near_sum.p, s))) return rc;
-    if (far && ((rc = run_m2m(p->tree, p->fmm, f)) || (rc = run_m2l(p->tree, p->lists, p->fmm, swapped, f)) ||
+    if (far && ((rc = run_m2m(p->tree, p->fmm, f)) || (rc = run_m2l(p->tree, p->lists, p->fmm, swapped, false, f)) ||
                 (rc = run_l2l(p->tree, p->fmm, f))))
         return rc;
     if (fork) {
@@ -920,7 +920,7 @@ int edfmm_targets_stage(edfmm_targets *t, int stage, void *out_dev, void *stream
     const int64_t M = t->tree.n_nodes;
     switch (stage) {
     case EDFMM_TARGETS_M2L:
-        return run_m2l_two(t->tree, p->tree, t->lists, p->fmm, t->buf, s);
+        return run_m2l_two(t->tree, p->tree, t->lists, p->fmm, t->buf, true, s);
     case EDFMM_TARGETS_L2L:
         return run_l2l(t->tree, t->buf, s);
     case EDFMM_TARGETS_L2P:
@@ -999,7 +999,7 @@ int edfmm_targets_potential(edfmm_targets *t, const void *sigma, const void *are
     if ((rc = set_charges(p->tree, sigma, areas, s))) return rc;
     if (far) {
         if ((rc = run_p2m(p->tree, p->fmm, s)) || (rc = run_m2m(p->tree, p->fmm, s)) ||
-            (rc = run_m2l_two(t->tree, p->tree, t->lists, p->fmm, t->buf, s)) || (rc = run_l2l(t->tree, t->buf, s)))
+            (rc = run_m2l_two(t->tree, p->tree, t->lists, p->fmm, t->buf, false, s)) || (rc = run_l2l(t->tree, t->buf, s)))
             return rc;
     }
     if (near && (rc = run_p2p(t->tree, t->lists, t->buf, &p->tree, t->near_sum.p, s))) return rc;
@@ -1026,7 +1026,7 @@ int edfmm_targets_field(edfmm_targets *t, const void *sigma, const void *areas, 
     if ((rc = set_charges(p->tree, sigma, areas, s))) return rc;
     if (far) {
         if ((rc = run_p2m(p->tree, p->fmm, s)) || (rc = run_m2m(p->tree, p->fmm, s)) ||
-            (rc = run_m2l_two(t->tree, p->tree, t->lists, p->fmm, t->buf, s)) || (rc = run_l2l(t->tree, t->buf, s)))
+            (rc = run_m2l_two(t->tree, p->tree, t->lists, p->fmm, t->buf, false, s)) || (rc = run_l2l(t->tree, t->buf, s)))
             return rc;
     }
     return run_targets_field(t->tree, t->lists, t->buf, p->tree, k_e, near, far, out, s);
