@@ -36,14 +36,17 @@ class DenseOperator:
         self.out = torch.empty(self.n, dtype=dtype, device=dev)
         self.table: Optional[Tensor] = None
 
+    def graph_state(self) -> tuple:
+        """What a captured graph of this operator depends on besides its buffers:
+        whether it applies the table."""
+        return (self.table is not None,)
+
     def tabulate(self, max_bytes: int = 4 << 30) -> bool:
         """Write out the operator's 1 / r (8 n^2 bytes) for a solve that applies
         it many times: an FP64 application is then a matrix-vector product (5,120
         panels: 63 us instead of 162; filling the table takes 180).  Not
         done in FP32 (distances are cheaper than the table's bytes), above
-        ``max_bytes``, or where the device would be left short of memory.  A
-        graph captured from the operator before holds the other kernel, so this
-        comes before the first application."""
+        ``max_bytes``, or where the device would be left short of memory."""
         if self.dtype != torch.float64 or self.table is not None or self.n == 0:
             return self.table is not None
         L = _lib.load_library()
