@@ -394,6 +394,7 @@ def _solve_pass(spec: Any, cfg: BEMConfig, mesh: TriMesh, h: float, *, dev, dtyp
                              "tile_size": int(getattr(cfg, "tile_size", 0) or 0),
                              "artifacts": (spec, C_dev, A_dev.to(dtype), Nrm, sigma, V_tot, mesh)},
             "operator": "fmm" if isinstance(op.base, FmmOperator) else "dense",
+            "dense_table": getattr(op.base, "table", None) is not None,
             "near_pairs": 0 if near is None else near.n_pairs, "charges": charges, "PV": PV}
 
 
@@ -422,6 +423,11 @@ def bem_solve(spec: Any, cfg: Optional[BEMConfig] = None, logger: Optional[Any] 
 
     Additions: ``mesh`` solves one pass on a given mesh; ``operator``
     ("auto": dense below ``fmm_threshold`` panels, FMM above);
+    a dense FP64 solve (not a mixed one) keeps a table of the operator's 1 / r
+    for its duration, 8 bytes a pair of panels and 4 GiB at most, where that much
+    memory and more is free (:meth:`DenseOperator.tabulate`), and says so in
+    ``mesh_stats["dense_table"]``: the sums of the two kernels differ in order, so
+    that two solves agree to the last bit only if both had the table or neither;
     ``self_integral`` "auto" follows the reference (quadrature self terms only
     when a near-quadrature option is on, else the equal-area disk value
     2 pi K_E sqrt(A / pi), bem.py:1747-1816) or forces "quadrature" / "disk";
@@ -539,7 +545,8 @@ def bem_solve(spec: Any, cfg: Optional[BEMConfig] = None, logger: Optional[Any] 
     idx = torch.arange(0, N_b, step, device=C_b.device)[:n_samples]
     mesh_stats = dict(n_panels=N_b, total_area=float(A_b.sum()), bc_residual_linf=float(best["bc_resid_linf"]),
                       h_final=float(best["h"]), tile_size_final=int(best["tile_size"]),
-                      operator=best_extra["operator"], near_pairs=best_extra["near_pairs"])
+                      operator=best_extra["operator"], dense_table=best_extra["dense_table"],
+                      near_pairs=best_extra["near_pairs"])
     if any(_cget(c, "type") == "plane" for c in (_cget(spec, "conductors", []) or [])) and mesh_stats["total_area"] > 0:
         mesh_stats["patch_L"] = math.sqrt(mesh_stats["total_area"])
     gmres_stats = dict(best.get("gmres_info", {}))

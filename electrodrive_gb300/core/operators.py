@@ -44,9 +44,11 @@ class DenseOperator:
     def tabulate(self, max_bytes: int = 4 << 30) -> bool:
         """Write out the operator's 1 / r (8 n^2 bytes) for a solve that applies
         it many times: an FP64 application is then a matrix-vector product (5,120
-        panels: 63 us instead of 162; filling the table takes 180).  Not
-        done in FP32 (distances are cheaper than the table's bytes), above
-        ``max_bytes``, or where the device would be left short of memory."""
+        panels: 63 us instead of 162; filling the table takes 180), whose sums
+        have another order.  Not done in FP32 (distances are cheaper than the
+        table's bytes), above ``max_bytes``, or where less than the table and
+        1 GiB would stay free, what the caching allocator holds unused counted
+        as free.  Returns whether the operator applies the table."""
         if self.dtype != torch.float64 or self.table is not None or self.n == 0:
             return self.table is not None
         L = _lib.load_library()
@@ -54,7 +56,9 @@ class DenseOperator:
         if nbytes == 0 or nbytes > max_bytes:
             return False
         try:
-            if torch.cuda.mem_get_info(self.device)[0] < 2 * nbytes + (1 << 30):
+            free = (torch.cuda.mem_get_info(self.device)[0] + torch.cuda.memory_reserved(self.device)
+                    - torch.cuda.memory_allocated(self.device))
+            if free < 2 * nbytes + (1 << 30):
                 return False
             table = torch.empty(nbytes // 8, dtype=torch.float64, device=self.device)
         except torch.OutOfMemoryError:
