@@ -439,12 +439,13 @@ int lists_impl(const DevTree &stree, const DevTree &tree, double theta, DevLists
     const TravTree<T> Tt{dptr<T4>(tree.center), dptr<uint8_t>(tree.is_leaf), dptr<int2>(tree.range),
                          dptr<int32_t>(tree.children)};
     L = DevLists();
-    if (M == 0 || stree.n_nodes == 0) {
-        if ((rc = L.p2p_off.reserve(sizeof(int32_t))) || (rc = L.m2l_off.reserve(sizeof(int32_t))) ||
-            (rc = L.p2p_src.reserve(4)) || (rc = L.m2l_src.reserve(4)))
+    if (M == 0 || stree.n_nodes == 0) {  // rows of nothing
+        const size_t rows = sizeof(int32_t) * (size_t)(M + 1);
+        if ((rc = L.p2p_off.reserve(rows)) || (rc = L.m2l_off.reserve(rows)) || (rc = L.p2p_src.reserve(4)) ||
+            (rc = L.m2l_src.reserve(4)))
             return rc;
-        EDFMM_CUDA_TRY(cudaMemsetAsync(L.p2p_off.p, 0, sizeof(int32_t), s));
-        EDFMM_CUDA_TRY(cudaMemsetAsync(L.m2l_off.p, 0, sizeof(int32_t), s));
+        EDFMM_CUDA_TRY(cudaMemsetAsync(L.p2p_off.p, 0, rows, s));
+        EDFMM_CUDA_TRY(cudaMemsetAsync(L.m2l_off.p, 0, rows, s));
         return EDFMM_OK;
     }
     // a same-tree forest (batched plan) starts from every (root, root) pair;
