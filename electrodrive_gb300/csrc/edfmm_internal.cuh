@@ -492,6 +492,7 @@ int upload_tables();
 struct edfmm_plan {
     edfmm::DevTree tree;
     edfmm::DevLists lists;
+    bool lists_ok = true;  // false after a rebuild that failed
     edfmm::FmmBuffers fmm;
     double mac_theta = 0.5;
     int leaf_size = 64;

@@ -169,6 +169,12 @@ int check_plan(const edfmm_plan *p) {
     if (!p) return fail(EDFMM_ERR_ARG, "plan is NULL");
     return EDFMM_OK;
 }
+int check_lists(const edfmm_plan *p) {
+    if (int rc = check_plan(p)) return rc;
+    if (!p->lists_ok)
+        return fail(EDFMM_ERR_STATE, "the plan's interaction lists could not be rebuilt; edfmm_plan_rebuild_lists tries again");
+    return EDFMM_OK;
+}
 
 }  // namespace
 
@@ -415,7 +421,7 @@ int edfmm_plan_create_batch(const void *points_dev, const int64_t *offsets, int 
 int edfmm_plan_convert(const edfmm_plan *src, int dtype, int expansion_order, void *stream, edfmm_plan **plan_out) {
     if (!plan_out) return fail(EDFMM_ERR_ARG, "plan_out is NULL");
     *plan_out = nullptr;
-    if (int rc = check_plan(src)) return rc;
+    if (int rc = check_lists(src)) return rc;
     if (dtype != EDFMM_F32 && dtype != EDFMM_F64) return fail(EDFMM_ERR_ARG, "dtype must be EDFMM_F32 or EDFMM_F64");
     if (expansion_order < 1 || expansion_order > 10)
         return fail(EDFMM_ERR_UNSUPPORTED, "expansion_order must be in [1, 10]");
@@ -525,7 +531,7 @@ int edfmm_plan_destroy(edfmm_plan *plan) {
 }
 
 int edfmm_plan_set_arithmetic(edfmm_plan *p, int mode, void *stream) {
-    if (int rc = check_plan(p)) return rc;
+    if (int rc = check_lists(p)) return rc;
     if (mode != EDFMM_ARITH_NATIVE && mode != EDFMM_ARITH_TWO_FLOAT)
         return fail(EDFMM_ERR_ARG, "mode must be EDFMM_ARITH_NATIVE or EDFMM_ARITH_TWO_FLOAT");
     cudaStream_t s = S(stream);
@@ -584,11 +590,16 @@ int edfmm_plan_get_launch(const edfmm_plan *p, int knob, int *value) {
 int edfmm_plan_rebuild_lists(edfmm_plan *p, double mac_theta, void *stream) {
     if (int rc = check_plan(p)) return rc;
     if (!(mac_theta > 0.0 && mac_theta < 1.0)) return fail(EDFMM_ERR_ARG, "mac_theta must be in (0, 1)");
-    if (mac_theta == p->mac_theta) return EDFMM_OK;
-    if (int rc = lists_build(p->tree, mac_theta, p->lists, S(stream))) return rc;
-    p->mac_theta = mac_theta;
+    if (mac_theta == p->mac_theta && p->lists_ok) return EDFMM_OK;
+    p->lists_ok = false;  // the old lists make room for the new
     p->fmm.extreme = ExtremeRows();
     p->fmm.extreme_swapped = ExtremeRows();
+    if (int rc = lists_build(p->tree, mac_theta, p->lists, S(stream))) {
+        p->lists = DevLists();
+        return rc;
+    }
+    p->lists_ok = true;
+    p->mac_theta = mac_theta;
     if (p->fmm.arith == EDFMM_ARITH_TWO_FLOAT) {
         if (int rc = prepare_extreme_rows(p->tree, p->lists, p->fmm, S(stream))) return rc;
     }
@@ -683,7 +694,7 @@ int edfmm_plan_export_tree(const edfmm_plan *p, int64_t *index_map, void *center
 }
 
 int edfmm_plan_export_lists(const edfmm_plan *p, int64_t *p2p_pairs, int64_t *m2l_pairs, void *stream) {
-    if (int rc = check_plan(p)) return rc;
+    if (int rc = check_lists(p)) return rc;
     const int64_t M = p->tree.n_nodes;
     if (M == 0) return EDFMM_OK;
     dim3 blk(32, 8);
@@ -737,7 +748,7 @@ int edfmm_plan_m2m(edfmm_plan *p, void *stream) {
 }
 
 int edfmm_plan_m2l(edfmm_plan *p, int flags, void *stream) {
-    if (int rc = check_plan(p)) return rc;
+    if (int rc = check_lists(p)) return rc;
     const bool swapped = (flags & EDFMM_REFERENCE_PAIR_ORDER) != 0;
     if (swapped) {
         if (int rc = lists_build_swapped(p->tree, p->lists, S(stream))) return rc;
@@ -759,14 +770,14 @@ int edfmm_plan_l2p(edfmm_plan *p, void *phi_far_tree, void *stream) {
 }
 
 int edfmm_plan_p2p(edfmm_plan *p, void *phi_near_tree, void *stream) {
-    if (int rc = check_plan(p)) return rc;
+    if (int rc = check_lists(p)) return rc;
     if (p->tree.n_points > 0 && !phi_near_tree) return fail(EDFMM_ERR_ARG, "output is NULL");
     return run_p2p(p->tree, p->lists, p->fmm, nullptr, phi_near_tree, S(stream));
 }
 
 int edfmm_plan_matvec(edfmm_plan *p, const void *sigma, const void *areas, const void *self_integrals, double k_e,
                       void *out, int flags, void *stream) {
-    if (int rc = check_plan(p)) return rc;
+    if (int rc = check_lists(p)) return rc;
     if (p->tree.n_points == 0) return EDFMM_OK;
     if (!sigma || !areas || !out) return fail(EDFMM_ERR_ARG, "sigma, areas and out must be non-NULL");
     cudaStream_t s = S(stream);
