@@ -16,15 +16,18 @@ timed region).  `--impl reference` times the CPU oracle's restatement of the
 operator (FP64, all host cores) on a bounded sample of the same workload.
 Under torchrun every rank runs its own replica (no data-path collective).
 
-At N = 1 the same line also carries the solve workloads, each a complete
-record of its own under ``workloads`` (``--matvec-only`` leaves them out):
+At N = 1 the solve workloads run too (``--matvec-only`` leaves them out): the
+line carries their throughputs under ``workloads``, and the complete record of
+each goes to stderr, a JSON line each, since the whole in one line is longer
+than what readers of a job's last line keep:
 ``torus_solve`` (200,000-panel torus, FMM p = 8 + near correction, mixed
 FP32/FP64 refinement with the learned warm start, solves/s to a 1e-6
 relative true residual, beside plain FP64 GMRES on the same GPU, the sigma
 error against the converged density, and the same solve run to 1e-7, whose
-sigma is within 1e-5), ``sphere_solve`` (5,120-panel icosphere, dense FP64)
-and ``batch_solve`` (256 sphere dimers of 2k-40k panels); ``torus_solve`` is
-summarised at the top level.  ``--workload`` runs one of them alone.
+sigma is within 1e-5), ``sphere_solve`` (5,120-panel icosphere, dense FP64),
+``batch_solve`` (256 sphere dimers of 2k-40k panels) and ``warm_start`` (the
+learned start on held-out geometries).  ``--workload`` runs one of them alone
+and prints its complete record.
 """
 from __future__ import annotations
 
@@ -1141,6 +1144,35 @@ def run_warm_start_workload(args, rank, world, local, emit=True):
     return out
 
 
+def _short(x):
+    """Numbers to six digits, recursively."""
+    if isinstance(x, dict):
+        return {k: _short(v) for k, v in x.items()}
+    if isinstance(x, (list, tuple)):
+        return [_short(v) for v in x]
+    return float(f"{x:.6g}") if isinstance(x, float) else x
+
+
+def headline(out, records):
+    """The line for stdout: the matvec's record and each workload's throughput."""
+    line = _short(out)
+    if not records:
+        return line
+    line["workloads"] = {}
+    for name, rec in records.items():
+        if "error" in rec:
+            line["workloads"][name] = {"error": rec["error"][:120]}
+            continue
+        w = {k: rec.get(k) for k in ("value", "unit", "ms_per_step")}
+        w["e2e"] = (rec.get("e2e") or {}).get("value")
+        solve = rec.get("solve") or {}
+        if "mixed_speedup_vs_plain_fp64_early_exit" in solve:
+            w["true_rel_resid"] = solve["true_rel_resid"]
+            w["speedup_vs_plain_fp64"] = solve["mixed_speedup_vs_plain_fp64_early_exit"]
+        line["workloads"][name] = _short(w)
+    return line
+
+
 def main():
     args = parse()
     rank = int(os.environ.get("RANK", "0"))
@@ -1309,12 +1341,12 @@ def main():
             "p2p_tflops": p2p_tflops,
             "cpu_baseline": cpu,
         }
+    records = {}
     if world == 1 and not args.matvec_only:
         # the solve workloads, each a full record of its own, timed after the
         # matvec on the same GPU (N = 1 only: the scaling runs time the matvec)
         del fmm, plan, sig_d, areas_d, out_d, flush
         torch.cuda.empty_cache()
-        out["workloads"] = {}
         for sub, steps in (("torus_solve", min(args.steps, 5)), ("sphere_solve", min(args.steps, 5)),
                            ("batch_solve", min(args.steps, 3)), ("warm_start", None)):
             sargs = argparse.Namespace(**vars(args))
@@ -1331,20 +1363,11 @@ def main():
                 rec["wall_s"] = time.perf_counter() - t0
             except Exception as e:  # a failing sub-record must not lose the headline line
                 rec = {"error": f"{type(e).__name__}: {str(e)[:300]}", "wall_s": time.perf_counter() - t0}
-            out["workloads"][sub] = rec
+            records[sub] = rec
+            print(json.dumps({"workload": sub, **rec}), file=sys.stderr, flush=True)
             torch.cuda.empty_cache()
-        tor = out["workloads"].get("torus_solve", {})
-        if "solve" in tor:
-            ts = tor["solve"]
-            out["torus_solve"] = {
-                "solves_per_s_rtol1e-6": tor["value"], "ms": tor["ms_per_step"],
-                "true_rel_resid": ts["true_rel_resid"], "sigma_rel_l2_vs_converged": ts["sigma_rel_l2_vs_converged"],
-                "plain_fp64_early_exit_solves_per_s": ts["plain_fp64_gmres_early_exit"]["solves_per_s"],
-                "speedup_vs_plain_fp64_early_exit": ts["mixed_speedup_vs_plain_fp64_early_exit"],
-                "accurate_rtol1e-7": ts["accurate_rtol1e-7"], "roofline": tor["roofline"], "e2e": tor["e2e"],
-                "cpu_baseline": tor["cpu_baseline"]}
     if rank == 0:
-        print(json.dumps(out), flush=True)
+        print(json.dumps(headline(out, records)), flush=True)
     if dist:
         dist.destroy_process_group()
 
