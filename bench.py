@@ -76,12 +76,13 @@ M2L_FLOPS_PER_PAIR = m2l_flops_per_pair(8)
 # taken from an ncu capture of k_m2l_rot<8> at N = 262,144 (44.64 MB moved for
 # 9,017,270 pairs)
 M2L_DRAM_BYTES_PER_PAIR = 44.64e6 / 9_017_270
-# DRAM bytes (read + write) per M2L pair of k_m2l_rot<p> on the
-# 200,000-panel torus (FP32 inner operator), from ncu captures of that kernel
-# on that mesh (median over the profile run's launches)
-M2L_DRAM_BYTES_PER_PAIR_TORUS = {(8, 64): 14_461_269 / 2_315_072, (6, 64): 12_600_576 / 2_315_072}  # (p, leaf)
-# the same for the 256-dimer batch (FP32 inner operator, autotuned order)
-M2L_DRAM_BYTES_PER_PAIR_BATCH = {(6, 64): (244_023_808 + 55_725_312) / 39_011_439}  # (p, leaf)
+# DRAM bytes (read + write) per M2L pair of k_m2l_rot<p> (multipoles by columns)
+# on the 200,000-panel torus (FP32 inner operator), from ncu captures of that
+# kernel on that mesh
+M2L_DRAM_BYTES_PER_PAIR_TORUS = {(8, 64): 14_508_032 / 2_315_072, (6, 64): 12_658_176 / 2_315_072}  # (p, leaf)
+# the same for the 256-dimer batch (FP32 inner operator, autotuned order), whose
+# columns and locals do not fit L2
+M2L_DRAM_BYTES_PER_PAIR_BATCH = {(6, 64): (2_804_471_808 + 69_571_840) / 39_009_433}  # (p, leaf)
 # DRAM bytes of one k_dense_f64 launch at n = 5,120 (ncu capture)
 DENSE_DRAM_BYTES_PER_MATVEC_5120 = 196_608
 # the FP64 dense kernel forms 1 / r on the FP32 pipe: 136 operations a pair there
