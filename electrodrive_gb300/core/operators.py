@@ -1,6 +1,6 @@
 """Graph-capturable single-layer operators for the device GMRES.
 
-Each operator owns its output (and scratch) buffers, launches only on the
+Each operator owns its output buffer, launches only on the
 current stream and allocates nothing per call, so ``gmres_restart`` can
 capture a whole restart cycle of ``A(v)`` + Arnoldi kernels in one CUDA
 graph.  ``capturable = True`` advertises that.
@@ -29,10 +29,6 @@ class DenseOperator:
         self.a = areas.to(dev, dtype).contiguous()
         self.si = None if self_integrals is None else self_integrals.to(dev, dtype).contiguous()
         self.n = int(self.a.shape[0])
-        L = _lib.load_library()
-        nbytes = int(L.edfmm_dense_workspace_bytes(self.n, _lib.dtype_code(dtype)))
-        self.ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=dev)
-        self.nbytes = nbytes
         self.out = torch.empty(self.n, dtype=dtype, device=dev)
         self.table: Optional[Tensor] = None
 
@@ -78,9 +74,9 @@ class DenseOperator:
                                                   _lib.ptr(self.si), self.n, self.k_e, _lib.ptr(o),
                                                   _lib.stream_handle(self.device)), "edfmm_dense_table_matvec")
             return o
-        _lib.check(L.edfmm_dense_matvec_ws(_lib.ptr(self.c), _lib.ptr(s), _lib.ptr(self.a), _lib.ptr(self.si), self.n,
-                                           _lib.dtype_code(self.dtype), self.k_e, _lib.ptr(o), _lib.ptr(self.ws),
-                                           self.nbytes, _lib.stream_handle(self.device)), "edfmm_dense_matvec_ws")
+        _lib.check(L.edfmm_dense_matvec(_lib.ptr(self.c), _lib.ptr(s), _lib.ptr(self.a), _lib.ptr(self.si), self.n,
+                                        _lib.dtype_code(self.dtype), self.k_e, _lib.ptr(o),
+                                        _lib.stream_handle(self.device)), "edfmm_dense_matvec")
         return o
 
 

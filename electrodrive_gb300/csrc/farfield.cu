@@ -6,20 +6,15 @@
 //   Mhat_n^m = M_n^m / a^n,  Lhat_n^m = L_n^m a^n.
 // This keeps every coefficient O(1) in FP32 at any tree depth.
 //
-// M2L (the dominant stage) is organised so that one lane owns one
-// (target, source) pair at a time and keeps the whole translation in
-// registers: the source multipole (scaled by (a_M/a_L)^k), the accumulator
-// for the 45 target coefficients (p = 8) and one column of irregular
-// harmonics of v = (c_L - c_M) / a_L, generated by recurrence.  A warp walks
-// one target's row of the interaction list; the 32 partial sums are reduced
-// with shuffles, so the result is deterministic.  With this scaling
+// M2L (the dominant stage) runs in the rotation form of m2l_rot.cuh for orders up
+// to 8, in FP32, FP64 or two-float arithmetic; FP32 and two-float read the
+// multipoles by columns (k_mult_columns).  With this scaling
 //   Lhat_n^m = (-1)^(n+m) / a_L  sum_pairs sum_{k,l} Mhat_k^l (a_M/a_L)^k I_{n+k}^{l-m}(v),
-// which is exact algebra; pairs whose source scale exceeds 256x the target's
-// (only in strongly adaptive trees) would overflow (a_M/a_L)^k in FP32 and are
-// instead translated by a shared-memory kernel using
+// v = (c_L - c_M) / a_L, which is exact algebra; pairs whose source scale exceeds
+// 256x the target's (only in strongly adaptive trees) would overflow (a_M/a_L)^k
+// in FP32 and are instead translated by a shared-memory kernel using
 //   Lhat_n^m = (-1)^(n+m) / a_L  (a_L/a_M)^(n+1) sum_{k,l} Mhat_k^l I_{n+k}^{l-m}((c_L - c_M)/a_M).
-// FP64 plans (p <= 8) translate every pair with an FP64 form of the fast
-// kernel; orders above 8 use the shared-memory kernel.
+// FP64 has the range for any ratio; orders above 8 use the shared-memory kernel.
 #include <algorithm>
 
 #include "edfmm_internal.cuh"
@@ -270,7 +265,7 @@ __global__ void __launch_bounds__(128) k_m2m(const int32_t *__restrict__ nodes, 
 
 // ---------------------------------------------------------------------------
 // pair helpers: (sr, si) += (xr, xi) * (c0, c1) on coefficients held in
-// separate re / im arrays; FP32 as one packed FMA (FFMA2), FP64 as two
+// separate re / im arrays, as one packed FMA (FFMA2)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 template <typename T> struct Pair {};
@@ -399,15 +394,6 @@ __device__ __forceinline__ void load_row(const float2 *row, AR &xr, AR &xi) {
     }
 }
 template <int P, typename AR>
-__device__ __forceinline__ void load_row(const double2 *row, AR &xr, AR &xi) {
-#pragma unroll
-    for (int q = 0; q < ncoef(P); ++q) {
-        const double2 v = row[q];
-        xr[q] = v.x;
-        xi[q] = v.y;
-    }
-}
-template <int P, typename AR>
 __device__ __forceinline__ void store_row(float2 *row, AR &xr, AR &xi) {
     constexpr int NC = ncoef(P);
     float4 *o4 = reinterpret_cast<float4 *>(row);
@@ -416,38 +402,27 @@ __device__ __forceinline__ void store_row(float2 *row, AR &xr, AR &xi) {
         o4[q] = make_float4(xr[2 * q], xi[2 * q], 2 * q + 1 < NC ? xr[2 * q + 1] : 0.0f,
                             2 * q + 1 < NC ? xi[2 * q + 1] : 0.0f);
 }
-template <int P, typename AR>
-__device__ __forceinline__ void store_row(double2 *row, AR &xr, AR &xi) {
-#pragma unroll
-    for (int q = 0; q < ncoef(P); ++q) row[q] = make_double2(xr[q], xi[q]);
-}
 
 // x_n^m <- e^{i m phi} f^n x_n^m  (f = 1 for the L2L)
-template <typename T, int P, typename AR>
-__device__ __forceinline__ void rotate_scale(AR &xr, AR &xi, T ec, T es, T f) {
-    T wr = 1, wi = 0;
+template <int P, typename AR>
+__device__ __forceinline__ void rotate_scale(AR &xr, AR &xi, float ec, float es, float f) {
+    float wr = 1, wi = 0;
 #pragma unroll
     for (int m = 0; m <= P; ++m) {
         if (m > 0) {
-            const T nr = wr * ec - wi * es, ni = wr * es + wi * ec;
+            const float nr = wr * ec - wi * es, ni = wr * es + wi * ec;
             wr = nr;
             wi = ni;
         }
-        T fk = 1;
+        float fk = 1;
 #pragma unroll
         for (int n = 0; n <= P; ++n) {
             if (n >= m) {
-                const T fr = wr * fk, fi = wi * fk;
-                if constexpr (sizeof(T) == 4) {
-                    const float2 x = f2(xr[tri(n, m)], xi[tri(n, m)]);
-                    const float2 y = __ffma2_rn(f2(x.y, x.x), f2(-fi, fi), __fmul2_rn(x, f2(fr, fr)));
-                    xr[tri(n, m)] = y.x;
-                    xi[tri(n, m)] = y.y;
-                } else {
-                    const T a = xr[tri(n, m)], b = xi[tri(n, m)];
-                    xr[tri(n, m)] = a * fr - b * fi;
-                    xi[tri(n, m)] = a * fi + b * fr;
-                }
+                const float fr = wr * fk, fi = wi * fk;
+                const float2 x = f2(xr[tri(n, m)], xi[tri(n, m)]);
+                const float2 y = __ffma2_rn(f2(x.y, x.x), f2(-fi, fi), __fmul2_rn(x, f2(fr, fr)));
+                xr[tri(n, m)] = y.x;
+                xi[tri(n, m)] = y.y;
             }
             fk *= f;
         }
@@ -479,20 +454,20 @@ __device__ __forceinline__ Shift<T> shift_of(typename Vec4<T>::type cc, typename
     return f;
 }
 
-template <typename T, int P, typename AR>
+template <int P, typename AR>
 __device__ __forceinline__ void m2m_node(int node, const uint8_t *__restrict__ is_leaf,
                                          const int32_t *__restrict__ children, const int32_t *__restrict__ parent,
-                                         const typename Vec4<T>::type *__restrict__ center,
-                                         const typename Vec4<T>::type *__restrict__ half,
-                                         typename Pair<T>::type *__restrict__ Mexp,
-                                         typename Pair<T>::type *__restrict__ moved, int nc_pad, AR &xr, AR &xi,
+                                         const float4 *__restrict__ center,
+                                         const float4 *__restrict__ half,
+                                         float2 *__restrict__ Mexp,
+                                         float2 *__restrict__ moved, int nc_pad, AR &xr, AR &xi,
                                          AR &Sr, AR &Si) {
     constexpr int NC = ncoef(P);
     if (is_leaf[node]) {
         load_row<P>(Mexp + (int64_t)node * nc_pad, xr, xi);
     } else {
 #pragma unroll
-        for (int q = 0; q < NC; ++q) xr[q] = xi[q] = (T)0;
+        for (int q = 0; q < NC; ++q) xr[q] = xi[q] = 0.0f;
         for (int o = 0; o < 8; ++o) {
             const int ch = children[8 * node + o];
             if (ch < 0) continue;
@@ -507,33 +482,33 @@ __device__ __forceinline__ void m2m_node(int node, const uint8_t *__restrict__ i
     }
     const int par = parent[node];
     if (par < 0) return;
-    const Shift<T> f = shift_of<T>(center[node], center[par], half[node].w, half[par].w);
-    rotate_scale<T, P>(xr, xi, f.ec, f.es, f.ratio);
+    const Shift<float> f = shift_of<float>(center[node], center[par], half[node].w, half[par].w);
+    rotate_scale<P>(xr, xi, f.ec, f.es, f.ratio);
 #pragma unroll
-    for (int q = 0; q < NC; ++q) Sr[q] = Si[q] = (T)0;
-    T diag = 1;
-    shift_column<T, P, false, 0>(xr, xi, f.s, f.z, f.r2, diag, Sr, Si);
-    rotate_scale<T, P>(Sr, Si, f.ec, -f.es, (T)1);  // e^{-i m phi}
+    for (int q = 0; q < NC; ++q) Sr[q] = Si[q] = 0.0f;
+    float diag = 1;
+    shift_column<float, P, false, 0>(xr, xi, f.s, f.z, f.r2, diag, Sr, Si);
+    rotate_scale<P>(Sr, Si, f.ec, -f.es, 1.0f);  // e^{-i m phi}
     store_row<P>(moved + (int64_t)node * nc_pad, Sr, Si);
 }
 
-template <typename T, int P, typename AR>
+template <int P, typename AR>
 __device__ __forceinline__ void l2l_node(int node, const int32_t *__restrict__ parent,
-                                         const typename Vec4<T>::type *__restrict__ center,
-                                         const typename Vec4<T>::type *__restrict__ half,
-                                         typename Pair<T>::type *__restrict__ Lexp, int nc_pad, AR &xr, AR &xi,
+                                         const float4 *__restrict__ center,
+                                         const float4 *__restrict__ half,
+                                         float2 *__restrict__ Lexp, int nc_pad, AR &xr, AR &xi,
                                          AR &Sr, AR &Si) {
     constexpr int NC = ncoef(P);
     const int par = parent[node];
     if (par < 0) return;
-    const Shift<T> f = shift_of<T>(center[node], center[par], half[node].w, half[par].w);
+    const Shift<float> f = shift_of<float>(center[node], center[par], half[node].w, half[par].w);
     load_row<P>(Lexp + (int64_t)par * nc_pad, xr, xi);
-    rotate_scale<T, P>(xr, xi, f.ec, f.es, (T)1);
+    rotate_scale<P>(xr, xi, f.ec, f.es, 1.0f);
 #pragma unroll
-    for (int q = 0; q < NC; ++q) Sr[q] = Si[q] = (T)0;
-    T diag = 1;
-    shift_column<T, P, true, 0>(xr, xi, f.s, f.z, f.r2, diag, Sr, Si);
-    rotate_scale<T, P>(Sr, Si, f.ec, -f.es, f.ratio);  // (a_C/a_P)^j e^{-i u phi}
+    for (int q = 0; q < NC; ++q) Sr[q] = Si[q] = 0.0f;
+    float diag = 1;
+    shift_column<float, P, true, 0>(xr, xi, f.s, f.z, f.r2, diag, Sr, Si);
+    rotate_scale<P>(Sr, Si, f.ec, -f.es, f.ratio);  // (a_C/a_P)^j e^{-i u phi}
     load_row<P>(Lexp + (int64_t)node * nc_pad, xr, xi);
 #pragma unroll
     for (int q = 0; q < NC; ++q) {
@@ -554,7 +529,7 @@ __global__ void __launch_bounds__(kFastThreads) k_m2m_fast(
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     float xr[NC], xi[NC], Sr[NC], Si[NC];
-    m2m_node<float, P>(nodes[i], is_leaf, children, parent, center, half, Mexp, moved, nc_pad, xr, xi, Sr, Si);
+    m2m_node<P>(nodes[i], is_leaf, children, parent, center, half, Mexp, moved, nc_pad, xr, xi, Sr, Si);
 }
 
 template <int P>
@@ -567,7 +542,7 @@ __global__ void __launch_bounds__(kFastThreads) k_l2l_fast(const int32_t *__rest
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     float xr[NC], xi[NC], Sr[NC], Si[NC];
-    l2l_node<float, P>(nodes[i], parent, center, half, Lexp, nc_pad, xr, xi, Sr, Si);
+    l2l_node<P>(nodes[i], parent, center, half, Lexp, nc_pad, xr, xi, Sr, Si);
 }
 
 // ---------------------------------------------------------------------------

@@ -552,8 +552,6 @@ __global__ void __launch_bounds__(32 * kNearWarps, near_blocks<MODE>())
         EDFMM_NEAR_R(2)
         EDFMM_NEAR_R(3)
         EDFMM_NEAR_R(4)
-        EDFMM_NEAR_R(5)
-        EDFMM_NEAR_R(6)
 #undef EDFMM_NEAR_R
     }
 }
