@@ -52,9 +52,11 @@ class DenseOperator:
         if nbytes == 0 or nbytes > max_bytes:
             return False
         try:
-            free = (torch.cuda.mem_get_info(self.device)[0] + torch.cuda.memory_reserved(self.device)
-                    - torch.cuda.memory_allocated(self.device))
-            if free < 2 * nbytes + (1 << 30):
+            need = 2 * nbytes + (1 << 30)
+            free = torch.cuda.mem_get_info(self.device)[0]
+            if free < need:  # the allocator's statistics take 100 us
+                free += torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
+            if free < need:
                 return False
             table = torch.empty(nbytes // 8, dtype=torch.float64, device=self.device)
         except torch.OutOfMemoryError:
