@@ -80,9 +80,10 @@ M2L_DRAM_BYTES_PER_PAIR = 44.64e6 / 9_017_270
 # on the 200,000-panel torus (FP32 inner operator), from ncu captures of that
 # kernel on that mesh
 M2L_DRAM_BYTES_PER_PAIR_TORUS = {(8, 64): 14_508_032 / 2_315_072, (6, 64): 12_658_176 / 2_315_072}  # (p, leaf)
-# the same for the 256-dimer batch (FP32 inner operator, autotuned order), whose
-# columns and locals do not fit L2
-M2L_DRAM_BYTES_PER_PAIR_BATCH = {(6, 64): (2_804_471_808 + 69_571_840) / 39_009_433}  # (p, leaf)
+# the same for the 256-dimer batch (FP32 inner operator, autotuned order and leaf
+# size); with leaves of 64 its columns and locals do not fit L2
+M2L_DRAM_BYTES_PER_PAIR_BATCH = {(6, 64): (2_804_471_808 + 69_571_840) / 39_009_433,
+                                 (6, 128): (120_345_600 + 22_391_552) / 16_951_111}  # (p, leaf)
 # DRAM bytes of one k_dense_f64 launch at n = 5,120 (ncu capture)
 DENSE_DRAM_BYTES_PER_MATVEC_5120 = 196_608
 # the FP64 dense kernel forms 1 / r on the FP32 pipe: 136 operations a pair there
