@@ -135,7 +135,9 @@ EDFMM_API int edfmm_plan_destroy(edfmm_plan *plan);
 /*
  * Rebuild the interaction lists of an existing plan for another MAC
  * parameter (build_interaction_lists(tree, tree, mac_theta=...),
- * electrodrive/fmm3d/interaction_lists.py:531-577).
+ * electrodrive/fmm3d/interaction_lists.py:531-577).  The old lists make room for
+ * the new: after a failure the plan has none, and calls that need them return
+ * EDFMM_ERR_STATE until a rebuild succeeds.
  */
 EDFMM_API int edfmm_plan_rebuild_lists(edfmm_plan *plan, double mac_theta, void *stream);
 
