@@ -421,10 +421,11 @@ int edfmm_plan_create_batch(const void *points_dev, const int64_t *offsets, int 
 int edfmm_plan_convert(const edfmm_plan *src, int dtype, int expansion_order, void *stream, edfmm_plan **plan_out) {
     if (!plan_out) return fail(EDFMM_ERR_ARG, "plan_out is NULL");
     *plan_out = nullptr;
-    if (int rc = check_lists(src)) return rc;
+    if (int rc = check_plan(src)) return rc;
     if (dtype != EDFMM_F32 && dtype != EDFMM_F64) return fail(EDFMM_ERR_ARG, "dtype must be EDFMM_F32 or EDFMM_F64");
     if (expansion_order < 1 || expansion_order > 10)
         return fail(EDFMM_ERR_UNSUPPORTED, "expansion_order must be in [1, 10]");
+    if (int rc = check_lists(src)) return rc;
     cudaStream_t s = S(stream);
     edfmm_plan *p = new edfmm_plan();
     cudaGetDevice(&p->device);
@@ -531,9 +532,10 @@ int edfmm_plan_destroy(edfmm_plan *plan) {
 }
 
 int edfmm_plan_set_arithmetic(edfmm_plan *p, int mode, void *stream) {
-    if (int rc = check_lists(p)) return rc;
+    if (int rc = check_plan(p)) return rc;
     if (mode != EDFMM_ARITH_NATIVE && mode != EDFMM_ARITH_TWO_FLOAT)
         return fail(EDFMM_ERR_ARG, "mode must be EDFMM_ARITH_NATIVE or EDFMM_ARITH_TWO_FLOAT");
+    if (int rc = check_lists(p)) return rc;
     cudaStream_t s = S(stream);
     // the split points' charges are doubles or pairs of floats
     auto split_charges = [&](bool tf) {
