@@ -321,9 +321,9 @@ __device__ __forceinline__ bool inst_active(const InstMask &m, int node) {
 // chain_launch may start while its predecessor in the stream still runs.  It
 // reads what the plan holds, calls chain_wait (all threads, before any return),
 // and only then reads or writes what other kernels of the chain do; chain_next
-// lets its own successor start.  A chain begins with an ordinary launch, so that
-// all that came before it is complete.  Without the launch attribute both do
-// nothing.
+// lets its own successor start.  A kernel that reads ahead what another may have
+// written since the plan's set-up (the M2L) has an ordinary launch between them.
+// Without the launch attribute both do nothing.
 // What the chain writes is read through pointers that are neither const
 // __restrict__ nor __ldg: those loads assume data that stay as they are for the
 // kernel's whole life, which here begins before its predecessor's end.
